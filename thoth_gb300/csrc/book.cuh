@@ -17,7 +17,7 @@ struct Smem {
     uint2* hs;      // [min(sobol_dims, HS_CHUNK)] tile parts of the current chunk of Sobol entries,
                     // for tile columns t and t + T/2 (see tile_high_bits)
     float* stk;     // [stack_depth][stack_factors][T]; after the time loop, the product partials
-    float* slots;   // [n_slots][T + 1]
+    float* slots;   // [n_slots][T + 1], here or in the CTA's part of DevPlan::slot_mem
     float* grp;     // [n_groups][T + 1]
     float* last;    // [n_last][T + 1] previous observation of each discretely observed variance group
     float* part;    // [T * 6] product partials: the bridge stack's space, free once the paths are built
@@ -64,6 +64,8 @@ __host__ __device__ inline size_t smem_bytes(int T, int sobol_dims, int stack_de
     return b;
 }
 
+// SLOT_MEM: a kernel whose plans may hold their slots in global memory
+template <bool SLOT_MEM>
 __device__ inline Smem carve(unsigned char* base, const DevPlan& P, int T)
 {
     Smem s;
@@ -74,7 +76,7 @@ __device__ inline Smem carve(unsigned char* base, const DevPlan& P, int T)
     s.part = s.stk;
     o += stack_part_bytes(T, P.stack_depth, P.stack_factors);
     s.slots = reinterpret_cast<float*>(base + o);
-    o += align16(sizeof(float) * (size_t)P.n_slots_used * (T + 1));
+    if (!SLOT_MEM || !P.slot_mem) o += align16(sizeof(float) * (size_t)P.n_slots_used * (T + 1));
     s.grp = reinterpret_cast<float*>(base + o);
     o += align16(sizeof(float) * (size_t)P.n_groups * (T + 1));
     s.last = reinterpret_cast<float*>(base + o);
@@ -686,15 +688,18 @@ __device__ __forceinline__ void pair_events(const DevPlan& P, const Smem& S, int
 // registers across the step and measured slower (2.93 against 2.75 ms for the 2^20-path Heston
 // grid). The other pass loads it one step ahead, which measured faster where the paths are
 // stored (GBM, 2^20 paths x 252 steps: 1.11 against 1.23 ms).
-template <int TB, int MODEL, bool UNIFORM, bool FAST>
+// AT: the pass is asset a0's of a multi-asset book; else the book's only asset. MODEL M_SEQ: the
+// asset's model is looked up (the passes of such books that are not FAST).
+template <int TB, int MODEL, bool UNIFORM, bool FAST, bool AT>
 __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairLane& L,
                                           const uint64_t (&n)[2], const bool (&valid)[2], int a0, float4 u0,
                                           float4 u1, float4 u2)
 {
     constexpr int T = 1 << TB, TH = T / 2;
     constexpr bool SEQ = MODEL == M_SEQ;
+    static_assert(!SEQ || AT, "a pass with its model looked up is one of several");
     const int t = threadIdx.x;
-    const int aid = SEQ ? a0 : 0;
+    const int aid = AT ? a0 : 0;
     const int model = SEQ ? P.model[aid] : MODEL;
     // the spot factor, and the variance factor where the model has one: compact stack row and
     // reference factor index (the dimension of a node is its bridge step * F + that index)
@@ -703,7 +708,7 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairL
     // rows 0 and 1 of a two-row stack and the asset's own factors.
     const bool act1 = MODEL == M_GBM ? false : (SEQ ? model != M_GBM : true);
     constexpr int ci0 = 0, ci1 = 1;
-    const int fid0 = SEQ ? P.fid_spot[aid] : 0, fid1 = SEQ ? P.fid_var[aid] : 1;
+    const int fid0 = AT ? P.fid_spot[aid] : 0, fid1 = AT ? P.fid_var[aid] : 1;
     constexpr int nfa = MODEL == M_GBM ? 1 : 2;
     float2* const stk = reinterpret_cast<float2*>(S.stk) + t; // this thread's column of the stack
     const bool degenerate = P.degenerate[aid] != 0;
@@ -885,9 +890,13 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
     constexpr int T = 1 << TB;  // paths per tile
     constexpr int TH = T / PP;  // threads per CTA; path p of thread t is tile column t + p * TH
     constexpr int FS = 2 * NA;
-    const Smem S = carve(smem_raw, P, T);
+    // two paths a thread, one pass per asset: the specialised passes, slots in global memory
+    // where the plan says so, and products summed as eval_threads threads would
+    constexpr bool SEQ2 = MODEL == M_SEQ && NA == 1 && PP == 2;
+    Smem S = carve<SEQ2>(smem_raw, P, T);
     const int t = threadIdx.x;
     const int stride = T + 1;
+    if (SEQ2 && P.slot_mem) S.slots = P.slot_mem + (size_t)blockIdx.x * P.n_slots_used * stride;
     __shared__ int s_cancel;
 
     for (int j = t; j < P.n_acc; j += TH) acc[j] = 0.0;
@@ -984,10 +993,22 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
             if constexpr (NA == 1 && PP == 2) {
                 // both passes in one kernel: the fast pass's own instantiation measured slower
                 // (Heston grid 2.91 against 2.75 ms, same box)
-                if (fast_pass(P))
-                    pair_pass<TB, MODEL, UNIFORM, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
-                else
-                    pair_pass<TB, MODEL, UNIFORM, false>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                if constexpr (SEQ) {
+                    // a pass of its own for each model: with the model looked up in the step loop,
+                    // and one path a thread, the five-asset LSV book took 34.1 ms (see SEQ2)
+                    if (!fast_pass(P))
+                        pair_pass<TB, M_SEQ, false, false, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                    else if (P.model[a0] == M_LSV)
+                        pair_pass<TB, M_LSV, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                    else if (P.model[a0] == M_HESTON)
+                        pair_pass<TB, M_HESTON, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                    else
+                        pair_pass<TB, M_GBM, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                } else if (fast_pass(P)) {
+                    pair_pass<TB, MODEL, UNIFORM, true, false>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                } else {
+                    pair_pass<TB, MODEL, UNIFORM, false, false>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                }
                 continue;
             }
             // ---- path state -------------------------------------------------
@@ -1283,12 +1304,14 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
             continue;
         }
         ++ntile;
-        for (int pc = 0; pc < C; pc += TH) {
-            const int CP = min(C - pc, TH);
-            const int G = TH / CP;
-            const int pl = t % CP, g = t / CP;
-            float a6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (g < G) {
+        const int VT = SEQ2 ? P.eval_threads : TH; // threads the sums are laid out for (TH or T)
+        for (int pc = 0; pc < C; pc += VT) {
+            const int CP = min(C - pc, VT);
+            const int G = VT / CP;
+            for (int w = t; w < VT; w += TH) {
+                const int pl = w % CP, g = w / CP;
+                if (g >= G) continue;
+                float a6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 if (P.vanilla_only) {
                     // lean vanilla loop: f = max(a S + b, 0), no dispatch
                     const VanTerm vt = P.vterms[pc + pl];
@@ -1328,13 +1351,13 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                 for (int j = 0; j < 6; ++j) S.part[(g * CP + pl) * 6 + j] = a6[j];
             }
             __syncthreads();
-            if (t < CP) {
+            for (int q0 = t; q0 < CP; q0 += TH) {
                 float cf = 0.f, cd = 0.f, cg = 0.f;
                 if (P.vanilla_only) {
-                    const VanTerm vt = P.vterms[pc + t];
+                    const VanTerm vt = P.vterms[pc + q0];
                     cf = fmaxf(fmaf(vt.a, S.slots[vt.slot * stride + k0], vt.b), 0.f);
                 } else {
-                    const DevProduct pr = P.products[pc + t];
+                    const DevProduct pr = P.products[pc + q0];
                     cf = payoff(P, pr, S.slots, S.grp, stride, k0);
                     if (P.greeks) greeks_of(P, pr, S.slots, stride, k0, cd, cg);
                 }
@@ -1344,7 +1367,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                 float f6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 for (int g2 = 0; g2 < G; ++g2)
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) f6[j] += S.part[(g2 * CP + t) * 6 + j];
+                    for (int j = 0; j < 6; ++j) f6[j] += S.part[(g2 * CP + q0) * 6 + j];
                 double s6[6];
 #pragma unroll
                 for (int j = 0; j < 6; ++j) s6[j] = (double)f6[j];
@@ -1356,7 +1379,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                     s6[2 * q] = d1 + (double)nv * c;
                 }
 #pragma unroll
-                for (int j = 0; j < 6; ++j) acc[(size_t)(pc + t) * 6 + j] += s6[j];
+                for (int j = 0; j < 6; ++j) acc[(size_t)(pc + q0) * 6 + j] += s6[j];
             }
             __syncthreads();
         }

@@ -179,6 +179,8 @@ struct DevPlan {
     double* acc;                 // [gridDim][n_acc] per-CTA FP64 sums
     int n_acc;
     int few_m;                   // > 0: few-product accumulation over few_m moments (see book_kernel)
+    int eval_threads;            // assets in turn, two paths a thread: threads the product sums are laid out for
+    float* slot_mem;             // assets in turn: [gridDim][n_slots][T + 1] observation slots (null: shared memory)
     float* path_out;             // [n_steps + 1][path_ld] spot of asset path_asset at every date (null: not stored)
     int64_t path_ld;             // paths per stored date (the book's path count)
     int path_asset;

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(1 << TB) bridge_kernel(const DevPlan P, float*
     constexpr int T = 1 << TB;
     constexpr int NA = 1; // factor slots 0..1 carry reference factors 0..1
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const Smem S = carve(smem_raw, P, T);
+    const Smem S = carve<false>(smem_raw, P, T);
     const int t = threadIdx.x;
     for (int64_t tile = blockIdx.x; tile < P.n_tiles; tile += gridDim.x) {
         const int64_t m = P.tile_first + tile;

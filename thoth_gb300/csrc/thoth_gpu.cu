@@ -455,6 +455,7 @@ struct Plan {
         o_sord;
     int variant = 1, base_variant = 1, shape = 0, T = 256;
     size_t smem = 0;
+    bool slots_global = false; // observation slots in global memory (slot_rows_bytes)
     int n_products = 0;
     int64_t paths = 0;
     std::vector<int> greek_mask;
@@ -464,7 +465,9 @@ bool finite(double x) { return std::isfinite(x); }
 
 // Untuned shape of a single-asset-kernel plan: (8, 2), unless shared memory
 // caps the CTAs per SM so low that (8, 1), with the same tile and twice the
-// threads per CTA, keeps more threads resident. Needs a device (else 0).
+// threads per CTA, keeps more threads resident. Needs a device (else 0). A book
+// whose assets run in turn then moves its slots to global memory instead and
+// keeps (8, 2) (slots_to_global).
 int default_shape(int variant, size_t smem)
 {
     static std::map<std::pair<int, size_t>, int> memo;
@@ -483,8 +486,29 @@ int default_shape(int variant, size_t smem)
     return shape;
 }
 
-// shape < 0: the autotuned shape for the book's size, else the default
-int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1)
+// Observation slots in global memory: one row of T + 1 floats a slot and CTA, written once a
+// path and read by the product sums, so they cost little there, while in shared memory the
+// slots of a book with many products decide how many CTAs fit an SM. The five-asset LSV book
+// (30 slots) holds 69 KB a CTA with its slots in shared memory, three CTAs of 128 threads an
+// SM, and 37 KB without, six. Taken for books whose assets run in turn, two paths a thread,
+// where shared memory caps the CTAs below the six their registers allow; books of at most
+// four products (few_m) and books whose slots would pass SLOT_MAX_BYTES keep them in shared
+// memory.
+constexpr size_t SLOT_MAX_BYTES = size_t(256) << 20;
+constexpr int SEQ_CTAS = 6;
+
+size_t slot_row_bytes(const Plan& P) { return sizeof(float) * (size_t)P.dp.n_slots_used * (P.T + 1); }
+
+bool slots_to_global(const Plan& P)
+{
+    if (P.variant != 6 || P.dp.few_m > 0 || (P.shape != 0 && P.shape != 3)) return false;
+    if (!g_dev.ready || book_occupancy(P.variant, P.shape, P.smem) >= SEQ_CTAS) return false;
+    return slot_row_bytes(P) * (size_t)(2 * SEQ_CTAS) * (size_t)g_dev.sms <= SLOT_MAX_BYTES;
+}
+
+// shape < 0: the autotuned shape for the book's size, else the default. own_memory: the plan's
+// memory is the caller's (the allocation-free entry point), its slots stay in shared memory
+int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1, bool own_memory = false)
 {
     const bool untuned = shape < 0;
     if (!d) return fail(THOTH_GPU_E_INVALID, "null descriptor");
@@ -1019,6 +1043,18 @@ int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1)
     P.o_sord = P.blob.put(order);
     // shapes 0 and 1 share the 256-path tile, so the plan above serves both
     if (untuned && !tuned && P.variant != 3 && P.shape == 0) P.shape = default_shape(P.variant, P.smem);
+    D.eval_threads = book_shape_threads(P.variant, P.shape);
+    if (!own_memory) {
+        // the product sums stay laid out as for the shape the plan would have had, so a book's
+        // results do not depend on where its slots are
+        const int shape_shared = P.shape;
+        if (untuned && !tuned && P.shape == 1) P.shape = 0;
+        P.slots_global = slots_to_global(P);
+        if (P.slots_global)
+            P.smem = book_smem_bytes(T, D.sobol_dims, D.stack_depth, D.stack_factors, 0, D.n_groups, D.n_last, D.few_m);
+        else
+            P.shape = shape_shared;
+    }
     return THOTH_GPU_OK;
 }
 
@@ -1134,7 +1170,21 @@ cudaError_t gather_low(const Plan& P, cudaStream_t st)
     return e;
 }
 
-// device layout of one priced book: [plan blob][low Sobol words][acc rows][out][status]
+// a book's per-CTA memory: its FP64 rows of sums, then (slots_global) its slots
+size_t sums_bytes(const Plan& P, int grid) { return (sizeof(double) * (size_t)grid * P.dp.n_acc + 255) & ~size_t(255); }
+size_t rows_bytes(const Plan& P, int grid)
+{
+    return sums_bytes(P, grid) + (P.slots_global ? (slot_row_bytes(P) * (size_t)grid + 255) & ~size_t(255) : 0);
+}
+
+// places it at `rows` (a region of rows_bytes(P, grid) bytes)
+void bind_rows(Plan& P, unsigned char* rows, int grid)
+{
+    P.dp.acc = reinterpret_cast<double*>(rows);
+    P.dp.slot_mem = P.slots_global ? reinterpret_cast<float*>(rows + sums_bytes(P, grid)) : nullptr;
+}
+
+// device layout of one priced book: [plan blob][low Sobol words][acc rows, slots][out][status]
 struct Layout {
     size_t o_lo, o_acc, o_out, o_st, total;
 };
@@ -1145,7 +1195,7 @@ Layout layout_of(const Plan& P, int grid)
     const size_t n_acc = (size_t)P.dp.n_acc;
     L.o_lo = (P.blob.bytes.size() + 255) & ~size_t(255);
     L.o_acc = L.o_lo + ((low_bytes(P) + 255) & ~size_t(255));
-    L.o_out = L.o_acc + ((sizeof(double) * grid * n_acc + 255) & ~size_t(255));
+    L.o_out = L.o_acc + rows_bytes(P, grid);
     L.o_st = L.o_out + ((sizeof(double) * n_acc + 255) & ~size_t(255));
     L.total = L.o_st + 256;
     return L;
@@ -1160,7 +1210,7 @@ int run_bound(Plan& P, unsigned char* base, const Layout& L, int grid, ThothBook
     int rc = ensure_pinned(sizeof(double) * n_acc + sizeof(int));
     if (rc) return rc;
     bind_low(P, base + L.o_lo);
-    P.dp.acc = reinterpret_cast<double*>(base + L.o_acc);
+    bind_rows(P, base + L.o_acc, grid);
     P.dp.status = reinterpret_cast<int*>(base + L.o_st);
     CUDA_TRY(cudaMemsetAsync(base + L.o_st, 0, sizeof(int), st));
     CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
@@ -1635,7 +1685,7 @@ static int price_noalloc_locked(const ThothBookDesc* book, ThothBookResult* out)
     int rc = noalloc_address(dev, &base);
     if (rc) return rc;
     Plan P;
-    rc = build_plan(book, P);
+    rc = build_plan(book, P, -1, true);
     if (rc) return rc;
     // direction numbers of the book's Sobol dimensions, from the embedded table
     std::vector<uint32_t> V, lo;
@@ -1873,10 +1923,6 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         grid[b] = grid_for(plans[b], g_batch.policy);
         o_blob[b] = off;
         off += up(plans[b].blob.bytes.size());
-        o_lo[b] = off;
-        off += up(low_bytes(plans[b]));
-        o_acc[b] = off;
-        off += up(sizeof(double) * (size_t)grid[b] * plans[b].dp.n_acc);
         sig += "|" + std::to_string(plans[b].variant) + "," + std::to_string(plans[b].shape) + "," +
                std::to_string(grid[b]) + "," +
                std::to_string(plans[b].smem) + "," + std::to_string(plans[b].blob.bytes.size()) + "," +
@@ -1909,6 +1955,14 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
                std::to_string(BL.items);
         for (int b : BL.books) sig += "," + std::to_string(b);
     }
+    // what is uploaded ends here; the books' low words, rows and slots are the device's own
+    const size_t up_bytes = off;
+    for (int b = 0; b < n; b++) {
+        o_lo[b] = off;
+        off += up(low_bytes(plans[b]));
+        o_acc[b] = off;
+        off += rows_bytes(plans[b], grid[b]);
+    }
     // outputs and status words (then the work counter) contiguous at the end: one device->host copy
     const size_t o_outs = off;
     size_t cur = o_outs;
@@ -1933,18 +1987,18 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         CUDA_TRY(dev_alloc(&g_batch.dev, total));
         g_batch.dev_size = total;
     }
-    if (std::max(o_outs, back) > g_batch.host_size) {
+    if (std::max(up_bytes, back) > g_batch.host_size) {
         if (g_batch.host) cudaFreeHost(g_batch.host);
         g_batch.host = nullptr;
         g_batch.host_size = 0;
-        CUDA_TRY(host_alloc(&g_batch.host, std::max(o_outs, back)));
-        g_batch.host_size = std::max(o_outs, back);
+        CUDA_TRY(host_alloc(&g_batch.host, std::max(up_bytes, back)));
+        g_batch.host_size = std::max(up_bytes, back);
     }
     for (int b = 0; b < n; b++) {
         std::memcpy(g_batch.host + o_blob[b], plans[b].blob.bytes.data(), plans[b].blob.bytes.size());
         bind(plans[b], g_batch.dev + o_blob[b]);
         bind_low(plans[b], g_batch.dev + o_lo[b]);
-        plans[b].dp.acc = reinterpret_cast<double*>(g_batch.dev + o_acc[b]);
+        bind_rows(plans[b], g_batch.dev + o_acc[b], grid[b]);
         plans[b].dp.status = reinterpret_cast<int*>(g_batch.dev + o_st[b]);
         // the kernel parameters are baked into the graph: a replay needs them byte-equal
         sig.append(reinterpret_cast<const char*>(&plans[b].dp), sizeof(DevPlan));
@@ -1968,7 +2022,7 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         }
     }
     cudaStream_t st = g_dev.stream;
-    CUDA_TRY(cudaMemcpyAsync(g_batch.dev, g_batch.host, o_outs, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(g_batch.dev, g_batch.host, up_bytes, cudaMemcpyHostToDevice, st));
     if (g_batch.signature != sig || !g_batch.exec) {
         if (g_batch.exec) cudaGraphExecDestroy(g_batch.exec);
         g_batch.exec = nullptr;
@@ -2022,7 +2076,7 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         r->book_premium = o[6 * (size_t)P.n_products] / np_;
         r->book_trust = trust_of(o[6 * (size_t)P.n_products], o[6 * (size_t)P.n_products + 1], np_);
         r->device_ms = ms; // the whole batch's device time
-        r->h2d_bytes = b == 0 ? (int64_t)o_outs : 0;
+        r->h2d_bytes = b == 0 ? (int64_t)up_bytes : 0;
         r->d2h_bytes = b == 0 ? (int64_t)back : 0;
     }
     return THOTH_GPU_OK;
@@ -2072,7 +2126,7 @@ static int autotune_book_locked(const ThothBookDesc* book, int reps, ThothTuneRe
         bind(P, g_dev.arena);
         bind_low(P, g_dev.arena + L.o_lo);
         CUDA_TRY(gather_low(P, st));
-        P.dp.acc = reinterpret_cast<double*>(g_dev.arena + L.o_acc);
+        bind_rows(P, g_dev.arena + L.o_acc, gmax);
         P.dp.status = reinterpret_cast<int*>(g_dev.arena + L.o_st);
         for (size_t c = 0; c < grids.size(); c++) {
             const int g = grids[c];
