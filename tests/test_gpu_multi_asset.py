@@ -46,13 +46,22 @@ def book(models, n_products, paths, skip=0, steps=36):
 @pytest.mark.parametrize("models,n_products,paths,skip", [
     (("lsv", "lsv"), 60, 4099, 0),              # no tile boundary at the last path
     (("gbm", "heston", "lsv"), 129, 2 ** 12, 5),  # more products than threads of a CTA
-    (("heston", "gbm", "lsv", "lsv"), 300, 1000, 255),  # more than a tile has columns
+    (("heston", "gbm", "lsv", "lsv"), 300, 1000, 255),  # slots beyond what shared memory may hold
+    (("lsv", "gbm"), 300, 1000, 255),  # more products than a tile has columns
     (("lsv", "heston"), 4, 300, 1),             # the few-product sums: slots stay shared
     (("lsv", "heston"), 5, 300, 1),
     (("heston",) * 8, 200, 513, 0),
+    (("heston",) * 8, 40, 513, 0),
 ])
 def test_assets_in_turn_slots_in_either_memory(gpu, models, n_products, paths, skip):
     b = book(models, n_products, paths, skip)
+    if n_products * len(models) > 1000:  # refused wherever its slots would go
+        with pytest.raises(gpu.ThothGpuError) as e:
+            gpu.price_book(b)
+        assert e.value.code == abi.THOTH_GPU_E_TOO_LARGE
+        return
+    if n_products > 256:
+        b = book(models, n_products, paths, skip, steps=20)
     r = gpu.price_book(b)
     ref = oracle.price_book(b, threads=THREADS)
     assert_shared_path_parity(r, ref["premium"], ref["trust"], "book", scale=1.0)

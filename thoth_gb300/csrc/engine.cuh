@@ -63,15 +63,23 @@ struct StepProg {
 
 // per-step record read once per step (at the step, or one step ahead): the first
 // bridge node inline, the node count (0 = pop), the remaining nodes' start,
-// 1/sqrt(dt) of the path generator, and whether any asset has events this date
+// 1/sqrt(dt) of the path generator, and the date's events, four bits an asset (SEV_*)
 struct alignas(16) StepRec {
     float lw, rw, sd;
     int dim;   // reference dimension of the first node for factor 0: bstep * F
     float isd;
     int count;
     int first; // index of the second node in nodes[] (when count > 1)
-    int ev;    // 1: events on this date
+    uint32_t ev; // SEV_* bits of asset a at 4 a
 };
+
+// A step's events of one asset, as the pair pass takes them. An asset's main running minimum,
+// maximum and sum of squared steps (its main groups) are updated on most dates of a book with
+// daily monitoring, so their updates need no event record: the bit says that the group takes
+// this date, and the group's row is in the plan. Their shifts (a quanto) come from ev_p where
+// the asset has any. The other events come from the event list, after the main ones.
+enum : uint32_t { SEV_MIN = 1, SEV_MAX = 2, SEV_SQ = 4, SEV_LIST = 8 };
+constexpr uint32_t SEV_MAIN = SEV_MIN | SEV_MAX | SEV_SQ;
 
 // path events, applied after the state at date i is known
 enum : int {
@@ -158,7 +166,10 @@ struct DevPlan {
     int uniform_steps;           // 1: every step's AssetStep equals step 1's
     const BridgeNode* nodes;     // time-ordered program
     const int2* ev_range;        // [(n_steps + 1)][n_assets] (first, count) into events; row 0 = date 0
-    const Event* events;
+    const Event* events;         // per (date, asset) the main groups' updates first
+    const float4* ev_p;          // [(n_steps + 1)][n_assets] shifts of the main groups' updates
+    int ev_shift[MAX_ASSETS];    // 1: the asset's main groups have shifts in ev_p
+    int main_row[3][MAX_ASSETS]; // groups of the main minimum, maximum and sum of squared steps
     const int* lev_layer;        // [n_assets][n_steps + 1] layer of date i
     const float2* lev_map;       // [n_assets][layers] (1/ln_step, lnS0/ln_step - offset)
     const float* lev_values;     // [n_assets][layers][lev_row_stride]

@@ -374,7 +374,7 @@ bool build_bridge(const std::vector<double>& t, BridgeProgram& out, std::string&
 
 // per-step records: first node inline, node count, 1/sqrt(dt), event flag; one zero record
 // past the last step, which a load one step ahead reads at the last step
-std::vector<StepRec> make_recs(const BridgeProgram& bp, const std::vector<float>& isd, const std::vector<char>& ev_flag,
+std::vector<StepRec> make_recs(const BridgeProgram& bp, const std::vector<float>& isd, const std::vector<uint32_t>& ev_flag,
                                int ref_factors)
 {
     const size_t N = isd.size();
@@ -451,7 +451,7 @@ struct Plan {
     DevPlan dp{};
     Blob blob;
     // offsets of the sections inside the blob
-    size_t o_steps, o_isd, o_prog, o_nodes, o_recs, o_evr, o_ev, o_lay, o_map, o_levv, o_ginit, o_prod, o_vterm, o_comp,
+    size_t o_steps, o_isd, o_prog, o_nodes, o_recs, o_evr, o_ev, o_evp, o_lay, o_map, o_levv, o_ginit, o_prod, o_vterm, o_comp,
         o_sord;
     int variant = 1, base_variant = 1, shape = 0, T = 256;
     size_t smem = 0;
@@ -991,17 +991,61 @@ int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1, bool own_memory 
     D.n_groups = (int)grp_init.size();
     if (grp_init.empty()) grp_init.push_back(0.f);
     D.n_products = d->n_products;
-    // events, ordered per (date, asset)
+    // each asset's main groups (engine.cuh, SEV_*): of each kind the group with the most dates (the
+    // first of them), -1 where it has none
+    auto main_kind = [](const Event& e) {
+        return e.type == EV_GRP_MIN ? 0 : e.type == EV_GRP_MAX ? 1 : e.type == EV_GRP_SQ_STEP ? 2 : -1;
+    };
+    for (int a = 0; a < NA; a++) {
+        std::map<int, int> dates; // group -> its updates
+        int most[3] = {0, 0, 0};
+        for (int k = 0; k < 3; k++) D.main_row[k][a] = -1;
+        for (int i = 1; i < nd; i++)
+            for (const Event& e : ev[(size_t)i * NA + a])
+                if (main_kind(e) >= 0) dates[e.a]++;
+        for (int i = 1; i < nd; i++)
+            for (const Event& e : ev[(size_t)i * NA + a]) {
+                const int k = main_kind(e);
+                // the allocation-free entry point's memory has no room for shifts
+                if (k < 0 || dates[e.a] <= most[k] || (own_memory && e.p != 0.f)) continue;
+                most[k] = dates[e.a];
+                D.main_row[k][a] = e.a;
+            }
+    }
+    // events, ordered per (date, asset): the main groups' updates, then the others as they came
+    // (a group's snapshot follows its update either way)
     std::vector<int2> ev_range((size_t)nd * NA);
     std::vector<Event> events;
-    std::vector<char> ev_flag(N, 0);
+    std::vector<uint32_t> ev_flag(N, 0);
+    std::vector<float4> ev_p((size_t)nd * NA, make_float4(0.f, 0.f, 0.f, 0.f));
     for (size_t k = 0; k < ev.size(); k++) {
-        ev_range[k] = make_int2((int)events.size(), (int)ev[k].size());
-        events.insert(events.end(), ev[k].begin(), ev[k].end());
         const size_t date = k / NA;
-        if (!ev[k].empty() && date >= 1) ev_flag[date - 1] = 1;
+        const int a = (int)(k % NA);
+        uint32_t flags = 0;
+        ev_range[k] = make_int2((int)events.size(), (int)ev[k].size());
+        std::vector<char> taken(ev[k].size(), 0);
+        for (int m = 0; m < 3; m++)
+            for (size_t e = 0; e < ev[k].size(); e++) {
+                const Event& E = ev[k][e];
+                if (main_kind(E) != m || E.a != D.main_row[m][a] || (own_memory && E.p != 0.f)) continue;
+                taken[e] = 1;
+                flags |= 1u << m;
+                events.push_back(E);
+                (m == 0 ? ev_p[k].x : m == 1 ? ev_p[k].y : ev_p[k].z) = E.p;
+                if (E.p != 0.f) D.ev_shift[a] = 1;
+                break;
+            }
+        for (size_t e = 0; e < ev[k].size(); e++)
+            if (!taken[e]) {
+                events.push_back(ev[k][e]);
+                flags |= SEV_LIST;
+            }
+        if (date >= 1) ev_flag[date - 1] |= flags << (4 * a);
     }
     if (events.empty()) events.push_back(Event{0, 0, 0.f, 0});
+    bool shifted = false;
+    for (int a = 0; a < NA; a++) shifted |= D.ev_shift[a] != 0;
+    if (!shifted) ev_p.clear(); // no date reads it
     const std::vector<StepRec> recs = make_recs(bp, isd, ev_flag, F);
     std::vector<int> order = sobol_order(bp, D, P.variant == 6);
     D.n_sobol = (int)order.size();
@@ -1033,6 +1077,7 @@ int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1, bool own_memory 
     P.o_recs = P.blob.put(recs);
     P.o_evr = P.blob.put(ev_range);
     P.o_ev = P.blob.put(events);
+    P.o_evp = P.blob.put(ev_p);
     P.o_lay = P.blob.put(lev_layer);
     P.o_map = P.blob.put(lev_map);
     P.o_levv = P.blob.put(lev_values);
@@ -1068,6 +1113,7 @@ void bind(Plan& P, unsigned char* base)
     D.recs = reinterpret_cast<const StepRec*>(base + P.o_recs);
     D.ev_range = reinterpret_cast<const int2*>(base + P.o_evr);
     D.events = reinterpret_cast<const Event*>(base + P.o_ev);
+    D.ev_p = reinterpret_cast<const float4*>(base + P.o_evp);
     D.lev_layer = reinterpret_cast<const int*>(base + P.o_lay);
     D.lev_map = reinterpret_cast<const float2*>(base + P.o_map);
     D.lev_values = reinterpret_cast<const float*>(base + P.o_levv);
@@ -3005,7 +3051,7 @@ int thoth_gpu_bridge_increments(const double* t, int32_t n_dates, int32_t factor
         P.o_isd = P.blob.put(isd);
         P.o_prog = P.blob.put(bp.prog);
         P.o_nodes = P.blob.put(bp.nodes);
-        P.o_recs = P.blob.put(make_recs(bp, isd, std::vector<char>(), factors));
+        P.o_recs = P.blob.put(make_recs(bp, isd, std::vector<uint32_t>(), factors));
         std::vector<int> order = sobol_order(bp, D);
         D.n_sobol = (int)order.size();
         P.o_sord = P.blob.put(order);
