@@ -185,3 +185,39 @@ def test_price_grid_pipeline_small(gpu):
     # the grid policy never takes over more buckets than the per-bucket one
     assert fails["grid"] <= fails["bucket"]
     m.close()
+
+
+@pytest.mark.parametrize("rows", [128, 640, 128 * 153])
+def test_gradient_tile_counts(gpu, rows):
+    """One tile, a few, and one more than the device has SMs: per-layer gradients against the
+    oracle (BF16 operands, as in test_gradient_matches_cpu_oracle)."""
+    m = S.Surrogate(seed=5)
+    p = m.params().astype(np.float64)
+    x, y, sc = _batch(rows, n=rows)
+    g, loss = m.gradient(x, y, sc)
+    go, lo = MO.gradient(p, x.astype(np.float64), y.astype(np.float64), sc.astype(np.float64))
+    assert abs(loss - lo) <= 1e-4 * lo
+    for a, b in [(MO.OFF_W1, MO.OFF_B1), (MO.OFF_B1, MO.OFF_W2), (MO.OFF_W2, MO.OFF_W5), (MO.OFF_W5, MO.N_PARAMS)]:
+        assert np.linalg.norm(g[a:b] - go[a:b]) <= 2e-3 * np.linalg.norm(go[a:b])
+    m.close()
+
+
+@pytest.mark.parametrize("n,batch", [(128, 128), (300, 128), (1000, 8192)])
+def test_training_step_is_adam_on_the_gradient(gpu, n, batch):
+    """The first step of a training call is Adam (FP32) on the gradient of its batch. Every element
+    moves by lr g / (|g| + eps) with eps 1e-8: equal to FP32 rounding wherever |g| is far above eps."""
+    x, y, sc = _batch(n, n=n)
+    rows = min(batch, n // 128 * 128)
+    x, y, sc = x[:rows], y[:rows], sc[:rows]  # one batch an epoch: the order only moves the sums' rounding
+    m, k = S.Surrogate(seed=6), S.Surrogate(seed=6)
+    p0 = m.params()
+    g, _ = m.gradient(x, y, sc)
+    g[:MO.OFF_B1] = 0.0
+    m.train(x, y, sc, epochs=1, batch=batch, lr=1e-3, seed=3)
+    d = m.params() - p0
+    lr = np.float32(1e-3 + 1e-6)
+    big = np.abs(g) > 1e-4 * np.abs(g).max()
+    assert big.sum() > 1000
+    np.testing.assert_allclose(d[big], -lr * np.sign(g[big]), rtol=2e-3)
+    k.close()
+    m.close()

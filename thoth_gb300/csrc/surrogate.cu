@@ -1,7 +1,6 @@
 // surrogate.cu — BF16 tensor-core (tcgen05) kernels of the learned Heston
 // surrogate: a validation GEMM, the fused MLP inference kernel, the training
-// layers (forward with bias + SiLU epilogue, backward for inputs and weights)
-// and Adam.
+// tile (forward, head, backward for inputs and weights) and Adam.
 #include "engine.cuh"
 #include "tc.cuh"
 
@@ -91,7 +90,8 @@ cudaError_t launch_tc_gemm_test(const void* A, const void* B, int N, int K, floa
 // The surrogate MLP: 7 inputs (padded to 16) -> 4 x 128 SiLU -> 1.
 // Parameters (FP32 master, offsets in floats):
 //   W1 [128][16], b1[128], W2..W4 [128][128] + b[128], w5[128], b5[1]
-// BF16 copies of W1..W4 are the tensor-core operands.
+// BF16 copies of W1..W4 are the tensor-core operands, kept in global memory in the operand
+// layout (tc::cm_offset), so a CTA's copy of them is a plain block copy.
 // ===========================================================================
 namespace mlp {
 
@@ -120,32 +120,6 @@ __device__ __forceinline__ float dsilu(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
-// stage an R x K row-major bf16 global tile (row stride ld elements, rows >= valid
-// are zero-filled) into the K-major core-matrix layout
-template <int R>
-__device__ __forceinline__ void stage(unsigned char* dst, const __nv_bfloat16* src, int ld, int K, int valid)
-{
-    const int kc = K / 8;
-    for (int c = threadIdx.x; c < R * kc; c += blockDim.x) {
-        const int r = c / kc, kb = c % kc;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < valid) v = *reinterpret_cast<const uint4*>(src + (size_t)r * ld + kb * 8);
-        *reinterpret_cast<uint4*>(dst + tc::cm_offset(r, kb * 8, R)) = v;
-    }
-}
-
-// stage the transpose: dst (R x K) element (r, k) = src[k][r], src row-major with
-// row stride ld, src rows >= valid_k are zero-filled
-template <int R>
-__device__ __forceinline__ void stage_t(unsigned char* dst, const __nv_bfloat16* src, int ld, int K, int valid_k)
-{
-    for (int e = threadIdx.x; e < R * K; e += blockDim.x) {
-        const int k = e / R, r = e % R; // consecutive threads read consecutive src columns
-        const __nv_bfloat16 v = (k < valid_k) ? src[(size_t)k * ld + r] : __float2bfloat16(0.f);
-        *reinterpret_cast<__nv_bfloat16*>(dst + tc::cm_offset(r, k, R)) = v;
-    }
-}
-
 struct Ctx {
     uint64_t* mbar;
     uint32_t tm;
@@ -153,276 +127,508 @@ struct Ctx {
     int* status;
 };
 
-// issue D (+)= A * B^T over K (single thread), then everyone waits for it
-__device__ __forceinline__ bool run_mma(Ctx& c, uint32_t dcol, const unsigned char* sA, int RA, const unsigned char* sB,
-                                        int RB, int K, bool accumulate_first)
+// ---------------------------------------------------------------------------
+// One training tile: 128 rows of the batch through the whole network and back, one CTA.
+//
+// Weights, activations and gradients of the tile never leave the SM: seven 32 KB operand
+// buffers in shared memory (W2, W3, W4, the activations a1..a3, and one that holds W1 and the
+// inputs during layer 1 and dz4 afterwards), and the four pre-activations' derivatives in the
+// 512 TMEM columns, where each layer's accumulator was. A buffer is reused as soon as the
+// products that read it are done: dz3 goes over W4, dz2 over W3, dz1 over dz4, the inputs (kept
+// in registers) over a3. dW = dz^T a and da = dz W read the same tiles as transposed operands
+// (tc::make_desc_mn), so nothing is transposed or stored twice. The da chain is the critical
+// path; each dW runs behind it into columns that are free by then, and is read out while the
+// next product runs.
+//
+// 512 threads do the epilogues: warp w owns rows 32 (w % 4) .. + 31 (its TMEM lanes) and columns
+// 32 (w / 4) .. + 31. The special-function unit bounds the forward half (two operations an
+// activation, 128 x 128 of them a layer at 16 a clock: 1.1 us); SiLU' is taken there as well,
+// from the same reciprocal, and kept, so the backward half has none. Four more warps add the bias
+// gradients, a column a thread in row order, beside the products that follow (in the epilogue
+// warps they held up every layer: 41 000 clocks a tile, about 33 000 beside them). Per-tile partial
+// gradients go to memory, dW as [in][out] so that a warp's lanes (out) store 128 consecutive
+// bytes; adam_kernel adds them in tile order. The two kernels are launched as programmatic
+// dependents: gathering the batch's rows and the launch itself overlap the other's end.
+//
+// As eight layer kernels with row-per-thread global accesses a step of 8192 rows took 0.50 ms
+// (64 CTAs, 12 to 29 warps stalled on global memory per issue); as this kernel and Adam, 35 us with
+// its host work.
+// ---------------------------------------------------------------------------
+struct TileArgs {
+    const __nv_bfloat16* x; // [n][16] normalised inputs of the training set
+    const float* y;         // [n] targets
+    const float* w;         // [n] loss weights 1 / scale^2
+    const int* perm;        // row r of the batch is perm[first + r] (null: first + r)
+    int64_t first;
+    int rows;               // batch rows (multiple of 128)
+    const float* params;    // FP32 master
+    const __nv_bfloat16* wbf; // bf16 W1..W4 in the operand layout
+    float* part;            // per-tile partial gradients, [tiles][N_PARAMS]
+    float* loss_part;       // [tiles]
+    int* status;
+};
+
+constexpr int TILE_MAIN = 512; // the epilogue threads
+constexpr int TILE_THREADS = TILE_MAIN + H;
+constexpr uint32_t TILE_BUF = H * H * 2; // one 128 x 128 bf16 operand
+constexpr size_t TILE_SMEM = 7 * (size_t)TILE_BUF;
+
+// issue D = A B^T over K (one thread); a tile of 128 rows is read as it lies (K along its
+// columns) or transposed (mn: K along its rows)
+__device__ __forceinline__ void issue(uint32_t d, const unsigned char* A, bool a_mn, const unsigned char* B, bool b_mn,
+                                      int N, int K)
 {
+    const uint32_t idesc = tc::make_idesc_bf16(128, N, a_mn, b_mn);
+    const uint32_t a0 = tc::smem_u32(A), b0 = tc::smem_u32(B);
+    for (uint32_t kk = 0; kk < (uint32_t)K / 16; ++kk) {
+        const uint64_t ad = a_mn ? tc::make_desc_mn(a0 + kk * 256, 128) : tc::make_desc(a0 + kk * 4096, 2048, 128);
+        const uint64_t bd = b_mn ? tc::make_desc_mn(b0 + kk * 256, 128) : tc::make_desc(b0 + kk * 4096, 2048, 128);
+        tc::mma_bf16(d, ad, bd, idesc, kk > 0 ? 1u : 0u);
+    }
+}
+
+// SiLU and its derivative from one reciprocal: z sigmoid(z) equals __fdividef(z, 1 + e^-z) bit for
+// bit (checked for every float z)
+__device__ __forceinline__ void silu_both(float z, float& a, float& d)
+{
+    const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+    a = z * s;
+    d = s * (1.0f + z * (1.0f - s));
+}
+
+// named barriers of the tile kernel: the epilogue threads' own; one for each dz tile, ready for its
+// bias gradient (each used once); dz4's bias gradient done, its buffer free
+enum : int { BAR_MAIN = 1, BAR_DZ = 2, BAR_D4_FREE = 6 };
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// 16 values of a row into columns c0 .. c0 + 15 of an operand tile, as bf16
+__device__ __forceinline__ void put16(unsigned char* tile, int row, int c0, const float (&v)[16])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        __align__(16) __nv_bfloat16 o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = __float2bfloat16(v[8 * h + j]);
+        *reinterpret_cast<uint4*>(tile + tc::cm_offset(row, c0 + 8 * h, ROWS)) = *reinterpret_cast<const uint4*>(o);
+    }
+}
+
+__global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileArgs A)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ uint64_t mb_w, mb_a, mb_b; // weights arrived; the da chain; the dW products
+    __shared__ uint32_t tm_s;
+    __shared__ float red[4][H];
+    __shared__ float red2[4][2];
+    float* const s_y = red[0];            // a row's partial head sum, then dL/dy
+    unsigned char *W2 = sm, *W3 = sm + TILE_BUF, *W4 = sm + 2 * TILE_BUF, *A1 = sm + 3 * TILE_BUF,
+                  *A2 = sm + 4 * TILE_BUF, *A3 = sm + 5 * TILE_BUF, *D4 = sm + 6 * TILE_BUF;
+    unsigned char *W1 = D4, *X = D4 + H * KIN * 2; // until dz4 is formed
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, cg = warp >> 2;
+    const int row = (warp & 3) * 32 + lane, c0 = cg * 32;
+    float* gp = A.part + (size_t)blockIdx.x * N_PARAMS;
+    if (t == 0) {
+        tc::mbar_init(&mb_w, 1);
+        tc::mbar_init(&mb_a, 1);
+        tc::mbar_init(&mb_b, 1);
+        tc::fence_mbar_init();
+        tc::fence_smem_async();
+    }
+    if (warp == 0) tc::tmem_alloc(&tm_s, 512);
+    // this thread's row of the set (perm and the set do not change while a step may overlap)
+    const int64_t r0 = A.first + (int64_t)blockIdx.x * ROWS;
+    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+    float yt = 0.f, wt = 0.f;
+    if (cg == 0 || cg == 3) {
+        const int64_t src = A.perm ? (int64_t)__ldg(A.perm + r0 + row) : r0 + row;
+        if (cg == 0) {
+            const uint4* xs = reinterpret_cast<const uint4*>(A.x + src * KIN);
+            x0 = __ldg(xs);
+            x1 = __ldg(xs + 1);
+            *reinterpret_cast<uint4*>(X + tc::cm_offset(row, 0, ROWS)) = x0;
+            *reinterpret_cast<uint4*>(X + tc::cm_offset(row, 8, ROWS)) = x1;
+        } else {
+            yt = __ldg(A.y + src);
+            wt = __ldg(A.w + src);
+        }
+    }
+    // The weights are there, and the partials free. Nothing the previous kernel writes is read
+    // before this, and the parameters never through the read-only path, which may run ahead of it.
+    tc::wait_previous();
+    if (t == 0) {
+        tc::mbar_expect(&mb_w, N_BF * 2);
+        tc::bulk_load(W1, A.wbf + OFF_BF_W1, H * KIN * 2, &mb_w);
+        tc::bulk_load(W2, A.wbf + OFF_BF_W2, 3 * TILE_BUF, &mb_w); // W2, W3, W4 follow on
+    }
     tc::fence_smem_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (threadIdx.x == 0) {
-        const uint32_t idesc = tc::make_idesc_bf16(RA, RB);
-        const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
-        for (int kk = 0; kk < K / 16; ++kk) {
-            const uint64_t ad = tc::make_desc(a0 + (uint32_t)(2 * kk) * (uint32_t)(RA * 16), (uint32_t)RA * 16, 128);
-            const uint64_t bd = tc::make_desc(b0 + (uint32_t)(2 * kk) * (uint32_t)(RB * 16), (uint32_t)RB * 16, 128);
-            tc::mma_bf16(c.tm + dcol, ad, bd, idesc, (kk > 0 || accumulate_first) ? 1u : 0u);
-        }
-        tc::mma_commit(c.mbar);
-    }
-    const bool ok = tc::mbar_wait(c.mbar, c.phase);
-    c.phase ^= 1u;
-    if (!ok && (threadIdx.x & 31) == 0) atomicExch(c.status, 1);
-    tc::fence_after_sync();
-    return ok;
-}
+    const uint32_t tm = tm_s;
+    bool ok = true;
 
-// 128-column row of this thread's TMEM lane (row = threadIdx.x) starting at col
-__device__ __forceinline__ void load_row(const Ctx& c, uint32_t col, int ncols, float* v)
-{
-    const int warp = threadIdx.x >> 5;
-    for (int c0 = 0; c0 < ncols; c0 += 16) {
-        float t[16];
-        tc::tmem_ld16(c.tm + ((uint32_t)(warp * 32) << 16) + col + (uint32_t)c0, t);
+    if (t >= TILE_MAIN) {
+        // db = the sum of dz over the tile's rows, in row order, a column a thread
+        const int o = t - TILE_MAIN;
+#pragma unroll 1
+        for (int l = 4; l >= 1; --l) {
+            bar_sync(BAR_DZ + 4 - l, TILE_THREADS);
+            const unsigned char* dz = l == 3 ? W4 : l == 2 ? W3 : D4;
+            float s = 0.f;
+#pragma unroll 16
+            for (int r = 0; r < ROWS; ++r)
+                s += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(dz + tc::cm_offset(r, o, ROWS)));
+            gp[b_off(l) + o] = s;
+            if (l == 4) bar_arrive(BAR_D4_FREE, TILE_THREADS);
+        }
+    } else {
+        uint32_t ph_a = 0, ph_b = 0;
+        auto operands_ready = [&] { // operand and TMEM accesses of every thread -> the next products
+            tc::fence_smem_async();
+            tc::fence_before_sync();
+            bar_sync(BAR_MAIN, TILE_MAIN);
+            tc::fence_after_sync();
+        };
+        auto wait_a = [&] {
+            ok = tc::mbar_wait(&mb_a, ph_a) && ok;
+            ph_a ^= 1u;
+            tc::fence_after_sync();
+        };
+        auto wait_b = [&] {
+            ok = tc::mbar_wait(&mb_b, ph_b) && ok;
+            ph_b ^= 1u;
+            tc::fence_after_sync();
+        };
+        const uint32_t at = tm + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0; // this thread's lane, column
+        ok = tc::mbar_wait(&mb_w, 0) && ok;
+
+        // ---- forward: layer l's accumulator in columns 128 (l - 1) ..; SiLU into the next operand,
+        // SiLU' over the accumulator ----------------------------------------------------------
+        unsigned char* const in[4] = {X, A1, A2, A3};
+        unsigned char* const wl[4] = {W1, W2, W3, W4};
+        const float4* w5 = reinterpret_cast<const float4*>(A.params + OFF_W5 + c0); // 16-byte aligned: OFF_W5 is a multiple of 4
+        static_assert(OFF_W5 % 4 == 0, "head weights are read four at a time");
+        float s4[32]; // layer 4: SiLU of this thread's columns
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[c0 + j] = t[j];
-    }
-}
-
-// write this thread's row of 128 bf16 values into a K-major core-matrix tile
-__device__ __forceinline__ void put_row(unsigned char* tile, int row, const float* v, int K)
-{
-    for (int kb = 0; kb < K / 8; ++kb) {
-        __align__(16) __nv_bfloat16 h[8];
+        for (int l = 1; l <= 4; ++l) {
+            if (t == 0) {
+                issue(tm + (uint32_t)(128 * (l - 1)), in[l - 1], false, wl[l - 1], false, H, l == 1 ? KIN : H);
+                tc::mma_commit(&mb_a);
+            }
+            const float* b = A.params + b_off(l) + c0;
+            float bv[16]; // requested before the wait, which covers their latency
 #pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16(v[kb * 8 + j]);
-        *reinterpret_cast<uint4*>(tile + tc::cm_offset(row, kb * 8, ROWS)) = *reinterpret_cast<const uint4*>(h);
-    }
-}
-
-struct TrainSched {
-    long long count;           // steps done in this training call
-    long long total;           // steps of the call
-    long long steps_per_epoch; // batches of one permutation
-    long long step0;           // Adam steps before the call
-    double lr0;                // peak learning rate
-    float lr_t, bc1, bc2;      // this step's learning rate and bias corrections
-    int rows;                  // batch rows
-    long long decay_steps;     // steps of the cosine decay (after them the rate stays at lr_lo)
-    double lr_lo;              // the rate the decay ends at
-};
-
-struct TrainArgs {
-    int rows;                       // batch rows (multiple of 128)
-    const __nv_bfloat16* x;         // [rows][16] normalised inputs
-    const float* y;                 // [rows] targets
-    const float* inv_w2;            // [rows] loss weights 1 / scale^2
-    const float* params;            // FP32 master
-    const __nv_bfloat16* wbf;       // bf16 W1..W4
-    float* z[5];                    // pre-activations of layers 1..4 ([rows][128]); index by layer
-    __nv_bfloat16* a[5];            // a[0] = x (alias), a[l] = SiLU(z[l]) ([rows][128])
-    __nv_bfloat16* dz[5];           // dL/dz of layers 1..4 ([rows][128])
-    float* part;                    // per-CTA partial gradients, [tiles][N_PARAMS]
-    float* loss_part;               // [tiles]
-    int* status;
-};
-
-// forward of hidden layer l for one 128-row tile; layer 4 also evaluates the head,
-// the loss and its gradient back to dz4, plus the head's weight gradients
-template <int L>
-__global__ void __launch_bounds__(128) fwd_layer_kernel(TrainArgs A)
-{
-    constexpr int K = (L == 1) ? KIN : H;
-    extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t tm_s;
-    __shared__ float red[4][H + 2];
-    unsigned char* sX = sm;                 // 128 x K
-    unsigned char* sW = sm + ROWS * K * 2;  // 128 x K
-    const int t = threadIdx.x, warp = t >> 5;
-    const int tile = blockIdx.x, r0 = tile * ROWS;
-    if (warp == 0) tc::tmem_alloc(&tm_s, 128);
-    if (t == 0) tc::mbar_init(&mbar, 1);
-    const __nv_bfloat16* src = (L == 1) ? A.x + (size_t)r0 * KIN : A.a[L - 1] + (size_t)r0 * H;
-    stage<ROWS>(sX, src, K, K, ROWS);
-    stage<ROWS>(sW, A.wbf + bf_off(L), K, K, H);
-    Ctx c{&mbar, 0, 0, A.status};
-    __syncthreads();
-    c.tm = tm_s;
-    const bool ok = run_mma(c, 0, sX, ROWS, sW, H, K, false);
-    float v[H];
-    if (ok) load_row(c, 0, H, v);
-    else
-        for (int j = 0; j < H; ++j) v[j] = 0.f;
-    const int row = r0 + t;
-    const float* b = A.params + b_off(L);
-    float* zr = A.z[L] + (size_t)row * H;
-    __nv_bfloat16* ar = A.a[L] + (size_t)row * H;
-    for (int j = 0; j < H; ++j) {
-        const float z = v[j] + b[j];
-        v[j] = z;
-        zr[j] = z;
-        ar[j] = __float2bfloat16(silu(z));
-    }
-    if (L == 4) {
-        // head y = w5 . a4 + b5, weighted MSE, dL/dy, dL/da4 = dy w5, dz4 = da4 * silu'(z4)
-        const float* w5 = A.params + OFF_W5;
-        float yhat = A.params[OFF_B5];
-        for (int j = 0; j < H; ++j) yhat = fmaf(w5[j], silu(v[j]), yhat);
-        const float e = yhat - A.y[row];
-        const float w = A.inv_w2[row];
-        const float dy = 2.f * e * w / (float)A.rows;
-        float* gp = A.part + (size_t)tile * N_PARAMS;
-        __nv_bfloat16* dzr = A.dz[4] + (size_t)row * H;
-        for (int j = 0; j < H; ++j) {
-            const float s = silu(v[j]);
-            dzr[j] = __float2bfloat16(dy * w5[j] * dsilu(v[j]));
-            v[j] = dy * s; // head weight gradient contribution of this row
+            for (int j = 0; j < 16; ++j) bv[j] = b[j];
+            wait_a();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float v[16], d[16];
+                const uint32_t col = at + (uint32_t)(128 * (l - 1) + 16 * h);
+                tc::tmem_ld16(col, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float z = v[j] + bv[j];
+                    silu_both(z, v[j], d[j]);
+                    if (l == 4) s4[16 * h + j] = v[j];
+                }
+                if (h == 0)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) bv[j] = b[16 + j];
+                if (l < 4) put16(in[l < 4 ? l : 0], row, c0 + 16 * h, v);
+                tc::tmem_st16(col, d);
+            }
+            tc::tmem_wait_st();
+            if (l < 4) operands_ready();
         }
-        // reduce over the tile's rows: warp shuffles then smem
-        const int lane = t & 31;
-        for (int j = 0; j < H; ++j) {
-            float s = v[j];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) red[warp][j] = s;
+        // ---- head: y = b5 + sum_j w5[j] a4[j], one column group after the other so that the sum
+        // runs in column order; weighted MSE, dL/dy ---------------------------------------------
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+            if (cg == g) {
+                float yh = g == 0 ? A.params[OFF_B5] : s_y[row];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float4 w = w5[j];
+                    yh = fmaf(w.x, s4[4 * j], yh);
+                    yh = fmaf(w.y, s4[4 * j + 1], yh);
+                    yh = fmaf(w.z, s4[4 * j + 2], yh);
+                    yh = fmaf(w.w, s4[4 * j + 3], yh);
+                }
+                if (g < 3) {
+                    s_y[row] = yh;
+                } else {
+                    const float e = yh - yt;
+                    const float dy = 2.f * e * wt / (float)A.rows;
+                    s_y[row] = dy;
+                    float sdy = dy, sl = e * e * wt;
+                    for (int o = 16; o > 0; o >>= 1) {
+                        sdy += __shfl_xor_sync(0xffffffffu, sdy, o);
+                        sl += __shfl_xor_sync(0xffffffffu, sl, o);
+                    }
+                    if (lane == 0) {
+                        red2[warp & 3][0] = sdy;
+                        red2[warp & 3][1] = sl;
+                    }
+                }
+            }
+            bar_sync(BAR_MAIN, TILE_MAIN);
         }
-        float sdy = dy, sl = e * e * w;
+        const float dy = s_y[row];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float d[16];
+            tc::tmem_ld16(at + (uint32_t)(384 + 16 * h), d);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 w = w5[4 * h + j];
+                d[4 * j] = dy * w.x * d[4 * j];
+                d[4 * j + 1] = dy * w.y * d[4 * j + 1];
+                d[4 * j + 2] = dy * w.z * d[4 * j + 2];
+                d[4 * j + 3] = dy * w.w * d[4 * j + 3];
+            }
+            put16(D4, row, c0 + 16 * h, d);
+        }
+        bar_arrive(BAR_DZ, TILE_THREADS);
+        operands_ready();
+        if (t == 0) { // da3 = dz4 W4
+            issue(tm + 384, D4, false, W4, true, H, H);
+            tc::mma_commit(&mb_a);
+        }
+        // the head's weight gradients: every column's sum over the warp's 32 rows by the butterfly
+        // tree of a shuffle reduction; at each level a lane keeps one half of its columns, so that
+        // lane k ends with column k
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s4[j] *= dy;
+#pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            sdy += __shfl_xor_sync(0xffffffffu, sdy, o);
-            sl += __shfl_xor_sync(0xffffffffu, sl, o);
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+                if (k < o) {
+                    const float keep = up ? s4[k + o] : s4[k], send = up ? s4[k] : s4[k + o];
+                    s4[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
         }
-        if (lane == 0) {
-            red[warp][H] = sdy;
-            red[warp][H + 1] = sl;
-        }
-        __syncthreads();
-        gp[OFF_W5 + t] = red[0][t] + red[1][t] + red[2][t] + red[3][t];
+        red[warp & 3][c0 + lane] = s4[0];
+
+        // ---- backward --------------------------------------------------------------------------
+        // dz_{l} = da_l SiLU'(z_l) into an operand tile: da_l in columns 384.., SiLU' in 128 (l - 1)..
+        auto input_grad = [&](int l, unsigned char* dst) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float v[16], d[16];
+                tc::tmem_ld16(at + (uint32_t)(384 + 16 * h), v);
+                tc::tmem_ld16(at + (uint32_t)(128 * (l - 1) + 16 * h), d);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] *= d[j];
+                put16(dst, row, c0 + 16 * h, v);
+            }
+            bar_arrive(BAR_DZ + 4 - l, TILE_THREADS);
+        };
+        // dW (rows out, columns in) from TMEM column dcol to the partials, [in][out]
+        auto weight_grad = [&](int l, uint32_t dcol) {
+            float* g = gp + w_off(l) + row;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float v[16];
+                tc::tmem_ld16(at + dcol + (uint32_t)(16 * h), v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) g[(c0 + 16 * h + j) * H] = v[j];
+            }
+        };
+        wait_a();
+        input_grad(3, W4);
+        operands_ready();
         if (t == 0) {
-            gp[OFF_B5] = red[0][H] + red[1][H] + red[2][H] + red[3][H];
-            A.loss_part[tile] = red[0][H + 1] + red[1][H + 1] + red[2][H + 1] + red[3][H + 1];
+            issue(tm + 384, W4, false, W3, true, H, H); // da2 = dz3 W3
+            tc::mma_commit(&mb_a);
+            issue(tm + 256, D4, true, A3, true, H, H);  // dW4 = dz4^T a3
+            tc::mma_commit(&mb_b);
+            gp[OFF_B5] = red2[0][0] + red2[1][0] + red2[2][0] + red2[3][0];
+            A.loss_part[blockIdx.x] = red2[0][1] + red2[1][1] + red2[2][1] + red2[3][1];
+        }
+        if (cg == 1) gp[OFF_W5 + row] = red[0][row] + red[1][row] + red[2][row] + red[3][row];
+        wait_a();
+        input_grad(2, W3);
+        wait_b();
+        if (cg == 0) { // a3 is done with: the inputs again, for dW1
+            *reinterpret_cast<uint4*>(A3 + tc::cm_offset(row, 0, ROWS)) = x0;
+            *reinterpret_cast<uint4*>(A3 + tc::cm_offset(row, 8, ROWS)) = x1;
+        }
+        operands_ready();
+        if (t == 0) {
+            issue(tm + 384, W3, false, W2, true, H, H); // da1 = dz2 W2
+            tc::mma_commit(&mb_a);
+            issue(tm + 128, W4, true, A2, true, H, H);  // dW3 = dz3^T a2
+            tc::mma_commit(&mb_b);
+        }
+        weight_grad(4, 256);
+        bar_sync(BAR_D4_FREE, TILE_THREADS);
+        wait_a();
+        tc::launch_dependents();
+        input_grad(1, D4);
+        wait_b();
+        operands_ready();
+        if (t == 0) {
+            issue(tm + 384, D4, true, A3, true, KIN, H); // dW1 = dz1^T x
+            issue(tm + 256, W3, true, A1, true, H, H);   // dW2 = dz2^T a1
+            tc::mma_commit(&mb_a);
+        }
+        weight_grad(3, 128);
+        wait_a();
+        weight_grad(2, 256);
+        if (cg == 0) {
+            float v[16];
+            tc::tmem_ld16(at + 384, v);
+#pragma unroll
+            for (int j = 0; j < KIN; ++j) gp[w_off(1) + j * H + row] = v[j];
         }
     }
+    if (!ok && lane == 0) atomicExch(A.status, 1);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(c.tm, 128);
+    if (warp == 0) tc::tmem_dealloc(tm, 512);
 }
 
-// backward of hidden layer l for one tile: partial dW_l = dz_l^T a_{l-1},
-// partial db_l = sum dz_l, and for l >= 2 dz_{l-1} = (dz_l W_l) * silu'(z_{l-1})
-template <int L>
-__global__ void __launch_bounds__(128) bwd_layer_kernel(TrainArgs A)
+// bf16 operand copy of parameter j (a weight of layer 1..4): its place in wbf, -1 for the others
+__host__ __device__ inline int bf_index(int j)
 {
-    constexpr int K = (L == 1) ? KIN : H; // input width of layer l
-    extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t tm_s;
-    unsigned char* sDzT = sm;                      // 128 (out) x 128 (rows): dz^T
-    unsigned char* sAT = sDzT + ROWS * H * 2;      // K (in) x 128 (rows): a_{l-1}^T
-    unsigned char* sDz = sAT + K * ROWS * 2;       // 128 (rows) x 128 (out): dz
-    unsigned char* sWT = sDz + ROWS * H * 2;       // K (in) x 128 (out): W^T
-    const int t = threadIdx.x, warp = t >> 5;
-    const int tile = blockIdx.x, r0 = tile * ROWS;
-    if (warp == 0) tc::tmem_alloc(&tm_s, 256);
-    if (t == 0) tc::mbar_init(&mbar, 1);
-    const __nv_bfloat16* dz = A.dz[L] + (size_t)r0 * H;
-    const __nv_bfloat16* ain = (L == 1) ? A.x + (size_t)r0 * KIN : A.a[L - 1] + (size_t)r0 * H;
-    stage_t<H>(sDzT, dz, H, ROWS, ROWS);           // (o, r) = dz[r][o]
-    stage_t<K>(sAT, ain, K, ROWS, ROWS);           // (i, r) = a[r][i]
-    if (L > 1) {
-        stage<ROWS>(sDz, dz, H, H, ROWS);          // (r, o) = dz[r][o]
-        stage_t<K>(sWT, A.wbf + bf_off(L), K, H, H); // (i, o) = W[o][i]
+    if (j < OFF_B1) return OFF_BF_W1 + (int)tc::cm_offset(j / KIN, j % KIN, H) / 2;
+    if (j < OFF_W2 || j >= OFF_W5) return -1;
+    const int l = (j - OFF_W2) / LAYER, o = (j - OFF_W2) % LAYER;
+    return o < H * H ? OFF_BF_W2 + l * H * H + (int)tc::cm_offset(o / H, o % H, H) / 2 : -1;
+}
+
+// The partial gradients lie [in][out] where the parameters lie [out][in]. Blocks of 32 (out) x 8
+// (in) weights: a warp sums one input's 32 outputs (128 consecutive bytes a tile), the sums cross
+// in shared memory, and each thread then has the parameter of its place in the parameters' order
+// (8 consecutive inputs of an output: 32 bytes). The last blocks take the biases and the head,
+// which lie alike. g: the block's sums; returns this thread's parameter, or -1.
+constexpr int GRAD_THREADS = 256;
+constexpr int GRAD_W1_BLOCKS = H / 32;            // inputs 0..6, with their low parts 7..13
+constexpr int GRAD_W_BLOCKS = (H / 32) * (H / 8); // per hidden layer
+constexpr int GRAD_VEC = 4 * H + H + 1;           // biases of layers 1..4, head weights, head bias
+constexpr int GRAD_BLOCKS = GRAD_W1_BLOCKS + 3 * GRAD_W_BLOCKS + (GRAD_VEC + GRAD_THREADS - 1) / GRAD_THREADS;
+
+// where a block's sums come from: the partials' index j of thread t's sum (-1: none), and whether
+// the low part's partials (7 inputs on) are added after it
+__device__ __forceinline__ int grad_source(int blk, int t, bool& lo)
+{
+    lo = false;
+    const int o = t & 31, i = t >> 5;
+    if (blk < GRAD_W1_BLOCKS) {
+        lo = true;
+        return i < 7 ? OFF_W1 + i * H + blk * 32 + o : -1;
     }
-    Ctx c{&mbar, 0, 0, A.status};
+    blk -= GRAD_W1_BLOCKS;
+    if (blk < 3 * GRAD_W_BLOCKS) {
+        const int l = blk / GRAD_W_BLOCKS, k = blk % GRAD_W_BLOCKS;
+        return OFF_W2 + l * LAYER + ((k >> 2) * 8 + i) * H + (k & 3) * 32 + o;
+    }
+    const int v = (blk - 3 * GRAD_W_BLOCKS) * GRAD_THREADS + t;
+    if (v >= GRAD_VEC) return -1;
+    return v < 4 * H ? b_off(1 + v / H) + v % H : OFF_W5 + v - 4 * H;
+}
+
+// the parameter that thread t of the block holds after the crossing (-1: none)
+__device__ __forceinline__ int grad_param(int blk, int t)
+{
+    const int o = t >> 3, i = t & 7;
+    if (blk < GRAD_W1_BLOCKS) return i < 7 ? OFF_W1 + (blk * 32 + o) * KIN + i : -1;
+    blk -= GRAD_W1_BLOCKS;
+    if (blk < 3 * GRAD_W_BLOCKS) {
+        const int l = blk / GRAD_W_BLOCKS, k = blk % GRAD_W_BLOCKS;
+        return OFF_W2 + l * LAYER + ((k & 3) * 32 + o) * H + (k >> 2) * 8 + i;
+    }
+    bool lo;
+    return grad_source(blk + GRAD_W1_BLOCKS, t, lo);
+}
+
+// SUM (float or double): the tiles' partials added in tile order
+template <class SUM>
+__device__ __forceinline__ SUM grad_sum(const float* part, int tiles, int j, SUM g)
+{
+    const float* p = part + j;
+    int tl = 0;
+    constexpr int F = 32; // loads in flight, added in order
+    for (; tl + F <= tiles; tl += F) {
+        float v[F];
+#pragma unroll
+        for (int k = 0; k < F; ++k) v[k] = __ldcg(p + (size_t)(tl + k) * N_PARAMS);
+#pragma unroll
+        for (int k = 0; k < F; ++k) g += (SUM)v[k];
+    }
+    for (; tl < tiles; ++tl) g += (SUM)__ldcg(p + (size_t)tl * N_PARAMS);
+    return g;
+}
+
+// a block's sums crossed from the partials' order into the parameters'
+template <class SUM>
+__device__ __forceinline__ SUM grad_cross(SUM (&s)[8][33], int blk, int t, SUM g)
+{
+    if (blk >= GRAD_W1_BLOCKS + 3 * GRAD_W_BLOCKS) return g; // the vectors lie alike
+    s[t >> 5][t & 31] = g;
     __syncthreads();
-    c.tm = tm_s;
-    // dW (128 out x K in) in TMEM columns [0, K)
-    bool ok = run_mma(c, 0, sDzT, H, sAT, K, ROWS, false);
-    float* gp = A.part + (size_t)tile * N_PARAMS;
-    {
-        float v[H];
-        if (ok) load_row(c, 0, K, v);
-        else
-            for (int j = 0; j < K; ++j) v[j] = 0.f;
-        float* gw = gp + w_off(L) + t * K; // row o = t
-        for (int j = 0; j < K; ++j) gw[j] = v[j];
-        // db_o = sum over rows of dz[r][o] (coalesced over o = t)
-        float s = 0.f;
-        for (int r = 0; r < ROWS; ++r) s += __bfloat162float(dz[(size_t)r * H + t]);
-        gp[b_off(L) + t] = s;
-    }
-    if (L > 1) {
-        // da_{l-1} (128 rows x K in) in TMEM columns [128, 128 + K)
-        ok = run_mma(c, 128, sDz, ROWS, sWT, K, H, false) && ok;
-        float v[H];
-        if (ok) load_row(c, 128, K, v);
-        else
-            for (int j = 0; j < K; ++j) v[j] = 0.f;
-        const int row = r0 + t;
-        const float* zp = A.z[L - 1] + (size_t)row * H;
-        __nv_bfloat16* out = A.dz[L - 1] + (size_t)row * H;
-        for (int j = 0; j < K; ++j) out[j] = __float2bfloat16(v[j] * dsilu(zp[j]));
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(c.tm, 256);
-}
-
-// the learning-rate schedule (a cosine decay from lr0 to lr_lo over decay_steps steps, then
-// lr_lo) and Adam's bias corrections of step `count` of a training call, computed where the
-// graph of one step can read them (its kernels' arguments stay the same from step to step)
-__host__ __device__ inline void sched_set(TrainSched& s)
-{
-    const double pi = 3.14159265358979323846;
-    const double step = (double)(s.step0 + s.count + 1);
-    const double c = (double)(s.count < s.decay_steps ? s.count : s.decay_steps);
-    s.lr_t = (float)(s.lr_lo + (s.lr0 - s.lr_lo) * 0.5 * (1.0 + cos(pi * c / (double)s.decay_steps)) + 1e-6);
-    s.bc1 = (float)(1.0 - pow(0.9, step));
-    s.bc2 = (float)(1.0 - pow(0.999, step));
-}
-
-__global__ void sched_advance_kernel(TrainSched* s)
-{
-    s->count += 1;
-    sched_set(*s);
+    return s[t & 7][t >> 3];
 }
 
 // grad[j] = sum over tiles of part[tile][j] (fixed order), then Adam on the FP32
 // master and refresh of the bf16 operand copies
-__global__ void adam_kernel(float* params, float* m, float* v, const float* part, int tiles, __nv_bfloat16* wbf,
-                            float lr, float b1, float b2, float eps, float bc1, float bc2, const TrainSched* sched)
+__global__ void __launch_bounds__(GRAD_THREADS) adam_kernel(float* params, float* m, float* v, const float* part,
+                                                            int tiles, __nv_bfloat16* wbf, float lr, float b1, float b2,
+                                                            float eps, float bc1, float bc2)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N_PARAMS) return;
-    if (sched) { // this step's learning rate and bias corrections, set by sched_advance_kernel
-        lr = sched->lr_t;
-        bc1 = sched->bc1;
-        bc2 = sched->bc2;
-    }
+    __shared__ float s[8][33];
+    const int t = threadIdx.x, blk = blockIdx.x;
+    bool lo;
+    const int js = grad_source(blk, t, lo);
     float g = 0.f;
-    for (int tl = 0; tl < tiles; ++tl) g += part[(size_t)tl * N_PARAMS + j];
-    // W1 columns f and f + 7 carry the hi and lo bf16 parts of feature f with one
-    // tied weight: column f's thread applies the summed gradient to both; columns
-    // 14 and 15 are padding and stay zero
-    if (j < OFF_B1) {
-        const int col = j % KIN;
-        if (col >= 7) return;
-        for (int tl = 0; tl < tiles; ++tl) g += part[(size_t)tl * N_PARAMS + j + 7];
+    tc::wait_previous();
+    if (js >= 0) {
+        g = grad_sum(part, tiles, js, g);
+        // W1 columns f and f + 7 carry the hi and lo bf16 parts of feature f with one
+        // tied weight: column f's thread applies the summed gradient to both; columns
+        // 14 and 15 are padding and stay zero
+        if (lo) g = grad_sum(part, tiles, js + 7 * H, g);
     }
+    tc::launch_dependents();
+    g = grad_cross(s, blk, t, g);
+    const int j = grad_param(blk, t);
+    if (j < 0) return;
     const float mj = fmaf(b1, m[j], (1.f - b1) * g);
     const float vj = fmaf(b2, v[j], (1.f - b2) * g * g);
     m[j] = mj;
     v[j] = vj;
     const float p = params[j] - lr * (mj / bc1) / (sqrtf(vj / bc2) + eps);
     params[j] = p;
-    // bf16 copies of W1..W4
+    const int bj = bf_index(j);
+    if (bj >= 0) wbf[bj] = __float2bfloat16(p);
     if (j < OFF_B1) {
         params[j + 7] = p;
-        wbf[OFF_BF_W1 + j] = __float2bfloat16(p);
-        wbf[OFF_BF_W1 + j + 7] = __float2bfloat16(p);
-    } else if (j >= OFF_W2 && j < OFF_W5) {
-        const int l = (j - OFF_W2) / LAYER, o = (j - OFF_W2) % LAYER;
-        if (o < H * H) wbf[OFF_BF_W2 + l * H * H + o] = __float2bfloat16(p);
+        wbf[bf_index(j + 7)] = __float2bfloat16(p);
+    }
+}
+
+// the gradient alone, in the parameters' order (W1's tied columns apart): the tiles' partials
+// summed in FP64 in tile order, rounded once
+__global__ void __launch_bounds__(GRAD_THREADS) gradient_kernel(const float* part, int tiles, float* grad)
+{
+    __shared__ double s[8][33];
+    const int t = threadIdx.x, blk = blockIdx.x;
+    bool lo;
+    const int js = grad_source(blk, t, lo);
+    const double g = grad_cross(s, blk, t, js >= 0 ? grad_sum(part, tiles, js, 0.0) : 0.0);
+    const int j = grad_param(blk, t);
+    if (j >= 0) grad[j] = (float)g;
+    if (blk < GRAD_W1_BLOCKS) { // the low parts' columns, and the padding's
+        for (int k = t; k < 9 * 32; k += GRAD_THREADS) {
+            const int i = 7 + k / 32, o = blk * 32 + k % 32;
+            grad[OFF_W1 + o * KIN + i] = (float)grad_sum(part, tiles, OFF_W1 + i * H + o, 0.0);
+        }
     }
 }
 
@@ -443,13 +649,11 @@ __global__ void weight_avg_finish_kernel(float* __restrict__ params, const float
     if (j < OFF_B1 && j % KIN >= 7) return; // the tied hi/lo columns are written by their partner
     const float p = avg[j];
     params[j] = p;
+    const int bj = bf_index(j);
+    if (bj >= 0) wbf[bj] = __float2bfloat16(p);
     if (j < OFF_B1) {
         params[j + 7] = p;
-        wbf[OFF_BF_W1 + j] = __float2bfloat16(p);
-        wbf[OFF_BF_W1 + j + 7] = __float2bfloat16(p);
-    } else if (j >= OFF_W2 && j < OFF_W5) {
-        const int l = (j - OFF_W2) / LAYER, o = (j - OFF_W2) % LAYER;
-        if (o < H * H) wbf[OFF_BF_W2 + l * H * H + o] = __float2bfloat16(p);
+        wbf[bf_index(j + 7)] = __float2bfloat16(p);
     }
 }
 
@@ -499,7 +703,7 @@ __global__ void __launch_bounds__(INFER_THREADS) infer_kernel(const __nv_bfloat1
                                                               float* __restrict__ y, int* status)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t mbar[INFER_WG];
+    __shared__ uint64_t mbar[INFER_WG], mb_w;
     __shared__ uint32_t tm_s;
     __shared__ __align__(16) float sb[4 * H + H + 1]; // biases of layers 1..4, head weights, head bias (pairs read as float2)
     unsigned char* sW1 = sm;                         // 128 x 16
@@ -508,10 +712,15 @@ __global__ void __launch_bounds__(INFER_THREADS) infer_kernel(const __nv_bfloat1
     unsigned char* sX = sW + 3 * H * H * 2 + wg * (ROWS * KIN * 2 + ROWS * H * 2); // this warpgroup's 128 x 16
     unsigned char* sAct = sX + ROWS * KIN * 2;                                    // and 128 x 128
     if (warp == 0) tc::tmem_alloc(&tm_s, INFER_TMEM_COLS);
-    if (t == 0)
+    if (t == 0) {
         for (int w = 0; w < INFER_WG; ++w) tc::mbar_init(&mbar[w], 1);
-    stage<H>(sW1, wbf + OFF_BF_W1, KIN, KIN, H);
-    for (int l = 0; l < 3; ++l) stage<H>(sW + l * H * H * 2, wbf + OFF_BF_W2 + l * H * H, H, H, H);
+        tc::mbar_init(&mb_w, 1);
+        tc::fence_mbar_init();
+        tc::fence_smem_async();
+        tc::mbar_expect(&mb_w, N_BF * 2);
+        for (int i = 0; i < N_BF * 2; i += 4096) // W1 and W2..W4 follow on in both memories
+            tc::bulk_load(sm + i, reinterpret_cast<const unsigned char*>(wbf) + i, 4096, &mb_w);
+    }
     for (int i = t; i < 4 * H; i += INFER_THREADS) sb[i] = params[b_off(1 + i / H) + i % H];
     for (int i = t; i < H; i += INFER_THREADS) sb[4 * H + i] = params[OFF_W5 + i];
     if (t == 0) sb[5 * H] = params[OFF_B5];
@@ -520,6 +729,8 @@ __global__ void __launch_bounds__(INFER_THREADS) infer_kernel(const __nv_bfloat1
     tc::fence_after_sync();
     Ctx c{&mbar[wg], tm_s + (uint32_t)(wg * 128), 0, status};
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16; // TMEM lanes of this warp
+    if (t == 0 && !tc::mbar_wait(&mb_w, 0)) atomicExch(status, 1);
+    __syncthreads(); // one thread waits for the weights: 2 % faster than every thread polling
     const int tiles = (n + ROWS - 1) / ROWS;
     for (int tile = INFER_WG * blockIdx.x + wg; tile < tiles; tile += INFER_WG * gridDim.x) {
         const int r0 = tile * ROWS;
@@ -598,63 +809,54 @@ __global__ void __launch_bounds__(INFER_THREADS) infer_kernel(const __nv_bfloat1
 } // namespace mlp
 
 // ---- launchers -----------------------------------------------------------------
-constexpr size_t kFwdSmem1 = (size_t)2 * mlp::ROWS * mlp::KIN * 2;
-constexpr size_t kFwdSmem = (size_t)2 * mlp::ROWS * mlp::H * 2;
-
-constexpr size_t kBwdSmem = (size_t)(mlp::ROWS * mlp::H + mlp::H * mlp::ROWS + mlp::ROWS * mlp::H + mlp::H * mlp::H) * 2;
-constexpr size_t kBwdSmem1 = (size_t)(mlp::ROWS * mlp::H + mlp::KIN * mlp::ROWS) * 2;
-
-// the layer kernels' shared-memory limits, set once per device (not inside a captured step)
-static cudaError_t train_attributes()
+// the tile kernel's shared-memory limit, once per device (not inside a training loop)
+cudaError_t mlp_train_prepare()
 {
-    using namespace mlp;
-    static bool set_on[64] = {};
-    int dev = 0;
-    cudaError_t e0 = cudaGetDevice(&dev);
-    if (e0 != cudaSuccess) return e0;
-    bool dummy = false;
-    bool& done = (dev >= 0 && dev < 64) ? set_on[dev] : dummy;
-    if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(fwd_layer_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fwd_layer_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fwd_layer_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fwd_layer_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_layer_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_layer_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_layer_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(bwd_layer_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem1);
-    done = e == cudaSuccess;
-    return e;
+    return cudaFuncSetAttribute(mlp::train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)mlp::TILE_SMEM);
 }
 
-cudaError_t mlp_train_prepare() { return train_attributes(); }
-
-// one training step: forward and backward layer by layer, Adam. With a schedule (sched not
-// null) the learning rate and bias corrections are read on the device, so the step's launches
-// have the same arguments every step and can be captured once into a graph.
-cudaError_t mlp_train_step(const mlp::TrainArgs& A, float* params, float* m, float* v, __nv_bfloat16* wbf, float lr,
-                           float b1, float b2, float eps, float bc1, float bc2, float* loss_out, cudaStream_t st,
-                           const mlp::TrainSched* sched)
+// a launch whose start may overlap the end of the stream's previous kernel (tc::wait_previous)
+template <class... P, class... Q>
+static cudaError_t launch_overlapped(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t st, Q... args)
 {
-    using namespace mlp;
-    const int tiles = A.rows / ROWS;
-    cudaError_t e = train_attributes();
-    if (e != cudaSuccess) return e;
-    fwd_layer_kernel<1><<<tiles, 128, kFwdSmem1, st>>>(A);
-    fwd_layer_kernel<2><<<tiles, 128, kFwdSmem, st>>>(A);
-    fwd_layer_kernel<3><<<tiles, 128, kFwdSmem, st>>>(A);
-    fwd_layer_kernel<4><<<tiles, 128, kFwdSmem, st>>>(A);
-    bwd_layer_kernel<4><<<tiles, 128, kBwdSmem, st>>>(A);
-    bwd_layer_kernel<3><<<tiles, 128, kBwdSmem, st>>>(A);
-    bwd_layer_kernel<2><<<tiles, 128, kBwdSmem, st>>>(A);
-    bwd_layer_kernel<1><<<tiles, 128, kBwdSmem1, st>>>(A);
-    adam_kernel<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(params, m, v, A.part, tiles, wbf, lr, b1, b2, eps, bc1, bc2,
-                                                         sched);
-    if (loss_out) sum_kernel<<<1, 256, 0, st>>>(A.loss_part, tiles, loss_out);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
+// the partial gradients and losses of a batch's tiles
+cudaError_t mlp_train_tiles(const mlp::TileArgs& A, cudaStream_t st)
+{
+    return launch_overlapped(mlp::train_tile_kernel, A.rows / mlp::ROWS, mlp::TILE_THREADS, mlp::TILE_SMEM, st, A);
+}
+
+cudaError_t mlp_adam(float* params, float* m, float* v, const float* part, int tiles, __nv_bfloat16* wbf, float lr,
+                     float b1, float b2, float eps, float bc1, float bc2, cudaStream_t st)
+{
+    return launch_overlapped(mlp::adam_kernel, mlp::GRAD_BLOCKS, mlp::GRAD_THREADS, 0, st, params, m, v, part, tiles, wbf,
+                             lr, b1, b2, eps, bc1, bc2);
+}
+
+cudaError_t mlp_gradient(const float* part, int tiles, float* grad, cudaStream_t st)
+{
+    mlp::gradient_kernel<<<mlp::GRAD_BLOCKS, mlp::GRAD_THREADS, 0, st>>>(part, tiles, grad);
     return cudaGetLastError();
 }
 
-void mlp_sched_init(mlp::TrainSched& s) { mlp::sched_set(s); }
+cudaError_t mlp_loss(const float* loss_part, int tiles, float* loss, cudaStream_t st)
+{
+    mlp::sum_kernel<<<1, 256, 0, st>>>(loss_part, tiles, loss);
+    return cudaGetLastError();
+}
 
 // sum = y (j == 0) or sum + y; at the last member (j == k - 1) the sum becomes the mean
 __global__ void mean_add_kernel(float* __restrict__ sum, const float* __restrict__ y, int64_t n, int j, int k)
@@ -684,12 +886,6 @@ cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16
     return cudaGetLastError();
 }
 
-cudaError_t mlp_sched_advance(mlp::TrainSched* s, cudaStream_t st)
-{
-    mlp::sched_advance_kernel<<<1, 1, 0, st>>>(s);
-    return cudaGetLastError();
-}
-
 cudaError_t mlp_infer(const __nv_bfloat16* x, int n, const float* params, const __nv_bfloat16* wbf, float* y,
                       int* status, int grid, cudaStream_t st)
 {
@@ -701,29 +897,34 @@ cudaError_t mlp_infer(const __nv_bfloat16* x, int n, const float* params, const 
     return cudaGetLastError();
 }
 
-// one training batch from the device-resident set: rows perm[first .. first + rows)
-__global__ void gather_batch_kernel(const __nv_bfloat16* __restrict__ X, const float* __restrict__ Y,
-                                    const float* __restrict__ W, const int* __restrict__ perm, int64_t first, int rows,
-                                    __nv_bfloat16* __restrict__ xb, float* __restrict__ yb, float* __restrict__ wb,
-                                    const mlp::TrainSched* sched)
+// a training set as the tile kernel reads it: each feature a bf16 pair hi + lo (columns f and
+// f + 7, tied weights), keeping about 16 significant bits of the input, and the loss weights
+// 1 / scale^2 (scale null: 1)
+__global__ void pack_set_kernel(const float* __restrict__ x, const float* __restrict__ scale, int64_t n,
+                                __nv_bfloat16* __restrict__ X, float* __restrict__ W)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    if (sched) first = (sched->count % sched->steps_per_epoch) * (int64_t)sched->rows; // this step's batch
-    const int64_t i = __ldg(perm + first + r);
-    const uint4* src = reinterpret_cast<const uint4*>(X + i * mlp::KIN);
-    uint4* dst = reinterpret_cast<uint4*>(xb + (int64_t)r * mlp::KIN);
-    dst[0] = __ldg(src);
-    dst[1] = __ldg(src + 1);
-    yb[r] = __ldg(Y + i);
-    wb[r] = __ldg(W + i);
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    __align__(16) __nv_bfloat16 h[mlp::KIN];
+#pragma unroll
+    for (int f = 0; f < 7; ++f) {
+        const float v = x[i * 7 + f];
+        h[f] = __float2bfloat16(v);
+        h[7 + f] = __float2bfloat16(v - __bfloat162float(h[f]));
+    }
+    h[14] = h[15] = __float2bfloat16(0.f);
+    uint4* dst = reinterpret_cast<uint4*>(X + i * mlp::KIN);
+    dst[0] = reinterpret_cast<const uint4*>(h)[0];
+    dst[1] = reinterpret_cast<const uint4*>(h)[1];
+    if (W) {
+        const double sc = scale ? (double)scale[i] : 1.0;
+        W[i] = (float)(1.0 / (sc * sc));
+    }
 }
 
-cudaError_t mlp_gather_batch(const __nv_bfloat16* X, const float* Y, const float* W, const int* perm, int64_t first,
-                             int rows, __nv_bfloat16* xb, float* yb, float* wb, cudaStream_t st,
-                             const mlp::TrainSched* sched)
+cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfloat16* X, float* W, cudaStream_t st)
 {
-    gather_batch_kernel<<<(rows + 127) / 128, 128, 0, st>>>(X, Y, W, perm, first, rows, xb, yb, wb, sched);
+    pack_set_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, scale, n, X, W);
     return cudaGetLastError();
 }
 

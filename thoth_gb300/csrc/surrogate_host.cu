@@ -18,43 +18,32 @@
 
 namespace thoth {
 namespace mlp {
-struct TrainArgs {
-    int rows;
+struct TileArgs {
     const __nv_bfloat16* x;
     const float* y;
-    const float* inv_w2;
+    const float* w;
+    const int* perm;
+    int64_t first;
+    int rows;
     const float* params;
     const __nv_bfloat16* wbf;
-    float* z[5];
-    __nv_bfloat16* a[5];
-    __nv_bfloat16* dz[5];
     float* part;
     float* loss_part;
     int* status;
 };
-struct TrainSched {
-    long long count, total, steps_per_epoch, step0;
-    double lr0;
-    float lr_t, bc1, bc2;
-    int rows;
-    long long decay_steps;
-    double lr_lo;
-};
 } // namespace mlp
-cudaError_t mlp_train_step(const mlp::TrainArgs& A, float* params, float* m, float* v, __nv_bfloat16* wbf, float lr,
-                           float b1, float b2, float eps, float bc1, float bc2, float* loss_out, cudaStream_t st,
-                           const mlp::TrainSched* sched = nullptr);
 cudaError_t mlp_train_prepare();
-void mlp_sched_init(mlp::TrainSched& s);
-cudaError_t mlp_sched_advance(mlp::TrainSched* s, cudaStream_t st);
+cudaError_t mlp_train_tiles(const mlp::TileArgs& A, cudaStream_t st);
+cudaError_t mlp_adam(float* params, float* m, float* v, const float* part, int tiles, __nv_bfloat16* wbf, float lr,
+                     float b1, float b2, float eps, float bc1, float bc2, cudaStream_t st);
+cudaError_t mlp_gradient(const float* part, int tiles, float* grad, cudaStream_t st);
+cudaError_t mlp_loss(const float* loss_part, int tiles, float* loss, cudaStream_t st);
+cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfloat16* X, float* W, cudaStream_t st);
 cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t st);
 cudaError_t mlp_mean_add(float* sum, const float* y, int64_t n, int j, int k, cudaStream_t st);
 cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16* wbf, cudaStream_t st);
 cudaError_t mlp_infer(const __nv_bfloat16* x, int n, const float* params, const __nv_bfloat16* wbf, float* y,
                       int* status, int grid, cudaStream_t st);
-cudaError_t mlp_gather_batch(const __nv_bfloat16* X, const float* Y, const float* W, const int* perm, int64_t first,
-                             int rows, __nv_bfloat16* xb, float* yb, float* wb, cudaStream_t st,
-                             const mlp::TrainSched* sched = nullptr);
 int mlp_n_params();
 int mlp_n_bf();
 struct LatticeArgs {
@@ -89,8 +78,7 @@ int sfail(int code, const std::string& m)
     } while (0)
 
 constexpr int H = 128, KIN = 16, NF = 7;
-constexpr int OFF_W1 = 0, OFF_B1 = H * KIN, OFF_W2 = OFF_B1 + H, LAYER = H * H + H, OFF_W5 = OFF_W2 + 3 * LAYER,
-              OFF_B5 = OFF_W5 + H;
+constexpr int OFF_W1 = 0, OFF_B1 = H * KIN, OFF_W2 = OFF_B1 + H, LAYER = H * H + H, OFF_W5 = OFF_W2 + 3 * LAYER;
 
 __nv_bfloat16 to_bf(float f)
 {
@@ -109,10 +97,11 @@ struct ThothSurrogate {
     int dev = 0; // the device current when the handle was created; every call sets it
     int sms = 0;
     int64_t step = 0;
-    // training buffers (grown on demand)
+    // training buffers (grown on demand): the tiles' partial gradients and losses
     int cap_rows = 0;
     unsigned char* tb = nullptr;
-    mlp::TrainArgs A{};
+    mlp::TileArgs A{};
+    float* grad = nullptr;
     float* loss = nullptr;
     // inference buffers
     int64_t cap_inf = 0;
@@ -120,8 +109,6 @@ struct ThothSurrogate {
     // lattice serving: parameter sets and lattice axes, scaled prices
     int64_t cap_lat = 0;
     unsigned char* lb = nullptr;
-    // the training schedule the captured step reads (learning rate, bias corrections, batch)
-    mlp::TrainSched* sched = nullptr;
     // the running average of the weights over a training call's last epochs
     float* avg = nullptr;
     // device copy of a training set and its per-epoch permutation (grown on demand)
@@ -135,10 +122,15 @@ namespace {
 
 void host_params_to_bf(const std::vector<float>& p, std::vector<__nv_bfloat16>& w)
 {
-    w.assign((size_t)H * KIN + 3 * (size_t)H * H, to_bf(0.f));
-    for (int j = 0; j < H * KIN; j++) w[j] = to_bf(p[OFF_W1 + j]);
-    for (int l = 0; l < 3; l++)
-        for (int j = 0; j < H * H; j++) w[(size_t)H * KIN + (size_t)l * H * H + j] = to_bf(p[OFF_W2 + l * LAYER + j]);
+    w.resize((size_t)H * KIN + 3 * (size_t)H * H);
+    __nv_bfloat16* to = w.data();
+    auto layer = [&](const float* from, int cols) { // the operand layout
+        for (int kb = 0; kb < cols; kb += 8)
+            for (int r = 0; r < H; r++)
+                for (int k = 0; k < 8; k++) *to++ = to_bf(from[(size_t)r * cols + kb + k]);
+    };
+    layer(p.data() + OFF_W1, KIN);
+    for (int l = 0; l < 3; l++) layer(p.data() + OFF_W2 + l * LAYER, H);
 }
 
 int upload_params(ThothSurrogate* s, const std::vector<float>& p)
@@ -164,68 +156,18 @@ int ensure_train(ThothSurrogate* s, int rows)
         off += (bytes + 255) & ~size_t(255);
         return o;
     };
-    const size_t ox = take((size_t)rows * KIN * 2), oy = take((size_t)rows * 4), ow = take((size_t)rows * 4);
-    size_t oz[5], oa[5], od[5];
-    for (int l = 1; l <= 4; l++) {
-        oz[l] = take((size_t)rows * H * 4);
-        oa[l] = take((size_t)rows * H * 2);
-        od[l] = take((size_t)rows * H * 2);
-    }
-    const size_t op = take((size_t)tiles * s->np * 4), ol = take((size_t)tiles * 4), oloss = take(4);
+    const size_t op = take((size_t)tiles * s->np * 4), ol = take((size_t)tiles * 4), og = take((size_t)s->np * 4),
+                 oloss = take(4);
     STRY(cudaMalloc(&s->tb, off));
     s->cap_rows = rows;
-    mlp::TrainArgs& A = s->A;
-    A.x = reinterpret_cast<const __nv_bfloat16*>(s->tb + ox);
-    A.y = reinterpret_cast<const float*>(s->tb + oy);
-    A.inv_w2 = reinterpret_cast<const float*>(s->tb + ow);
-    for (int l = 1; l <= 4; l++) {
-        A.z[l] = reinterpret_cast<float*>(s->tb + oz[l]);
-        A.a[l] = reinterpret_cast<__nv_bfloat16*>(s->tb + oa[l]);
-        A.dz[l] = reinterpret_cast<__nv_bfloat16*>(s->tb + od[l]);
-    }
-    A.z[0] = nullptr;
-    A.a[0] = nullptr;
-    A.dz[0] = nullptr;
+    mlp::TileArgs& A = s->A;
     A.part = reinterpret_cast<float*>(s->tb + op);
     A.loss_part = reinterpret_cast<float*>(s->tb + ol);
+    s->grad = reinterpret_cast<float*>(s->tb + og);
     s->loss = reinterpret_cast<float*>(s->tb + oloss);
     A.params = s->params;
     A.wbf = s->wbf;
     A.status = s->status;
-    return THOTH_GPU_OK;
-}
-
-// pack rows [i0, i0 + rows) of a (possibly permuted) host dataset into pinned-free host staging
-void pack(const float* x, const float* y, const float* scale, const int64_t* idx, int64_t i0, int rows,
-          std::vector<__nv_bfloat16>& hx, std::vector<float>& hy, std::vector<float>& hw)
-{
-    hx.assign((size_t)rows * KIN, to_bf(0.f));
-    hy.resize(rows);
-    hw.resize(rows);
-    for (int r = 0; r < rows; r++) {
-        const int64_t i = idx ? idx[i0 + r] : i0 + r;
-        for (int f = 0; f < NF; f++) {
-            // each feature enters as a bf16 pair hi + lo (columns f and f + 7, tied weights),
-            // keeping about 16 significant bits of the input
-            const float v = x[i * NF + f];
-            const __nv_bfloat16 hi = to_bf(v);
-            hx[(size_t)r * KIN + f] = hi;
-            hx[(size_t)r * KIN + NF + f] = to_bf(v - __bfloat162float(hi));
-        }
-        hy[r] = y[i];
-        const double sc = scale ? scale[i] : 1.0;
-        hw[r] = (float)(1.0 / (sc * sc));
-    }
-}
-
-int upload_batch(ThothSurrogate* s, const std::vector<__nv_bfloat16>& hx, const std::vector<float>& hy,
-                 const std::vector<float>& hw)
-{
-    mlp::TrainArgs& A = s->A;
-    STRY(cudaMemcpyAsync(const_cast<__nv_bfloat16*>(A.x), hx.data(), hx.size() * 2, cudaMemcpyHostToDevice, s->st));
-    STRY(cudaMemcpyAsync(const_cast<float*>(A.y), hy.data(), hy.size() * 4, cudaMemcpyHostToDevice, s->st));
-    STRY(cudaMemcpyAsync(const_cast<float*>(A.inv_w2), hw.data(), hw.size() * 4, cudaMemcpyHostToDevice, s->st));
-    A.a[0] = const_cast<__nv_bfloat16*>(A.x);
     return THOTH_GPU_OK;
 }
 
@@ -238,27 +180,62 @@ int check_status(ThothSurrogate* s)
     return THOTH_GPU_OK;
 }
 
+// the handle's device copy of a training set of n rows: inputs packed to bf16 pairs, targets, loss
+// weights, and a permutation; raw is where the caller's inputs and scales land before the packing
+struct SetBuffers {
+    __nv_bfloat16* x;
+    float *y, *w;
+    int* perm;
+    float *raw_x, *raw_scale;
+};
+
+int upload_set(ThothSurrogate* s, const float* x, const float* y, const float* scale, int64_t n, SetBuffers& D)
+{
+    if (n > s->cap_ds) {
+        if (s->ds) cudaFree(s->ds);
+        if (s->perm_host) cudaFreeHost(s->perm_host);
+        s->ds = nullptr;
+        s->perm_host = nullptr;
+        s->cap_ds = 0;
+        STRY(cudaMalloc(&s->ds, (size_t)n * (KIN * 2 + 4 + 4 + 4 + NF * 4 + 4) + 2048));
+        STRY(cudaHostAlloc(&s->perm_host, sizeof(int) * (size_t)n, cudaHostAllocDefault));
+        if (!s->perm_copied) STRY(cudaEventCreateWithFlags(&s->perm_copied, cudaEventDisableTiming));
+        s->cap_ds = n;
+    }
+    unsigned char* at = s->ds;
+    auto take = [&](size_t bytes) {
+        unsigned char* p = at;
+        at += (bytes + 255) & ~size_t(255);
+        return p;
+    };
+    D.x = reinterpret_cast<__nv_bfloat16*>(take((size_t)n * KIN * 2));
+    D.y = reinterpret_cast<float*>(take((size_t)n * 4));
+    D.w = reinterpret_cast<float*>(take((size_t)n * 4));
+    D.perm = reinterpret_cast<int*>(take((size_t)n * 4));
+    D.raw_x = reinterpret_cast<float*>(take((size_t)n * NF * 4));
+    D.raw_scale = scale ? reinterpret_cast<float*>(take((size_t)n * 4)) : nullptr;
+    STRY(cudaMemcpyAsync(D.raw_x, x, (size_t)n * NF * 4, cudaMemcpyHostToDevice, s->st));
+    STRY(cudaMemcpyAsync(D.y, y, (size_t)n * 4, cudaMemcpyHostToDevice, s->st));
+    if (scale) STRY(cudaMemcpyAsync(D.raw_scale, scale, (size_t)n * 4, cudaMemcpyHostToDevice, s->st));
+    STRY(mlp_pack_set(D.raw_x, D.raw_scale, n, D.x, D.w, s->st));
+    return THOTH_GPU_OK;
+}
 
 // one network's training call in three phases, so that several networks can train side by side
 struct TrainRun {
     ThothSurrogate* s = nullptr;
-    int64_t n = 0, steps_per_epoch = 0, total = 0;
-    int epochs = 0, avg_epochs = 0;
-    int* dP = nullptr;              // the device permutation of the current epoch
-    std::vector<int> idx;           // the host permutation
+    int64_t n = 0, steps_per_epoch = 0, total = 0, done = 0;
+    int epochs = 0, avg_epochs = 0, batch = 0;
+    // a cosine decay from lr to lr_lo over decay_steps steps, then lr_lo
+    double lr = 0, lr_lo = 0;
+    int64_t decay_steps = 1;
+    SetBuffers D{};
+    std::vector<int> idx; // the host permutation
     std::mt19937_64 rng;
-    cudaGraphExec_t exec = nullptr; // one captured step: gather, forward, backward, Adam, loss, schedule
-    TrainRun() = default;
-    TrainRun(const TrainRun&) = delete;
-    TrainRun& operator=(const TrainRun&) = delete;
-    ~TrainRun()
-    {
-        if (exec) cudaGraphExecDestroy(exec);
-    }
 };
 
 // the training set up once on the member's device memory (bf16 hi/lo inputs, targets, loss
-// weights), the schedule of this call, and the captured step
+// weights) and the schedule of this call
 int train_setup(TrainRun& R, ThothSurrogate* s, const float* x, const float* y, const float* scale, int64_t n,
                 int epochs, int batch, double lr, uint64_t seed, int avg_epochs, double lr_avg)
 {
@@ -266,77 +243,30 @@ int train_setup(TrainRun& R, ThothSurrogate* s, const float* x, const float* y, 
     R.n = n;
     R.epochs = epochs;
     R.avg_epochs = avg_epochs;
-    const int B = (int)std::min<int64_t>(batch, n / 128 * 128);
-    int rc = ensure_train(s, B);
+    R.batch = (int)std::min<int64_t>(batch, n / 128 * 128);
+    int rc = ensure_train(s, R.batch);
     if (rc) return rc;
     if (avg_epochs > 0 && !s->avg) STRY(cudaMalloc(&s->avg, sizeof(float) * s->np));
-    // each epoch uploads one permutation and every step gathers its rows on the device
-    if (n > s->cap_ds) {
-        if (s->ds) cudaFree(s->ds);
-        if (s->perm_host) cudaFreeHost(s->perm_host);
-        s->ds = nullptr;
-        s->perm_host = nullptr;
-        s->cap_ds = 0;
-        STRY(cudaMalloc(&s->ds, (size_t)n * (KIN * 2 + 4 + 4 + 4) + 1024));
-        STRY(cudaHostAlloc(&s->perm_host, sizeof(int) * (size_t)n, cudaHostAllocDefault));
-        if (!s->perm_copied) STRY(cudaEventCreateWithFlags(&s->perm_copied, cudaEventDisableTiming));
-        s->cap_ds = n;
-    }
-    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-    __nv_bfloat16* dX = reinterpret_cast<__nv_bfloat16*>(s->ds);
-    float* dY = reinterpret_cast<float*>(s->ds + up((size_t)n * KIN * 2));
-    float* dW = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(dY) + up((size_t)n * 4));
-    R.dP = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(dW) + up((size_t)n * 4));
-    {
-        std::vector<__nv_bfloat16> hx;
-        std::vector<float> hy, hw;
-        pack(x, y, scale, nullptr, 0, (int)n, hx, hy, hw);
-        STRY(cudaMemcpy(dX, hx.data(), hx.size() * 2, cudaMemcpyHostToDevice));
-        STRY(cudaMemcpy(dY, hy.data(), hy.size() * 4, cudaMemcpyHostToDevice));
-        STRY(cudaMemcpy(dW, hw.data(), hw.size() * 4, cudaMemcpyHostToDevice));
-    }
+    rc = upload_set(s, x, y, scale, n, R.D);
+    if (rc) return rc;
     R.idx.resize(n);
     for (int64_t i = 0; i < n; i++) R.idx[i] = (int)i;
     R.rng.seed(seed);
-    R.steps_per_epoch = n / B;
+    R.steps_per_epoch = n / R.batch;
     R.total = R.steps_per_epoch * epochs;
-    mlp::TrainArgs& A = s->A;
-    A.a[0] = const_cast<__nv_bfloat16*>(A.x);
-    A.rows = B;
-    // the schedule of this call on the device: the captured step reads its batch offset,
-    // learning rate and bias corrections there and advances it
-    if (!s->sched) STRY(cudaMalloc(&s->sched, sizeof(mlp::TrainSched)));
-    mlp::TrainSched sc{};
-    sc.count = 0;
-    sc.total = R.total;
-    sc.steps_per_epoch = R.steps_per_epoch;
-    sc.step0 = s->step;
-    sc.lr0 = lr;
-    sc.rows = B;
     // without averaging the decay runs over every step down to zero; with it, over the steps
     // before the averaged epochs, down to lr_avg, which then holds
-    sc.decay_steps = avg_epochs > 0 ? R.steps_per_epoch * (int64_t)(epochs - avg_epochs) : R.total;
-    sc.lr_lo = avg_epochs > 0 ? lr_avg : 0.0;
-    if (sc.decay_steps < 1) sc.decay_steps = 1;
-    mlp_sched_init(sc);
-    STRY(cudaMemcpyAsync(s->sched, &sc, sizeof sc, cudaMemcpyHostToDevice, s->st));
+    R.lr = lr;
+    R.lr_lo = avg_epochs > 0 ? lr_avg : 0.0;
+    R.decay_steps = std::max<int64_t>(1, avg_epochs > 0 ? R.steps_per_epoch * (int64_t)(epochs - avg_epochs) : R.total);
+    mlp::TileArgs& A = s->A;
+    A.x = R.D.x;
+    A.y = R.D.y;
+    A.w = R.D.w;
+    A.perm = R.D.perm;
+    A.rows = R.batch;
     STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
     STRY(mlp_train_prepare());
-    // one step (gather, forward, backward, Adam, loss, schedule) captured once, replayed
-    // for every step: its launches' arguments do not change from step to step
-    cudaGraph_t graph = nullptr;
-    STRY(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-    cudaError_t ce = mlp_gather_batch(dX, dY, dW, R.dP, 0, B, const_cast<__nv_bfloat16*>(A.x),
-                                      const_cast<float*>(A.y), const_cast<float*>(A.inv_w2), s->st, s->sched);
-    if (ce == cudaSuccess)
-        ce = mlp_train_step(A, s->params, s->m, s->v, s->wbf, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f, s->loss, s->st,
-                            s->sched);
-    if (ce == cudaSuccess) ce = mlp_sched_advance(s->sched, s->st);
-    const cudaError_t ee = cudaStreamEndCapture(s->st, &graph);
-    if (ce == cudaSuccess) ce = ee;
-    if (ce == cudaSuccess) ce = cudaGraphInstantiate(&R.exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (ce != cudaSuccess) return sfail(THOTH_GPU_E_CUDA, std::string("training step graph: ") + cudaGetErrorString(ce));
     STRY(cudaEventRecord(s->perm_copied, s->st));
     return THOTH_GPU_OK;
 }
@@ -346,12 +276,21 @@ int train_setup(TrainRun& R, ThothSurrogate* s, const float* x, const float* y, 
 int train_epoch(TrainRun& R, int e)
 {
     ThothSurrogate* s = R.s;
+    const double pi = 3.14159265358979323846;
     std::shuffle(R.idx.begin(), R.idx.end(), R.rng);
     STRY(cudaEventSynchronize(s->perm_copied)); // the previous permutation has left the pinned buffer
     std::memcpy(s->perm_host, R.idx.data(), sizeof(int) * (size_t)R.n);
-    STRY(cudaMemcpyAsync(R.dP, s->perm_host, sizeof(int) * (size_t)R.n, cudaMemcpyHostToDevice, s->st));
+    STRY(cudaMemcpyAsync(R.D.perm, s->perm_host, sizeof(int) * (size_t)R.n, cudaMemcpyHostToDevice, s->st));
     STRY(cudaEventRecord(s->perm_copied, s->st));
-    for (int64_t b = 0; b < R.steps_per_epoch; b++) STRY(cudaGraphLaunch(R.exec, s->st));
+    const int tiles = R.batch / 128;
+    for (int64_t b = 0; b < R.steps_per_epoch; b++, R.done++) {
+        const double c = (double)std::min(R.done, R.decay_steps), step = (double)(s->step + R.done + 1);
+        const float lr = (float)(R.lr_lo + (R.lr - R.lr_lo) * 0.5 * (1.0 + std::cos(pi * c / (double)R.decay_steps)) + 1e-6);
+        s->A.first = b * R.batch;
+        STRY(mlp_train_tiles(s->A, s->st));
+        STRY(mlp_adam(s->params, s->m, s->v, s->A.part, tiles, s->wbf, lr, 0.9f, 0.999f, 1e-8f,
+                      (float)(1.0 - std::pow(0.9, step)), (float)(1.0 - std::pow(0.999, step)), s->st));
+    }
     if (R.avg_epochs > 0 && e >= R.epochs - R.avg_epochs)
         STRY(mlp_weight_avg(s->params, s->avg, e - (R.epochs - R.avg_epochs), s->st));
     return THOTH_GPU_OK;
@@ -363,6 +302,7 @@ int train_finish(TrainRun& R, double* final_loss)
     if (R.avg_epochs > 0) STRY(mlp_weight_avg_finish(s->params, s->avg, s->wbf, s->st));
     s->step += R.total;
     float l = 0;
+    STRY(mlp_loss(s->A.loss_part, R.batch / 128, s->loss, s->st)); // the last step's
     STRY(cudaMemcpyAsync(&l, s->loss, sizeof(float), cudaMemcpyDeviceToHost, s->st));
     STRY(cudaStreamSynchronize(s->st));
     const int rc = check_status(s);
@@ -448,7 +388,6 @@ int thoth_gpu_surrogate_destroy(ThothSurrogate* s)
         if (s->tb) cudaFree(s->tb);
         if (s->ib) cudaFree(s->ib);
         if (s->lb) cudaFree(s->lb);
-        if (s->sched) cudaFree(s->sched);
         if (s->avg) cudaFree(s->avg);
         if (s->ds) cudaFree(s->ds);
         if (s->perm_host) cudaFreeHost(s->perm_host);
@@ -505,31 +444,27 @@ int thoth_gpu_surrogate_gradient(ThothSurrogate* s, const float* x, const float*
         STRY(cudaSetDevice(s->dev));
         int rc = ensure_train(s, rows);
         if (rc) return rc;
-        std::vector<__nv_bfloat16> hx;
-        std::vector<float> hy, hw;
-        pack(x, y, scale, nullptr, 0, rows, hx, hy, hw);
-        rc = upload_batch(s, hx, hy, hw);
+        SetBuffers D{};
+        rc = upload_set(s, x, y, scale, rows, D);
         if (rc) return rc;
-        s->A.rows = rows;
-        // a step with lr = 0 leaves the parameters unchanged but fills the partial gradients
-        std::vector<float> keep_m(2 * (size_t)s->np);
-        STRY(cudaMemcpyAsync(keep_m.data(), s->m, sizeof(float) * 2 * s->np, cudaMemcpyDeviceToHost, s->st));
-        STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
-        STRY(mlp_train_step(s->A, s->params, s->m, s->v, s->wbf, 0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f, s->loss, s->st));
-        rc = check_status(s);
-        if (rc) return rc;
+        mlp::TileArgs A = s->A;
+        A.x = D.x;
+        A.y = D.y;
+        A.w = D.w;
+        A.perm = nullptr;
+        A.first = 0;
+        A.rows = rows;
         const int tiles = rows / 128;
-        std::vector<float> part((size_t)tiles * s->np);
-        STRY(cudaMemcpyAsync(part.data(), s->A.part, sizeof(float) * part.size(), cudaMemcpyDeviceToHost, s->st));
+        STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
+        STRY(mlp_train_prepare());
+        STRY(mlp_train_tiles(A, s->st));
+        STRY(mlp_gradient(A.part, tiles, s->grad, s->st));
+        STRY(mlp_loss(A.loss_part, tiles, s->loss, s->st));
         float l = 0;
         STRY(cudaMemcpyAsync(&l, s->loss, sizeof(float), cudaMemcpyDeviceToHost, s->st));
-        STRY(cudaMemcpyAsync(s->m, keep_m.data(), sizeof(float) * 2 * s->np, cudaMemcpyHostToDevice, s->st));
-        STRY(cudaStreamSynchronize(s->st));
-        for (int j = 0; j < s->np; j++) {
-            double g = 0;
-            for (int t = 0; t < tiles; t++) g += part[(size_t)t * s->np + j];
-            grad[j] = (float)g;
-        }
+        STRY(cudaMemcpyAsync(grad, s->grad, sizeof(float) * s->np, cudaMemcpyDeviceToHost, s->st));
+        rc = check_status(s);
+        if (rc) return rc;
         if (loss) *loss = l / rows;
         return THOTH_GPU_OK;
     } catch (const std::bad_alloc&) {

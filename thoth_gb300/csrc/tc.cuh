@@ -41,12 +41,20 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
     return d;
 }
 
-// instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N)
+// The same tile read as the transposed operand (MN-major, no swizzle): a core matrix holds 8
+// elements along M or N (its contiguous 16 bytes) by 8 along K (its rows). So for a tile of
+// cm_offset layout the stride between 8-element groups along M or N is the K-major LBO (R * 16
+// bytes) and goes into the SBO field, and the stride between 8-row groups along K is 128 bytes
+// and goes into the LBO field. One K = 16 slice starts every 256 bytes.
+__device__ __forceinline__ uint64_t make_desc_mn(uint32_t saddr, uint32_t R) { return make_desc(saddr, 128, R * 16); }
+
+// instruction descriptor, kind::f16: D = F32, A = B = BF16; a_mn / b_mn: that operand is MN-major
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool a_mn = false, bool b_mn = false)
 {
     return (1u << 4)                      // D format: F32
            | (1u << 7)                    // A format: BF16
            | (1u << 10)                   // B format: BF16
+           | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16)
            | ((uint32_t)(N >> 3) << 17)   // N / 8
            | ((uint32_t)(M >> 4) << 24);  // M / 16
 }
@@ -101,11 +109,48 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
     return false;
 }
 
+// programmatic dependent launch: the next kernel of the stream may be scheduled; everything of the
+// previous one is done and visible. Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;"); }
 
 // generic-proxy smem writes -> visible to the tensor core's async proxy
 __device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// one-dimensional bulk copy global -> shared (16-byte aligned, a multiple of 16 bytes), completing
+// on the mbarrier, and the barrier's expected byte count with its one arrival
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* mbar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(uint64_t* mbar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
+}
+
+// barrier initialisation visible to the async proxy
+__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+// 16 consecutive FP32 columns of this thread's TMEM lane, written
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16])
+{
+    uint32_t r[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(v[i]);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+                   "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 16 consecutive FP32 columns of this thread's TMEM lane (32x32b shape)
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
