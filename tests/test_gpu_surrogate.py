@@ -221,3 +221,29 @@ def test_training_step_is_adam_on_the_gradient(gpu, n, batch):
     np.testing.assert_allclose(d[big], -lr * np.sign(g[big]), rtol=2e-3)
     k.close()
     m.close()
+
+
+@pytest.mark.parametrize("sets,n_lm,n_T,members", [
+    (1, 1, 1, 1),        # one cell
+    (127, 1, 1, 2),      # one short of a tile
+    (43, 3, 1, 1),       # one more than a tile
+    (5, 21, 12, 3),      # tiles that end inside a set
+    (153, 128, 3, 1),    # more tiles than fit the device's slots at once
+])
+def test_lattice_cells_equal_the_same_rows(gpu, sets, n_lm, n_T, members):
+    """A lattice cell is the network on the clipped, normalised features (the same BF16 words as
+    the rows' path) times the price scale; both round the product to FP32 once, from FP64 scales
+    equal to a few ulp: within one FP32 ulp. Some parameters lie outside the training box."""
+    rng = np.random.default_rng(sets)
+    P = S.BOX_LO[2:] + rng.uniform(-0.1, 1.1, (sets, 5)) * (S.BOX_HI[2:] - S.BOX_LO[2:])
+    lms, Ts = np.linspace(-0.6, 0.55, n_lm), np.linspace(0.05, 3.1, n_T)
+    E = S.Ensemble(members, seed=9)
+    got, _ = E.price_lattice(P, lms, Ts) if members > 1 else E.members[0].price_lattice(P, lms, Ts)
+    X = np.clip(S.grid_features(P, lms, Ts), S.BOX_LO, S.BOX_HI)
+    y = E.members[0].predict(S.normalise(X))[0]
+    for m in E.members[1:]:
+        y = y + m.predict(S.normalise(X))[0]
+    if members > 1:
+        y = y * np.float32(1.0 / members)
+    np.testing.assert_allclose(got, y.astype(np.float64) * S.price_scale(X), rtol=1.3e-7, atol=0)
+    E.close()

@@ -7,6 +7,9 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+
 namespace thoth {
 
 // ---------------------------------------------------------------------------
@@ -174,17 +177,20 @@ constexpr uint32_t TILE_BUF = H * H * 2; // one 128 x 128 bf16 operand
 constexpr size_t TILE_SMEM = 7 * (size_t)TILE_BUF;
 
 // issue D = A B^T over K (one thread); a tile of 128 rows is read as it lies (K along its
-// columns) or transposed (mn: K along its rows)
+// columns) or transposed (mn: K along its rows). The descriptors of a K slice differ from the
+// first's in the start address alone (16-byte units): formed per slice, in a loop, the issuing
+// thread held the products up (inference of 2^20 cells 198 us, 185 like this)
+template <int K>
 __device__ __forceinline__ void issue(uint32_t d, const unsigned char* A, bool a_mn, const unsigned char* B, bool b_mn,
-                                      int N, int K)
+                                      int N)
 {
     const uint32_t idesc = tc::make_idesc_bf16(128, N, a_mn, b_mn);
     const uint32_t a0 = tc::smem_u32(A), b0 = tc::smem_u32(B);
-    for (uint32_t kk = 0; kk < (uint32_t)K / 16; ++kk) {
-        const uint64_t ad = a_mn ? tc::make_desc_mn(a0 + kk * 256, 128) : tc::make_desc(a0 + kk * 4096, 2048, 128);
-        const uint64_t bd = b_mn ? tc::make_desc_mn(b0 + kk * 256, 128) : tc::make_desc(b0 + kk * 4096, 2048, 128);
-        tc::mma_bf16(d, ad, bd, idesc, kk > 0 ? 1u : 0u);
-    }
+    const uint64_t ad = a_mn ? tc::make_desc_mn(a0, 128) : tc::make_desc(a0, 2048, 128);
+    const uint64_t bd = b_mn ? tc::make_desc_mn(b0, 128) : tc::make_desc(b0, 2048, 128);
+#pragma unroll
+    for (uint32_t kk = 0; kk < K / 16; ++kk)
+        tc::mma_bf16(d, ad + kk * (a_mn ? 16u : 256u), bd + kk * (b_mn ? 16u : 256u), idesc, kk > 0 ? 1u : 0u);
 }
 
 // SiLU and its derivative from one reciprocal: z sigmoid(z) equals __fdividef(z, 1 + e^-z) bit for
@@ -316,7 +322,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileA
 #pragma unroll
         for (int l = 1; l <= 4; ++l) {
             if (t == 0) {
-                issue(tm + (uint32_t)(128 * (l - 1)), in[l - 1], false, wl[l - 1], false, H, l == 1 ? KIN : H);
+                const uint32_t d = tm + (uint32_t)(128 * (l - 1));
+                if (l == 1) issue<KIN>(d, X, false, W1, false, H);
+                else issue<H>(d, in[l - 1], false, wl[l - 1], false, H);
                 tc::mma_commit(&mb_a);
             }
             const float* b = A.params + b_off(l) + c0;
@@ -395,7 +403,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileA
         bar_arrive(BAR_DZ, TILE_THREADS);
         operands_ready();
         if (t == 0) { // da3 = dz4 W4
-            issue(tm + 384, D4, false, W4, true, H, H);
+            issue<H>(tm + 384, D4, false, W4, true, H);
             tc::mma_commit(&mb_a);
         }
         // the head's weight gradients: every column's sum over the warp's 32 rows by the butterfly
@@ -444,9 +452,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileA
         input_grad(3, W4);
         operands_ready();
         if (t == 0) {
-            issue(tm + 384, W4, false, W3, true, H, H); // da2 = dz3 W3
+            issue<H>(tm + 384, W4, false, W3, true, H); // da2 = dz3 W3
             tc::mma_commit(&mb_a);
-            issue(tm + 256, D4, true, A3, true, H, H);  // dW4 = dz4^T a3
+            issue<H>(tm + 256, D4, true, A3, true, H);  // dW4 = dz4^T a3
             tc::mma_commit(&mb_b);
             gp[OFF_B5] = red2[0][0] + red2[1][0] + red2[2][0] + red2[3][0];
             A.loss_part[blockIdx.x] = red2[0][1] + red2[1][1] + red2[2][1] + red2[3][1];
@@ -461,9 +469,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileA
         }
         operands_ready();
         if (t == 0) {
-            issue(tm + 384, W3, false, W2, true, H, H); // da1 = dz2 W2
+            issue<H>(tm + 384, W3, false, W2, true, H); // da1 = dz2 W2
             tc::mma_commit(&mb_a);
-            issue(tm + 128, W4, true, A2, true, H, H);  // dW3 = dz3^T a2
+            issue<H>(tm + 128, W4, true, A2, true, H);  // dW3 = dz3^T a2
             tc::mma_commit(&mb_b);
         }
         weight_grad(4, 256);
@@ -474,8 +482,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) train_tile_kernel(const TileA
         wait_b();
         operands_ready();
         if (t == 0) {
-            issue(tm + 384, D4, true, A3, true, KIN, H); // dW1 = dz1^T x
-            issue(tm + 256, W3, true, A1, true, H, H);   // dW2 = dz2^T a1
+            issue<H>(tm + 384, D4, true, A3, true, KIN); // dW1 = dz1^T x
+            issue<H>(tm + 256, W3, true, A1, true, H);   // dW2 = dz2^T a1
             tc::mma_commit(&mb_a);
         }
         weight_grad(3, 128);
@@ -671,20 +679,6 @@ __global__ void sum_kernel(const float* x, int n, float* out)
     if (threadIdx.x == 0) *out = s[0];
 }
 
-// fused inference: persistent CTAs of three warpgroups, one CTA per SM. The weights
-// are resident in shared memory and shared by all; each warpgroup walks its own
-// 128-cell tiles with its own TMEM accumulator (128 columns each), mbarrier and
-// named barrier, so the warpgroups' bias + SiLU epilogues overlap one another's
-// MMAs. The epilogue streams 16 accumulator columns at a time straight into the
-// next layer's A operand (K-major core-matrix layout); the last layer folds the head.
-// Three warpgroups: 208 KB of shared memory (the weights and three tiles of
-// activations) and 384 of the 512 TMEM columns.
-constexpr int INFER_WG = 3;
-constexpr int INFER_THREADS = 128 * INFER_WG;
-constexpr uint32_t INFER_TMEM_COLS = 512; // a power of two >= 128 x INFER_WG
-
-__device__ __forceinline__ void wg_sync(int wg) { asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory"); }
-
 // SiLU of two columns at once for inference: silu(z) = z sigmoid(z), sigmoid(z) = (1 + tanh(z/2)) / 2,
 // with one special-function-unit tanh per value (the exponential and reciprocal form takes two)
 // and the arithmetic on packed pairs. tanh.approx is within about 2^-11 of tanh, well inside the
@@ -698,112 +692,260 @@ __device__ __forceinline__ float2 silu2_infer(float2 z)
     return __ffma2_rn(h, make_float2(t0, t1), h); // z/2 (1 + tanh(z/2))
 }
 
-__global__ void __launch_bounds__(INFER_THREADS) infer_kernel(const __nv_bfloat16* __restrict__ x, int n,
-                                                              const float* params, const __nv_bfloat16* wbf,
-                                                              float* __restrict__ y, int* status)
+// ---------------------------------------------------------------------------
+// Fused inference: one persistent CTA per SM, three tiles of 128 cells in flight, each with its
+// own 256 threads, TMEM accumulator (128 columns), mbarrier and named barrier; the weights are
+// resident in shared memory and shared by all. Two warps share a tile's 32 rows, one half of the
+// columns each: an epilogue (bias, SiLU, the next operand) is bound by the latency of its column
+// blocks rather than by the special-function unit (16 tanh a clock: 1024 clocks for a tile's
+// layer), so it has two warps a scheduler and tile, and each block's accumulator is requested
+// while the one before it is worked on. With one warp and no request ahead an epilogue took 3800
+// clocks beside two others, and 2^20 cells 0.22 ms; like this 0.185. (What holds it above the
+// special-function bound of 0.11 ms is the queue that those operations share with shared memory,
+// which the products' operand reads fill.)
+//
+// Cells come as rows of normalised features, or as a lattice: its features are one word (the bf16
+// pair hi, lo) a log-moneyness, maturity and parameter, from tables that a small kernel fills, so
+// a tile's rows are put together from seven words and no feature is stored. Building them per
+// cell, in FP64 with seven divisions, took 0.23 ms for 2^20 cells.
+//
+// An ensemble's members run one after the other in the same launch, their outputs added in member
+// order. The price scale of a lattice cell is FP64 work (two normal distribution functions), and
+// FP64 issues at 1/64 of the FP32 rate; four more warps do it beside the networks, whose pipes it
+// does not use, and the outputs are scaled at the end. As a kernel of its own, with the library's
+// normcdf, it took 0.48 ms.
+// ---------------------------------------------------------------------------
+constexpr int INFER_TILES = 3;                 // tiles in flight
+constexpr int INFER_GROUP = 256;               // threads a tile
+constexpr int INFER_MAIN = INFER_TILES * INFER_GROUP;
+constexpr int INFER_LATTICE_THREADS = INFER_MAIN + ROWS; // and the scale's
+constexpr uint32_t INFER_TMEM_COLS = 512;      // a power of two >= 128 x INFER_TILES
+constexpr int MAX_MEMBERS = 64;
+
+// Phi(x) by its Taylor polynomials about x0 = k / 8: Phi(x0) + phi(x0) sum_n (-1)^(n-1)
+// He_(n-1)(x0) h^n / n!, |h| <= 1/16, He the Hermite polynomials. Ten coefficients leave less than
+// 2.3e-16 anywhere; beyond +-69/8 Phi is 0 or 1 to 1e-17.
+constexpr int PHI_NODES = 139, PHI_COEF = 10, PHI_MID = 69;
+
+struct LatticeTables {
+    const uint32_t* f_lm;  // [n_lm] feature words (bf16 hi, lo << 16), clipped and normalised
+    const uint32_t* f_T;   // [n_T]
+    const uint32_t* f_set; // [n_sets][5]
+    const double2* set_T;  // [n_sets][n_T] 1 / sd, sd / 2 of the price scale
+    const double2* lm;     // [n_lm] clipped log-moneyness, its exponential
+    const double* phi;     // [PHI_NODES][PHI_COEF]
+    double floor2;         // squared scale floor
+    uint32_t n_lm, n_T;
+};
+
+struct InferArgs {
+    const float* x;   // [n][7] normalised rows (not a lattice)
+    LatticeTables L;  // a lattice
+    int n;            // cells
+    int members;
+    float* y;         // [n] outputs, the members' mean
+    double* scale;    // [n] a lattice's price scale
+    float* price;     // [n] a lattice's prices
+    int* status;
+    const float* params[MAX_MEMBERS];
+    const __nv_bfloat16* wbf[MAX_MEMBERS];
+};
+
+__device__ __forceinline__ uint32_t feature_word(float v)
+{
+    const __nv_bfloat16 h = __float2bfloat16(v), l = __float2bfloat16(v - __bfloat162float(h));
+    return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
+}
+
+__device__ __forceinline__ double phi_table(const double* tab, double x)
+{
+    const double u = fmin(fmax(x, -8.625), 8.625);
+    const int k = __double2int_rn(u * 8.0);
+    const double h = fma((double)k, -0.125, u); // exact
+    const double2* c = reinterpret_cast<const double2*>(tab + (k + PHI_MID) * PHI_COEF);
+    double p = c[4].y;
+#pragma unroll
+    for (int i = 4; i >= 0; --i) {
+        p = i == 4 ? fma(p, h, c[4].x) : fma(fma(p, h, c[i].y), h, c[i].x);
+    }
+    return x == x ? p : x;
+}
+
+template <bool LATTICE>
+__global__ void __launch_bounds__(LATTICE ? INFER_LATTICE_THREADS : INFER_MAIN, 1) infer_kernel(const InferArgs A)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ uint64_t mbar[INFER_WG], mb_w;
+    __shared__ uint64_t mbar[INFER_TILES], mb_w;
     __shared__ uint32_t tm_s;
-    __shared__ __align__(16) float sb[4 * H + H + 1]; // biases of layers 1..4, head weights, head bias (pairs read as float2)
-    unsigned char* sW1 = sm;                         // 128 x 16
-    unsigned char* sW = sW1 + H * KIN * 2;           // 3 x (128 x 128)
-    const int t = threadIdx.x, warp = t >> 5, wg = t >> 7, r = t & 127;
-    unsigned char* sX = sW + 3 * H * H * 2 + wg * (ROWS * KIN * 2 + ROWS * H * 2); // this warpgroup's 128 x 16
-    unsigned char* sAct = sX + ROWS * KIN * 2;                                    // and 128 x 128
+    __shared__ __align__(16) float sb[4 * H + H + 4]; // biases of layers 1..4, head weights, head bias
+    unsigned char* sW1 = sm;               // 128 x 16
+    unsigned char* sW = sW1 + H * KIN * 2; // 3 x (128 x 128)
+    unsigned char* tiles_sm = sW + 3 * H * H * 2;
+    double* s_phi = reinterpret_cast<double*>(tiles_sm + INFER_TILES * (ROWS * KIN * 2 + ROWS * H * 2));
+    const int t = threadIdx.x, warp = t >> 5, g = t / INFER_GROUP; // g: the tile slot, or 3 for the scale's warps
+    const int half = (t >> 7) & 1, r = t & 127;
     if (warp == 0) tc::tmem_alloc(&tm_s, INFER_TMEM_COLS);
     if (t == 0) {
-        for (int w = 0; w < INFER_WG; ++w) tc::mbar_init(&mbar[w], 1);
+        for (int w = 0; w < INFER_TILES; ++w) tc::mbar_init(&mbar[w], 1);
         tc::mbar_init(&mb_w, 1);
         tc::fence_mbar_init();
         tc::fence_smem_async();
-        tc::mbar_expect(&mb_w, N_BF * 2);
-        for (int i = 0; i < N_BF * 2; i += 4096) // W1 and W2..W4 follow on in both memories
-            tc::bulk_load(sm + i, reinterpret_cast<const unsigned char*>(wbf) + i, 4096, &mb_w);
     }
-    for (int i = t; i < 4 * H; i += INFER_THREADS) sb[i] = params[b_off(1 + i / H) + i % H];
-    for (int i = t; i < H; i += INFER_THREADS) sb[4 * H + i] = params[OFF_W5 + i];
-    if (t == 0) sb[5 * H] = params[OFF_B5];
+    if (LATTICE)
+        for (int i = t; i < PHI_NODES * PHI_COEF; i += INFER_LATTICE_THREADS) s_phi[i] = A.L.phi[i];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    Ctx c{&mbar[wg], tm_s + (uint32_t)(wg * 128), 0, status};
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16; // TMEM lanes of this warp
-    if (t == 0 && !tc::mbar_wait(&mb_w, 0)) atomicExch(status, 1);
-    __syncthreads(); // one thread waits for the weights: 2 % faster than every thread polling
-    const int tiles = (n + ROWS - 1) / ROWS;
-    for (int tile = INFER_WG * blockIdx.x + wg; tile < tiles; tile += INFER_WG * gridDim.x) {
-        const int r0 = tile * ROWS;
-        const int valid = min(ROWS, n - r0);
-        // this warpgroup stages its input tile (row r by thread r: two 16-byte chunks)
-        for (int kb = 0; kb < KIN / 8; ++kb) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (r < valid) v = *reinterpret_cast<const uint4*>(x + (size_t)(r0 + r) * KIN + kb * 8);
-            *reinterpret_cast<uint4*>(sX + tc::cm_offset(r, kb * 8, ROWS)) = v;
-        }
-        float o = sb[5 * H];
-        for (int l = 1; l <= 4; ++l) {
-            const unsigned char* A = (l == 1) ? sX : sAct;
-            const unsigned char* W = (l == 1) ? sW1 : sW + (l - 2) * H * H * 2;
-            const int K = (l == 1) ? KIN : H;
-            // operand writes of every thread of the warpgroup -> visible to the tensor core
-            tc::fence_smem_async();
-            tc::fence_before_sync();
-            wg_sync(wg);
-            tc::fence_after_sync();
-            if (r == 0) {
-                const uint32_t idesc = tc::make_idesc_bf16(ROWS, H);
-                const uint32_t a0 = tc::smem_u32(A), b0 = tc::smem_u32(W);
-                for (int kk = 0; kk < K / 16; ++kk) {
-                    const uint64_t ad = tc::make_desc(a0 + (uint32_t)(2 * kk) * (ROWS * 16), ROWS * 16, 128);
-                    const uint64_t bd = tc::make_desc(b0 + (uint32_t)(2 * kk) * (H * 16), H * 16, 128);
-                    tc::mma_bf16(c.tm, ad, bd, idesc, kk > 0 ? 1u : 0u);
-                }
-                tc::mma_commit(c.mbar);
+    const int tiles = (A.n + ROWS - 1) / ROWS;
+    const int stride = INFER_TILES * gridDim.x;
+    const uint32_t per = LATTICE ? A.L.n_lm * A.L.n_T : 1;
+
+    if (LATTICE && g == INFER_TILES) {
+        // the price scale of every cell of this CTA's tiles
+        for (int tile0 = INFER_TILES * blockIdx.x; tile0 < tiles; tile0 += stride)
+            for (int tile = tile0; tile < min(tile0 + INFER_TILES, tiles); ++tile) {
+                const uint32_t c = (uint32_t)tile * ROWS + (uint32_t)r;
+                if (c >= (uint32_t)A.n) break;
+                const uint32_t set = c / per, q = c % per, j = q / A.L.n_lm, k = q % A.L.n_lm;
+                const double2 v = A.L.set_T[(size_t)set * A.L.n_T + j], m = A.L.lm[k];
+                const double d1 = fma(-m.x, v.x, v.y);
+                const double bs = fma(-m.y, phi_table(s_phi, fma(-2.0, v.y, d1)), phi_table(s_phi, d1));
+                A.scale[c] = sqrt(fma(bs, bs, A.L.floor2));
             }
-            const bool ok = tc::mbar_wait(c.mbar, c.phase);
-            c.phase ^= 1u;
-            if (!ok && (t & 31) == 0) atomicExch(c.status, 1);
-            tc::fence_after_sync();
-            const float* bias = sb + (l - 1) * H;
-            for (int c0 = 0; c0 < H; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(c.tm + lane_base + (uint32_t)c0, v);
-                if (!ok) {
+    } else {
+        unsigned char* sX = tiles_sm + g * (ROWS * KIN * 2 + ROWS * H * 2); // this tile's 128 x 16
+        unsigned char* sAct = sX + ROWS * KIN * 2;                          // and 128 x 128
+        const uint32_t acc = tm_s + (uint32_t)(g * 128);
+        const uint32_t at = acc + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * 64); // this thread's columns
+        uint32_t phase = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int m = 0; m < A.members; ++m) {
+            // the member's weights, once every tile of the one before is done
+            if (m > 0) asm volatile("bar.sync 8, %0;" ::"n"(INFER_MAIN) : "memory");
+            if (t == 0) {
+                tc::fence_smem_async();
+                tc::mbar_expect(&mb_w, N_BF * 2);
+                for (int i = 0; i < N_BF * 2; i += 4096) // W1 and W2..W4 follow on in both memories
+                    tc::bulk_load(sm + i, reinterpret_cast<const unsigned char*>(A.wbf[m]) + i, 4096, &mb_w);
+            }
+            const float* params = A.params[m];
+            for (int i = t; i < 4 * H; i += INFER_MAIN) sb[i] = params[b_off(1 + i / H) + i % H];
+            for (int i = t; i <= H; i += INFER_MAIN) sb[4 * H + i] = params[OFF_W5 + i]; // and the head bias
+            if (t == 0) ok = tc::mbar_wait(&mb_w, (uint32_t)(m & 1)) && ok;
+            asm volatile("bar.sync 8, %0;" ::"n"(INFER_MAIN) : "memory");
+#pragma unroll 1
+            for (int tile = INFER_TILES * blockIdx.x + g; tile < tiles; tile += stride) {
+                const int64_t c = (int64_t)tile * ROWS + r;
+                // row r of the input tile: hi parts in columns 0..6, lo parts in 7..13; each half of
+                // the group stores one 16-byte chunk
+                uint32_t f[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
+                if (c < A.n) {
+                    if (LATTICE) {
+                        const uint32_t set = (uint32_t)c / per, q = (uint32_t)c % per;
+                        f[0] = __ldg(A.L.f_lm + q % A.L.n_lm);
+                        f[1] = __ldg(A.L.f_T + q / A.L.n_lm);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = 0.f;
-                }
+                        for (int i = 0; i < 5; ++i) f[2 + i] = __ldg(A.L.f_set + (size_t)set * 5 + i);
+                    } else {
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    const float2 z = __fadd2_rn(make_float2(v[j], v[j + 1]),
-                                                *reinterpret_cast<const float2*>(bias + c0 + j));
-                    const float2 a = silu2_infer(z);
-                    v[j] = a.x;
-                    v[j + 1] = a.y;
-                }
-                if (l < 4) {
-                    // the MMA that read sAct has completed: overwrite it in place with the next operand
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        __align__(16) __nv_bfloat162 hv[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) hv[j] = __floats2bfloat162_rn(v[h * 8 + 2 * j], v[h * 8 + 2 * j + 1]);
-                        *reinterpret_cast<uint4*>(sAct + tc::cm_offset(r, c0 + h * 8, ROWS)) =
-                            *reinterpret_cast<const uint4*>(hv);
+                        for (int i = 0; i < 7; ++i) f[i] = feature_word(__ldg(A.x + c * 7 + i));
                     }
-                } else {
+                }
+                uint4 v;
+                if (half == 0) // hi 0..6, lo 0
+                    v = make_uint4(__byte_perm(f[0], f[1], 0x5410), __byte_perm(f[2], f[3], 0x5410),
+                                   __byte_perm(f[4], f[5], 0x5410), __byte_perm(f[6], f[0], 0x7610));
+                else // lo 1..6, padding
+                    v = make_uint4(__byte_perm(f[1], f[2], 0x7632), __byte_perm(f[3], f[4], 0x7632),
+                                   __byte_perm(f[5], f[6], 0x7632), 0u);
+                *reinterpret_cast<uint4*>(sX + tc::cm_offset(r, 8 * half, ROWS)) = v;
+                float o = sb[5 * H];
+#pragma unroll 1
+                for (int l = 1; l <= 4; ++l) {
+                    // operand writes of every thread of the group -> visible to the tensor core
+                    tc::fence_smem_async();
+                    tc::fence_before_sync();
+                    bar_sync(1 + g, INFER_GROUP);
+                    tc::fence_after_sync();
+                    if ((t & (INFER_GROUP - 1)) == 0) {
+                        if (l == 1) issue<KIN>(acc, sX, false, sW1, false, H);
+                        else issue<H>(acc, sAct, false, sW + (l - 2) * H * H * 2, false, H);
+                        tc::mma_commit(&mbar[g]);
+                    }
+                    ok = tc::mbar_wait(&mbar[g], phase) && ok;
+                    phase ^= 1u;
+                    tc::fence_after_sync();
+                    const float* bias = sb + (l - 1) * H + half * 64;
+                    uint32_t u[2][16];
+                    tc::tmem_ld16_start(at, u[0]);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) o = fmaf(sb[4 * H + c0 + j], v[j], o);
+                    for (int q = 0; q < 4; ++q) { // blocks of 16 columns, the next one's load in flight
+                        tc::tmem_ld16_wait(u[q & 1]);
+                        if (q < 3) tc::tmem_ld16_start(at + (uint32_t)(16 * (q + 1)), u[(q + 1) & 1]);
+                        float a[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4) {
+                            const float4 b4 = *reinterpret_cast<const float4*>(bias + 16 * q + j);
+                            const float2 z0 = __fadd2_rn(make_float2(__uint_as_float(u[q & 1][j]), __uint_as_float(u[q & 1][j + 1])),
+                                                         make_float2(b4.x, b4.y));
+                            const float2 z1 = __fadd2_rn(make_float2(__uint_as_float(u[q & 1][j + 2]), __uint_as_float(u[q & 1][j + 3])),
+                                                         make_float2(b4.z, b4.w));
+                            const float2 s0 = silu2_infer(z0), s1 = silu2_infer(z1);
+                            a[j] = s0.x;
+                            a[j + 1] = s0.y;
+                            a[j + 2] = s1.x;
+                            a[j + 3] = s1.y;
+                        }
+                        if (l < 4) {
+                            // the products that read sAct are done: the next operand goes over it
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                __align__(16) __nv_bfloat162 hv[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                    hv[j] = __floats2bfloat162_rn(a[h * 8 + 2 * j], a[h * 8 + 2 * j + 1]);
+                                *reinterpret_cast<uint4*>(sAct + tc::cm_offset(r, half * 64 + 16 * q + h * 8, ROWS)) =
+                                    *reinterpret_cast<const uint4*>(hv);
+                            }
+                        } else if (half == 0) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) o = fmaf(sb[4 * H + 16 * q + j], a[j], o);
+                        } else {
+                            tc::tmem_st16(at + (uint32_t)(16 * q), a); // for the head's sum, in column order
+                        }
+                    }
+                }
+                // the head: columns 0..63 are in o; the same thread goes on with the other half's
+                if (half) tc::tmem_wait_st();
+                tc::fence_before_sync();
+                bar_sync(1 + g, INFER_GROUP);
+                tc::fence_after_sync();
+                if (half == 0) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        float a[16];
+                        tc::tmem_ld16(at + (uint32_t)(64 + 16 * q), a);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) o = fmaf(sb[4 * H + 64 + 16 * q + j], a[j], o);
+                    }
+                    if (c < A.n) {
+                        float s = m == 0 ? o : A.y[c] + o;
+                        if (m == A.members - 1) s *= 1.0f / (float)A.members;
+                        A.y[c] = s;
+                    }
                 }
             }
-            // every lane has read the accumulator before the next MMA overwrites it
-            tc::fence_before_sync();
         }
-        if (r < valid) y[r0 + r] = o;
+        if (!ok && (t & 31) == 0) atomicExch(A.status, 1);
     }
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tm_s, INFER_TMEM_COLS);
+    if (LATTICE) // the CTA's own tiles, outputs times scale
+        for (int tile0 = INFER_TILES * blockIdx.x; tile0 < tiles; tile0 += stride)
+            for (int c = tile0 * ROWS + t; c < min((tile0 + INFER_TILES) * ROWS, A.n); c += INFER_LATTICE_THREADS)
+                A.price[c] = (float)((double)A.y[c] * A.scale[c]);
 }
 
 } // namespace mlp
@@ -858,22 +1000,6 @@ cudaError_t mlp_loss(const float* loss_part, int tiles, float* loss, cudaStream_
     return cudaGetLastError();
 }
 
-// sum = y (j == 0) or sum + y; at the last member (j == k - 1) the sum becomes the mean
-__global__ void mean_add_kernel(float* __restrict__ sum, const float* __restrict__ y, int64_t n, int j, int k)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float a = j == 0 ? y[i] : sum[i] + y[i];
-    if (j == k - 1) a *= 1.0f / (float)k;
-    sum[i] = a;
-}
-
-cudaError_t mlp_mean_add(float* sum, const float* y, int64_t n, int j, int k, cudaStream_t st)
-{
-    mean_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sum, y, n, j, k);
-    return cudaGetLastError();
-}
-
 cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t st)
 {
     mlp::weight_avg_kernel<<<(mlp::N_PARAMS + 255) / 256, 256, 0, st>>>(params, avg, k);
@@ -883,17 +1009,6 @@ cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t 
 cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16* wbf, cudaStream_t st)
 {
     mlp::weight_avg_finish_kernel<<<(mlp::N_PARAMS + 255) / 256, 256, 0, st>>>(params, avg, wbf);
-    return cudaGetLastError();
-}
-
-cudaError_t mlp_infer(const __nv_bfloat16* x, int n, const float* params, const __nv_bfloat16* wbf, float* y,
-                      int* status, int grid, cudaStream_t st)
-{
-    using namespace mlp;
-    const size_t smem = (size_t)(H * KIN + 3 * H * H + INFER_WG * (ROWS * KIN + ROWS * H)) * 2;
-    cudaError_t e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    infer_kernel<<<grid, INFER_THREADS, smem, st>>>(x, n, params, wbf, y, status);
     return cudaGetLastError();
 }
 
@@ -934,76 +1049,98 @@ int mlp_n_bf() { return mlp::N_BF; }
 // ---------------------------------------------------------------------------
 // Lattice serving: the cells of n_sets parameter sets x n_T maturities x n_lm
 // log-moneyness, cell c = (set * n_T + j) * n_lm + k with raw features
-// (lm[k], T[j], kappa, theta, xi, rho, v0 of the set), built, clipped to the
-// training box and normalised on the device (the network's hi/lo bf16 input
-// split), and the network's output scaled back to a price in units of spot.
+// (lm[k], T[j], kappa, theta, xi, rho, v0 of the set), clipped to the training
+// box and normalised, and the network's output scaled back to a price in units
+// of spot. Everything a cell needs is one word or number per axis value or per
+// (set, maturity); this kernel fills those tables, one thread an entry.
 // ---------------------------------------------------------------------------
 struct LatticeArgs {
     const double* params; // [n_sets][5] kappa, theta, xi, rho, v0
     const double* lms;    // [n_lm]
     const double* Ts;     // [n_T]
     double lo[7], hi[7];  // training box
-    double floor;         // scale floor (units of spot)
-    int64_t n;            // cells
-    int n_lm, n_T;
+    int n_sets, n_lm, n_T;
+    uint32_t *f_lm, *f_T, *f_set;
+    double2 *set_T, *lm;
 };
 
-__device__ __forceinline__ void lattice_cell(const LatticeArgs& A, int64_t c, double (&f)[7])
+__device__ __forceinline__ double clip(const LatticeArgs& A, int q, double f)
 {
-    const int64_t per = (int64_t)A.n_lm * A.n_T;
-    const int64_t set = c / per;
-    const int r = (int)(c % per);
-    f[0] = A.lms[r % A.n_lm];
-    f[1] = A.Ts[r / A.n_lm];
-    for (int q = 0; q < 5; ++q) f[2 + q] = A.params[set * 5 + q];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) f[q] = fmin(fmax(f[q], A.lo[q]), A.hi[q]);
+    return fmin(fmax(f, A.lo[q]), A.hi[q]);
 }
 
-__global__ void lattice_features_kernel(const LatticeArgs A, __nv_bfloat16* __restrict__ x)
+// 2 (f - lo) / (hi - lo) - 1 in FP64, then to FP32, as the host normalisation
+__device__ __forceinline__ uint32_t lattice_word(const LatticeArgs& A, int q, double f)
 {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= A.n) return;
-    double f[7];
-    lattice_cell(A, c, f);
-    __nv_bfloat16* row = x + c * mlp::KIN;
-#pragma unroll
-    for (int q = 0; q < 7; ++q) {
-        // 2 (f - lo) / (hi - lo) - 1 in FP64, then to FP32, as the host normalisation
-        const float v = (float)(2.0 * (f[q] - A.lo[q]) / (A.hi[q] - A.lo[q]) - 1.0);
-        const __nv_bfloat16 h = __float2bfloat16(v);
-        row[q] = h;
-        row[7 + q] = __float2bfloat16(v - __bfloat162float(h));
+    return mlp::feature_word((float)(2.0 * (clip(A, q, f) - A.lo[q]) / (A.hi[q] - A.lo[q]) - 1.0));
+}
+
+__global__ void __launch_bounds__(256) lattice_tables_kernel(const LatticeArgs A)
+{
+    const int n_st = A.n_sets * A.n_T; // at most the cells
+    const int64_t total = (int64_t)n_st + (int64_t)A.n_sets * 5 + A.n_lm + A.n_T;
+    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+        if (e < n_st) {
+            // the expected average Heston variance over [0, T]: sd of the Black-Scholes price
+            const double* p = A.params + (e / A.n_T) * 5;
+            const double T = clip(A, 1, A.Ts[e % A.n_T]), kappa = clip(A, 2, p[0]), theta = clip(A, 3, p[1]),
+                         v0 = clip(A, 6, p[4]);
+            const double kt = kappa * T;
+            const double var = theta + (v0 - theta) * (1.0 - exp(-kt)) / kt;
+            const double sd = sqrt(fmax(var, 1e-8) * T);
+            A.set_T[e] = make_double2(1.0 / sd, 0.5 * sd);
+            continue;
+        }
+        int64_t i = e - n_st;
+        if (i < (int64_t)A.n_sets * 5) {
+            A.f_set[i] = lattice_word(A, 2 + (int)(i % 5), A.params[i]);
+        } else if ((i -= (int64_t)A.n_sets * 5) < A.n_lm) {
+            const double f = clip(A, 0, A.lms[i]);
+            A.f_lm[i] = lattice_word(A, 0, A.lms[i]);
+            A.lm[i] = make_double2(f, exp(f));
+        } else {
+            i -= A.n_lm;
+            A.f_T[i] = lattice_word(A, 1, A.Ts[i]);
+        }
     }
-    row[14] = row[15] = __float2bfloat16(0.f);
 }
 
-// y (the network's normalised price) times sqrt(bs^2 + floor^2), bs the Black-Scholes call
-// (S = 1, r = q = 0) at the expected average Heston variance over [0, T]
-__global__ void lattice_scale_kernel(const LatticeArgs A, const float* __restrict__ y, float* __restrict__ price)
+cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st)
 {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= A.n) return;
-    double f[7];
-    lattice_cell(A, c, f);
-    const double lm = f[0], T = f[1], kappa = f[2], theta = f[3], v0 = f[6];
-    const double kt = kappa * T;
-    const double var = theta + (v0 - theta) * (1.0 - exp(-kt)) / kt;
-    const double sd = sqrt(fmax(var, 1e-8) * T);
-    const double d1 = -lm / sd + 0.5 * sd;
-    const double bs = normcdf(d1) - exp(lm) * normcdf(d1 - sd);
-    price[c] = (float)((double)y[c] * sqrt(bs * bs + A.floor * A.floor));
-}
-
-cudaError_t lattice_features(const LatticeArgs& A, __nv_bfloat16* x, cudaStream_t st)
-{
-    lattice_features_kernel<<<(unsigned)((A.n + 255) / 256), 256, 0, st>>>(A, x);
+    const int64_t total = (int64_t)A.n_sets * (A.n_T + 5) + A.n_lm + A.n_T;
+    lattice_tables_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8 * sms), 256, 0, st>>>(A);
     return cudaGetLastError();
 }
 
-cudaError_t lattice_scale(const LatticeArgs& A, const float* y, float* price, cudaStream_t st)
+// Phi's Taylor coefficients about the nodes k / 8 (mlp::phi_table)
+void phi_coefficients(double* out)
 {
-    lattice_scale_kernel<<<(unsigned)((A.n + 255) / 256), 256, 0, st>>>(A, y, price);
+    for (int k = -mlp::PHI_MID; k <= mlp::PHI_MID; ++k, out += mlp::PHI_COEF) {
+        const double x = k / 8.0, phi = std::exp(-0.5 * x * x) / std::sqrt(2.0 * 3.14159265358979323846);
+        double he0 = 1.0, he1 = x, f = 1.0; // He_0, He_1; n!
+        out[0] = 0.5 * std::erfc(-x / std::sqrt(2.0));
+        for (int n = 1; n < mlp::PHI_COEF; ++n) {
+            f *= n;
+            out[n] = (n % 2 ? phi : -phi) * he0 / f;
+            const double he2 = x * he1 - n * he0;
+            he0 = he1;
+            he1 = he2;
+        }
+    }
+}
+
+int phi_size() { return mlp::PHI_NODES * mlp::PHI_COEF; }
+
+cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st)
+{
+    using namespace mlp;
+    const size_t smem = (size_t)N_BF * 2 + INFER_TILES * (size_t)(ROWS * KIN + ROWS * H) * 2 +
+                        (lattice ? sizeof(double) * PHI_NODES * PHI_COEF : 0);
+    auto k = lattice ? infer_kernel<true> : infer_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int tiles = (A.n + ROWS - 1) / ROWS, grid = std::min((tiles + INFER_TILES - 1) / INFER_TILES, sms);
+    k<<<grid, lattice ? INFER_LATTICE_THREADS : INFER_MAIN, smem, st>>>(A);
     return cudaGetLastError();
 }
 

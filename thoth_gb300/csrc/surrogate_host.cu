@@ -40,23 +40,43 @@ cudaError_t mlp_gradient(const float* part, int tiles, float* grad, cudaStream_t
 cudaError_t mlp_loss(const float* loss_part, int tiles, float* loss, cudaStream_t st);
 cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfloat16* X, float* W, cudaStream_t st);
 cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t st);
-cudaError_t mlp_mean_add(float* sum, const float* y, int64_t n, int j, int k, cudaStream_t st);
 cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16* wbf, cudaStream_t st);
-cudaError_t mlp_infer(const __nv_bfloat16* x, int n, const float* params, const __nv_bfloat16* wbf, float* y,
-                      int* status, int grid, cudaStream_t st);
 int mlp_n_params();
 int mlp_n_bf();
+namespace mlp {
+constexpr int MAX_MEMBERS = 64;
+struct LatticeTables {
+    const uint32_t *f_lm, *f_T, *f_set;
+    const double2 *set_T, *lm;
+    const double* phi;
+    double floor2;
+    uint32_t n_lm, n_T;
+};
+struct InferArgs {
+    const float* x;
+    LatticeTables L;
+    int n, members;
+    float* y;
+    double* scale;
+    float* price;
+    int* status;
+    const float* params[MAX_MEMBERS];
+    const __nv_bfloat16* wbf[MAX_MEMBERS];
+};
+} // namespace mlp
 struct LatticeArgs {
     const double* params;
     const double* lms;
     const double* Ts;
     double lo[7], hi[7];
-    double floor;
-    int64_t n;
-    int n_lm, n_T;
+    int n_sets, n_lm, n_T;
+    uint32_t *f_lm, *f_T, *f_set;
+    double2 *set_T, *lm;
 };
-cudaError_t lattice_features(const LatticeArgs& A, __nv_bfloat16* x, cudaStream_t st);
-cudaError_t lattice_scale(const LatticeArgs& A, const float* y, float* price, cudaStream_t st);
+cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st);
+void phi_coefficients(double* out);
+int phi_size();
+cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st);
 } // namespace thoth
 
 using namespace thoth;
@@ -103,12 +123,9 @@ struct ThothSurrogate {
     mlp::TileArgs A{};
     float* grad = nullptr;
     float* loss = nullptr;
-    // inference buffers
-    int64_t cap_inf = 0;
+    // inference buffer (grown on demand)
+    size_t cap_inf = 0;
     unsigned char* ib = nullptr;
-    // lattice serving: parameter sets and lattice axes, scaled prices
-    int64_t cap_lat = 0;
-    unsigned char* lb = nullptr;
     // the running average of the weights over a training call's last epochs
     float* avg = nullptr;
     // device copy of a training set and its per-epoch permutation (grown on demand)
@@ -176,6 +193,46 @@ int check_status(ThothSurrogate* s)
     int st = 0;
     STRY(cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     STRY(cudaStreamSynchronize(s->st));
+    if (st) return sfail(THOTH_GPU_E_CUDA, "tensor-core MMA did not complete (bounded wait expired)");
+    return THOTH_GPU_OK;
+}
+
+int ensure_infer(ThothSurrogate* s, size_t bytes)
+{
+    if (bytes <= s->cap_inf) return THOTH_GPU_OK;
+    if (s->ib) cudaFree(s->ib);
+    s->ib = nullptr;
+    s->cap_inf = 0; // stays empty if the allocation fails
+    STRY(cudaMalloc(&s->ib, bytes));
+    s->cap_inf = bytes;
+    return THOTH_GPU_OK;
+}
+
+// a timed region of the handle's stream: its two events, destroyed on every way out
+struct Timed {
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    ~Timed()
+    {
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+    }
+    cudaError_t create()
+    {
+        const cudaError_t e = cudaEventCreate(&e0);
+        return e == cudaSuccess ? cudaEventCreate(&e1) : e;
+    }
+};
+
+// the results and the status word back in one wait, and the region's device time
+int finish_infer(ThothSurrogate* s, Timed& T, const float* from, float* to, int64_t n, double* device_ms)
+{
+    int st = 0;
+    STRY(cudaMemcpyAsync(to, from, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s->st));
+    STRY(cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    STRY(cudaStreamSynchronize(s->st));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, T.e0, T.e1);
+    if (device_ms) *device_ms = ms;
     if (st) return sfail(THOTH_GPU_E_CUDA, "tensor-core MMA did not complete (bounded wait expired)");
     return THOTH_GPU_OK;
 }
@@ -387,7 +444,6 @@ int thoth_gpu_surrogate_destroy(ThothSurrogate* s)
         cudaFree(s->status);
         if (s->tb) cudaFree(s->tb);
         if (s->ib) cudaFree(s->ib);
-        if (s->lb) cudaFree(s->lb);
         if (s->avg) cudaFree(s->avg);
         if (s->ds) cudaFree(s->ds);
         if (s->perm_host) cudaFreeHost(s->perm_host);
@@ -538,42 +594,26 @@ int thoth_gpu_surrogate_predict(ThothSurrogate* s, const float* x, int64_t n, fl
         if (!s || !x || !y || n < 1 || n > ((int64_t)1 << 30)) return sfail(THOTH_GPU_E_INVALID, "bad predict arguments");
         std::lock_guard<std::mutex> lk(s_mu);
         STRY(cudaSetDevice(s->dev));
-        if (n > s->cap_inf) {
-            if (s->ib) cudaFree(s->ib);
-            s->ib = nullptr;
-            s->cap_inf = 0;
-            const int64_t cap = (n + 127) / 128 * 128;
-            STRY(cudaMalloc(&s->ib, (size_t)cap * (KIN * 2 + 8) + 512));
-            s->cap_inf = cap;
-        }
-        __nv_bfloat16* dx = reinterpret_cast<__nv_bfloat16*>(s->ib);
-        float* dy = reinterpret_cast<float*>(s->ib + (size_t)s->cap_inf * KIN * 2);
-        std::vector<__nv_bfloat16> hx((size_t)n * KIN, to_bf(0.f));
-        for (int64_t i = 0; i < n; i++)
-            for (int f = 0; f < NF; f++) {
-                const float v = x[i * NF + f];
-                const __nv_bfloat16 hi = to_bf(v);
-                hx[(size_t)i * KIN + f] = hi;
-                hx[(size_t)i * KIN + NF + f] = to_bf(v - __bfloat162float(hi));
-            }
-        STRY(cudaMemcpyAsync(dx, hx.data(), hx.size() * 2, cudaMemcpyHostToDevice, s->st));
+        auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+        const size_t o_y = up(sizeof(float) * NF * (size_t)n);
+        int rc = ensure_infer(s, o_y + sizeof(float) * (size_t)n);
+        if (rc) return rc;
+        mlp::InferArgs A{};
+        A.x = reinterpret_cast<const float*>(s->ib);
+        A.n = (int)n;
+        A.members = 1;
+        A.y = reinterpret_cast<float*>(s->ib + o_y);
+        A.status = s->status;
+        A.params[0] = s->params;
+        A.wbf[0] = s->wbf;
+        Timed T;
+        STRY(T.create());
+        STRY(cudaMemcpyAsync(s->ib, x, sizeof(float) * NF * (size_t)n, cudaMemcpyHostToDevice, s->st));
         STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
-        cudaEvent_t e0, e1;
-        STRY(cudaEventCreate(&e0));
-        STRY(cudaEventCreate(&e1));
-        const int tiles = (int)((n + 127) / 128);
-        const int grid = std::min(tiles, s->sms);
-        STRY(cudaEventRecord(e0, s->st));
-        STRY(mlp_infer(dx, (int)n, s->params, s->wbf, dy, s->status, grid, s->st));
-        STRY(cudaEventRecord(e1, s->st));
-        STRY(cudaMemcpyAsync(y, dy, sizeof(float) * n, cudaMemcpyDeviceToHost, s->st));
-        STRY(cudaStreamSynchronize(s->st));
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        if (device_ms) *device_ms = ms;
-        return check_status(s);
+        STRY(cudaEventRecord(T.e0, s->st));
+        STRY(mlp_infer(A, false, s->sms, s->st));
+        STRY(cudaEventRecord(T.e1, s->st));
+        return finish_infer(s, T, A.y, y, n, device_ms);
     } catch (const std::bad_alloc&) {
         return sfail(THOTH_GPU_E_NOMEM, "out of host memory");
     } catch (const std::exception& e) {
@@ -609,74 +649,66 @@ int thoth_gpu_surrogate_price_lattice_mean(ThothSurrogate* const* members, int32
             if (!(box_hi[q] > box_lo[q])) return sfail(THOTH_GPU_E_INVALID, "empty training box");
         std::lock_guard<std::mutex> lk(s_mu);
         STRY(cudaSetDevice(s->dev));
+        // [inputs: sets, axes, Phi's table][feature words][per set and maturity][per log-moneyness]
+        // [outputs][scales][prices]
         auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-        if (n > s->cap_inf) {
-            if (s->ib) cudaFree(s->ib);
-            s->ib = nullptr;
-            s->cap_inf = 0;
-            const int64_t cap = (n + 127) / 128 * 128;
-            STRY(cudaMalloc(&s->ib, (size_t)cap * (KIN * 2 + 8) + 512));
-            s->cap_inf = cap;
-        }
-        const size_t in_bytes = up(sizeof(double) * ((size_t)n_sets * 5 + n_lm + n_T));
-        const int64_t need = (int64_t)(in_bytes + up(sizeof(float) * (size_t)n));
-        if (need > s->cap_lat) {
-            if (s->lb) cudaFree(s->lb);
-            s->lb = nullptr;
-            s->cap_lat = 0;
-            STRY(cudaMalloc(&s->lb, (size_t)need));
-            s->cap_lat = need;
-        }
-        double* dp = reinterpret_cast<double*>(s->lb);
-        double* dlm = dp + (size_t)n_sets * 5;
-        double* dT = dlm + n_lm;
-        float* dprice = reinterpret_cast<float*>(s->lb + in_bytes);
-        STRY(cudaMemcpyAsync(dp, params, sizeof(double) * (size_t)n_sets * 5, cudaMemcpyHostToDevice, s->st));
-        STRY(cudaMemcpyAsync(dlm, lms, sizeof(double) * n_lm, cudaMemcpyHostToDevice, s->st));
-        STRY(cudaMemcpyAsync(dT, Ts, sizeof(double) * n_T, cudaMemcpyHostToDevice, s->st));
-        LatticeArgs A{};
-        A.params = dp;
-        A.lms = dlm;
-        A.Ts = dT;
+        const size_t n_par = (size_t)n_sets * 5, n_in = n_par + n_lm + n_T + phi_size();
+        size_t off = 0;
+        auto take = [&](size_t bytes) {
+            const size_t o = off;
+            off += up(bytes);
+            return o;
+        };
+        const size_t o_in = take(sizeof(double) * n_in), o_w = take(sizeof(uint32_t) * (n_par + n_lm + n_T)),
+                     o_st = take(sizeof(double2) * (size_t)n_sets * n_T), o_lm = take(sizeof(double2) * n_lm),
+                     o_y = take(sizeof(float) * (size_t)n), o_sc = take(sizeof(double) * (size_t)n),
+                     o_p = take(sizeof(float) * (size_t)n);
+        int rc = ensure_infer(s, off);
+        if (rc) return rc;
+        std::vector<double> in(n_in);
+        std::copy(params, params + n_par, in.begin());
+        std::copy(lms, lms + n_lm, in.begin() + n_par);
+        std::copy(Ts, Ts + n_T, in.begin() + n_par + n_lm);
+        phi_coefficients(in.data() + n_par + n_lm + n_T);
+        const double* d_in = reinterpret_cast<const double*>(s->ib + o_in);
+        LatticeArgs B{};
+        B.params = d_in;
+        B.lms = d_in + n_par;
+        B.Ts = d_in + n_par + n_lm;
         for (int q = 0; q < 7; q++) {
-            A.lo[q] = box_lo[q];
-            A.hi[q] = box_hi[q];
+            B.lo[q] = box_lo[q];
+            B.hi[q] = box_hi[q];
         }
-        A.floor = floor;
-        A.n = n;
-        A.n_lm = n_lm;
-        A.n_T = n_T;
-        __nv_bfloat16* dx = reinterpret_cast<__nv_bfloat16*>(s->ib);
-        float* dy = reinterpret_cast<float*>(s->ib + (size_t)s->cap_inf * KIN * 2);
+        B.n_sets = n_sets;
+        B.n_lm = n_lm;
+        B.n_T = n_T;
+        B.f_set = reinterpret_cast<uint32_t*>(s->ib + o_w);
+        B.f_lm = B.f_set + n_par;
+        B.f_T = B.f_lm + n_lm;
+        B.set_T = reinterpret_cast<double2*>(s->ib + o_st);
+        B.lm = reinterpret_cast<double2*>(s->ib + o_lm);
+        mlp::InferArgs A{};
+        A.L = mlp::LatticeTables{B.f_lm, B.f_T, B.f_set, B.set_T, B.lm, d_in + n_par + n_lm + n_T, floor * floor,
+                                 (uint32_t)n_lm, (uint32_t)n_T};
+        A.n = (int)n;
+        A.members = k;
+        A.y = reinterpret_cast<float*>(s->ib + o_y);
+        A.scale = reinterpret_cast<double*>(s->ib + o_sc);
+        A.price = reinterpret_cast<float*>(s->ib + o_p);
+        A.status = s->status;
+        for (int j = 0; j < k; j++) {
+            A.params[j] = members[j]->params;
+            A.wbf[j] = members[j]->wbf;
+        }
+        Timed T;
+        STRY(T.create());
+        STRY(cudaMemcpyAsync(s->ib + o_in, in.data(), sizeof(double) * n_in, cudaMemcpyHostToDevice, s->st));
         STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
-        cudaEvent_t e0, e1;
-        STRY(cudaEventCreate(&e0));
-        STRY(cudaEventCreate(&e1));
-        const int tiles = (int)((n + 127) / 128);
-        const int grid = std::min(tiles, s->sms);
-        STRY(cudaEventRecord(e0, s->st));
-        STRY(lattice_features(A, dx, s->st));
-        if (k == 1) {
-            STRY(mlp_infer(dx, (int)n, s->params, s->wbf, dy, s->status, grid, s->st));
-            STRY(lattice_scale(A, dy, dprice, s->st));
-        } else {
-            // each member's normalised prices, added in member order into the mean
-            float* dsum = reinterpret_cast<float*>(s->ib + ((size_t)s->cap_inf * (KIN * 2 + 4) + 255) / 256 * 256);
-            for (int j = 0; j < k; j++) {
-                STRY(mlp_infer(dx, (int)n, members[j]->params, members[j]->wbf, dy, s->status, grid, s->st));
-                STRY(mlp_mean_add(dsum, dy, n, j, k, s->st));
-            }
-            STRY(lattice_scale(A, dsum, dprice, s->st));
-        }
-        STRY(cudaEventRecord(e1, s->st));
-        STRY(cudaMemcpyAsync(prices, dprice, sizeof(float) * n, cudaMemcpyDeviceToHost, s->st));
-        STRY(cudaStreamSynchronize(s->st));
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        if (device_ms) *device_ms = ms;
-        return check_status(s);
+        STRY(cudaEventRecord(T.e0, s->st));
+        STRY(lattice_tables(B, s->sms, s->st));
+        STRY(mlp_infer(A, true, s->sms, s->st));
+        STRY(cudaEventRecord(T.e1, s->st));
+        return finish_infer(s, T, A.price, prices, n, device_ms);
     } catch (const std::bad_alloc&) {
         return sfail(THOTH_GPU_E_NOMEM, "out of host memory");
     } catch (const std::exception& e) {
