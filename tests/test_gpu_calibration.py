@@ -112,3 +112,32 @@ def test_uneven_ensembles_and_thin_bins_match_the_oracle(gpu, particles, bins, m
     c.bins, c.min_bin_count = bins, min_count
     L, _ = gpu.calibrate_leverage(c)
     np.testing.assert_allclose(L, oracle.calibrate_leverage(c), rtol=1e-9, atol=0)
+
+
+@pytest.mark.parametrize("particles,points", [
+    (16384, 2),          # the smallest layer
+    (129, 201),          # one particle more than a CTA
+    (77825, 64),         # more than one a thread: the ensemble in memory
+])
+def test_ensemble_and_layer_edges_match_the_oracle(gpu, particles, points):
+    """The particles' places (registers, memory), a CTA with one particle, and the smallest layer,
+    against the oracle; rounding differences alone, as in the tests above."""
+    c = W.lsv_calibration(horizon_days=6, particles=particles)
+    c.local_vol = np.ascontiguousarray(c.local_vol[:, (201 - points) // 2:][:, :points])
+    c.offset = np.ascontiguousarray(c.offset + (201 - points) // 2)
+    c.leverage = np.zeros_like(c.local_vol)
+    L, _ = gpu.calibrate_leverage(c)
+    np.testing.assert_allclose(L, oracle.calibrate_leverage(c), rtol=1e-9, atol=0)
+
+
+def test_vanishing_vol_of_vol_keeps_its_errors_and_limits(gpu):
+    """xi = 0 leaves no variance (psi = 0): refused, as the step's ratio is not a number; a tiny xi
+    is the deterministic variance (the exact limit of the step)."""
+    for xi, ok in ((0.0, False), (1e-100, True), (1e-13, True)):
+        c = W.lsv_calibration(horizon_days=5, particles=1024, heston=dict(v0=0.04, kappa=1.0, theta=0.04, xi=xi, rho=0.0))
+        if not ok:
+            with pytest.raises(gpu.ThothGpuError):
+                gpu.calibrate_leverage(c)
+            continue
+        L, _ = gpu.calibrate_leverage(c)
+        np.testing.assert_allclose(L, oracle.calibrate_leverage(c), rtol=1e-9, atol=0)

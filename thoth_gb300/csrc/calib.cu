@@ -2,13 +2,24 @@
 // Single::CalibrateLeverage and its helpers (pricer/src/marketdata/single.cpp:240-473) with
 // the reference Rng (helpers/rng.hpp) and inverse normal (helpers/distributions.cpp:37-81).
 //
-// One cooperative launch walks the dates. Per date, two publish-and-release rounds build
-// the conditional variance of the current ensemble: (A) the extremes of ln S and the sum of
-// v, (B) per-bin counts and sums of v between those extremes. The last CTA to publish in a
-// round adds every CTA's contribution (exact integer sums), and after round B computes the
-// bin means, fills thin bins and writes layer k of the surface; the others wait for its
-// release flag. Every CTA then steps its particles into date k with layer k, read from
-// shared memory.
+// One cooperative launch walks the dates. Per date, two rounds build the conditional variance of
+// the current ensemble: (A) the extremes of ln S and the sum of v, (B) per-bin counts and sums of
+// v between those extremes. In a round every CTA adds its contribution into the date's totals
+// (exact integer sums), arrives at a counter and waits for the others there; every CTA then forms
+// the bin means and the layer itself, from the same totals. Everything of the step into the date
+// that needs no layer runs between an arrival and its wait: the Gaussians, the generator's jump
+// and the layer coordinate behind round A, the variance step behind round B.
+//
+// GB300 issues FP64 at 1/64 of the FP32 rate: an FP64 instruction holds its scheduler's pipe for
+// 64 clocks, and 16384 particles are one warp a scheduler on 128 SMs, so the FP64 instructions of
+// a date are what it costs. The step is therefore kept short: constants of a date come from the
+// host; the tail of the inverse normal (its logarithm and square root, 4.85 % of draws) runs on
+// draws collected over the CTA; the layer is looked up from ln S - ln S0, which the ensemble
+// carries, instead of from the logarithm of a spot kept through an exponential; the part of the
+// log-spot step that no leverage enters waits ready for it; a CTA builds the layer only where the
+// ensemble is (a CTA without particles writes the whole of it out). Per date 29 us as a
+// restatement of the reference's expressions, both branches of the inverse normal evaluated and a
+// last CTA building the layer: 13.3 ms for 16384 particles x 365 dates; like this 18 us, 6.5 ms.
 //
 // The Gaussians are the reference's stream: xoshiro256++ seeded by splitmix64, one 64-bit
 // draw per Gaussian through Acklam's inverse normal, two per particle per date in particle
@@ -18,10 +29,14 @@
 // evaluated at the transition: 256 transitions and XORs (F. Haramoto et al., "Efficient jump
 // ahead for F2-linear random number generators", INFORMS J. Computing 20(3), 2008).
 //
-// Compiled without FMA contraction: every expression rounds as the reference's does, so the
-// ensemble differs from the reference's only where CUDA's exp, log and erfc differ from the
-// host's in the last bit. The sums of v are exact (exact.cuh), independent of the grid.
+// Compiled without FMA contraction (the book kernel's tail Gaussians round as the reference's do);
+// the ensemble's own arithmetic uses fused multiply-adds where written. It differs from the
+// reference's in rounding only, about one part in 10^16 an operation; the sums of v are exact
+// (exact.cuh), independent of the grid.
 #include "calib.cuh"
+#include "phi.cuh"
+
+#include <cmath>
 
 #include <mutex>
 #include <vector>
@@ -29,6 +44,7 @@
 namespace {
 
 constexpr int CALIB_WARPS = CALIB_THREADS / 32;
+static_assert(CALIB_WARPS == 4, "four warps share the results of round A");
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull; // 2 s
 
 __host__ __device__ __forceinline__ uint64_t rotl64(uint64_t x, int k) { return (x << k) | (x >> (64 - k)); }
@@ -106,89 +122,123 @@ __device__ __forceinline__ void xo_jump_tab(const uint64_t* tab, uint64_t* s)
     s[3] = r3;
 }
 
-// Acklam's inverse normal as the reference evaluates it (NormalCdfInv). Both the tail and
-// the central rational are evaluated and one is selected: the selected value is the same
-// expression the reference evaluates, and without branches the compiler can interleave the
-// particle's independent FP64 chains (two Gaussians, the layer lookup).
-__device__ double normal_cdf_inv(double P)
+constexpr double ACKLAM_P_LOW = 0.02425;
+
+// Acklam's inverse normal (the reference's NormalCdfInv), its two branches apart, each the
+// expression the reference evaluates there
+__device__ __forceinline__ double acklam_central(double P) // P in [p_low, 1 - p_low]
 {
     const double a0 = -3.969683028665376e+01, a1 = 2.209460984245205e+02, a2 = -2.759285104469687e+02,
                  a3 = 1.383577518672690e+02, a4 = -3.066479806614716e+01, a5 = 2.506628277459239e+00;
     const double b0 = -5.447609879822406e+01, b1 = 1.615858368580409e+02, b2 = -1.556989798598866e+02,
                  b3 = 6.680131188771972e+01, b4 = -1.328068155288572e+01;
-    const double c0 = -7.784894002430293e-03, c1 = -3.223964580411365e-01, c2 = -2.400758277161838e+00,
-                 c3 = -2.549732539343734e+00, c4 = 4.374664141464968e+00, c5 = 2.938163982698783e+00;
-    const double d0 = 7.784695709041462e-03, d1 = 3.224671290700398e-01, d2 = 2.445134137142996e+00,
-                 d3 = 3.754408661907416e+00;
-    const double p_low = 0.02425, p_high = 1.0 - p_low;
-    const bool lower = P < p_low, upper = !(P <= p_high);
-    // tail: q = sqrt(-2 ln P) below, sqrt(-2 ln(1 - P)) above (1 - P is exact where it is used)
-    const double qt = sqrt(-2.0 * log(lower ? P : 1.0 - P));
-    const double tn = ((((c0 * qt + c1) * qt + c2) * qt + c3) * qt + c4) * qt + c5;
-    const double td = (((d0 * qt + d1) * qt + d2) * qt + d3) * qt + 1.0;
     const double q = P - 0.5;
     const double r = q * q;
     const double cn = (((((a0 * r + a1) * r + a2) * r + a3) * r + a4) * r + a5) * q;
     const double cd = ((((b0 * r + b1) * r + b2) * r + b3) * r + b4) * r + 1.0;
-    const double num = lower ? tn : (upper ? -tn : cn);
-    const double den = (lower || upper) ? td : cd;
-    return num / den;
+    return cn / cd;
 }
 
-// Rng::Gaussian: a 53-bit uniform in (0, 1) through the inverse normal
-__device__ __forceinline__ double gaussian(uint64_t* s)
+__device__ __forceinline__ double acklam_tail(double P) // P < p_low or P > 1 - p_low
+{
+    const double c0 = -7.784894002430293e-03, c1 = -3.223964580411365e-01, c2 = -2.400758277161838e+00,
+                 c3 = -2.549732539343734e+00, c4 = 4.374664141464968e+00, c5 = 2.938163982698783e+00;
+    const double d0 = 7.784695709041462e-03, d1 = 3.224671290700398e-01, d2 = 2.445134137142996e+00,
+                 d3 = 3.754408661907416e+00;
+    const bool lower = P < ACKLAM_P_LOW;
+    const double qt = sqrt(-2.0 * log(lower ? P : 1.0 - P));
+    const double tn = ((((c0 * qt + c1) * qt + c2) * qt + c3) * qt + c4) * qt + c5;
+    const double td = (((d0 * qt + d1) * qt + d2) * qt + d3) * qt + 1.0;
+    return (lower ? tn : -tn) / td;
+}
+
+// a uniform in (0, 1) of 53 bits, as Rng::Gaussian forms it
+__device__ __forceinline__ double uniform53(uint64_t* s)
 {
     const double u0 = (double)(xo_next(s) >> 11) * (1.0 / 9007199254740992.0);
-    return normal_cdf_inv(u0 > 0.0 ? u0 : (1.0 / 9007199254740992.0));
+    return u0 > 0.0 ? u0 : (1.0 / 9007199254740992.0);
 }
 
-// QeVarianceStep (single.cpp:344-368) with e = exp(-kappa Dt) rounded on the host
-__device__ double qe_step(double V, double Z, double e, const CalibArgs& A)
+__device__ __forceinline__ bool in_tail(double u) { return u < ACKLAM_P_LOW || !(u <= 1.0 - ACKLAM_P_LOW); }
+
+// the inverse normal's branches with fused multiply-adds
+__device__ __forceinline__ double gauss_tail(double P)
 {
-    const double m = A.theta + (V - A.theta) * e;
-    const double s2 = V * A.xi * A.xi * e / A.kappa * (1 - e) + A.theta * A.xi * A.xi / (2 * A.kappa) * (1 - e) * (1 - e);
-    const double psi = (m > 0) ? s2 / (m * m) : 0;
-    if (psi <= 1.5) {
-        const double c = 2.0 / psi;
-        const double b2 = c - 1.0 + sqrt(c) * sqrt(c - 1.0);
-        const double a = m / (1.0 + b2);
+    const bool lower = P < ACKLAM_P_LOW;
+    const double q = sqrt(-2.0 * log(lower ? P : 1.0 - P));
+    double n = -7.784894002430293e-03, d = 7.784695709041462e-03;
+    n = fma(n, q, -3.223964580411365e-01);
+    d = fma(d, q, 3.224671290700398e-01);
+    n = fma(n, q, -2.400758277161838e+00);
+    d = fma(d, q, 2.445134137142996e+00);
+    n = fma(n, q, -2.549732539343734e+00);
+    d = fma(d, q, 3.754408661907416e+00);
+    n = fma(n, q, 4.374664141464968e+00);
+    d = fma(d, q, 1.0);
+    n = fma(n, q, 2.938163982698783e+00);
+    return (lower ? n : -n) / d;
+}
+
+__device__ __forceinline__ double gauss_central(double P)
+{
+    const double q = P - 0.5, r = q * q;
+    double n = -3.969683028665376e+01, d = -5.447609879822406e+01;
+    n = fma(n, r, 2.209460984245205e+02);
+    d = fma(d, r, 1.615858368580409e+02);
+    n = fma(n, r, -2.759285104469687e+02);
+    d = fma(d, r, -1.556989798598866e+02);
+    n = fma(n, r, 1.383577518672690e+02);
+    d = fma(d, r, 6.680131188771972e+01);
+    n = fma(n, r, -3.066479806614716e+01);
+    d = fma(d, r, -1.328068155288572e+01);
+    n = fma(n, r, 2.506628277459239e+00);
+    d = fma(d, r, 1.0);
+    return n * q / d;
+}
+
+// QeVarianceStep (single.cpp:344-368): psi = s2 / m^2 <= 1.5 is tested as s2 <= 1.5 m^2, and the
+// quadratic branch takes c = 2 / psi from m and s2 and sqrt(c) sqrt(c - 1) as one square root (c
+// capped where its square would overflow: the step's random part is below FP64 there)
+__device__ double qe_step(double V, double Z, const CalibStep& C, const double* phi)
+{
+    const double m = fma(V, C.e, C.th1e), s2 = fma(V, C.qa, C.qb), m2 = m * m;
+    if (s2 <= 1.5 * m2) {
+        double c = 2.0 * m2 / s2;
+        if (c > 1e150 && c < INFINITY) c = 1e150;
+        const double b2 = c - 1.0 + sqrt(c * (c - 1.0));
         const double bz = sqrt(b2) + Z;
-        return a * bz * bz;
+        return m / (1.0 + b2) * bz * bz;
     }
-    const double p = (psi - 1.0) / (psi + 1.0);
-    const double beta = (1.0 - p) / m;
-    const double u = 0.5 * erfc(-Z / sqrt(2.0));
-    return (u <= p) ? 0.0 : log((1.0 - p) / (1.0 - u)) / beta;
+    // 1 - p = 2 m^2 / (s2 + m^2), 1 - u = Phi(-Z), 1 / beta = (s2 + m^2) / (2 m)
+    const double num = s2 + m2;
+    const double r = 2.0 * m2 / (num * thoth::phi_table(phi, -Z)); // (1 - p) / (1 - u)
+    return r <= 1.0 ? 0.0 : log(r) * (num / (2.0 * m));
 }
 
-// LeveragedLogSpotStep (single.cpp:370-388)
-__device__ double spot_step(double Vp, double Vc, double Dt, double Carry, double L, double Z, const CalibArgs& A)
+// LeveragedLogSpotStep (single.cpp:370-388) as carry + L b - L^2 d: its parts b and d
+__device__ __forceinline__ void spot_parts(double Vp, double Vc, double Z, const CalibStep& C, double& b, double& d)
 {
-    if (A.xi > 1e-12) {
-        const double g = 0.5;
-        const double k0 = -L * A.rho * A.kappa * A.theta / A.xi * Dt;
-        const double a = g * Dt * (L * A.kappa * A.rho / A.xi - 0.5 * L * L);
-        const double k1 = a - L * A.rho / A.xi;
-        const double k2 = a + L * A.rho / A.xi;
-        const double k3 = g * Dt * (1.0 - A.rho * A.rho) * L * L;
-        double var = k3 * (Vp + Vc);
-        if (var < 0) var = 0;
-        return Carry + k0 + k1 * Vp + k2 * Vc + sqrt(var) * Z;
+    if (C.flat == 0.0) {
+        const double s = Vp + Vc;
+        const double var = C.k3 * s;
+        b = fma(sqrt(var < 0 ? 0.0 : var), Z, fma(C.r, Vc - Vp, fma(C.a1, s, C.k0)));
+        d = C.a2 * s;
+    } else {
+        b = sqrt(Vp * C.dt) * Z;
+        d = 0.5 * Vp * C.dt;
     }
-    return Carry - 0.5 * L * L * Vp * Dt + L * sqrt(Vp * Dt) * Z;
 }
 
-// LeverageSurface::LayerAt (leverage_surface.cpp:19-40) on a layer in shared memory: the
-// clamps select instead of branching (the interpolation index is clamped to the layer, and
-// its value is only selected where the reference interpolates)
-__device__ __forceinline__ double layer_at(const double* lev, int points, double ln_step, int64_t offset, double S)
+// LeverageSurface::LayerAt (leverage_surface.cpp:19-40) at grid coordinate f on a layer in shared
+// memory: the clamps select instead of branching (the interpolation index is clamped to the layer,
+// and its value is only selected where the reference interpolates)
+__device__ __forceinline__ double layer_at(const double* lev, int points, double f)
 {
-    const double f = log(S) / ln_step - (double)offset;
     const int last = points - 1;
     const bool inside = f > 0.0 && f < (double)last;
     const int i = inside ? (int)f : 0;
     const double w = f - (double)i;
-    const double mid = (1.0 - w) * lev[i] + w * lev[i + 1];
+    const double mid = fma(w, lev[i + 1] - lev[i], lev[i]);
     return !(f > 0.0) ? lev[0] : (f >= (double)last ? lev[last] : mid);
 }
 
@@ -214,11 +264,6 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // wait until *flag >= want; false (status 2) after 2 s, or at once when another CTA failed
@@ -248,19 +293,24 @@ __device__ __forceinline__ double from_key(long long k)
     return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 
-// exact 128-bit add into global memory: the low word's returned old value gives the carry
-__device__ __forceinline__ void fx_atomic_add(Fx128* dst, const Fx128& a)
+// An exact 128-bit sum added into global memory as limbs of 42, 42 and 44 bits, each into a word
+// of its own by a reduction that returns nothing (as in american.cu): a CTA's sum is below 2^108,
+// so fewer than 2^20 CTAs cannot overflow a word.
+__device__ __forceinline__ void fx_red3(unsigned long long* dst, const Fx128& a)
 {
-    unsigned long long* w = reinterpret_cast<unsigned long long*>(dst);
-    const unsigned long long old = atomicAdd(w, (unsigned long long)a.lo);
-    const unsigned long long carry = (old + (unsigned long long)a.lo < old) ? 1ull : 0ull;
-    if (a.hi + carry) atomicAdd(w + 1, (unsigned long long)(a.hi + carry));
+    const uint64_t m = (1ull << 42) - 1;
+    atomicAdd(dst, (unsigned long long)(a.lo & m));
+    atomicAdd(dst + 1, (unsigned long long)((a.lo >> 42) | ((a.hi & ((1ull << 20) - 1)) << 22)));
+    atomicAdd(dst + 2, (unsigned long long)(a.hi >> 20));
 }
 
-__device__ __forceinline__ Fx128 fx_load_cg(const Fx128* p)
+__device__ __forceinline__ Fx128 fx_load3(const unsigned long long* p)
 {
-    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(p);
-    return Fx128{(uint64_t)__ldcg(w), (uint64_t)__ldcg(w + 1)};
+    const uint64_t l0 = __ldcg(p), l1 = __ldcg(p + 1), l2 = __ldcg(p + 2);
+    Fx128 r = {l0, 0};
+    fx_add(r, l1 << 42, l1 >> 22);
+    fx_add(r, 0, l2 << 20);
+    return r;
 }
 
 // the two 64-bit words x adds to an Fx128 (x >= 0, truncated to 2^-64); bad when out of range
@@ -272,237 +322,335 @@ __device__ __forceinline__ void fx_words(double x, uint64_t& lo, uint64_t& hi, b
     hi = t.hi;
 }
 
-// layer k from the conditional variance cv(x) of the published bins (all threads of the CTA)
-__device__ void build_layer(const CalibArgs& A, int k, bool flat, double fallback, double x0, double dx,
-                            const double* mean)
+// A bin's sum of v in shared memory, one particle a thread: v's fixed-point value (below 2^36 by
+// its check, in units of 2^-64) as five 20-bit limbs, each added into its own 32-bit word, which
+// 2^12 addends cannot overflow. (A 64-bit shared atomic is a compare-and-swap loop, and the
+// particles crowd into a few bins.)
+constexpr int BIN_LIMBS = 5;
+static_assert(CALIB_THREADS <= 4096, "a limb's word holds 2^12 addends");
+
+__device__ __forceinline__ uint64_t limb_bits(uint64_t lo, uint64_t hi, int i)
 {
-    const double ls = A.ln_step[k];
-    const int64_t off = A.offset[k];
-    for (int i = threadIdx.x; i < A.points; i += CALIB_THREADS) {
-        const double x = (double)(off + i) * ls;
-        double ev;
-        if (flat) {
-            ev = fallback;
-        } else {
-            const double f = (x - x0) / dx;
-            const double last = (double)(A.bins - 1);
-            if (f <= 0) {
-                ev = mean[0];
-            } else if (f >= last) {
-                ev = mean[A.bins - 1];
-            } else {
-                const int j = (int)f;
-                const double w = f - (double)j;
-                ev = (1.0 - w) * mean[j] + w * mean[j + 1];
-            }
-        }
-        if (ev < A.min_cv) ev = A.min_cv;
-        const double L = A.local_vol[(size_t)k * A.points + i] / sqrt(ev);
-        A.lev[(size_t)k * A.points + i] = L < A.lmin ? A.lmin : (L > A.lmax ? A.lmax : L);
-    }
+    const int b = 20 * i;
+    const uint64_t w = b >= 64 ? hi >> (b - 64) : (b == 0 ? lo : (lo >> b) | (hi << (64 - b)));
+    return w & 0xfffffu;
 }
 
-__global__ void __launch_bounds__(CALIB_THREADS) lsv_calib_kernel(const CalibArgs A)
+// one particle's state and what its next step has so far
+struct Particle {
+    double x, var, lns;
+    double z1, z2, vc, sb, sd;
+    uint64_t s[4];
+};
+
+// ONE: at most one particle a thread, held in registers
+template <bool ONE>
+__global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const CalibArgs A, int G)
 {
     extern __shared__ __align__(16) unsigned char s_dyn[]; // the jump table, then the layer [points]
     uint64_t* s_jtab = reinterpret_cast<uint64_t*>(s_dyn);
     double* s_layer = reinterpret_cast<double*>(s_dyn + sizeof(uint64_t) * CALIB_JTAB_WORDS);
-    __shared__ double s_min[CALIB_WARPS], s_max[CALIB_WARPS];
+    __shared__ long long s_min[CALIB_WARPS], s_max[CALIB_WARPS];
     __shared__ Fx128 s_sum[CALIB_WARPS];
+    static_assert(CALIB_MAX_BINS >= CALIB_THREADS, "the tail queue fits the bins' arrays");
     __shared__ unsigned s_cnt[CALIB_MAX_BINS];
-    __shared__ unsigned long long s_blo[CALIB_MAX_BINS], s_bhi[CALIB_MAX_BINS];
-    __shared__ double s_bsum[CALIB_MAX_BINS], s_mean[CALIB_MAX_BINS];
-    __shared__ double s_bc[4];
-    __shared__ int s_last, s_ok;
-    const int G = gridDim.x;
-    const int T = G * CALIB_THREADS;
-    const int gt = blockIdx.x * CALIB_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int P = A.P, bins = A.bins;
+    __shared__ unsigned long long s_bin[2 * CALIB_MAX_BINS]; // 64-bit sums, or three of the limbs
+    __shared__ double s_two[2 * CALIB_MAX_BINS];             // the others; then sums and means
+    unsigned long long *s_blo = s_bin, *s_bhi = s_bin + CALIB_MAX_BINS;
+    unsigned *s_l0 = reinterpret_cast<unsigned*>(s_bin), *s_l4 = reinterpret_cast<unsigned*>(s_two); // limbs 0..3, 4
+    double *s_bsum = s_two, *s_mean = s_two + CALIB_MAX_BINS;
+    // behind round A, when the bins are not in use: the tail draws, whose they are, their Gaussians
+    double *s_qu = reinterpret_cast<double*>(s_bin), *s_z = s_two;
+    unsigned short* s_qi = reinterpret_cast<unsigned short*>(s_cnt);
+    __shared__ int s_qn[2];    // how many
+    __shared__ double s_bc[4]; // min ln S, bin width and its reciprocal, ensemble mean of v
+    __shared__ int s_ok; // 0: a wait failed; 1; 2: every particle at one spot
+    const int T = G * CALIB_THREADS; // the CTAs past G have no particles and take no part in the rounds
+    const int t = threadIdx.x, gt = blockIdx.x * CALIB_THREADS + t;
+    const int lane = t & 31, warp = t >> 5;
+    const int P = (int)blockIdx.x < G ? A.P : 0, bins = A.bins;
+    const bool writes = (int)blockIdx.x == A.writer;
+    const int R = ONE ? 1 : (A.P + T - 1) / T; // particles a thread, the same for every thread
     bool bad = false;
+    int tog = 0;
+    Particle q{};
 
-    for (int i = threadIdx.x; i < (int)CALIB_JTAB_WORDS; i += CALIB_THREADS) s_jtab[i] = A.jtab[i];
+    for (int i = t; i < (int)CALIB_JTAB_WORDS; i += CALIB_THREADS) s_jtab[i] = A.jtab[i];
+    if (t < 2) s_qn[t] = 0;
     __syncthreads();
     // the ensemble at today; particle p's generator at draw 2p of the stream
     for (int p = gt; p < P; p += T) {
-        A.spot[p] = A.s0;
-        A.var[p] = A.v0;
-        A.lns[p] = A.ln_s0;
-        uint64_t s[4] = {A.seed_state[0], A.seed_state[1], A.seed_state[2], A.seed_state[3]};
+        q.x = 0.0;
+        q.var = A.v0;
+        q.lns = A.ln_s0;
+        for (int w = 0; w < 4; w++) q.s[w] = A.seed_state[w];
         const uint64_t off = 2ull * (uint64_t)p;
         for (int i = 0; i < CALIB_JUMP_BITS; i++)
-            if ((off >> i) & 1u) xo_jump(A.jpow + 4 * i, s);
-        for (int w = 0; w < 4; w++) A.rng[(size_t)w * P + p] = s[w];
+            if ((off >> i) & 1u) xo_jump(A.jpow + 4 * i, q.s);
+        if (!ONE) {
+            A.x[p] = q.x;
+            A.var[p] = q.var;
+            A.lns[p] = q.lns;
+            for (int w = 0; w < 4; w++) A.rng[(size_t)w * P + p] = q.s[w];
+        }
     }
 
     unsigned round = 0;
-    for (int k = 0; k < A.n; k++) {
-        // ---- round A: extremes of ln S, sum of v ----
-        double mn = INFINITY, mx = -INFINITY;
-        Fx128 sv = {0, 0};
-        for (int p = gt; p < P; p += T) {
-            const double x = A.lns[p];
-            mn = fmin(mn, x);
-            mx = fmax(mx, x);
-            fx_add_checked(sv, A.var[p], bad);
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
-        warp_sum(sv);
-        if (lane == 0) {
-            s_min[warp] = mn;
-            s_max[warp] = mx;
-            s_sum[warp] = sv;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double cm = s_min[0], cx = s_max[0];
-            Fx128 cs = s_sum[0];
-            for (int w = 1; w < CALIB_WARPS; w++) {
-                cm = fmin(cm, s_min[w]);
-                cx = fmax(cx, s_max[w]);
-                fx_add(cs, s_sum[w]);
-            }
-            if (cm <= cx) { // a CTA without particles adds nothing
-                atomicMin(A.kmin + k, order_key(cm));
-                atomicMax(A.kmax + k, order_key(cx));
-                fx_atomic_add(A.vsum + k, cs);
-            }
-            __threadfence();
-        }
-        if (bad) atomicExch(A.status, 3);
+    auto arrive = [&] { // after a __syncthreads that follows every contribution's fence
         ++round;
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicAdd(A.bar, 1u) == round * (unsigned)G - 1;
-        __syncthreads();
-        if (s_last) {
-            if (threadIdx.x == 0) {
-                __threadfence();
-                const double gmn = from_key((long long)__ldcg((const unsigned long long*)(A.kmin + k)));
-                const double gmx = from_key((long long)__ldcg((const unsigned long long*)(A.kmax + k)));
-                s_bc[0] = gmn;
-                s_bc[1] = (gmx - gmn) / bins;
-                s_bc[2] = fx_to_double(fx_load_cg(A.vsum + k)) / (double)P;
-                s_bc[3] = (gmx - gmn < 1e-10) ? 1.0 : 0.0;
-                for (int j = 0; j < 4; j++) A.bc[j] = s_bc[j];
-            }
-            __syncthreads();
-            if (s_bc[3] != 0.0) build_layer(A, k, true, s_bc[2], 0.0, 1.0, s_mean);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                st_release(A.done, round);
-            }
-        } else if (threadIdx.x == 0) {
-            const bool ok = wait_for(A.done, round, A.status);
-            if (ok)
-                for (int j = 0; j < 4; j++) s_bc[j] = __ldcg(A.bc + j);
-            s_ok = ok;
-        }
-        __syncthreads();
-        if (!s_last && !s_ok) return;
-
-        if (s_bc[3] == 0.0) {
-            // ---- round B: per-bin counts and sums of v ----
-            const double bmn = s_bc[0], width = s_bc[1];
-            for (int b = threadIdx.x; b < bins; b += CALIB_THREADS) {
-                s_cnt[b] = 0;
-                s_blo[b] = 0;
-                s_bhi[b] = 0;
-            }
-            __syncthreads();
+        if (t == 0 && P > 0) atomicAdd(A.bar, 1u);
+    };
+    for (int k = 0; k < A.n; k++) {
+        // ---- round A: extremes of ln S (as integer keys), sum of v ----
+        if (P > 0) {
+            long long mn = 0x7fffffffffffffffll, mx = -0x7fffffffffffffffll;
+            Fx128 sv = {0, 0};
             for (int p = gt; p < P; p += T) {
-                int b = (int)((A.lns[p] - bmn) / width);
-                b = b < 0 ? 0 : (b > bins - 1 ? bins - 1 : b);
-                uint64_t lo, hi;
-                fx_words(A.var[p], lo, hi, bad);
-                atomicAdd(&s_cnt[b], 1u);
-                const unsigned long long old = atomicAdd(&s_blo[b], (unsigned long long)lo);
-                atomicAdd(&s_bhi[b], (unsigned long long)(hi + ((uint64_t)old + lo < lo ? 1u : 0u)));
-            }
-            __syncthreads();
-            for (int b = threadIdx.x; b < bins; b += CALIB_THREADS) {
-                if (s_cnt[b]) {
-                    atomicAdd(A.bcnt + (size_t)k * bins + b, s_cnt[b]);
-                    fx_atomic_add(A.bsum + (size_t)k * bins + b, Fx128{s_blo[b], s_bhi[b]});
+                if (!ONE) {
+                    q.lns = A.lns[p];
+                    q.var = A.var[p];
                 }
-                __threadfence();
+                const long long key = order_key(q.lns);
+                mn = min(mn, key);
+                mx = max(mx, key);
+                fx_add_checked(sv, q.var, bad);
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            warp_sum(sv);
+            if (lane == 0) {
+                s_min[warp] = mn;
+                s_max[warp] = mx;
+                s_sum[warp] = sv;
             }
             if (bad) atomicExch(A.status, 3);
-            ++round;
             __syncthreads();
-            if (threadIdx.x == 0) s_last = atomicAdd(A.bar, 1u) == round * (unsigned)G - 1;
-            __syncthreads();
-            if (s_last) {
+            if (t == 0) {
+                long long cm = s_min[0], cx = s_max[0];
+                Fx128 cs = s_sum[0];
+                for (int w = 1; w < CALIB_WARPS; w++) {
+                    cm = min(cm, s_min[w]);
+                    cx = max(cx, s_max[w]);
+                    fx_add(cs, s_sum[w]);
+                }
+                atomicMin(A.kmin + k, cm);
+                atomicMax(A.kmax + k, cx);
+                fx_red3(A.vsum + 3 * (size_t)k, cs);
                 __threadfence();
-                for (int b = threadIdx.x; b < bins; b += CALIB_THREADS) {
-                    s_bsum[b] = fx_to_double(fx_load_cg(A.bsum + (size_t)k * bins + b));
-                    s_cnt[b] = __ldcg(A.bcnt + (size_t)k * bins + b);
-                }
-                __syncthreads();
-                __syncthreads();
-                // populated bins, then each thin bin from its nearest populated one, left first
-                // (one thread a bin: the fill reads only populated bins)
-                const unsigned mc = (unsigned)A.min_count;
-                for (int b = threadIdx.x; b < bins; b += CALIB_THREADS) {
-                    double mv = s_bc[2];
-                    if (s_cnt[b] >= mc) {
-                        mv = s_bsum[b] / s_cnt[b];
-                    } else {
-                        for (int d = 1; d < bins; d++) {
-                            if (b - d >= 0 && s_cnt[b - d] >= mc) {
-                                mv = s_bsum[b - d] / s_cnt[b - d];
-                                break;
-                            }
-                            if (b + d < bins && s_cnt[b + d] >= mc) {
-                                mv = s_bsum[b + d] / s_cnt[b + d];
-                                break;
-                            }
-                        }
+            }
+        }
+        arrive();
+        // ---- behind round A: the Gaussians of the step into date k in draw order (the variance's
+        // first) and the generator's jump ----
+        if (k > 0 && P > 0)
+            for (int it = 0; it < R; ++it, tog ^= 1) {
+                const int p = gt + it * T;
+                const bool act = p < P;
+                bool tail1 = false, tail2 = false;
+                if (act) {
+                    if (!ONE)
+                        for (int w = 0; w < 4; w++) q.s[w] = A.rng[(size_t)w * P + p];
+                    const double u1 = uniform53(q.s), u2 = uniform53(q.s);
+                    tail1 = in_tail(u1);
+                    tail2 = in_tail(u2);
+                    if (tail1) {
+                        const int o = atomicAdd(&s_qn[tog], 1);
+                        s_qu[o] = u1;
+                        s_qi[o] = (unsigned short)(2 * t);
                     }
-                    s_mean[b] = mv;
+                    if (tail2) {
+                        const int o = atomicAdd(&s_qn[tog], 1);
+                        s_qu[o] = u2;
+                        s_qi[o] = (unsigned short)(2 * t + 1);
+                    }
+                    q.z1 = gauss_central(u1);
+                    q.z2 = gauss_central(u2);
                 }
                 __syncthreads();
-                build_layer(A, k, false, s_bc[2], bmn + 0.5 * width, width, s_mean);
+                // the CTA's tail draws, a dozen of 256: one warp's work while the others go on
+                for (int o = t; o < s_qn[tog]; o += CALIB_THREADS) s_z[s_qi[o]] = gauss_tail(s_qu[o]);
+                if (t == 0) s_qn[tog ^ 1] = 0;
+                if (act) xo_jump_tab(s_jtab, q.s);
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    __threadfence();
-                    st_release(A.done, round);
+                if (tail1) q.z1 = s_z[2 * t];
+                if (tail2) q.z2 = s_z[2 * t + 1];
+                if (!ONE && act) {
+                    for (int w = 0; w < 4; w++) A.rng[(size_t)w * P + p] = q.s[w];
+                    A.z1[p] = q.z1;
+                    A.z2[p] = q.z2;
                 }
-            } else if (threadIdx.x == 0) {
-                s_ok = wait_for(A.done, round, A.status);
+            }
+        __syncthreads(); // the Gaussians are read: the arrays below are theirs
+        for (int b = t; b < CALIB_MAX_BINS; b += CALIB_THREADS) {
+            s_cnt[b] = 0;
+            s_blo[b] = 0; // or limbs 0..3
+            s_bhi[b] = 0;
+            s_l4[b] = 0;
+        }
+        // one thread a warp forms its share of the round's results: the bins' origin and width; their
+        // reciprocal; the layer's points around the ensemble (below the lowest, above the highest);
+        // the ensemble's mean
+        if (lane == 0) {
+            const bool ok = wait_for(A.bar, round * (unsigned)G, A.status);
+            if (ok && warp == 1) {
+                s_bc[3] = fx_to_double(fx_load3(A.vsum + 3 * (size_t)k)) * A.rP;
+            } else if (ok) {
+                const double gmn = from_key((long long)__ldcg((const unsigned long long*)(A.kmin + k)));
+                const double gmx = from_key((long long)__ldcg((const unsigned long long*)(A.kmax + k)));
+                if (warp == 0) {
+                    s_bc[0] = gmn;
+                    s_bc[1] = (gmx - gmn) * A.rbins;
+                    s_ok = gmx - gmn < 1e-10 ? 2 : 1;
+                } else if (warp == 2) {
+                    s_bc[2] = 1.0 / ((gmx - gmn) * A.rbins);
+                } else {
+                    const double off = (double)A.offset[k], top = (double)A.points;
+                    s_min[0] = (long long)fmin(fmax(floor(fma(gmn, A.rln_step[k], -off)) - 1.0, 0.0), top - 1.0);
+                    s_max[0] = (long long)fmin(fmax(floor(fma(gmx, A.rln_step[k], -off)) + 3.0, 1.0), top);
+                }
+            } else if (warp == 0) {
+                s_ok = 0;
+            }
+        }
+        __syncthreads();
+        if (!s_ok) return;
+        const bool flat = s_ok == 2;
+        const double bmn = s_bc[0], width = s_bc[1], rwidth = s_bc[2], fallback = s_bc[3];
+        // the layer's points this CTA needs: those around the ensemble, or all to write out
+        const int i0 = writes ? 0 : (int)s_min[0];
+        const int i1 = writes ? A.points : (int)s_max[0];
+
+        if (!flat) {
+            // ---- round B: per-bin counts and sums of v ----
+            if (P > 0) {
+                for (int p = gt; p < P; p += T) {
+                    if (!ONE) {
+                        q.lns = A.lns[p];
+                        q.var = A.var[p];
+                    }
+                    int b = (int)((q.lns - bmn) * rwidth);
+                    b = b < 0 ? 0 : (b > bins - 1 ? bins - 1 : b);
+                    uint64_t lo, hi;
+                    fx_words(q.var, lo, hi, bad);
+                    atomicAdd(&s_cnt[b], 1u);
+                    if (ONE) {
+#pragma unroll
+                        for (int i = 0; i < BIN_LIMBS; i++)
+                            atomicAdd(i < 4 ? s_l0 + i * CALIB_MAX_BINS + b : s_l4 + b, (unsigned)limb_bits(lo, hi, i));
+                    } else {
+                        const unsigned long long old = atomicAdd(&s_blo[b], (unsigned long long)lo);
+                        atomicAdd(&s_bhi[b], (unsigned long long)(hi + ((uint64_t)old + lo < lo ? 1u : 0u)));
+                    }
+                }
+                __syncthreads();
+                for (int b = t; b < bins; b += CALIB_THREADS)
+                    if (s_cnt[b]) {
+                        atomicAdd(A.bcnt + (size_t)k * bins + b, s_cnt[b]);
+                        Fx128 v = {0, 0};
+                        if (ONE) {
+                            for (int i = 0; i < BIN_LIMBS; i++) {
+                                const uint64_t w = i < 4 ? s_l0[i * CALIB_MAX_BINS + b] : s_l4[b];
+                                const int sh = 20 * i;
+                                if (sh >= 64) fx_add(v, 0, w << (sh - 64));
+                                else fx_add(v, w << sh, sh ? w >> (64 - sh) : 0);
+                            }
+                        } else {
+                            v = Fx128{s_blo[b], s_bhi[b]};
+                        }
+                        fx_red3(A.bsum + 3 * ((size_t)k * bins + b), v);
+                        __threadfence();
+                    }
+                if (bad) atomicExch(A.status, 3);
             }
             __syncthreads();
-            if (!s_last && !s_ok) return;
+            arrive();
         }
+        // ---- behind round B: the variance step and the log-spot step's parts ----
+        const CalibStep C = A.steps[k];
+        if (k > 0)
+            for (int p = gt; p < P; p += T) {
+                if (!ONE) {
+                    q.var = A.var[p];
+                    q.z1 = A.z1[p];
+                    q.z2 = A.z2[p];
+                }
+                q.vc = qe_step(q.var, q.z1, C, A.phi);
+                spot_parts(q.var, q.vc, q.z2, C, q.sb, q.sd);
+                if (!ONE) {
+                    A.vc[p] = q.vc;
+                    A.sb[p] = q.sb;
+                    A.sd[p] = q.sd;
+                }
+            }
+        if (!flat) {
+            // the layer's points on the bins' grid
+            const double x0 = fma(0.5, width, bmn), ls = A.ln_step[k];
+            const int64_t off = A.offset[k];
+            for (int i = i0 + t; i < i1; i += CALIB_THREADS) s_layer[i] = ((double)(off + i) * ls - x0) * rwidth;
+            if (t == 0) s_ok = wait_for(A.bar, round * (unsigned)G, A.status);
+            __syncthreads();
+            if (!s_ok) return;
+            for (int b = t; b < bins; b += CALIB_THREADS) {
+                s_bsum[b] = fx_to_double(fx_load3(A.bsum + 3 * ((size_t)k * bins + b)));
+                s_cnt[b] = __ldcg(A.bcnt + (size_t)k * bins + b);
+            }
+            __syncthreads();
+            // populated bins, then each thin bin from its nearest populated one, left first
+            // (one thread a bin: the fill reads only populated bins)
+            const unsigned mc = (unsigned)A.min_count;
+            for (int b = t; b < bins; b += CALIB_THREADS) {
+                int from = s_cnt[b] >= mc ? b : -1;
+                for (int d = 1; d < bins && from < 0; d++) {
+                    if (b - d >= 0 && s_cnt[b - d] >= mc) from = b - d;
+                    else if (b + d < bins && s_cnt[b + d] >= mc) from = b + d;
+                }
+                s_mean[b] = from >= 0 ? s_bsum[from] / s_cnt[from] : fallback;
+            }
+            __syncthreads();
+        }
+        // ---- layer k from the conditional variance of the bins (the same in every CTA) ----
+        for (int i = i0 + t; i < i1; i += CALIB_THREADS) {
+            double ev = fallback;
+            if (!flat) {
+                // linear between bin centres, the outer bins' means beyond them
+                const double f = fmin(fmax(s_layer[i], 0.0), (double)(bins - 1));
+                const int j = min((int)f, max(bins - 2, 0));
+                const double m0 = s_mean[j];
+                ev = fma(f - (double)j, s_mean[min(j + 1, bins - 1)] - m0, m0);
+            }
+            if (ev < A.min_cv) ev = A.min_cv;
+            double L = A.local_vol[(size_t)k * A.points + i] * rsqrt(ev);
+            L = L < A.lmin ? A.lmin : (L > A.lmax ? A.lmax : L);
+            s_layer[i] = L;
+            if (writes) A.lev[(size_t)k * A.points + i] = L;
+        }
+        __syncthreads();
         if (k == 0) continue;
 
         // ---- the step into date k with layer k ----
-        for (int i = threadIdx.x; i < A.points; i += CALIB_THREADS) s_layer[i] = __ldcg(A.lev + (size_t)k * A.points + i);
-        __syncthreads();
-        const double dt = A.dt[k], carry = A.carry[k], e = A.qe_e[k], ls = A.ln_step[k];
-        const int64_t off = A.offset[k];
+        const double rls = A.rln_step[k], f0 = A.f0[k];
         for (int p = gt; p < P; p += T) {
-            uint64_t s[4];
-            for (int w = 0; w < 4; w++) s[w] = A.rng[(size_t)w * P + p];
-            // both Gaussians in draw order (the variance's first) and the layer lookup before
-            // the branched QE step: three independent chains in one block
-            const double z1 = gaussian(s);
-            const double z2 = gaussian(s);
-            const double lp = layer_at(s_layer, A.points, ls, off, A.spot[p]);
-            const double vp = A.var[p];
-            const double vc = qe_step(vp, z1, e, A);
-            const double step = spot_step(vp, vc, dt, carry, lp, z2, A);
-            A.var[p] = vc;
-            A.spot[p] *= exp(step);
-            A.lns[p] += step;
-            xo_jump_tab(s_jtab, s);
-            for (int w = 0; w < 4; w++) A.rng[(size_t)w * P + p] = s[w];
+            if (!ONE) {
+                q.x = A.x[p];
+                q.lns = A.lns[p];
+                q.vc = A.vc[p];
+                q.sb = A.sb[p];
+                q.sd = A.sd[p];
+            }
+            const double L = layer_at(s_layer, A.points, fma(q.x, rls, f0));
+            const double step = fma(-L * L, q.sd, fma(L, q.sb, C.carry));
+            q.var = q.vc;
+            q.x += step;
+            q.lns += step;
+            if (!ONE) {
+                A.var[p] = q.var;
+                A.x[p] = q.x;
+                A.lns[p] = q.lns;
+            }
         }
-        __syncthreads();
     }
 }
 
@@ -593,35 +741,6 @@ struct TailSeed {
 constexpr int TAIL_THREADS = 128;
 constexpr int TAIL_WARPS = TAIL_THREADS / 32;
 constexpr int TAIL_PATHS_PER_THREAD = 16;
-constexpr double ACKLAM_P_LOW = 0.02425;
-
-// normal_cdf_inv's two branches apart, each the same expression the reference evaluates there
-__device__ __forceinline__ double acklam_central(double P) // P in [p_low, 1 - p_low]
-{
-    const double a0 = -3.969683028665376e+01, a1 = 2.209460984245205e+02, a2 = -2.759285104469687e+02,
-                 a3 = 1.383577518672690e+02, a4 = -3.066479806614716e+01, a5 = 2.506628277459239e+00;
-    const double b0 = -5.447609879822406e+01, b1 = 1.615858368580409e+02, b2 = -1.556989798598866e+02,
-                 b3 = 6.680131188771972e+01, b4 = -1.328068155288572e+01;
-    const double q = P - 0.5;
-    const double r = q * q;
-    const double cn = (((((a0 * r + a1) * r + a2) * r + a3) * r + a4) * r + a5) * q;
-    const double cd = ((((b0 * r + b1) * r + b2) * r + b3) * r + b4) * r + 1.0;
-    return cn / cd;
-}
-
-__device__ __forceinline__ double acklam_tail(double P) // P < p_low or P > 1 - p_low
-{
-    const double c0 = -7.784894002430293e-03, c1 = -3.223964580411365e-01, c2 = -2.400758277161838e+00,
-                 c3 = -2.549732539343734e+00, c4 = 4.374664141464968e+00, c5 = 2.938163982698783e+00;
-    const double d0 = 7.784695709041462e-03, d1 = 3.224671290700398e-01, d2 = 2.445134137142996e+00,
-                 d3 = 3.754408661907416e+00;
-    const bool lower = P < ACKLAM_P_LOW;
-    const double qt = sqrt(-2.0 * log(lower ? P : 1.0 - P));
-    const double tn = ((((c0 * qt + c1) * qt + c2) * qt + c3) * qt + c4) * qt + c5;
-    const double td = (((d0 * qt + d1) * qt + d2) * qt + d3) * qt + 1.0;
-    return (lower ? tn : -tn) / td;
-}
-
 // thread k draws the tail Gaussians of paths [16 k, 16 k + 16): one jump to its first path's
 // place in the stream (p dt draws in: the binary powers of x), then its paths' draws in stream
 // order, as the reference's NextPath draws them. A draw in the central region is inverted at
@@ -748,18 +867,23 @@ void xo_jump_table(const uint64_t poly[4], uint64_t* tab)
 
 int calib_max_grid(int sms, size_t smem)
 {
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lsv_calib_kernel, CALIB_THREADS, smem) != cudaSuccess)
+    int per = 0, per1 = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lsv_calib_kernel<false>, CALIB_THREADS, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, lsv_calib_kernel<true>, CALIB_THREADS, smem) != cudaSuccess)
         return 0;
-    return per * sms;
+    return (per < per1 ? per : per1) * sms;
 }
 
-cudaError_t launch_calib(const CalibArgs& A, int grid, size_t smem, cudaStream_t st)
+cudaError_t launch_calib(const CalibArgs& A, int grid, int cap, size_t smem, cudaStream_t st)
 {
+    // one more CTA, without particles, writes the layers out where the device has room for it
     CalibArgs a = A;
-    void* args[] = {&a};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lsv_calib_kernel), dim3(grid),
-                                       dim3(CALIB_THREADS), args, smem, st);
+    int G = grid;
+    if (grid < cap) ++grid;
+    a.writer = grid - 1;
+    void* args[] = {&a, &G};
+    auto k = (int64_t)G * CALIB_THREADS >= A.P ? lsv_calib_kernel<true> : lsv_calib_kernel<false>;
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(grid), dim3(CALIB_THREADS), args, smem, st);
 }
 
 cudaError_t tail_normals_prepare()

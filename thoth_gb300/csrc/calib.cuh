@@ -11,18 +11,31 @@ constexpr int CALIB_THREADS = 128;
 constexpr int CALIB_MAX_BINS = 128;
 constexpr int CALIB_JUMP_BITS = 40; // x^(2^i) mod chi for i < 40: particle offsets below 2^40
 
+// Date constants of one step, rounded from FP64 expressions on the host. Variance (QE, Andersen):
+// m = th + (v - theta) e as fma(v, e, th1e), s2 = fma(v, qa, qb). Log-spot with leverage L:
+// step = carry + L (k0 + a1 s + r (vc - v) + sqrt(k3 s) z) - L^2 a2 s, s = v + vc; for a vanishing
+// vol of vol (flat != 0) step = carry + L sqrt(v dt) z - L^2 v dt / 2.
+struct CalibStep {
+    double e, th1e, qa, qb, carry, k0, a1, a2, k3, r, dt, flat;
+};
+
 struct CalibArgs {
     int P, n, points, bins, min_count;
-    double s0, ln_s0, v0, kappa, theta, xi, rho, min_cv, lmin, lmax;
-    const double* dt;        // [n] year fraction of the step into date k (dt[0] unused)
-    const double* carry;     // [n] cumulative carry of date k minus date k-1
-    const double* qe_e;      // [n] exp(-kappa dt[k]), rounded on the host like the reference
+    double ln_s0, v0, min_cv, lmin, lmax;
+    double rP, rbins;        // 1 / P, 1 / bins
+    const CalibStep* steps;  // [n] constants of the step into date k (steps[0] unused)
     const double* ln_step;   // [n]
+    const double* f0;        // [n] ln S0 / ln_step - offset: the grid coordinate of ln S - ln S0 = 0
+    const double* rln_step;  // [n] 1 / ln_step
     const int64_t* offset;   // [n]
     const double* local_vol; // [n][points]
     double* lev;             // [n][points] out
-    double *spot, *var, *lns; // [P] the ensemble
-    uint64_t* rng;           // [4][P] each particle's Rng state
+    // the ensemble where a thread has several particles (else it is in registers): ln S - ln S0,
+    // variance, ln S, the date's two Gaussians, next variance, the step's two parts; the Rng states
+    // [4][P]
+    double *x, *var, *lns, *z1, *z2, *vc, *sb, *sd;
+    uint64_t* rng;
+    int writer;              // the CTA that writes the layers out
     const uint64_t* jpow;    // [CALIB_JUMP_BITS][4] x^(2^i) mod chi
     // the jump from a particle's draws of one date to the next (2P - 2 draws) as a nibble
     // table of its GF(2) matrix: jtab[(n 16 + v) 4 + w] = word w of the jump of the state
@@ -32,18 +45,19 @@ struct CalibArgs {
     // per-date totals the CTAs add into with integer atomics (order-independent, exact):
     long long *kmin, *kmax;  // [n] order-preserving integer keys of the extremes of ln S
                              // (initialised to 0x7f.. / 0x80.. bytes: neutral for min / max)
-    Fx128* vsum;             // [n] sum of v (zero at launch)
+    unsigned long long* vsum; // [n][3] sum of v, in limbs (zero at launch)
     unsigned* bcnt;          // [n][bins] particles per bin (zero at launch)
-    Fx128* bsum;             // [n][bins] sum of v per bin (zero at launch)
-    double* bc;              // [4] published: min ln S, bin width, ensemble mean of v, degenerate
-    unsigned *bar, *done;    // arrivals and releases, all rounds (zero at launch)
+    unsigned long long* bsum; // [n][bins][3] sum of v per bin (zero at launch)
+    const double* phi;       // the normal distribution's table (phi.cuh)
+    unsigned* bar;           // arrivals, all rounds (zero at launch)
     int* status;             // 0 ok, 2 a wait timed out, 3 a sum out of range
 };
 
 constexpr size_t CALIB_JTAB_WORDS = 64 * 16 * 4;
 
 int calib_max_grid(int sms, size_t smem);
-cudaError_t launch_calib(const CalibArgs& A, int grid, size_t smem, cudaStream_t st);
+// grid CTAs for the particles, of at most cap resident ones
+cudaError_t launch_calib(const CalibArgs& A, int grid, int cap, size_t smem, cudaStream_t st);
 
 // host: the reference Rng's transition, seeding, and jump polynomials
 void xo_seed_state(uint64_t seed, uint64_t s[4]);

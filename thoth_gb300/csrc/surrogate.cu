@@ -2,6 +2,7 @@
 // surrogate: a validation GEMM, the fused MLP inference kernel, the training
 // tile (forward, head, backward for inputs and weights) and Adam.
 #include "engine.cuh"
+#include "phi.cuh"
 #include "tc.cuh"
 
 #include <cuda_bf16.h>
@@ -722,11 +723,6 @@ constexpr int INFER_LATTICE_THREADS = INFER_MAIN + ROWS; // and the scale's
 constexpr uint32_t INFER_TMEM_COLS = 512;      // a power of two >= 128 x INFER_TILES
 constexpr int MAX_MEMBERS = 64;
 
-// Phi(x) by its Taylor polynomials about x0 = k / 8: Phi(x0) + phi(x0) sum_n (-1)^(n-1)
-// He_(n-1)(x0) h^n / n!, |h| <= 1/16, He the Hermite polynomials. Ten coefficients leave less than
-// 2.3e-16 anywhere; beyond +-69/8 Phi is 0 or 1 to 1e-17.
-constexpr int PHI_NODES = 139, PHI_COEF = 10, PHI_MID = 69;
-
 struct LatticeTables {
     const uint32_t* f_lm;  // [n_lm] feature words (bf16 hi, lo << 16), clipped and normalised
     const uint32_t* f_T;   // [n_T]
@@ -755,20 +751,6 @@ __device__ __forceinline__ uint32_t feature_word(float v)
 {
     const __nv_bfloat16 h = __float2bfloat16(v), l = __float2bfloat16(v - __bfloat162float(h));
     return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
-}
-
-__device__ __forceinline__ double phi_table(const double* tab, double x)
-{
-    const double u = fmin(fmax(x, -8.625), 8.625);
-    const int k = __double2int_rn(u * 8.0);
-    const double h = fma((double)k, -0.125, u); // exact
-    const double2* c = reinterpret_cast<const double2*>(tab + (k + PHI_MID) * PHI_COEF);
-    double p = c[4].y;
-#pragma unroll
-    for (int i = 4; i >= 0; --i) {
-        p = i == 4 ? fma(p, h, c[4].x) : fma(fma(p, h, c[i].y), h, c[i].x);
-    }
-    return x == x ? p : x;
 }
 
 template <bool LATTICE>
@@ -1112,14 +1094,14 @@ cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// Phi's Taylor coefficients about the nodes k / 8 (mlp::phi_table)
+// Phi's Taylor coefficients about the nodes k / 8 (phi.cuh)
 void phi_coefficients(double* out)
 {
-    for (int k = -mlp::PHI_MID; k <= mlp::PHI_MID; ++k, out += mlp::PHI_COEF) {
+    for (int k = -PHI_MID; k <= PHI_MID; ++k, out += PHI_COEF) {
         const double x = k / 8.0, phi = std::exp(-0.5 * x * x) / std::sqrt(2.0 * 3.14159265358979323846);
         double he0 = 1.0, he1 = x, f = 1.0; // He_0, He_1; n!
         out[0] = 0.5 * std::erfc(-x / std::sqrt(2.0));
-        for (int n = 1; n < mlp::PHI_COEF; ++n) {
+        for (int n = 1; n < PHI_COEF; ++n) {
             f *= n;
             out[n] = (n % 2 ? phi : -phi) * he0 / f;
             const double he2 = x * he1 - n * he0;
@@ -1128,8 +1110,6 @@ void phi_coefficients(double* out)
         }
     }
 }
-
-int phi_size() { return mlp::PHI_NODES * mlp::PHI_COEF; }
 
 cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st)
 {

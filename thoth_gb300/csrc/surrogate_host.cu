@@ -2,6 +2,7 @@
 // SiLU -> 1 MLP trained and served by the tcgen05 kernels of surrogate.cu.
 // No reference counterpart: the reference has no learned pricer.
 #include "thoth_gpu.h"
+#include "phi.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -74,8 +75,6 @@ struct LatticeArgs {
     double2 *set_T, *lm;
 };
 cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st);
-void phi_coefficients(double* out);
-int phi_size();
 cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st);
 } // namespace thoth
 
@@ -652,7 +651,7 @@ int thoth_gpu_surrogate_price_lattice_mean(ThothSurrogate* const* members, int32
         // [inputs: sets, axes, Phi's table][feature words][per set and maturity][per log-moneyness]
         // [outputs][scales][prices]
         auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-        const size_t n_par = (size_t)n_sets * 5, n_in = n_par + n_lm + n_T + phi_size();
+        const size_t n_par = (size_t)n_sets * 5, n_in = n_par + n_lm + n_T + PHI_NODES * PHI_COEF;
         size_t off = 0;
         auto take = [&](size_t bytes) {
             const size_t o = off;

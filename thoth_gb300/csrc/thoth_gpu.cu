@@ -9,6 +9,7 @@
 #include "engine.cuh"
 #include "american.cuh"
 #include "calib.cuh"
+#include "phi.cuh"
 
 #include <cuda_runtime.h>
 
@@ -2421,11 +2422,30 @@ int calibrate_locked(ThothLeverageCalib* c)
         if (!(c->ln_step[k] > 0)) return fail(THOTH_GPU_E_INVALID, "layer grid spacing must be positive");
     int rc = ensure_device();
     if (rc) return rc;
-    std::vector<double> dt(n, 0.0), carry(n, 0.0), qe(n, 1.0);
+    const double ln_s0 = std::log(c->spot);
+    std::vector<double> f0(n), rls(n);
+    std::vector<CalibStep> steps(n);
+    for (int k = 0; k < n; k++) {
+        rls[k] = 1.0 / c->ln_step[k];
+        f0[k] = ln_s0 / c->ln_step[k] - (double)c->offset[k];
+    }
     for (int k = 1; k < n; k++) {
-        dt[k] = (double)(c->days[k] - c->days[k - 1]) / 365.0;
-        carry[k] = c->carry[k] * ((double)c->days[k] / 365.0) - c->carry[k - 1] * ((double)c->days[k - 1] / 365.0);
-        qe[k] = std::exp(-c->kappa * dt[k]);
+        CalibStep& S = steps[k];
+        const double g = 0.5;
+        S.dt = (double)(c->days[k] - c->days[k - 1]) / 365.0;
+        S.carry = c->carry[k] * ((double)c->days[k] / 365.0) - c->carry[k - 1] * ((double)c->days[k - 1] / 365.0);
+        S.e = std::exp(-c->kappa * S.dt);
+        S.th1e = c->theta * (1 - S.e);
+        S.qa = c->xi * c->xi * S.e / c->kappa * (1 - S.e);
+        S.qb = c->theta * c->xi * c->xi / (2 * c->kappa) * (1 - S.e) * (1 - S.e);
+        S.flat = c->xi > 1e-12 ? 0.0 : 1.0;
+        if (c->xi > 1e-12) {
+            S.k0 = -c->rho * c->kappa * c->theta / c->xi * S.dt;
+            S.a1 = g * S.dt * c->kappa * c->rho / c->xi;
+            S.a2 = g * S.dt * 0.5;
+            S.k3 = g * S.dt * (1.0 - c->rho * c->rho);
+            S.r = c->rho / c->xi;
+        }
     }
     uint64_t jpow[CALIB_JUMP_BITS][4], jdate[4];
     for (int i = 0; i < CALIB_JUMP_BITS; i++)
@@ -2437,6 +2457,7 @@ int calibrate_locked(ThothLeverageCalib* c)
     const int cap = calib_max_grid(g_dev.sms, smem);
     if (cap < 1) return fail(THOTH_GPU_E_TOO_LARGE, "layer too large for shared memory");
     const int grid = std::max(1, std::min(cap, (P + CALIB_THREADS - 1) / CALIB_THREADS));
+    const bool several = (int64_t)grid * CALIB_THREADS < P; // particles a thread: the ensemble in memory
     // device layout: inputs | layers | ensemble | generators | partial sums | control
     const size_t nd = (size_t)n, np = (size_t)P, npt = (size_t)pts;
     size_t o = 0;
@@ -2445,16 +2466,15 @@ int calibrate_locked(ThothLeverageCalib* c)
         o = align256(o + bytes);
         return at;
     };
-    const size_t o_dt = take(8 * nd), o_carry = take(8 * nd), o_qe = take(8 * nd), o_ls = take(8 * nd);
+    const size_t o_steps = take(sizeof(CalibStep) * nd), o_ls = take(8 * nd), o_f0 = take(8 * nd), o_rls = take(8 * nd);
     const size_t o_off = take(8 * nd), o_lv = take(8 * nd * npt), o_jp = take(8 * 4 * CALIB_JUMP_BITS),
-                 o_jt = take(8 * CALIB_JTAB_WORDS);
+                 o_jt = take(8 * CALIB_JTAB_WORDS), o_phi = take(8 * PHI_NODES * PHI_COEF);
     const size_t up_bytes = o; // everything above is uploaded in one copy
-    const size_t o_lev = take(8 * nd * npt), o_spot = take(8 * np), o_var = take(8 * np), o_lns = take(8 * np);
-    const size_t o_rng = take(8 * 4 * np), o_bc = take(8 * 4);
+    const size_t o_lev = take(8 * nd * npt), o_ens = take(several ? 8 * 12 * np : 0);
     // per-date totals: zeroed (sums, counts, control) or set to the neutral keys (extremes)
     const size_t o_kmin = take(8 * nd), o_kmax = take(8 * nd);
-    const size_t o_zero = o, o_vsum = take(sizeof(Fx128) * nd), o_bcnt = take(4 * nd * (size_t)bins);
-    const size_t o_bsum = take(sizeof(Fx128) * nd * (size_t)bins), o_ctl = take(16);
+    const size_t o_zero = o, o_vsum = take(24 * nd), o_bcnt = take(4 * nd * (size_t)bins);
+    const size_t o_bsum = take(24 * nd * (size_t)bins), o_ctl = take(16);
     if (o > g_dev.calib_size) {
         if (g_dev.calib) cudaFree(g_dev.calib);
         g_dev.calib = nullptr;
@@ -2466,14 +2486,15 @@ int calibrate_locked(ThothLeverageCalib* c)
     if (rc) return rc;
     unsigned char* h = g_dev.pinned;
     std::memset(h, 0, up_bytes);
-    std::memcpy(h + o_dt, dt.data(), 8 * nd);
-    std::memcpy(h + o_carry, carry.data(), 8 * nd);
-    std::memcpy(h + o_qe, qe.data(), 8 * nd);
+    std::memcpy(h + o_steps, steps.data(), sizeof(CalibStep) * nd);
     std::memcpy(h + o_ls, c->ln_step, 8 * nd);
+    std::memcpy(h + o_f0, f0.data(), 8 * nd);
+    std::memcpy(h + o_rls, rls.data(), 8 * nd);
     std::memcpy(h + o_off, c->offset, 8 * nd);
     std::memcpy(h + o_lv, c->local_vol, 8 * nd * npt);
     std::memcpy(h + o_jp, jpow, sizeof jpow);
     std::memcpy(h + o_jt, jtab.data(), 8 * CALIB_JTAB_WORDS);
+    phi_coefficients(reinterpret_cast<double*>(h + o_phi));
     unsigned char* base = g_dev.calib;
     cudaStream_t st = g_dev.stream;
     CUDA_TRY(cudaMemcpyAsync(base, h, up_bytes, cudaMemcpyHostToDevice, st));
@@ -2486,42 +2507,41 @@ int calibrate_locked(ThothLeverageCalib* c)
     A.points = pts;
     A.bins = bins;
     A.min_count = min_count;
-    A.s0 = c->spot;
-    A.ln_s0 = std::log(c->spot);
+    A.ln_s0 = ln_s0;
     A.v0 = c->v0;
-    A.kappa = c->kappa;
-    A.theta = c->theta;
-    A.xi = c->xi;
-    A.rho = c->rho;
+    A.rP = 1.0 / (double)P;
+    A.rbins = 1.0 / (double)bins;
     A.min_cv = c->min_cond_variance > 0 ? c->min_cond_variance : 1e-6;
     A.lmin = c->lev_min > 0 ? c->lev_min : 0.05;
     A.lmax = c->lev_max > 0 ? c->lev_max : 10.0;
-    A.dt = reinterpret_cast<const double*>(base + o_dt);
-    A.carry = reinterpret_cast<const double*>(base + o_carry);
-    A.qe_e = reinterpret_cast<const double*>(base + o_qe);
+    A.steps = reinterpret_cast<const CalibStep*>(base + o_steps);
+    A.f0 = reinterpret_cast<const double*>(base + o_f0);
     A.ln_step = reinterpret_cast<const double*>(base + o_ls);
     A.offset = reinterpret_cast<const int64_t*>(base + o_off);
     A.local_vol = reinterpret_cast<const double*>(base + o_lv);
     A.lev = reinterpret_cast<double*>(base + o_lev);
-    A.spot = reinterpret_cast<double*>(base + o_spot);
-    A.var = reinterpret_cast<double*>(base + o_var);
-    A.lns = reinterpret_cast<double*>(base + o_lns);
-    A.rng = reinterpret_cast<uint64_t*>(base + o_rng);
+    A.rln_step = reinterpret_cast<const double*>(base + o_rls);
+    double* ens = reinterpret_cast<double*>(base + o_ens); // several only
+    double** arr[] = {&A.x, &A.var, &A.lns, &A.z1, &A.z2, &A.vc, &A.sb, &A.sd};
+    for (double** v : arr) {
+        *v = ens;
+        ens += np;
+    }
+    A.rng = reinterpret_cast<uint64_t*>(ens);
     A.jpow = reinterpret_cast<const uint64_t*>(base + o_jp);
     A.jtab = reinterpret_cast<const uint64_t*>(base + o_jt);
     xo_seed_state(c->seed, A.seed_state);
     A.kmin = reinterpret_cast<long long*>(base + o_kmin);
     A.kmax = reinterpret_cast<long long*>(base + o_kmax);
-    A.vsum = reinterpret_cast<Fx128*>(base + o_vsum);
+    A.vsum = reinterpret_cast<unsigned long long*>(base + o_vsum);
     A.bcnt = reinterpret_cast<unsigned*>(base + o_bcnt);
-    A.bsum = reinterpret_cast<Fx128*>(base + o_bsum);
-    A.bc = reinterpret_cast<double*>(base + o_bc);
+    A.bsum = reinterpret_cast<unsigned long long*>(base + o_bsum);
+    A.phi = reinterpret_cast<const double*>(base + o_phi);
     A.bar = reinterpret_cast<unsigned*>(base + o_ctl);
-    A.done = reinterpret_cast<unsigned*>(base + o_ctl + 4);
     A.status = reinterpret_cast<int*>(base + o_ctl + 8);
     A.min_count = min_count;
     CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
-    CUDA_TRY(launch_calib(A, grid, smem, st));
+    CUDA_TRY(launch_calib(A, grid, cap, smem, st));
     CUDA_TRY(cudaEventRecord(g_dev.ev1, st));
     CUDA_TRY(cudaMemcpyAsync(h, base + o_lev, 8 * nd * npt, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(h + 8 * nd * npt, base + o_ctl + 8, sizeof(int), cudaMemcpyDeviceToHost, st));
