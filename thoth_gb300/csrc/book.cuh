@@ -25,6 +25,7 @@ struct Smem {
     float* fa;      // few-product mode: [few_m][T] per-thread FP32 moment sums since the last flush
     float* fw;      // few-product mode: [T / 32][few_m][2] per-warp Kahan (sum, compensation)
     float* fshift;  // few-product mode: [few_m / 2] the CTA's shift of each quantity
+    unsigned char* end;
 };
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -90,7 +91,9 @@ __device__ inline Smem carve(unsigned char* base, const DevPlan& P, int T)
         s.fw = reinterpret_cast<float*>(base + o);
         o += align16(sizeof(float) * 2 * (size_t)P.few_m * (T / 32));
         s.fshift = reinterpret_cast<float*>(base + o);
+        o += align16(sizeof(float) * (size_t)(P.few_m / 2));
     }
+    s.end = base + o;
     return s;
 }
 
@@ -114,17 +117,38 @@ __device__ inline Smem carve(unsigned char* base, const DevPlan& P, int T)
 // hs[j] ^ V[d][TB-1] ^ V[d][TB-2]: a thread with two paths (columns t and
 // t + T/2) reads one low word per entry, and one 8-byte broadcast of the pair.
 // ---------------------------------------------------------------------------
-template <int TB>
+// WIDE: a lone tile's first chunk waits for its direction numbers, so they are loaded four at a
+// time and all together (one after the other, every set bit of the tile index cost a round trip);
+// elsewhere other CTAs cover the wait, and the narrow form's registers are worth more.
+template <int TB, bool WIDE = false>
 __device__ inline void tile_high_bits(const DevPlan& P, uint2* hs, int64_t m, int j0)
 {
     const uint64_t g = (uint64_t)m ^ ((uint64_t)m >> 1);
     const int j1 = min(j0 + HS_CHUNK, P.n_sobol);
     for (int j = j0 + (int)threadIdx.x; j < j1; j += blockDim.x) {
         const uint32_t* V = P.sobol_v + __ldg(P.sobol_order + j) * SOBOL_BITS;
-        uint32_t acc = (m & 1) ? __ldg(V + TB - 1) : 0u;
-        uint64_t gg = g;
-        for (int k = 0; gg != 0 && k < SOBOL_BITS - TB; ++k, gg >>= 1)
-            if (gg & 1u) acc ^= __ldg(V + TB + k);
+        uint32_t acc;
+        if constexpr (WIDE) {
+            const uint4* V4 = reinterpret_cast<const uint4*>(V); // rows of 32 words
+            acc = (m & 1) ? __ldg(V + TB - 1) : 0u;
+            const uint32_t gb = (uint32_t)g;
+            const int nb = 32 - __clz(gb);
+#pragma unroll
+            for (int q = 0; q < (SOBOL_BITS - TB + 3) / 4; ++q)
+                if (4 * q < nb + TB % 4) {
+                    const uint4 v = __ldg(V4 + TB / 4 + q);
+                    const int k = 4 * q - TB % 4; // Gray bit of v.x
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (k + i >= 0) acc ^= (0u - ((gb >> (k + i)) & 1u)) & w[i];
+                }
+        } else {
+            acc = (m & 1) ? __ldg(V + TB - 1) : 0u;
+            uint64_t gg = g;
+            for (int k = 0; gg != 0 && k < SOBOL_BITS - TB; ++k, gg >>= 1)
+                if (gg & 1u) acc ^= __ldg(V + TB + k);
+        }
         hs[j - j0] = make_uint2(acc, acc ^ __ldg(V + TB - 1) ^ __ldg(V + TB - 2));
     }
 }
@@ -381,20 +405,15 @@ __device__ __forceinline__ void leverage(const DevPlan& P, int a, float4 c3, flo
     const float* v = P.lev_values + __float_as_int(c3.z);
     const int npts = P.lev_points[a];
     const float f = fmaf(x, mp.x, mp.y);
+    // both ends select instead of branching, so that a thread's two lookups overlap
     const int last = npts - 1;
-    if (f <= 0.f) {
-        L = __ldg(v);
-        dL = 0.f;
-    } else if (f >= (float)last) {
-        L = __ldg(v + last);
-        dL = 0.f;
-    } else {
-        const int k = (int)f;
-        const float w = f - (float)k;
-        const float v0 = __ldg(v + k), v1 = __ldg(v + k + 1);
-        L = fmaf(w, v1 - v0, v0);
-        dL = (v1 - v0) * mp.x;
-    }
+    const int k = min(max((int)f, 0), last - 1);
+    const float w = f - (float)k;
+    const float v0 = __ldg(v + k), v1 = __ldg(v + k + 1);
+    const float mid = fmaf(w, v1 - v0, v0), slope = (v1 - v0) * mp.x;
+    const bool below = f <= 0.f, above = f >= (float)last;
+    L = below ? v0 : (above ? v1 : mid); // k is 0 below and last - 1 above
+    dL = below || above ? 0.f : slope;
 }
 
 __device__ __forceinline__ float intrinsic(const DevProduct& pr, float s)
@@ -567,52 +586,105 @@ __device__ __forceinline__ float2 comb2(float lw, float rw, float sd, float2 wp,
 
 // The Sobol lane of a thread with two paths: a running pointer into the tile parts in shared
 // memory (refilled HS_CHUNK entries at a time, uniformly across the CTA as in gauss) and a
-// running pointer into the book's low words, whose table carries two rows of padding so that
-// the load two entries ahead needs no bounds test.
+// running pointer into the book's low words. With LD = 2 the next two words are in registers (the
+// move of one into the other waits for its load, so the load is one entry ahead in effect); else
+// LD - 1 entries are on their way into this thread's ring in shared memory by asynchronous copies,
+// which no register waits for. The table carries rows of padding behind the last entry, so the
+// loads ahead need no bounds test.
+template <int LD>
 struct PairLane {
     const uint2* hs;      // tile part of the next entry
     const uint2* hs_end;  // end of the chunk in shared memory
-    const uint32_t* lo;   // low word of the entry two ahead (this thread's column)
-    uint32_t cur, nxt;    // low words of the next two entries
+    const uint32_t* lo;   // low word of the entry LD (ring: LD - 1) ahead (this thread's column)
+    uint32_t cur, nxt;    // LD = 2: low words of the next two entries
+    uint32_t ring, slot;  // ring: shared address of the thread's slot 0; byte offset of the next entry
     int jc;               // first entry of the chunk in shared memory
     int64_t m;            // tile index
 };
 
-template <int T>
-__device__ __forceinline__ PairLane pair_lane(const DevPlan& P, const uint2* hs, int64_t m)
+__host__ __device__ constexpr size_t ring_bytes(int threads, int LD) { return LD > 2 ? sizeof(uint32_t) * (size_t)threads * LD : 0; }
+
+__device__ __forceinline__ void copy_word(uint32_t dst, const uint32_t* src)
 {
-    PairLane L;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n\tcp.async.commit_group;" ::"r"(dst), "l"(src) : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int T, int LD>
+__device__ __forceinline__ PairLane<LD> pair_lane(const DevPlan& P, const uint2* hs, int64_t m, uint32_t* ring)
+{
+    PairLane<LD> L;
     L.hs = hs;
     L.hs_end = hs + HS_CHUNK;
-    L.lo = P.sobol_lo + 2 * T + threadIdx.x;
-    L.cur = __ldg(P.sobol_lo + threadIdx.x);
-    L.nxt = __ldg(P.sobol_lo + T + threadIdx.x);
+    const uint32_t* lo = P.sobol_lo + threadIdx.x;
+    if constexpr (LD > 2) {
+        constexpr uint32_t STEP = T / 2 * sizeof(uint32_t);
+        L.ring = static_cast<uint32_t>(__cvta_generic_to_shared(ring + threadIdx.x));
+        L.slot = 0;
+        copy_wait<0>(); // the tile before left copies of padding on their way
+#pragma unroll
+        for (int i = 0; i + 1 < LD; ++i) copy_word(L.ring + i * STEP, lo + i * T);
+        L.lo = lo + (LD - 1) * T;
+    } else {
+        L.cur = __ldg(lo);
+        L.nxt = __ldg(lo + T);
+        L.lo = lo + 2 * T;
+    }
     L.jc = 0;
     L.m = m;
     return L;
 }
 
+// the next entry's low word, and the load of the one LD (or LD - 1) ahead
+template <int T, int LD>
+__device__ __forceinline__ uint32_t next_word(PairLane<LD>& L)
+{
+    uint32_t w;
+    if constexpr (LD > 2) {
+        constexpr uint32_t STEP = T / 2 * sizeof(uint32_t), MASK = LD * STEP - 1;
+        static_assert((LD & (LD - 1)) == 0, "the ring's offset is masked");
+        copy_word(L.ring + ((L.slot + (LD - 1) * STEP) & MASK), L.lo);
+        copy_wait<LD - 1>();
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(L.ring + L.slot) : "memory");
+        L.slot = (L.slot + STEP) & MASK;
+    } else {
+        w = L.cur;
+        L.cur = L.nxt;
+        L.nxt = __ldg(L.lo);
+    }
+    L.lo += T;
+    return w;
+}
+
+// the next chunk of tile parts (uniform across the CTA)
+template <int TB, int LD>
+__device__ __forceinline__ void next_chunk(const DevPlan& P, uint2* hs_base, PairLane<LD>& L)
+{
+    L.jc += HS_CHUNK;
+    __syncthreads();
+    tile_high_bits<TB, (LD > 2)>(P, hs_base, L.m, L.jc);
+    __syncthreads();
+    L.hs = hs_base;
+}
+
 // ALL: every dimension of the book is a Sobol dimension (the bound test is dropped)
-template <int TB, bool ALL>
-__device__ __forceinline__ float2 pair_gauss(const DevPlan& P, uint2* hs_base, PairLane& L, const uint64_t (&n)[2],
+template <int TB, bool ALL, int LD>
+__device__ __forceinline__ float2 pair_gauss(const DevPlan& P, uint2* hs_base, PairLane<LD>& L, const uint64_t (&n)[2],
                                              int dim)
 {
     constexpr int T = 1 << TB;
     uint32_t x0, x1;
     if (ALL || dim < P.sobol_dims) {
-        if (L.hs == L.hs_end) { // next chunk of tile parts (uniform across the CTA)
-            L.jc += HS_CHUNK;
-            __syncthreads();
-            tile_high_bits<TB>(P, hs_base, L.m, L.jc);
-            __syncthreads();
-            L.hs = hs_base;
-        }
+        if (L.hs == L.hs_end) next_chunk<TB>(P, hs_base, L);
         const uint2 h = *L.hs++;
-        x0 = h.x ^ L.cur; // columns t and t + T/2 share the low word through the tile-part pair
-        x1 = h.y ^ L.cur;
-        L.cur = L.nxt;
-        L.nxt = __ldg(L.lo);
-        L.lo += T;
+        const uint32_t w = next_word<T, LD>(L);
+        x0 = h.x ^ w; // columns t and t + T/2 share the low word through the tile-part pair
+        x1 = h.y ^ w;
     } else if (P.tail) {
         return f2(tail_gauss(P, n[0], dim), tail_gauss(P, n[1], dim));
     } else {
@@ -622,6 +694,22 @@ __device__ __forceinline__ float2 pair_gauss(const DevPlan& P, uint2* hs_base, P
     float z0, z1;
     quantile_pair(x0, x1, z0, z1);
     return f2(z0, z1);
+}
+
+// A node's two draws of a book with one asset and two factors, all in Sobol: its entries come in
+// pairs, which a chunk holds whole, so one test, one 16-byte read of the tile parts and one test
+// for the tail serve both, and the two quantiles' chains of ~150 clocks overlap (with one draw
+// after the other: small Heston books 224 against 199 us, the ragged batch 30.4 against 28.6 ms).
+template <int TB, int LD>
+__device__ __forceinline__ void pair_gauss2(const DevPlan& P, uint2* hs_base, PairLane<LD>& L, float2& z0, float2& z1)
+{
+    constexpr int T = 1 << TB;
+    static_assert(HS_CHUNK % 2 == 0, "a chunk holds whole pairs");
+    if (L.hs == L.hs_end) next_chunk<TB>(P, hs_base, L);
+    const uint4 h = *reinterpret_cast<const uint4*>(L.hs);
+    L.hs += 2;
+    const uint32_t w0 = next_word<T, LD>(L), w1 = next_word<T, LD>(L);
+    quantile_quad(h.x ^ w0, h.y ^ w0, h.z ^ w1, h.w ^ w1, z0, z1);
 }
 
 // The path events of date i for asset a on both tile columns of a thread (t and t + TH), from
@@ -715,6 +803,32 @@ __device__ __forceinline__ void step_events(const DevPlan& P, const Smem& S, uin
     if (ev & SEV_LIST) pair_events<TH>(P, S, i, a, __popc(ev & SEV_MAIN), x, step, w, y);
 }
 
+// A book's step program as a deep launch reads it: staged in shared memory by the CTA where it
+// fits (there a load costs some 30 clocks, and no other warp covers the hundreds that a miss
+// takes), else where it lies. Other launches read the plan's own pointers.
+struct Program {
+    const float4* recs;      // StepRec [n_steps + 1]
+    const BridgeNode* nodes;
+    const float4* steps;     // AssetStep [n_steps][n_assets]
+};
+
+template <bool STAGED>
+__device__ __forceinline__ StepRec program_rec(const DevPlan& P, const Program& G, int i)
+{
+    if constexpr (!STAGED) return load_rec(P, i);
+    const float4 a = G.recs[2 * (i - 1)], b = G.recs[2 * (i - 1) + 1];
+    StepRec s;
+    s.lw = a.x;
+    s.rw = a.y;
+    s.sd = a.z;
+    s.dim = __float_as_int(a.w);
+    s.isd = b.x;
+    s.count = __float_as_int(b.y);
+    s.first = __float_as_int(b.z);
+    s.ev = __float_as_uint(b.w);
+    return s;
+}
+
 // FAST: the book is in Sobol mode with every dimension a Sobol dimension, and stores no paths.
 // There each step's record is loaded at the step: loading it one step ahead holds eight more
 // registers across the step and measured slower (2.93 against 2.75 ms for the 2^20-path Heston
@@ -722,8 +836,10 @@ __device__ __forceinline__ void step_events(const DevPlan& P, const Smem& S, uin
 // stored (GBM, 2^20 paths x 252 steps: 1.11 against 1.23 ms).
 // AT: the pass is asset a0's of a multi-asset book; else the book's only asset. MODEL M_SEQ: the
 // asset's model is looked up (the passes of such books that are not FAST).
-template <int TB, int MODEL, bool UNIFORM, bool FAST, bool AT>
-__device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairLane& L,
+//
+// LD > 2: the pass of a launch of few CTAs (DEEP_CTAS), where no other warp covers a load.
+template <int TB, int MODEL, bool UNIFORM, bool FAST, bool AT, int LD>
+__device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const Program& G, PairLane<LD>& L,
                                           const uint64_t (&n)[2], const bool (&valid)[2], int a0, float4 u0,
                                           float4 u1, float4 u2)
 {
@@ -755,25 +871,46 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairL
         for (int p = 0; p < 2; ++p)
             if (valid[p]) P.path_out[n[p] - (uint64_t)P.skip - 1] = P.s0[aid];
 
-    StepRec rec;
-    if constexpr (!FAST) rec = load_rec(P, 1);
+    constexpr bool DEEP = LD > 2;
+    StepRec rec; // the next step's record
+    const BridgeNode* const nodes = DEEP ? G.nodes : P.nodes;
+    auto load_consts = [&](int i, float4& a, float4& b, float4& c, float4& d) {
+        if constexpr (DEEP) {
+            const float4* cs = G.steps + 4 * ((i - 1) * P.n_assets + aid);
+            a = cs[0];
+            b = cs[1];
+            c = cs[2];
+            if (MODEL == M_LSV || (SEQ && model == M_LSV)) d = cs[3];
+        } else {
+            const float4* cs = reinterpret_cast<const float4*>(P.steps[(i - 1) * P.n_assets + aid].c);
+            a = __ldg(cs);
+            b = __ldg(cs + 1);
+            c = __ldg(cs + 2);
+            if (MODEL == M_LSV || (SEQ && model == M_LSV)) d = __ldg(cs + 3);
+        }
+    };
+    if constexpr (!FAST || DEEP) rec = program_rec<DEEP>(P, G, 1);
+    // the draws of a node whose first dimension (factor 0) is dim
+    auto draw = [&](int dim, float2& z0, float2& z1) {
+        if constexpr (FAST && !AT && MODEL != M_GBM) {
+            pair_gauss2<TB>(P, S.hs, L, z0, z1);
+        } else {
+            z0 = pair_gauss<TB, FAST, LD>(P, S.hs, L, n, dim + fid0);
+            z1 = f2s(0.f);
+            if (act1) z1 = pair_gauss<TB, FAST, LD>(P, S.hs, L, n, dim + fid1);
+        }
+    };
     for (int i = 1; i <= P.n_steps; ++i) {
         StepRec cur;
-        if constexpr (FAST) {
+        if constexpr (FAST && !DEEP) {
             cur = load_rec(P, i);
         } else {
             cur = rec;
-            rec = load_rec(P, i + 1); // the record past the last step is padding
+            rec = program_rec<DEEP>(P, G, i + 1); // the record past the last step is padding
         }
         // this step's constants, requested before the bridge work that covers their latency
         float4 c0 = u0, c1 = u1, c2 = u2, c3 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!UNIFORM) {
-            const float4* cs = reinterpret_cast<const float4*>(P.steps[(i - 1) * P.n_assets + aid].c);
-            c0 = __ldg(cs);
-            c1 = __ldg(cs + 1);
-            c2 = __ldg(cs + 2);
-            if (MODEL == M_LSV || (SEQ && model == M_LSV)) c3 = __ldg(cs + 3);
-        }
+        if (!UNIFORM) load_consts(i, c0, c1, c2, c3);
         // LSV: the leverage at the step's start, requested before the bridge work (see book_kernel)
         float lvL[2] = {1.f, 1.f}, lvD[2] = {0.f, 0.f};
         if (MODEL == M_LSV || (SEQ && model == M_LSV)) {
@@ -794,23 +931,27 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairL
                 }
                 --sp;
             } else if (cur.count == 1) {
-                Wi0 = comb2(cur.lw, cur.rw, cur.sd, Wp0, T0, pair_gauss<TB, FAST>(P, S.hs, L, n, cur.dim + fid0));
-                if (act1) Wi1 = comb2(cur.lw, cur.rw, cur.sd, Wp1, T1, pair_gauss<TB, FAST>(P, S.hs, L, n, cur.dim + fid1));
+                float2 z0, z1;
+                draw(cur.dim, z0, z1);
+                Wi0 = comb2(cur.lw, cur.rw, cur.sd, Wp0, T0, z0);
+                if (act1) Wi1 = comb2(cur.lw, cur.rw, cur.sd, Wp1, T1, z1);
             } else {
                 float lw = cur.lw, rw = cur.rw, sd = cur.sd;
                 int dim = cur.dim;
-                BridgeNode nd = P.nodes[cur.first]; // node 1 of the chain, loaded one node ahead
+                BridgeNode nd = nodes[cur.first]; // node 1 of the chain, loaded one node ahead
                 for (int k = 0; k < cur.count; ++k) {
                     if (k > 0) {
                         lw = nd.lw;
                         rw = nd.rw;
                         sd = nd.sd;
                         dim = nd.bstep * P.ref_factors;
-                        if (k + 1 < cur.count) nd = P.nodes[cur.first + k];
+                        if (k + 1 < cur.count) nd = nodes[cur.first + k];
                     }
-                    const float2 w0 = comb2(lw, rw, sd, Wp0, T0, pair_gauss<TB, FAST>(P, S.hs, L, n, dim + fid0));
+                    float2 z0, z1;
+                    draw(dim, z0, z1);
+                    const float2 w0 = comb2(lw, rw, sd, Wp0, T0, z0);
                     float2 w1 = f2s(0.f);
-                    if (act1) w1 = comb2(lw, rw, sd, Wp1, T1, pair_gauss<TB, FAST>(P, S.hs, L, n, dim + fid1));
+                    if (act1) w1 = comb2(lw, rw, sd, Wp1, T1, z1);
                     if (k + 1 < cur.count) {
                         const int base = sp * nfa;
                         stk[(base + ci0) * TH] = T0;
@@ -905,6 +1046,18 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, PairL
 //           with correlated GBM names, M_SEQ for other multi-asset books
 //   UNIFORM every step has the same per-asset constants (kept in registers)
 // ---------------------------------------------------------------------------
+// DEEP_CTAS: a launch of at most this many CTAs an SM is bound by the latency of a path's steps,
+// not by throughput: 16384 paths x 250 Heston steps took 2000 clocks a step, 875 of them waiting
+// for global loads (records, low words), and as long as 131072 paths. It runs the deep variant of
+// the (8, 2) shape: DEEP_WORDS - 1 low words on their way by asynchronous copies (a load into a
+// register that later moves waits for all of them), the step program in shared memory. 250 steps,
+// before and after: 16384 paths of GBM 149 and 117 us, Heston 272 and 199, LSV 313 and 222; the 391-tile Heston
+// surface 355 and 325 (its kernel alone). The line is the CTAs of 128 threads that an SM's
+// registers allow at the 160 a thread this form wants; above it the ordinary kernel's six CTAs an
+// SM hide the same waits.
+constexpr int DEEP_CTAS = 3;
+constexpr int DEEP_WORDS = 8;
+constexpr size_t DEEP_SMEM = 74 * 1024; // shared memory a CTA, DEEP_CTAS of which fit an SM
 // resident CTAs per SM the registers are bounded for: 768 threads per SM worth for one or two
 // paths a thread, 7 CTAs of 64 threads (146 registers each) for four, 3 for the mixed kernel
 template <int TB, int NA, int PP>
@@ -916,7 +1069,7 @@ struct MinBlocks {
 // product evaluated on each tile's paths, the FP64 sums in the row acc (zeroed here). A book's
 // own launch runs it with tile0 = blockIdx.x and tile_step = gridDim.x; the batch kernel runs
 // the same work items from a shared work list. Returns false when the cancel word stopped it.
-template <int TB, int NA, int MODEL, bool UNIFORM, int PP>
+template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
 __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_raw, int64_t tile0, int64_t tile_step,
                                           double* acc)
 {
@@ -933,6 +1086,23 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
     __shared__ int s_cancel;
 
     for (int j = t; j < P.n_acc; j += TH) acc[j] = 0.0;
+
+    Program G{reinterpret_cast<const float4*>(P.recs), P.nodes, reinterpret_cast<const float4*>(P.steps)};
+    if constexpr (LD > 2) {
+        float4* to = reinterpret_cast<float4*>(S.end + ring_bytes(TH, LD));
+        auto stage = [&](const void* from, int bytes) {
+            const float4* src = reinterpret_cast<const float4*>(from);
+            for (int i = t; i < bytes / 16; i += TH) to[i] = __ldg(src + i);
+            const float4* at = to;
+            to += bytes / 16;
+            return at;
+        };
+        if (P.deep_prog) { // read after the first tile's barrier
+            G.recs = stage(P.recs, (int)sizeof(StepRec) * (P.n_steps + 1));
+            G.nodes = reinterpret_cast<const BridgeNode*>(stage(P.nodes, (int)sizeof(BridgeNode) * P.n_nodes));
+        }
+        if (P.deep_consts) G.steps = stage(P.steps, (int)sizeof(AssetStep) * P.n_steps * P.n_assets);
+    }
 
     // uniform step constants (UNIFORM: step 1's for every step)
     float4 u0[NA], u1[NA], u2[NA];
@@ -966,7 +1136,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
             s_cancel = cancel_ahead;
             if (P.cancel != nullptr) cancel_ahead = *P.cancel;
         }
-        if (P.use_sobol) tile_high_bits<TB>(P, S.hs, m, 0);
+        if (P.use_sobol) tile_high_bits<TB, (LD > 2)>(P, S.hs, m, 0);
         __syncthreads();
         if (s_cancel) {
             if (t == 0) atomicExch(P.status, 1);
@@ -1021,7 +1191,8 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
         // one pass per asset for M_SEQ (asset a0), one pass for every asset otherwise
         constexpr bool SEQ = (MODEL == M_SEQ);
         const int n_pass = SEQ ? P.n_assets : 1;
-        PairLane PL = pair_lane<T>(P, S.hs, m); // unused (and dropped) unless NA == 1 and PP == 2
+        // unused (and dropped) unless NA == 1 and PP == 2; the ring lies behind the plan's shared memory
+        PairLane<LD> PL = pair_lane<T, LD>(P, S.hs, m, reinterpret_cast<uint32_t*>(S.end));
         for (int a0 = 0; a0 < n_pass; ++a0) {
             if constexpr (NA == 1 && PP == 2) {
                 // both passes in one kernel: the fast pass's own instantiation measured slower
@@ -1030,17 +1201,17 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                     // a pass of its own for each model: with the model looked up in the step loop,
                     // and one path a thread, the five-asset LSV book took 34.1 ms (see SEQ2)
                     if (!fast_pass(P))
-                        pair_pass<TB, M_SEQ, false, false, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                        pair_pass<TB, M_SEQ, false, false, true, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                     else if (P.model[a0] == M_LSV)
-                        pair_pass<TB, M_LSV, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                        pair_pass<TB, M_LSV, false, true, true, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                     else if (P.model[a0] == M_HESTON)
-                        pair_pass<TB, M_HESTON, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                        pair_pass<TB, M_HESTON, false, true, true, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                     else
-                        pair_pass<TB, M_GBM, false, true, true>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                        pair_pass<TB, M_GBM, false, true, true, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                 } else if (fast_pass(P)) {
-                    pair_pass<TB, MODEL, UNIFORM, true, false>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                    pair_pass<TB, MODEL, UNIFORM, true, false, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                 } else {
-                    pair_pass<TB, MODEL, UNIFORM, false, false>(P, S, PL, n, valid, a0, u0[0], u1[0], u2[0]);
+                    pair_pass<TB, MODEL, UNIFORM, false, false, LD>(P, S, G, PL, n, valid, a0, u0[0], u1[0], u2[0]);
                 }
                 continue;
             }
@@ -1492,11 +1663,13 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
     return true;
 }
 
-template <int TB, int NA, int MODEL, bool UNIFORM, int PP>
-__global__ void __launch_bounds__((1 << TB) / PP, MinBlocks<TB, NA, PP>::value) book_kernel(const DevPlan P)
+template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
+__global__ void __launch_bounds__((1 << TB) / PP, LD > 2 ? DEEP_CTAS : MinBlocks<TB, NA, PP>::value)
+    book_kernel(const DevPlan P)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    book_body<TB, NA, MODEL, UNIFORM, PP>(P, smem_raw, blockIdx.x, gridDim.x, P.acc + (size_t)blockIdx.x * P.n_acc);
+    book_body<TB, NA, MODEL, UNIFORM, PP, LD>(P, smem_raw, blockIdx.x, gridDim.x,
+                                             P.acc + (size_t)blockIdx.x * P.n_acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1572,7 +1745,7 @@ constexpr int SHAPE_TB[N_SHAPES] = {8, 8, 7, 7, 8};
 constexpr int SHAPE_PP[N_SHAPES] = {2, 1, 1, 2, 4};
 
 
-template <int TB, int NA, int MODEL, bool UNIFORM, int PP>
+template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
 static cudaError_t smem_attr_t()
 {
     // once per variant: allow the device's opt-in maximum, so that launches of
@@ -1583,20 +1756,21 @@ static cudaError_t smem_attr_t()
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa;
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, book_kernel<TB, NA, MODEL, UNIFORM, PP>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, book_kernel<TB, NA, MODEL, UNIFORM, PP, LD>);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(book_kernel<TB, NA, MODEL, UNIFORM, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(book_kernel<TB, NA, MODEL, UNIFORM, PP, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  mx - (int)fa.sharedSizeBytes);
     done = e == cudaSuccess;
     return e;
 }
 
-template <int TB, int NA, int MODEL, bool UNIFORM, int PP>
+template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
 static cudaError_t launch_book_t(const DevPlan& P, int grid, size_t smem, cudaStream_t st)
 {
-    cudaError_t e = smem_attr_t<TB, NA, MODEL, UNIFORM, PP>();
+    cudaError_t e = smem_attr_t<TB, NA, MODEL, UNIFORM, PP, LD>();
     if (e != cudaSuccess) return e;
-    book_kernel<TB, NA, MODEL, UNIFORM, PP><<<grid, (1 << TB) / PP, smem, st>>>(P);
+    book_kernel<TB, NA, MODEL, UNIFORM, PP, LD>
+        <<<grid, (1 << TB) / PP, smem + (LD > 2 ? ring_bytes((1 << TB) / PP, LD) + P.deep_prog + P.deep_consts : 0), st>>>(P);
     return cudaGetLastError();
 }
 
@@ -1610,11 +1784,18 @@ static int occ_t(size_t smem)
     return n < 1 ? 1 : n;
 }
 
-// one single-asset model in each of the four shapes: launch (grid > 0) or occupancy (grid == 0)
+// shape DEEP_SHAPE is the deep variant of shape 0: the same tiles, threads and results. A plan runs
+// it where its launch is small (DEEP_CTAS) and nothing runs beside it; it is no shape of a plan.
+constexpr int DEEP_SHAPE = -1;
+
+// one single-asset model in each of the shapes: launch (grid > 0) or occupancy (grid == 0)
 template <int MODEL, bool UNIFORM>
 static int single_t(const DevPlan* P, int shape, int grid, size_t smem, cudaStream_t st, cudaError_t* err)
 {
     switch (shape) {
+    case DEEP_SHAPE:
+        if (grid) *err = launch_book_t<8, 1, MODEL, UNIFORM, 2, DEEP_WORDS>(*P, grid, smem, st);
+        return grid ? 0 : occ_t<8, 1, MODEL, UNIFORM, 2>(smem);
     case 0:
         if (grid) *err = launch_book_t<8, 1, MODEL, UNIFORM, 2>(*P, grid, smem, st);
         return grid ? 0 : occ_t<8, 1, MODEL, UNIFORM, 2>(smem);

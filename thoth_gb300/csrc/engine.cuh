@@ -165,6 +165,8 @@ struct DevPlan {
     const StepRec* recs;         // [n_steps + 1] (the last is padding for a load one step ahead)
     int uniform_steps;           // 1: every step's AssetStep equals step 1's
     const BridgeNode* nodes;     // time-ordered program
+    int n_nodes;
+    int deep_prog, deep_consts;  // deep launches: bytes of recs + nodes, and of steps, staged in shared memory (0: not)
     const int2* ev_range;        // [(n_steps + 1)][n_assets] (first, count) into events; row 0 = date 0
     const Event* events;         // per (date, asset) the main groups' updates first
     const float4* ev_p;          // [(n_steps + 1)][n_assets] shifts of the main groups' updates
@@ -358,6 +360,31 @@ __device__ __forceinline__ void quantile_pair(uint32_t x0, uint32_t x1, float& z
     zz = __fmul2_rn(zz, sv);
     z0 = zz.x;
     z1 = zz.y;
+}
+
+// two quantile_pairs as one straight-line block with one test for the rare tail (same expressions,
+// same results): the two factors' draws of a bridge node
+__device__ __forceinline__ void quantile_quad(uint32_t x0, uint32_t x1, uint32_t y0, uint32_t y1, float2& z, float2& w)
+{
+    const uint32_t q0 = min(x0, 0u - x0), q1 = min(x1, 0u - x1), p0 = min(y0, 0u - y0), p1 = min(y1, 0u - y1);
+    const float2 su = __fmul2_rn(f2(__int2float_rn((int)(x0 ^ 0x80000000u)), __int2float_rn((int)(x1 ^ 0x80000000u))),
+                                 f2s(4.656612873077393e-10f));
+    const float2 sv = __fmul2_rn(f2(__int2float_rn((int)(y0 ^ 0x80000000u)), __int2float_rn((int)(y1 ^ 0x80000000u))),
+                                 f2s(4.656612873077393e-10f));
+    const float2 qf = f2(__uint2float_rn(q0), __uint2float_rn(q1)), pf = f2(__uint2float_rn(p0), __uint2float_rn(p1));
+    const float2 a = __fmul2_rn(qf, __ffma2_rn(qf, f2s(-2.168404344971009e-19f), f2s(9.313225746154785e-10f)));
+    const float2 b = __fmul2_rn(pf, __ffma2_rn(pf, f2s(-2.168404344971009e-19f), f2s(9.313225746154785e-10f)));
+    const float2 la = f2(fminf(__log2f(a.x), 0.0f), fminf(__log2f(a.y), 0.0f));
+    const float2 lb = f2(fminf(__log2f(b.x), 0.0f), fminf(__log2f(b.y), 0.0f));
+    float2 za = quantile_central2(la), zb = quantile_central2(lb);
+    if (!(fminf(fminf(la.x, la.y), fminf(lb.x, lb.y)) > QUANTILE_TAIL_LG)) {
+        if (!(la.x > QUANTILE_TAIL_LG)) za.x = quantile_tail(la.x);
+        if (!(la.y > QUANTILE_TAIL_LG)) za.y = quantile_tail(la.y);
+        if (!(lb.x > QUANTILE_TAIL_LG)) zb.x = quantile_tail(lb.x);
+        if (!(lb.y > QUANTILE_TAIL_LG)) zb.y = quantile_tail(lb.y);
+    }
+    z = __fmul2_rn(za, su);
+    w = __fmul2_rn(zb, sv);
 }
 
 // quantile_n for an even number of paths a thread: their quantiles in pairs

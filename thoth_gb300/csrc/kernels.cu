@@ -213,7 +213,7 @@ int book_shape_threads(int variant, int shape) { return variant == 3 ? 128 : (1 
 static int dispatch(const DevPlan* P, int variant, int shape, int grid, size_t smem, cudaStream_t st, cudaError_t* err)
 {
     *err = cudaSuccess;
-    if (variant != 3 && (shape < 0 || shape >= N_SHAPES)) {
+    if (variant != 3 && shape != DEEP_SHAPE && (shape < 0 || shape >= N_SHAPES)) {
         *err = cudaErrorInvalidValue;
         return 1;
     }
@@ -234,11 +234,33 @@ static int dispatch(const DevPlan* P, int variant, int shape, int grid, size_t s
 //           5 GBM with uniform steps, 6 multi-asset with independent assets (one pass per asset)
 cudaError_t launch_book(const DevPlan& P, int variant, int shape, int grid, size_t smem, cudaStream_t st)
 {
-    if (grid < 1) return cudaErrorInvalidValue;
+    if (grid < 1 || shape < 0) return cudaErrorInvalidValue;
     cudaError_t e;
     dispatch(&P, variant, shape, grid, smem, st, &e);
     return e;
 }
+
+// the launch of a book that has the device to itself, on a plan whose low words carry
+// book_low_padding() rows: the deep variant where its CTAs are few (DEEP_CTAS)
+cudaError_t launch_book_alone(const DevPlan& P, int variant, int shape, int grid, int sms, size_t smem, cudaStream_t st)
+{
+    const size_t ring = ring_bytes(book_shape_threads(variant, 0), DEEP_WORDS);
+    if (variant == 3 || shape != 0 || grid < 1 || grid > DEEP_CTAS * sms || smem + ring > DEEP_SMEM)
+        return launch_book(P, variant, shape, grid, smem, st);
+    // the step program, and the steps' constants where they differ, into the shared memory left
+    DevPlan Q = P;
+    size_t left = DEEP_SMEM - smem - ring;
+    const size_t prog = sizeof(StepRec) * (size_t)(P.n_steps + 1) + sizeof(BridgeNode) * (size_t)P.n_nodes;
+    const size_t consts = P.uniform_steps ? 0 : sizeof(AssetStep) * (size_t)P.n_steps * (size_t)P.n_assets;
+    Q.deep_prog = prog <= left ? (int)prog : 0;
+    left -= (size_t)Q.deep_prog;
+    Q.deep_consts = consts <= left ? (int)consts : 0;
+    cudaError_t e;
+    dispatch(&Q, variant, DEEP_SHAPE, grid, smem, st, &e);
+    return e;
+}
+
+int book_low_padding() { return DEEP_WORDS; }
 
 // resident CTAs per SM of a variant and shape at a given dynamic shared-memory size
 int book_occupancy(int variant, int shape, size_t smem)

@@ -27,6 +27,8 @@
 
 namespace thoth {
 cudaError_t launch_book(const DevPlan& P, int variant, int shape, int grid, size_t smem, cudaStream_t st);
+cudaError_t launch_book_alone(const DevPlan& P, int variant, int shape, int grid, int sms, size_t smem, cudaStream_t st);
+int book_low_padding();
 int book_shape_count(int variant);
 int book_shape_tile_bits(int variant, int shape);
 int book_shape_threads(int variant, int shape);
@@ -456,6 +458,7 @@ struct Plan {
         o_sord;
     int variant = 1, base_variant = 1, shape = 0, T = 256;
     size_t smem = 0;
+    int low_pad = 2; // rows of padding behind the low Sobol words (8 for launch_book_alone)
     bool slots_global = false; // observation slots in global memory (slot_rows_bytes)
     int n_products = 0;
     int64_t paths = 0;
@@ -1071,6 +1074,7 @@ int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1, bool own_memory 
 
     // pack
     if (bp.nodes.empty()) bp.nodes.push_back(BridgeNode{0, 0, 0, 0});
+    D.n_nodes = (int)bp.nodes.size();
     P.o_steps = P.blob.put(steps);
     P.o_isd = P.blob.put(isd);
     P.o_prog = P.blob.put(bp.prog);
@@ -1090,6 +1094,7 @@ int build_plan(const ThothBookDesc* d, Plan& P, int shape = -1, bool own_memory 
     // shapes 0 and 1 share the 256-path tile, so the plan above serves both
     if (untuned && !tuned && P.variant != 3 && P.shape == 0) P.shape = default_shape(P.variant, P.smem);
     D.eval_threads = book_shape_threads(P.variant, P.shape);
+    P.low_pad = own_memory ? 2 : book_low_padding();
     if (!own_memory) {
         // the product sums stay laid out as for the shape the plan would have had, so a book's
         // results do not depend on where its slots are
@@ -1180,11 +1185,11 @@ double trust_of(double s1, double s2, double n)
 }
 
 // bytes of a book's low Sobol words in consumption order ([n_sobol][T])
-// the book's low words in consumption order, and two rows of padding that the kernel's
-// load two entries ahead may read past the last entry
+// the book's low words in consumption order, and the rows of padding that the kernel's loads two
+// (or, in the deep variant, eight) entries ahead may read past the last entry
 // a book's own device tables after its plan blob: its low Sobol words in consumption order, then
 // (aligned) its tail Gaussians
-size_t low_words_bytes(const Plan& P) { return sizeof(uint32_t) * ((size_t)P.dp.n_sobol + 2) * P.T; }
+size_t low_words_bytes(const Plan& P) { return sizeof(uint32_t) * ((size_t)P.dp.n_sobol + P.low_pad) * P.T; }
 size_t low_bytes(const Plan& P)
 {
     const size_t lo = low_words_bytes(P);
@@ -1262,7 +1267,7 @@ int run_bound(Plan& P, unsigned char* base, const Layout& L, int grid, ThothBook
     CUDA_TRY(cudaMemsetAsync(base + L.o_st, 0, sizeof(int), st));
     CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
     if (gather) CUDA_TRY(gather_low(P, st));
-    CUDA_TRY(launch_book(P.dp, P.variant, P.shape, grid, P.smem, st));
+    CUDA_TRY(launch_book_alone(P.dp, P.variant, P.shape, grid, g_dev.sms, P.smem, st));
     CUDA_TRY(launch_reduce(P.dp.acc, grid, (int)n_acc, reinterpret_cast<double*>(base + L.o_out), st));
     CUDA_TRY(cudaEventRecord(g_dev.ev1, st));
     CUDA_TRY(cudaMemcpyAsync(g_dev.pinned, base + L.o_out, sizeof(double) * n_acc, cudaMemcpyDeviceToHost, st));
@@ -2178,10 +2183,10 @@ static int autotune_book_locked(const ThothBookDesc* book, int reps, ThothTuneRe
         for (size_t c = 0; c < grids.size(); c++) {
             const int g = grids[c];
             CUDA_TRY(cudaMemsetAsync(g_dev.arena + L.o_st, 0, sizeof(int), st));
-            CUDA_TRY(launch_book(P.dp, P.variant, P.shape, g, P.smem, st)); // warm-up
+            CUDA_TRY(launch_book_alone(P.dp, P.variant, P.shape, g, g_dev.sms, P.smem, st)); // warm-up
             CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
             for (int r = 0; r < reps; r++) {
-                CUDA_TRY(launch_book(P.dp, P.variant, P.shape, g, P.smem, st));
+                CUDA_TRY(launch_book_alone(P.dp, P.variant, P.shape, g, g_dev.sms, P.smem, st));
                 CUDA_TRY(launch_reduce(P.dp.acc, g, P.dp.n_acc, reinterpret_cast<double*>(g_dev.arena + L.o_out), st));
             }
             CUDA_TRY(cudaEventRecord(g_dev.ev1, st));
