@@ -1,0 +1,63 @@
+"""The exercise fit at the edges of its shares of paths, in shared and in global memory.
+
+A CTA walks a run of whole 32-path chunks, split over its warps; the paths' cashflows and lists are
+in shared memory where they fit (about 1.3 million paths of one contract on 152 SMs) and in global
+memory beyond. The sums are exact and the arithmetic the reference's, so every case equals the
+oracle on the stored paths bit for bit.
+"""
+import numpy as np
+import pytest
+
+from oracle import american as am
+from thoth_gb300 import abi
+from tests.test_gpu_american import DAYS, assert_same_fit, rates_of, vanilla_book
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("paths,K,typ,model", [
+    (2, 100.0, abi.PUT, "gbm"),
+    (31, 100.0, abi.PUT, "gbm"),
+    (33, 103.7, abi.PUT, "heston"),             # a strike that is no float, a normaliser of 53 bits
+    (129, 100.0, abi.CALL, "gbm"),              # a second CTA of one path
+    (128 * 152, 96.25, abi.PUT, "heston"),      # one chunk a scheduler on every SM
+    (128 * 152 + 1, 96.25, abi.CALL, "heston"),
+    (100003, 99.9, abi.PUT, "gbm"),
+    (60000, 260.0, abi.PUT, "gbm"),             # every path in the money, most below half the strike
+    (700000, 100.0, abi.PUT, "heston"),
+])
+def test_fit_over_ragged_shares(gpu, paths, K, typ, model):
+    b = vanilla_book(K=K, typ=typ, model=model, paths=paths, r=0.08 if typ == abi.PUT else 0.02)
+    if typ == abi.CALL:
+        b.assets[0]["carry"] = b.assets[0]["carry"] - 0.06
+    r = gpu.price_american(b, 0, min_itm=5)
+    S, _ = gpu.simulate_paths(b, 0)
+    o = am.fit(S, b.t, rates_of(b), K, typ == abi.CALL, K, min_itm=5)
+    if o["has_fit"].any():
+        assert_same_fit(r, o, b.n_dates)
+    else:
+        assert r["fitted_dates"] == 0 and r["premium"] == o["premium"]
+
+
+def test_fit_of_paths_in_global_memory(gpu):
+    b = vanilla_book(paths=1500001, days=[0, 100, 200, 300, 365])
+    r = gpu.price_american(b, 0)
+    S, _ = gpu.simulate_paths(b, 0)
+    assert_same_fit(r, am.fit(S, b.t, rates_of(b), 100.0, False, 100.0), b.n_dates)
+
+
+@pytest.mark.parametrize("paths,n", [(20001, 3), (120000, 20)])  # shared; the 20 contracts' paths global
+def test_contracts_that_share_a_fit(gpu, paths, n):
+    b = abi.Book(days=np.asarray(DAYS), paths=paths)
+    a = b.add_gbm(100.0, 0.30, 0.06)
+    for k in range(n):
+        b.add_vanilla(a, 80.0 + 2.37 * k, [13, 1, 7, 2][k % 4], abi.PUT if k % 3 else abi.CALL, zero_rate=0.06)
+    together = gpu.price_american_book(b, list(range(n)))
+    S, _ = gpu.simulate_paths(b, 0)
+    for p in range(n):
+        P = b.products[p]
+        M = P["maturity"] + 1
+        o = am.fit(S[:M], b.t, rates_of(b), P["strike"], P["option_type"] == abi.CALL, P["strike"])
+        assert together[p]["premium"] == o["premium"] and together[p]["european"] == o["european"], p
+        assert together[p]["fitted_dates"] == int(o["has_fit"].sum())
+        np.testing.assert_array_equal(together[p]["beta"][:M][o["has_fit"]], o["beta"][o["has_fit"]])

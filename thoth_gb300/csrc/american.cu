@@ -3,17 +3,22 @@
 // with the normal-equation solve of helpers/maths.cpp:354-381 and 419-470.
 //
 // Fit: one cooperative, persistent launch fits every contract of an asset on the same stored
-// paths, walking the exercise dates backwards. At each date, for each contract whose grid
-// reaches the date, every CTA discounts its paths' cashflows, queues the in-the-money paths so
-// that full warps do the FP64 work, and adds the regression moments into the contract's
-// per-date totals (exact 128-bit integer atomics). The last CTA to publish solves every
-// contract's 3x3 system, one thread each, and releases the others with a flag; every CTA then
-// rolls its paths' cashflows back through each contract's exercise decision. The dates are
-// sequential and the contracts share them, so one launch with one publish-and-release per
-// date replaces a launch per contract and date. The exercise decisions of the backward pass
-// are the frozen policy's decisions on the same paths (the same test at the same dates), so
-// the earliest exercise the pass records per path is the value the reference's apply step
-// finds: the premium comes out of the fit without a second walk over the paths.
+// paths, walking the exercise dates backwards. A date's regression needs the sums of the powers of
+// the in-the-money paths' moneyness, which no decision changes, and the sums with their cashflows,
+// which date t + 1's decisions change. So while date t's policy is being found, the CTAs already
+// list date t - 1's in-the-money paths and form its moneyness sums, and the normal equations'
+// matrix is factored beside the cashflow sums: the round of all CTAs that each date needs (publish,
+// wait, solve) lies behind the next date's work. Every CTA solves from the contracts' per-date
+// totals (exact 128-bit integer atomics) itself, one contract a lane, so no CTA releases the
+// others. The decision at date t + 1 is taken where its cashflow is used, on the way to date t, and
+// a path keeps the date of its earliest exercise: the frozen policy's exercise on the same paths
+// (the same test at the same dates), so the premium comes out of the fit without a second walk.
+//
+// What bounds the fit is FP64: an SM finishes one warp's instruction in 16 clocks, and a date needs
+// one product a path and eight operations an in-the-money path (2^20 paths, half of them in the
+// money: 16.6 thousand clocks of the 25 thousand a date takes; with a publish-and-release per date,
+// FP64 decisions, FP64 conversions and branches between the products it took 71 thousand).
+// 2^20 Heston paths x 365 dates: 13.4 ms before, 4.7 ms.
 //
 // Apply: the frozen policy on another path set (the bumped scenarios of the Greeks), one
 // forward walk per path that stops at the first exercise.
@@ -24,17 +29,17 @@
 // multiply-adds (those inside the moneyness quotient give its correctly rounded value).
 // GB300 runs FP64 at a small fraction of its FP32 rate, so the per-path work keeps FP64
 // to what the result depends on: the in-the-money test is an integer compare on the
-// spot's bits, and the quotient S / norm is one multiply and four fused multiply-adds. In
-// the apply the exercise test runs in FP32 wherever a proven margin shows that it decides as
-// the FP64 test (screen_exercise), which then runs only in a thin band around the boundary.
-// (The fit's test, on its compacted lists of full warps, measured faster in FP64.)
+// spot's bits, the quotient S / norm is two operations where norm has few digits and five
+// elsewhere, spots widen by integer operations, and the exercise test runs in FP32 wherever a
+// proven margin shows that it decides as the FP64 test (screen_exercise), which then runs only in a
+// thin band around the boundary (0.3 paths in a thousand).
 #include "american.cuh"
+
+#include <type_traits>
 
 namespace {
 
 constexpr int LSM_WARPS = LSM_THREADS / 32;
-static_assert(LSM_WARPS >= LSM_PART, "one warp per regression sum in the cross-CTA reduction");
-constexpr int LSM_QCAP = 64; // per-warp queue of in-the-money paths waiting for a full warp
 constexpr unsigned long long BARRIER_LIMIT_NS = 2000000000ull; // 2 s
 
 // max(phi (S - K), 0): payoff_vanilla with a floor at 0 (helpers/finance.cpp:9-32)
@@ -53,7 +58,8 @@ __device__ __forceinline__ bool in_the_money(float s, const K& A)
     return A.call ? b >= A.itm_bits : b <= A.itm_bits;
 }
 
-// S / norm rounded to nearest, from y = 1 / norm rounded to nearest. q0 = RN(S y) may be
+// S / norm rounded to nearest, from y = 1 / norm rounded to nearest (see moneyness_short for a norm
+// of few digits). q0 = RN(S y) may be
 // more than one ulp off near a power of two; one correction step q1 = RN(q0 + RN(S - norm q0) y)
 // brings it within one ulp, and then the remainder S - norm q1 is exact and the second step
 // q1 + r y rounded once is the correctly rounded quotient (P. Markstein, IBM J. Res. Dev.
@@ -66,6 +72,15 @@ __device__ __forceinline__ double moneyness(double s, const K& A)
     const double q0 = __dmul_rn(s, y);
     const double q1 = __fma_rn(__fma_rn(-q0, b, s), y, q0);
     return __fma_rn(__fma_rn(-q1, b, s), y, q1);
+}
+
+// The same for a norm of at most 45 significant bits, from y and ylo = RN(1 / norm - y): the sum
+// before its one rounding is within 2^-105 of S / norm, and a quotient of a 24-bit by a 45-bit number
+// is never nearer than 2^-99 to a midpoint of two doubles (it would have to be a fraction with the
+// 54-bit midpoint's numerator), so it rounds as the quotient does. Two FP64 operations.
+__device__ __forceinline__ double moneyness_short(double s, double y, double ylo)
+{
+    return __fma_rn(s, y, __dmul_rn(s, ylo));
 }
 
 // b0 + b1 m + b2 m m, evaluated left to right
@@ -103,58 +118,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// wait until *flag >= want; false (status 2) after 2 s, or at once when another CTA
-// has failed: the caller returns, so no wait outlives the limit
+// wait until *flag >= want; false (status 2) after 2 s, or soon when another CTA has failed: the
+// caller returns, so no wait outlives the limit
 __device__ bool wait_for(const unsigned* flag, unsigned want, int* status)
 {
     const unsigned long long t0 = now_ns();
-    while (ld_acquire(flag) < want) {
+    for (unsigned polls = 1; ld_acquire(flag) < want; ++polls) {
+        if (polls % 64) continue;
         if (*(volatile int*)status != 0) return false;
         if (now_ns() - t0 > BARRIER_LIMIT_NS) {
             atomicExch(status, 2);
             return false;
         }
-        __nanosleep(32);
-    }
-    return true;
-}
-
-// (X^T X) beta = X^T y for X = {1, m, m^2}: Cholesky A = L L^T in place of the lower
-// triangle, forward then back substitution (maths.cpp:354-381, 419-470). False when a pivot
-// is not positive (the date keeps no regression).
-__device__ bool solve3(const double* tot, double* beta)
-{
-    const double n = tot[LSM_NQ];
-    const double s1 = tot[0], s2 = tot[1], s3 = tot[2], s4 = tot[3];
-    double A[3][3] = {{n, s1, s2}, {s1, s2, s3}, {s2, s3, s4}};
-    const double g[3] = {tot[4], tot[5], tot[6]};
-    for (int i = 0; i < 3; i++) {
-        for (int j = 0; j <= i; j++) {
-            double sum = A[i][j];
-            for (int k = 0; k < j; k++) sum = __dsub_rn(sum, __dmul_rn(A[i][k], A[j][k]));
-            if (i == j) {
-                if (sum <= 0.0) return false;
-                A[i][j] = __dsqrt_rn(sum);
-            } else {
-                A[i][j] = __ddiv_rn(sum, A[j][j]);
-            }
-        }
-    }
-    double z[3];
-    for (int i = 0; i < 3; i++) {
-        double s = g[i];
-        for (int k = 0; k < i; k++) s = __dsub_rn(s, __dmul_rn(A[i][k], z[k]));
-        z[i] = __ddiv_rn(s, A[i][i]);
-    }
-    for (int i = 2; i >= 0; i--) {
-        double s = z[i];
-        for (int k = i + 1; k < 3; k++) s = __dsub_rn(s, __dmul_rn(A[k][i], beta[k]));
-        beta[i] = __ddiv_rn(s, A[i][i]);
     }
     return true;
 }
@@ -183,24 +158,21 @@ __device__ __forceinline__ Fx128 fx_from3(const unsigned long long* src)
 
 // The exercise test iv >= b0 + b1 m + b2 m^2 (iv = phi (S - K), m = S / norm) of an
 // in-the-money spot sf, in single precision: 1 exercise, 0 hold, -1 too close to call.
-// With u = 2^-24 and mag = |K| + |S| + |b0| + |b1 m| + |b2| m^2, the single-precision
-// difference d = iv - c (the inputs rounded to float, then five rounded operations) is within
-// 8 u mag of the real iv - c, and the reference's double-precision operands are within
-// 6 * 2^-53 mag of it. So |d| > 2^-19 mag (four times that bound, computed from the rounded
-// inputs) fixes the sign of the double-precision difference and hence the reference's test;
-// an absolute floor keeps underflow out of the bound. Inputs too large for single precision
-// give an infinite or NaN d or bound and come back undecided, as does the thin band around
-// the exercise boundary: the caller then runs the double-precision test.
+// With u = 2^-24, x = S - K_f (one rounding, relative) and h = x / norm, the inputs rounded to float
+// and the rounded operations leave iv with 2 u (|iv| + |K_f - K|), a0 with 2 u, a1 h with 6 u and
+// a2 h^2 with 9 u of their sizes, and the difference with one u of iv and c: below 10 u of each term,
+// against 32 u in the bound (lsm_screen), which also holds the reference's own rounding. So |d| above
+// the bound fixes the sign of the double-precision difference and hence the reference's test; inputs
+// too large for single precision give an infinite or NaN d or bound and come back undecided, as does
+// the thin band around the exercise boundary: the caller then runs the double-precision test.
 template <class K>
-__device__ __forceinline__ int screen_exercise(float sf, float b0, float b1, float b2, const K& A)
+__device__ __forceinline__ int screen_exercise(float sf, const LsmScreen& P, const K& A)
 {
-    const float m = sf * A.inv_norm_f;
-    const float iv = A.call ? sf - A.strike_f : A.strike_f - sf;
-    const float c = fmaf(fmaf(b2, m, b1), m, b0);
-    const float d = iv - c;
-    const float am = fabsf(m);
-    const float mag = fmaf(fabsf(b2) * am, am, fmaf(fabsf(b1), am, fabsf(b0))) + (fabsf(A.strike_f) + fabsf(sf));
-    const float e = fmaf(mag, 0x1p-19f, 1e-30f);
+    const float x = sf - A.strike_f, v = x + A.strike_lo;
+    const float iv = A.call ? v : -v;
+    const float h = x * A.inv_norm_f, ah = fabsf(h);
+    const float d = iv - fmaf(fmaf(P.a2, h, P.a1), h, P.a0);
+    const float e = fmaf(fabsf(iv), 0x1p-19f, fmaf(fmaf(P.e2, ah, P.e1), ah, P.e0));
     return d > e ? 1 : (d < -e ? 0 : -1);
 }
 
@@ -212,28 +184,9 @@ __device__ __forceinline__ double itm_value(float sf, const K& A)
     return A.call ? __dsub_rn(s, A.strike) : __dsub_rn(A.strike, s);
 }
 
-// one in-the-money path of contract K at the current date: its regression terms into the
-// lane's sums, its moneyness and intrinsic value into the warp's compacted list at entry o
-__device__ __forceinline__ void itm_item(int p, float sf, double y, const LsmContract& K, Fx128* q, int64_t o,
-                                         bool& bad)
-{
-    const double s = (double)sf;
-    const double iv = K.call ? __dsub_rn(s, K.strike) : __dsub_rn(K.strike, s);
-    const double m = moneyness(s, K), m2 = __dmul_rn(m, m);
-    K.c_idx[o] = p;
-    K.c_m[o] = m;
-    K.c_iv[o] = iv;
-    fx_add_checked(q[0], m, bad);
-    fx_add_checked(q[1], m2, bad);
-    fx_add_checked(q[2], __dmul_rn(m2, m), bad);
-    fx_add_checked(q[3], __dmul_rn(m2, m2), bad);
-    fx_add_checked(q[4], y, bad);
-    fx_add_checked(q[5], __dmul_rn(m, y), bad);
-    fx_add_checked(q[6], __dmul_rn(m2, y), bad);
-}
-
 // CTA-wide exact sum of one accumulator per thread into out (thread 0 writes)
-__device__ void block_sum(Fx128 a, Fx128 (*s_w)[LSM_PART], int slot, Fx128* out)
+template <int WARPS>
+__device__ void block_sum(Fx128 a, Fx128 (&s_w)[WARPS][LSM_NACC], int slot, Fx128* out)
 {
     warp_sum(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -241,213 +194,587 @@ __device__ void block_sum(Fx128 a, Fx128 (*s_w)[LSM_PART], int slot, Fx128* out)
     __syncthreads();
     if (threadIdx.x == 0) {
         Fx128 s = {0, 0};
-        for (int w = 0; w < LSM_WARPS; w++) fx_add(s, s_w[w][slot]);
+        for (int w = 0; w < WARPS; w++) fx_add(s, s_w[w][slot]);
         *out = s;
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(LSM_THREADS, 1) lsm_fit_kernel(const LsmFitArgs A)
+// The fit's CTA: 16 warps walk the paths; two more publish the CTA's sums, wait for the others' and
+// find the policies, one (the factorer) from the moneyness sums, one (the solver) from the cashflow
+// sums. Both are on the SM's scheduler 0 (warps 0 and 4).
+constexpr int FIT_WARPS = 18, FIT_FACTORER = 0, FIT_SOLVER = 4;
+constexpr int FIT_THREADS = 32 * FIT_WARPS;
+constexpr int FIT_WALKERS = FIT_THREADS - 64;
+constexpr int FIT_MIN_PATHS = 128; // paths a CTA walks before the grid grows: a chunk a scheduler
+constexpr int FIT_SOLVER_CHUNKS = 24; // see lsm_fit_kernel
+constexpr int SUM_LIMBS = 5; // a warp's 128-bit sum in 26-bit limbs, added in shared memory
+
+constexpr int FIT_X = 5, FIT_Y = 3; // a date's moneyness sums (with the count), its cashflow sums
+static_assert(FIT_X + FIT_Y == LSM_PART, "the totals hold both");
+// A contract's sums in shared memory: the moneyness sums of even and of odd dates, the cashflow
+// sums. The walkers form date t - 1's moneyness sums before they wait for date t's policy, and the
+// solver may still hold date t's then; date t - 2's and the next cashflow sums come behind that wait.
+constexpr int FIT_SUMS = 2 * FIT_X + FIT_Y;
+
+// named barriers: date t's moneyness sums are in shared memory (by the parity of t, as the
+// sums); its cashflow sums; its policy; its factors, from factorer to solver (by parity)
+enum { BAR_X = 1, BAR_Y = 3, BAR_POLICY = 4, BAR_FACTOR = 5 };
+constexpr int FIT_HANDOVER = FIT_WALKERS + 32; // the walkers and one of the two
+template <int N>
+__device__ __forceinline__ void bar_sync(int id)
 {
-    __shared__ Fx128 s_w[LSM_WARPS][LSM_PART];
-    __shared__ int q_idx[LSM_WARPS][LSM_QCAP];
-    __shared__ float q_s[LSM_WARPS][LSM_QCAP];
-    __shared__ double q_y[LSM_WARPS][LSM_QCAP];
-    __shared__ LsmContract s_ct[LSM_MAX_CONTRACTS];
-    __shared__ int s_nout[LSM_WARPS][LSM_MAX_CONTRACTS];
-    __shared__ double s_b[LSM_MAX_CONTRACTS][3];
-    __shared__ double s_tot[LSM_MAX_CONTRACTS][LSM_PART];
-    __shared__ int s_fit[LSM_MAX_CONTRACTS];
-    __shared__ int s_ok, s_last;
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bar_arrive(int id)
+{
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(N) : "memory");
+}
+
+// A divisor and its reciprocal in two pieces: r = 1 / l rounded, rl = 1 / l - r rounded.
+struct Pivot {
+    double l, r, rl;
+};
+__device__ __forceinline__ Pivot pivot(double l)
+{
+    const double r = __ddiv_rn(1.0, l);
+    return Pivot{l, r, __dmul_rn(__fma_rn(-l, r, 1.0), r)};
+}
+
+// a / P.l from the two-piece reciprocal: within half an ulp and 2^-50 of one, so the correctly
+// rounded quotient unless a tie is nearer than that. `sure` stays set where the exact remainder
+// a - q l is below half an ulp of q (of the ulp below a power of two) times l by a clear margin,
+// which an integer comparison of its bits decides; elsewhere, and near the ends of the range, the
+// caller takes the division. Two dependent FP64 operations, the test beside the next ones: the
+// solver's chain of six divisions is on every date's critical path (a division takes about nine).
+__device__ __forceinline__ double divide_by(double a, const Pivot& P, bool& sure)
+{
+    const double q = __fma_rn(a, P.r, __dmul_rn(a, P.rl));
+    const unsigned long long rem = (unsigned long long)__double_as_longlong(__fma_rn(-q, P.l, a)) & 0x7fffffffffffffffull;
+    const unsigned long long qb = (unsigned long long)__double_as_longlong(q), lb = (unsigned long long)__double_as_longlong(P.l);
+    const int ea = (int)(__double2hiint(a) >> 20 & 0x7ff), eq = (int)(qb >> 52 & 0x7ff), el = (int)(lb >> 52 & 0x7ff);
+    // half an ulp of q times |l|, less 2^-19 of it; half that at a power of two
+    const long long half = (long long)(lb & 0x7fffffffffffffffull) - (1ll << 34) +
+                           ((long long)(eq - 1023 - 53 - ((qb << 12) == 0)) << 52);
+    sure &= (unsigned)(ea - 623) <= 800u && (unsigned)(el - 623) <= 800u && (long long)rem < half;
+    return q;
+}
+
+// the Cholesky factor of one date's normal equations
+struct FitFactor {
+    Pivot p1, p2, p3;
+    double l21, l31, l32;
+    int ok;
+};
+
+// one contract's policy at a date: coefficients and screen
+struct FitPolicy {
+    double b[3], df; // df: the discount from this date to the one before
+    LsmScreen s;
+};
+
+// shared memory of one contract beside its paths
+constexpr size_t FIT_CONTRACT_BYTES = sizeof(LsmContract) + 2 * sizeof(FitFactor) + sizeof(FitPolicy) +
+                                      sizeof(unsigned) * FIT_SUMS * SUM_LIMBS + sizeof(int) * FIT_WARPS;
+
+__host__ __device__ inline size_t fit_control_bytes(int C) { return (FIT_CONTRACT_BYTES * (size_t)C + 15) & ~size_t(15); }
+
+// and of its paths: spots of two dates, then per contract cashflow, list moneyness and list index
+__host__ __device__ inline size_t fit_path_bytes(int C, int64_t ppc)
+{
+    return (size_t)ppc * (2 * sizeof(float) + (size_t)C * (2 * sizeof(double) + sizeof(uint16_t)));
+}
+
+// a float spot as a double, without the conversion's pass through the FP64 unit (out of line where
+// it is needed: the compiler would convert every spot and select)
+__device__ __noinline__ double widen_rare(float s) { return (double)s; }
+__device__ __forceinline__ double widen(float s)
+{
+    const unsigned b = (unsigned)__float_as_int(s), a = b & 0x7fffffffu;
+    if (a - 0x00800000u < 0x7f000000u)
+        return __hiloint2double((int)((a >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
+    return widen_rare(s); // zero, subnormal, infinite or NaN
+}
+
+// the warp's sums of four accumulators: halves of them change hands, so a lane adds 5 values where
+// four butterflies add 20; lanes 0, 8, 16, 24 are left with sums 0..3, which they add into dst
+__device__ __forceinline__ void warp_sum4(Fx128 (&q)[4], int lane, unsigned* dst, int n)
+{
+    auto swap = [](const Fx128& give, int o) {
+        Fx128 r;
+        r.lo = __shfl_xor_sync(0xffffffffu, (unsigned long long)give.lo, o);
+        r.hi = __shfl_xor_sync(0xffffffffu, (unsigned long long)give.hi, o);
+        return r;
+    };
+    const bool up = lane & 16, odd = lane & 8;
+    Fx128 k0 = up ? q[2] : q[0], k1 = up ? q[3] : q[1];
+    const Fx128 g0 = up ? q[0] : q[2], g1 = up ? q[1] : q[3];
+    fx_add(k0, swap(g0, 16));
+    fx_add(k1, swap(g1, 16));
+    Fx128 k = odd ? k1 : k0;
+    const Fx128 g = odd ? k0 : k1;
+    fx_add(k, swap(g, 8));
+#pragma unroll
+    for (int o = 4; o; o >>= 1) fx_add(k, swap(k, o));
+    const int i = lane >> 3;
+    if ((lane & 7) == 0 && i < n) {
+        constexpr unsigned L26 = (1u << 26) - 1;
+        unsigned* d = dst + i * SUM_LIMBS;
+        atomicAdd(d, (unsigned)k.lo & L26);
+        atomicAdd(d + 1, (unsigned)(k.lo >> 26) & L26);
+        atomicAdd(d + 2, (unsigned)((k.lo >> 52) | (k.hi << 12)) & L26);
+        atomicAdd(d + 3, (unsigned)(k.hi >> 14) & L26);
+        atomicAdd(d + 4, (unsigned)(k.hi >> 40));
+    }
+}
+
+// the limbs' value (each below 2^30: 16 warps), and the limbs cleared for the next date
+__device__ __forceinline__ Fx128 take_limbs(unsigned* d)
+{
+    Fx128 r = {d[0], 0};
+    fx_add(r, (uint64_t)d[1] << 26, 0);
+    fx_add(r, (uint64_t)d[2] << 52, (uint64_t)d[2] >> 12);
+    fx_add(r, 0, (uint64_t)d[3] << 14);
+    fx_add(r, 0, (uint64_t)d[4] << 40);
+#pragma unroll
+    for (int i = 0; i < SUM_LIMBS; i++) d[i] = 0;
+    return r;
+}
+
+// the factor of (X^T X) for X = {1, m, m^2}: Cholesky A = L L^T (maths.cpp:354-381), the
+// operations of a column loop in its order
+__device__ void factor3(double n, double s1, double s2, double s3, double s4, FitFactor& F)
+{
+    F.ok = 0;
+    if (n <= 0.0) return;
+    F.p1 = pivot(__dsqrt_rn(n));
+    F.l21 = __ddiv_rn(s1, F.p1.l);
+    F.l31 = __ddiv_rn(s2, F.p1.l);
+    const double p22 = __dsub_rn(s2, __dmul_rn(F.l21, F.l21));
+    if (p22 <= 0.0) return;
+    F.p2 = pivot(__dsqrt_rn(p22));
+    F.l32 = __ddiv_rn(__dsub_rn(s3, __dmul_rn(F.l31, F.l21)), F.p2.l);
+    const double p33 = __dsub_rn(__dsub_rn(s4, __dmul_rn(F.l31, F.l31)), __dmul_rn(F.l32, F.l32));
+    if (p33 <= 0.0) return;
+    F.p3 = pivot(__dsqrt_rn(p33));
+    F.ok = 1;
+}
+
+// beta of L L^T beta = g: forward, then back substitution (maths.cpp:419-470)
+template <class Divide>
+__device__ __forceinline__ void substitute3(const FitFactor& F, double g0, double g1, double g2, double* beta, Divide div)
+{
+    const double z0 = div(g0, F.p1);
+    const double z1 = div(__dsub_rn(g1, __dmul_rn(F.l21, z0)), F.p2);
+    const double z2 = div(__dsub_rn(__dsub_rn(g2, __dmul_rn(F.l31, z0)), __dmul_rn(F.l32, z1)), F.p3);
+    beta[2] = div(z2, F.p3);
+    beta[1] = div(__dsub_rn(z1, __dmul_rn(F.l32, beta[2])), F.p2);
+    beta[0] = div(__dsub_rn(__dsub_rn(z0, __dmul_rn(F.l21, beta[1])), __dmul_rn(F.l31, beta[2])), F.p1);
+}
+
+__device__ __noinline__ void substitute3_divisions(const FitFactor* F, double g0, double g1, double g2, double* beta)
+{
+    substitute3(*F, g0, g1, g2, beta, [](double a, const Pivot& P) { return __ddiv_rn(a, P.l); });
+}
+
+// what the walk's loops need of a contract, in registers (their stores to shared memory would make
+// every use of the contract there a load again)
+struct FitScreen {
+    int call, itm_bits, float_strike;
+    float strike_f, strike_lo, inv_norm_f;
+};
+__device__ __forceinline__ FitScreen screen_of(const LsmContract& K)
+{
+    return FitScreen{K.call, K.itm_bits, K.float_strike, K.strike_f, K.strike_lo, K.inv_norm_f};
+}
+
+// S - K in single precision, and 1 where it is exact and a normal number: where the strike is a
+// float that holds for S within a factor of two of K (and often beyond: the rounding error, the
+// two-sum's, is zero). It is then the double-precision difference.
+__device__ __forceinline__ int difference(float sf, const FitScreen& E, float& d)
+{
+    d = sf - E.strike_f;
+    const float bv = d - sf;
+    const float err = (sf - (d - bv)) - (E.strike_f + bv);
+    return (int)(err == 0.0f) & E.float_strike & (int)(((unsigned)__float_as_int(d) & 0x7fffffffu) - 0x00800000u < 0x7f000000u);
+}
+
+// the test that the screen leaves open, out of the walk's line
+__device__ __noinline__ bool exercises_exactly(float sf, const FitPolicy* Q, const LsmContract* K)
+{
+    return itm_value(sf, *K) >= continuation(Q->b[0], Q->b[1], Q->b[2], moneyness((double)sf, *K));
+}
+
+// IN_SMEM: the CTA's paths (spots of two dates, every contract's cashflows and in-the-money list)
+// live in shared memory, wherever they fit: 26 bytes a path of one contract, 18 more a contract. Else
+// in global memory, with the spots read from their rows.
+template <bool IN_SMEM>
+__global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArgs A)
+{
+    extern __shared__ __align__(16) unsigned char fit_smem[];
+    __shared__ Fx128 s_w[FIT_WARPS][LSM_NACC];
+    __shared__ int s_ok;
+    using Index = typename std::conditional<IN_SMEM, uint16_t, int32_t>::type;
     const int G = gridDim.x;
     const int C = A.C;
-    const int64_t T = (int64_t)G * LSM_THREADS;
-    const int64_t g0 = (int64_t)blockIdx.x * LSM_THREADS + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t gw = (int64_t)blockIdx.x * LSM_WARPS + warp; // global warp: paths gw 32 + lane + k T
-    const int64_t seg = gw * A.seg_len;
     const unsigned below = (1u << lane) - 1u;
+    LsmContract* const s_ct = reinterpret_cast<LsmContract*>(fit_smem);
+    FitFactor* const s_fac = reinterpret_cast<FitFactor*>(s_ct + C); // [2][C], by the parity of the date
+    FitPolicy* const s_pol = reinterpret_cast<FitPolicy*>(s_fac + 2 * C);
+    unsigned* const s_limb = reinterpret_cast<unsigned*>(s_pol + C); // [C][FIT_SUMS][SUM_LIMBS]
+    int* const s_nout = reinterpret_cast<int*>(s_limb + C * FIT_SUMS * SUM_LIMBS); // [C][FIT_WARPS]
+    unsigned char* const paths = fit_smem + fit_control_bytes(C);
+    float* const s_spot = reinterpret_cast<float*>(paths);                              // [2][ppc]
+    double* const s_cf = reinterpret_cast<double*>(paths + 2 * sizeof(float) * A.ppc);  // [C][2][ppc]
+    uint16_t* const s_idx = reinterpret_cast<uint16_t*>(s_cf + 2 * (size_t)C * A.ppc);  // [C][ppc]
+
+    // this CTA's paths: [p0, p0 + len); a warp's: [la, lb) of them, whole chunks of 32 (the last
+    // may end early). The factorer and the solver on scheduler 0 issue FP64 work worth
+    // FIT_SOLVER_CHUNKS chunks of a contract a date, so that scheduler's three walkers take that much
+    // less than the five, four and four of the others (2^20 paths x 365 dates, fit alone: 0 chunks
+    // 5.83 ms, 12 5.70, 24 5.54, 40 5.79).
+    const int64_t p0 = (int64_t)blockIdx.x * A.ppc;
+    const int len = (int)max((int64_t)0, min(A.ppc, A.n - p0));
+    int la, lb;
+    {
+        const int chunks = (len + 31) / 32;
+        const int first = max(0, (chunks - 3 * ((FIT_SOLVER_CHUNKS + C - 1) / C)) / 4); // scheduler 0's
+        const int s = warp & 3, k = s ? warp >> 2 : (warp >> 2) - 2, of = s == 0 ? 3 : (s == 1 ? 5 : 4);
+        const int from = s ? first + (chunks - first) * (s - 1) / 3 : 0;
+        const int to = s ? first + (chunks - first) * s / 3 : first;
+        la = 32 * (from + (to - from) * k / of);
+        lb = min(len, 32 * (from + (to - from) * (k + 1) / of));
+    }
     bool bad = false;
-    for (int c = threadIdx.x; c < C; c += LSM_THREADS) s_ct[c] = A.ct[c];
+
+    for (int c = threadIdx.x; c < C; c += FIT_THREADS) s_ct[c] = A.ct[c];
+    for (int i = threadIdx.x; i < C * FIT_SUMS * SUM_LIMBS; i += FIT_THREADS) s_limb[i] = 0;
+    if (threadIdx.x == 0) s_ok = 1;
     __syncthreads();
 
-    // maturity: each contract's cashflow is its payoff, and its value if never exercised earlier
-    for (int c = 0; c < C; ++c) {
-        const LsmContract K = s_ct[c];
-        Fx128 eu = {0, 0};
-        const float* row = A.S + (int64_t)(K.M - 1) * A.ld;
-        const double dT = K.disc[K.M - 1];
-        for (int64_t p = g0; p < A.n; p += T) {
-            const double iv = intrinsic((double)row[p], K.strike, K.call);
-            const double v = __dmul_rn(iv, dT);
-            K.cf[p] = iv;
-            K.val[p] = v;
-            fx_add_checked(eu, v, bad);
-        }
-        block_sum(eu, s_w, 2, K.acc + (size_t)blockIdx.x * LSM_NACC + 2);
-    }
+    auto spots = [&](int t) -> const float* { // date t's spots of this CTA
+        if constexpr (IN_SMEM) return s_spot + (size_t)(t & 1) * A.ppc;
+        return A.S + (int64_t)t * A.ld + p0;
+    };
+    auto cashflows = [&](const LsmContract& K, int c) -> double* {
+        if constexpr (IN_SMEM) return s_cf + (size_t)(2 * c) * A.ppc;
+        return K.cf + p0;
+    };
+    auto list_m = [&](const LsmContract& K, int c) -> double* {
+        if constexpr (IN_SMEM) return s_cf + (size_t)(2 * c + 1) * A.ppc + la;
+        return K.c_m + p0 + la;
+    };
+    auto list_idx = [&](const LsmContract& K, int c) -> Index* {
+        if constexpr (IN_SMEM) return s_idx + (size_t)c * A.ppc + la;
+        else return K.c_idx + p0 + la;
+    };
 
-    unsigned phase = 0; // dates done
-    for (int t = A.Tmax - 2; t >= 1; --t) {
-        const float* row = A.S + (int64_t)t * A.ld;
-        // every contract whose exercise grid reaches date t: discount, queue, sum, publish
-        for (int c = 0; c < C; ++c) {
-            const LsmContract K = s_ct[c];
-            if (t > K.M - 2) continue;
-            const double d = K.df[t];
-            Fx128 q[LSM_NQ];
-#pragma unroll
-            for (int i = 0; i < LSM_NQ; i++) q[i] = Fx128{0, 0};
-            // in-the-money paths queue until a full warp of them does the FP64 work (the
-            // warp's count qn and list length nout are uniform)
-            int qn = 0, nout = 0;
-            // each lane's next cashflow and spot are loaded one iteration ahead
-            double cf_next = gw * 32 + lane < A.n ? K.cf[gw * 32 + lane] : 0.0;
-            float s_next = gw * 32 + lane < A.n ? row[gw * 32 + lane] : 0.0f;
-            for (int64_t base = gw * 32; base < A.n; base += T) {
-                const int64_t p = base + lane;
-                const double cf_p = cf_next;
-                const float s_p = s_next;
-                if (p + T < A.n) {
-                    cf_next = K.cf[p + T];
-                    s_next = row[p + T];
-                }
-                bool itm = false;
-                float sf = 0.0f;
-                double y = 0.0;
-                if (p < A.n) {
-                    y = __dmul_rn(cf_p, d);
-                    K.cf[p] = y;
-                    sf = s_p;
-                    itm = in_the_money(sf, K);
-                }
-                const unsigned mk = __ballot_sync(0xffffffffu, itm);
-                if (itm) {
-                    const int k = qn + __popc(mk & below);
-                    q_idx[warp][k] = (int)p;
-                    q_s[warp][k] = sf;
-                    q_y[warp][k] = y;
-                }
-                qn += __popc(mk);
-                __syncwarp();
-                if (qn >= 32) {
-                    qn -= 32;
-                    const int k = qn + lane;
-                    itm_item(q_idx[warp][k], q_s[warp][k], q_y[warp][k], K, q, seg + nout + lane, bad);
-                    nout += 32;
-                    __syncwarp();
-                }
-            }
-            if (lane < qn) itm_item(q_idx[warp][lane], q_s[warp][lane], q_y[warp][lane], K, q, seg + nout + lane, bad);
-            nout += qn;
-#pragma unroll
-            for (int i = 0; i < LSM_NQ; i++) warp_sum(q[i]);
-            if (lane == 0) {
-#pragma unroll
-                for (int i = 0; i < LSM_NQ; i++) s_w[warp][i] = q[i];
-                s_w[warp][LSM_NQ] = Fx128{(uint64_t)nout, 0};
-                s_nout[warp][c] = nout;
-            }
-            __syncthreads();
-            if (threadIdx.x < LSM_PART) {
-                Fx128 sm = {0, 0};
-                for (int w = 0; w < LSM_WARPS; w++) fx_add(sm, s_w[w][threadIdx.x]);
-                fx_red3(K.tot + ((size_t)t * LSM_PART + threadIdx.x) * 3, sm);
-                __threadfence();
-            }
-            __syncthreads();
+    // the CTA's sums at `slot` of each contract into the totals of date t at `first`
+    auto publish = [&](int t, int slot, int first, int count, unsigned* bar) {
+        for (int x = lane; x < C * count; x += 32) {
+            const int c = x / count, i = x - c * count;
+            if (t > s_ct[c].M - 2) continue;
+            fx_red3(s_ct[c].tot + ((size_t)t * LSM_PART + first + i) * 3,
+                    take_limbs(s_limb + (c * FIT_SUMS + slot + i) * SUM_LIMBS));
         }
-        if (bad) atomicExch(A.status, 3);
-        ++phase;
-        if (threadIdx.x == 0) s_last = atomicAdd(A.bar, 1u) == phase * (unsigned)G - 1;
-        // while the regressions are solved: pull the next date's spots of this warp's paths
-        // into L2 (lane k takes the warp's k-th, (k+32)-th, ... line of 32 paths)
-        if (t > 1) {
-            const float* next = A.S + (int64_t)(t - 1) * A.ld;
-            for (int64_t pp = gw * 32 + (int64_t)lane * T; pp < A.n; pp += 32 * T) prefetch_l2(next + pp);
-        }
-        __syncthreads();
-        if (s_last) {
-            // the last CTA to publish rounds every active contract's sums (one thread a sum)
-            // and solves every contract's system (one thread a contract)
-            __threadfence();
-            for (int x = threadIdx.x; x < C * LSM_PART; x += LSM_THREADS) {
-                const int c = x / LSM_PART, i = x - c * LSM_PART;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicAdd(bar, 1u);
+    };
+    auto await = [&](const unsigned* bar, unsigned want) {
+        int ok = 1;
+        if (lane == 0) ok = wait_for(bar, want, A.status);
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp(); // lane 0's acquire orders the warp's reads of the totals
+        if (!ok) s_ok = 0;
+        return ok != 0;
+    };
+    auto total = [&](int c, int t, int i) { return fx_from3(s_ct[c].tot + ((size_t)t * LSM_PART + i) * 3); };
+
+    if (warp == FIT_FACTORER) {
+        // the moneyness sums of a date are complete while the CTAs still form its cashflow sums:
+        // the normal equations' matrix is factored beside them
+        unsigned phase = 0;
+        for (int t = A.Tmax - 2; t >= 1; --t) {
+            phase += (unsigned)G;
+            bar_sync<FIT_HANDOVER>(BAR_X + (t & 1));
+            publish(t, (t & 1) * FIT_X, 0, FIT_X, A.bar_x);
+            const bool ok = await(A.bar_x, phase);
+            for (int c = lane; ok && c < C; c += 32) {
                 if (t > s_ct[c].M - 2) continue;
-                const Fx128 v = fx_from3(s_ct[c].tot + ((size_t)t * LSM_PART + i) * 3);
-                s_tot[c][i] = i == LSM_NQ ? (double)v.lo : fx_to_double(v);
+                const Fx128 a1 = total(c, t, 0), a2 = total(c, t, 1), a3 = total(c, t, 2), a4 = total(c, t, 3);
+                const double n = (double)total(c, t, 4).lo;
+                FitFactor& F = s_fac[(t & 1) * C + c];
+                F.ok = 0;
+                if (n >= (double)s_ct[c].min_itm)
+                    factor3(n, fx_to_double(a1), fx_to_double(a2), fx_to_double(a3), fx_to_double(a4), F);
             }
-            __syncthreads();
-            for (int c = threadIdx.x; c < C; c += LSM_THREADS) {
-                const LsmContract K = s_ct[c];
+            bar_arrive<64>(BAR_FACTOR + (t & 1));
+            if (!ok) return;
+        }
+    } else if (warp == FIT_SOLVER) {
+        unsigned phase = 0;
+        for (int t = A.Tmax - 2; t >= 1; --t) {
+            phase += (unsigned)G;
+            bar_sync<FIT_HANDOVER>(BAR_Y);
+            publish(t, 2 * FIT_X, FIT_X, FIT_Y, A.bar_y);
+            bool ok = await(A.bar_y, phase);
+            bar_sync<64>(BAR_FACTOR + (t & 1));
+            ok = ok && *(volatile int*)&s_ok;
+            for (int c = lane; ok && c < C; c += 32) {
+                const LsmContract& K = s_ct[c];
                 if (t > K.M - 2) continue;
+                const Fx128 g0 = total(c, t, FIT_X), g1 = total(c, t, FIT_X + 1), g2 = total(c, t, FIT_X + 2);
                 double b[3] = {0.0, 0.0, 0.0};
-                const int f = s_tot[c][LSM_NQ] >= (double)K.min_itm && solve3(s_tot[c], b);
-                K.fit[t] = f;
-                K.beta[3 * t] = b[0];
-                K.beta[3 * t + 1] = b[1];
-                K.beta[3 * t + 2] = b[2];
-                s_fit[c] = f;
-                s_b[c][0] = b[0];
-                s_b[c][1] = b[1];
-                s_b[c][2] = b[2];
-                __threadfence();
+                const FitFactor& F = s_fac[(t & 1) * C + c];
+                const int f = F.ok;
+                const double df = K.df[t - 1];
+                if (f) {
+                    const double h0 = fx_to_double(g0), h1 = fx_to_double(g1), h2 = fx_to_double(g2);
+                    bool sure = true;
+                    substitute3(F, h0, h1, h2, b, [&](double a, const Pivot& P) { return divide_by(a, P, sure); });
+                    if (!sure) substitute3_divisions(&F, h0, h1, h2, b);
+                }
+                FitPolicy& Q = s_pol[c];
+                Q.s = lsm_screen(b, f, K.strike, K.norm, K.m0);
+                Q.df = df;
+                for (int i = 0; i < 3; i++) Q.b[i] = b[i];
+                if (blockIdx.x == 0) {
+                    K.fit[t] = f;
+                    for (int i = 0; i < 3; i++) K.beta[3 * t + i] = b[i];
+                }
             }
-            __syncthreads();
-            if (threadIdx.x == 0) st_release(A.done, phase);
-        } else {
-            if (threadIdx.x == 0) s_ok = wait_for(A.done, phase, A.status);
-            __syncthreads();
-            if (!s_ok) return;
-            for (int c = threadIdx.x; c < C; c += LSM_THREADS) {
-                const LsmContract K = s_ct[c];
+            bar_arrive<FIT_HANDOVER>(BAR_POLICY);
+            if (!ok) return;
+        }
+    } else {
+        // ---- the walkers -----------------------------------------------------------
+        auto request_spots = [&](int t) { // each thread copies the spots it will screen itself
+            if constexpr (IN_SMEM) {
+                float* const dst = s_spot + (size_t)(t & 1) * A.ppc;
+                const float* const row = A.S + (int64_t)t * A.ld + p0;
+                for (int l = la + lane; l < lb; l += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                     (unsigned)__cvta_generic_to_shared(dst + l)),
+                                 "l"(row + l)
+                                 : "memory");
+            }
+            if (t > 1) // the date after next: into L2
+                for (int l = la + 32 * lane; l < lb; l += 1024) prefetch_l2(A.S + (int64_t)(t - 1) * A.ld + p0 + l);
+        };
+        // the moneyness sums of date t for every contract whose exercise grid reaches it: list
+        // the in-the-money paths, then full warps of them do the FP64 work
+        auto moneyness_sums = [&](int t) {
+            if constexpr (IN_SMEM) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncwarp();
+            }
+            const float* const S = spots(t);
+            for (int c = 0; c < C; ++c) {
+                const LsmContract& K = s_ct[c];
                 if (t > K.M - 2) continue;
-                s_fit[c] = __ldcg(K.fit + t);
-                s_b[c][0] = __ldcg(K.beta + 3 * t);
-                s_b[c][1] = __ldcg(K.beta + 3 * t + 1);
-                s_b[c][2] = __ldcg(K.beta + 3 * t + 2);
+                Index* const idx = list_idx(K, c);
+                double* const lm = list_m(K, c);
+                const FitScreen E = screen_of(K);
+                int nout = 0;
+#pragma unroll 4
+                for (int l0 = la; l0 < lb; l0 += 32) {
+                    const int l = l0 + lane;
+                    const bool itm = l < lb && in_the_money(S[l < lb ? l : la], E);
+                    const unsigned mk = __ballot_sync(0xffffffffu, itm);
+                    if (itm) idx[nout + __popc(mk & below)] = (Index)l;
+                    nout += __popc(mk);
+                }
+                __syncwarp();
+                Fx128 q[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+                auto sums = [&](auto money) {
+                    for (int j = lane; j < nout; j += 32) {
+                        const double m = money(widen(S[idx[j]])), m2 = __dmul_rn(m, m);
+                        const double m3 = __dmul_rn(m2, m), m4 = __dmul_rn(m2, m2);
+                        lm[j] = m;
+                        fx_add_checked(q[0], m, bad);
+                        fx_add_checked(q[1], m2, bad);
+                        fx_add_checked(q[2], m3, bad);
+                        fx_add_checked(q[3], m4, bad);
+                    }
+                };
+                if (K.short_norm)
+                    sums([y = K.inv_norm, lo = K.inv_norm_lo](double s) { return moneyness_short(s, y, lo); });
+                else
+                    sums([&K](double s) { return moneyness(s, K); });
+                __syncwarp();
+                unsigned* const limb = s_limb + (c * FIT_SUMS + (t & 1) * FIT_X) * SUM_LIMBS;
+                warp_sum4(q, lane, limb, 4);
+                if (lane == 0) {
+                    s_nout[c * FIT_WARPS + warp] = nout;
+                    atomicAdd(limb + 4 * SUM_LIMBS, (unsigned)nout);
+                }
             }
-        }
-        __syncthreads();
-        // every active contract's exercise decision on its list
+        };
+        // every path through date t + 1's decision and to date t
+        auto roll = [&](int t) {
+            const float* const Sn = spots(t + 1);
+            for (int c = 0; c < C; ++c) {
+                const LsmContract& K = s_ct[c];
+                if (t > K.M - 2) continue;
+                const bool last = t == K.M - 2; // the date before maturity: no decision to take
+                const FitPolicy& Q = s_pol[c];
+                const double d = last ? K.df[t] : Q.df;
+                const bool decide = !last && Q.s.fit;
+                double* const cf = cashflows(K, c);
+                const LsmScreen P = Q.s;
+                const FitScreen E = screen_of(K);
+                const int sign = E.call ? 0 : (int)0x80000000; // K - S rounds to -(S - K)
+                int32_t* const tau = K.tau + p0;
+                // without a branch from the screen to the product, so that the chunks' chains of
+                // single-precision operations overlap and an FP64 instruction serves a whole warp
+                constexpr int U = 4;
+                for (int l0 = la + lane; l0 - lane < lb; l0 += 32 * U) {
+                    double v[U];
+                    float sf[U];
+                    int ex[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int l = min(l0 + 32 * u, lb - 1);
+                        v[u] = cf[l];
+                        sf[u] = Sn[decide ? l : 0];
+                    }
+                    if (decide) {
+                        int open = 0, rest = 0;
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            ex[u] = screen_exercise(sf[u], P, E) & -(int)((l0 + 32 * u < lb) & in_the_money(sf[u], E));
+                            open |= ex[u];
+                        }
+                        if (__any_sync(0xffffffffu, open < 0)) {
+#pragma unroll
+                            for (int u = 0; u < U; ++u)
+                                if (ex[u] < 0) ex[u] = exercises_exactly(sf[u], &Q, &K);
+                            __syncwarp();
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            float x;
+                            const int exact = difference(sf[u], E, x);
+                            const unsigned xb = (unsigned)__float_as_int(x);
+                            const int hi = (int)(((xb & 0x7fffffffu) >> 3) + 0x38000000u | (xb & 0x80000000u)) ^ sign;
+                            const bool now = ex[u] & exact;
+                            v[u] = __hiloint2double(now ? hi : __double2hiint(v[u]), now ? (int)(xb << 29) : __double2loint(v[u]));
+                            rest |= ex[u] & (exact ^ 1);
+                        }
+                        if (__any_sync(0xffffffffu, rest)) {
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                float x;
+                                if (ex[u] && !difference(sf[u], E, x)) v[u] = itm_value(sf[u], K);
+                            }
+                            __syncwarp();
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            if (ex[u]) tau[l0 + 32 * u] = t + 1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        v[u] = __dmul_rn(v[u], d);
+                        if (l0 + 32 * u < lb) cf[l0 + 32 * u] = v[u];
+                    }
+                }
+            }
+            __syncwarp();
+        };
+        // the cashflow sums of date t over the lists
+        auto cashflow_sums = [&](int t) {
+            for (int c = 0; c < C; ++c) {
+                const LsmContract& K = s_ct[c];
+                if (t > K.M - 2) continue;
+                const double* const cf = cashflows(K, c);
+                const Index* const idx = list_idx(K, c);
+                const double* const lm = list_m(K, c);
+                const int nout = s_nout[c * FIT_WARPS + warp];
+                Fx128 q[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+                for (int j = lane; j < nout; j += 32) {
+                    const double y = cf[idx[j]], m = lm[j], m2 = __dmul_rn(m, m);
+                    const double my = __dmul_rn(m, y), m2y = __dmul_rn(m2, y);
+                    fx_add_checked(q[0], y, bad);
+                    fx_add_checked(q[1], my, bad);
+                    fx_add_checked(q[2], m2y, bad);
+                }
+                __syncwarp();
+                warp_sum4(q, lane, s_limb + (c * FIT_SUMS + 2 * FIT_X) * SUM_LIMBS, FIT_Y);
+            }
+            if (bad) atomicExch(A.status, 3);
+        };
+
+        // maturity: each contract's cashflow is its payoff
         for (int c = 0; c < C; ++c) {
-            const LsmContract K = s_ct[c];
-            if (t > K.M - 2 || !s_fit[c]) continue;
-            const double b0 = s_b[c][0], b1 = s_b[c][1], b2 = s_b[c][2];
-            const double dt = K.disc[t];
-            const int nout = s_nout[warp][c];
-            // two entries a lane per pass, their loads issued together
-            for (int j = lane; j < nout; j += 64) {
-                const int64_t o0 = seg + j, o1 = o0 + 32;
-                const bool h1 = j + 32 < nout;
-                const double iv0 = K.c_iv[o0], m0 = K.c_m[o0];
-                const double iv1 = h1 ? K.c_iv[o1] : 0.0, m1 = h1 ? K.c_m[o1] : 0.0;
-                if (iv0 >= continuation(b0, b1, b2, m0)) {
-                    const int p = K.c_idx[o0];
-                    K.cf[p] = iv0;
-                    K.val[p] = __dmul_rn(iv0, dt);
-                }
-                if (h1 && iv1 >= continuation(b0, b1, b2, m1)) {
-                    const int p = K.c_idx[o1];
-                    K.cf[p] = iv1;
-                    K.val[p] = __dmul_rn(iv1, dt);
-                }
+            const LsmContract& K = s_ct[c];
+            const float* row = A.S + (int64_t)(K.M - 1) * A.ld + p0;
+            double* const cf = cashflows(K, c);
+            for (int l = la + lane; l < lb; l += 32) {
+                cf[l] = intrinsic((double)row[l], K.strike, K.call);
+                K.tau[p0 + l] = 0;
             }
         }
-        __syncthreads();
+        const int t0 = A.Tmax - 2;
+        if (t0 >= 1) {
+            request_spots(t0);
+            moneyness_sums(t0);
+            bar_arrive<FIT_HANDOVER>(BAR_X + (t0 & 1));
+        }
+        for (int t = t0; t >= 1; --t) {
+            if (t < t0) {
+                bar_sync<FIT_HANDOVER>(BAR_POLICY);
+                if (!s_ok) return;
+            }
+            roll(t);
+            // date t + 1's spots have been used: date t - 1's take their place
+            if (t > 1) request_spots(t - 1);
+            cashflow_sums(t);
+            bar_arrive<FIT_HANDOVER>(BAR_Y);
+            if (t > 1) { // the next date's moneyness sums, while this date's policy is found
+                moneyness_sums(t - 1);
+                bar_arrive<FIT_HANDOVER>(BAR_X + ((t - 1) & 1));
+            }
+        }
+        if (t0 >= 1) {
+            bar_sync<FIT_HANDOVER>(BAR_POLICY);
+            if (!s_ok) return;
+        }
     }
 
+    // the value of each path's earliest exercise (date 1's decision here), else of its maturity
     for (int c = 0; c < C; ++c) {
-        const LsmContract K = s_ct[c];
-        Fx128 v = {0, 0}, v2 = {0, 0};
-        for (int64_t p = g0; p < A.n; p += T) {
-            const double x = K.val[p];
-            fx_add_checked(v, x, bad);
-            fx_add_checked(v2, __dmul_rn(x, x), bad);
+        const LsmContract& K = s_ct[c];
+        Fx128 v = {0, 0}, v2 = {0, 0}, eu = {0, 0};
+        if (warp != FIT_FACTORER && warp != FIT_SOLVER) {
+            const bool decide = K.M > 2 && s_pol[c].s.fit;
+            const float* const S1 = spots(1);
+            const float* const last = A.S + (int64_t)(K.M - 1) * A.ld + p0;
+            const double dT = K.disc[K.M - 1];
+            for (int l = la + lane; l < lb; l += 32) {
+                int t = K.tau[p0 + l];
+                if (decide && in_the_money(S1[l], K)) {
+                    const FitPolicy& Q = s_pol[c];
+                    int ex = screen_exercise(S1[l], Q.s, K);
+                    if (ex < 0) ex = exercises_exactly(S1[l], &Q, &K);
+                    if (ex) t = 1;
+                }
+                const double e = __dmul_rn(intrinsic((double)last[l], K.strike, K.call), dT);
+                const double x = t ? __dmul_rn(itm_value(A.S[(int64_t)t * A.ld + p0 + l], K), K.disc[t]) : e;
+                fx_add_checked(v, x, bad);
+                fx_add_checked(v2, __dmul_rn(x, x), bad);
+                fx_add_checked(eu, e, bad);
+            }
         }
-        Fx128* acc = K.acc + (size_t)blockIdx.x * LSM_NACC;
+        Fx128* const acc = K.acc + (size_t)blockIdx.x * LSM_NACC;
         block_sum(v, s_w, 0, acc);
         block_sum(v2, s_w, 1, acc + 1);
+        block_sum(eu, s_w, 2, acc + 2);
     }
     if (bad) atomicExch(A.status, 3);
 }
@@ -456,7 +783,7 @@ constexpr int APPLY_UNROLL = 8; // dates whose spots one thread loads together
 
 __global__ void __launch_bounds__(LSM_THREADS) lsm_apply_kernel(const LsmArgs A)
 {
-    __shared__ Fx128 s_w[LSM_WARPS][LSM_PART];
+    __shared__ Fx128 s_w[LSM_WARPS][LSM_NACC];
     const int64_t T = (int64_t)gridDim.x * LSM_THREADS;
     const int64_t g0 = (int64_t)blockIdx.x * LSM_THREADS + threadIdx.x;
     bool bad = false;
@@ -477,9 +804,10 @@ __global__ void __launch_bounds__(LSM_THREADS) lsm_apply_kernel(const LsmArgs A)
             for (int u = 0; u < APPLY_UNROLL; ++u) {
                 const int tu = t + u;
                 if (tu >= tend) break;
-                const float4 b = __ldg(A.screen + tu);
-                if (b.w == 0.f || !in_the_money(sv[u], A)) continue;
-                int ex = screen_exercise(sv[u], b.x, b.y, b.z, A);
+                if (!in_the_money(sv[u], A)) continue;
+                const LsmScreen P = A.screen[tu];
+                if (!P.fit) continue;
+                int ex = screen_exercise(sv[u], P, A);
                 if (ex < 0)
                     ex = itm_value(sv[u], A) >= continuation(A.beta[3 * tu], A.beta[3 * tu + 1], A.beta[3 * tu + 2],
                                                              moneyness((double)sv[u], A));
@@ -504,19 +832,43 @@ __global__ void __launch_bounds__(LSM_THREADS) lsm_apply_kernel(const LsmArgs A)
 
 } // namespace
 
-int lsm_fit_max_grid(int sms)
+// dynamic shared memory of a fit whose CTAs walk ppc paths each (in_smem: the paths' too)
+static size_t fit_smem(int C, int64_t ppc, bool in_smem)
 {
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lsm_fit_kernel, LSM_THREADS, 0) != cudaSuccess) return 0;
-    return per * sms;
+    return fit_control_bytes(C) + (in_smem ? fit_path_bytes(C, ppc) : 0);
 }
 
-cudaError_t launch_lsm_fit(const LsmFitArgs& A, int grid, cudaStream_t st)
+cudaError_t lsm_fit_shape(int64_t n, int C, int sms, LsmFitShape* out)
+{
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes at;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, lsm_fit_kernel<true>);
+    if (e != cudaSuccess) return e;
+    // one CTA an SM, all resident
+    const int64_t want = (n + FIT_MIN_PATHS - 1) / FIT_MIN_PATHS;
+    out->grid = (int)(want < 1 ? 1 : (want < sms ? want : sms));
+    out->ppc = ((n + out->grid - 1) / out->grid + 31) / 32 * 32;
+    out->in_smem = fit_smem(C, out->ppc, true) + at.sharedSizeBytes <= (size_t)most;
+    const size_t smem = fit_smem(C, out->ppc, out->in_smem);
+    const void* fn = out->in_smem ? reinterpret_cast<const void*>(lsm_fit_kernel<true>)
+                                  : reinterpret_cast<const void*>(lsm_fit_kernel<false>);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most - (int)at.sharedSizeBytes));
+    int per = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, FIT_THREADS, smem);
+    if (e == cudaSuccess && per < 1) e = cudaErrorLaunchOutOfResources;
+    return e;
+}
+
+cudaError_t launch_lsm_fit(const LsmFitArgs& A, const LsmFitShape& shape, cudaStream_t st)
 {
     LsmFitArgs a = A;
     void* args[] = {&a};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lsm_fit_kernel), dim3(grid), dim3(LSM_THREADS),
-                                       args, 0, st);
+    const void* fn = shape.in_smem ? reinterpret_cast<const void*>(lsm_fit_kernel<true>)
+                                   : reinterpret_cast<const void*>(lsm_fit_kernel<false>);
+    return cudaLaunchCooperativeKernel(fn, dim3(shape.grid), dim3(FIT_THREADS), args,
+                                       fit_smem(A.C, A.ppc, shape.in_smem), st);
 }
 
 cudaError_t launch_lsm_apply(const LsmArgs& A, int grid, cudaStream_t st)

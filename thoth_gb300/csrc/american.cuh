@@ -2,6 +2,7 @@
 // launchers (american.cu), shared with the host pass in thoth_gpu.cu.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <vector>
@@ -12,11 +13,44 @@
 
 constexpr int LSM_THREADS = 512;
 // regression sums of one date: sum m, m^2, m^3, m^4, y, y m, y m^2 over the in-the-money
-// paths (m = S / norm, y = discounted continuation), then the path count
-constexpr int LSM_NQ = 7;
-constexpr int LSM_PART = LSM_NQ + 1;
+// paths (m = S / norm, y = discounted continuation), with the path count behind the powers of m
+constexpr int LSM_PART = 8;
 // per-CTA result sums: discounted exercise values, their squares, discounted maturity payoffs
 constexpr int LSM_NACC = 3;
+
+// One date's exercise test in single precision (screen_exercise), with h = (S - K) / norm:
+// continuation a0 + a1 h + a2 h^2, and its error bound 2^-19 |iv| + e0 + e1 |h| + e2 h^2.
+struct LsmScreen {
+    float a0, a1, a2, e0, e1, e2;
+    int fit; // 1 where the date has a regression
+};
+
+// the screen of beta; m0 = (float) strike / norm. The expansion about the strike keeps the terms at
+// the size of the values that are compared: about 0 they are tens of times larger and cancel (near
+// the exercise boundary the polynomial hugs the payoff), and 4 % of the in-the-money paths of a daily
+// Heston put stayed open. The e's carry 2^-19 of each term (32 units of single precision; a term has
+// at most 10) and 2^-48 of the terms about 0, where the reference's own rounding and that of the
+// shift lie.
+__host__ __device__ inline LsmScreen lsm_screen(const double* beta, int fit, double strike, double norm, double m0)
+{
+    LsmScreen s;
+    const double a1 = fma(2.0 * beta[2], m0, beta[1]), a0 = fma(fma(beta[2], m0, beta[1]), m0, beta[0]);
+    s.a0 = (float)a0;
+    s.a1 = (float)a1;
+    s.a2 = (float)beta[2];
+    s.fit = fit;
+    constexpr float U = 0x1p-19f, D = 0x1p-48f;
+    const float k = fabsf((float)strike), q = fabsf((float)norm), m = fabsf((float)m0);
+    const float b0 = fabsf((float)beta[0]), b1 = fabsf((float)beta[1]), b2 = fabsf(s.a2);
+    s.e0 = U * (fabsf(s.a0) + fabsf((float)((double)(float)strike - strike))) + D * (2.0f * k + b0 + (b1 + b2 * m) * m) +
+           1e-30f;
+    s.e1 = U * fabsf(s.a1) + D * (q + b1 + 2.0f * b2 * m);
+    s.e2 = U * b2;
+    // far from single precision's range: the test stays open
+    if (!(fmaxf(fmaxf(fmaxf(fabsf(s.a0), fabsf(s.a1)), fmaxf(b0, b1)), fmaxf(fmaxf(k, q), fmaxf(b2, m))) < 1e30f))
+        s.e0 = INFINITY;
+    return s;
+}
 
 // The frozen-policy apply of one contract (lsm_apply_kernel).
 struct LsmArgs {
@@ -38,8 +72,9 @@ struct LsmArgs {
     Fx128* acc;           // [grid][LSM_NACC] per-CTA result sums
     int* status;          // 0 ok; 3 an addend out of range
     // apply only: the exercise test in single precision first (exercise_screened)
-    const float4* screen; // [M] b0, b1, b2 rounded to float; w = 1 where date t has a regression
+    const LsmScreen* screen; // [M]
     float strike_f;       // strike rounded to float
+    float strike_lo;      // strike_f - strike
     float inv_norm_f;     // 1 / norm rounded to float
 };
 
@@ -49,34 +84,46 @@ constexpr int LSM_MAX_CONTRACTS = 64;
 struct LsmContract {
     int M, call, min_itm, itm_bits; // as in LsmArgs
     double strike, norm, inv_norm;
+    double inv_norm_lo;             // 1 / norm - inv_norm, rounded to nearest
+    int short_norm;                 // norm has at most 45 significant bits (moneyness_short)
+    int float_strike;               // strike is a float
+    float strike_f, strike_lo, inv_norm_f; // as in LsmArgs
+    double m0;                      // strike_f / norm
     const double* df;               // [M]
     const double* disc;             // [M]
     double* beta;                   // [3M] out
     int* fit;                       // [M] out (zero at launch)
-    double *cf, *val;               // [n] scratch
-    int32_t* c_idx;                 // [n_list] compacted in-the-money lists, per warp
-    double *c_m, *c_iv;             // [n_list]
+    int32_t* tau;                   // [n] scratch: a path's earliest exercise date so far (0: none)
+    double* cf;                     // [n] scratch, as the lists only where the paths are not in
+    int32_t* c_idx;                 // shared memory: the cashflows; [n] each warp's in-the-money
+    double* c_m;                    // paths and [n] their moneyness
     unsigned long long* tot;        // [M][LSM_PART][3] per-date regression sums as 42/42/44-bit
                                     // limbs (zero at launch)
     Fx128* acc;                     // [grid][LSM_NACC] per-CTA result sums
 };
 
 // The batched fit: every contract fitted on the same stored paths in one launch, each date
-// one publish-and-release for all of them.
+// two publishes for all of them.
 struct LsmFitArgs {
     const float* S;
     int64_t ld, n;
     int C;                          // contracts, <= LSM_MAX_CONTRACTS
     int Tmax;                       // the largest M
     const LsmContract* ct;          // [C]
-    int64_t seg_len;                // list entries of one warp, 32 ceil(n / threads)
-    unsigned *bar, *done;           // arrivals and releases, all dates (zero at launch)
+    int64_t ppc;                    // paths of one CTA, a multiple of 32
+    unsigned *bar_x, *bar_y;        // CTAs that published their moneyness and their cashflow sums,
+                                    // all dates (zero at launch)
     int* status;                    // 0 ok; 2 a wait timed out; 3 an addend out of range
 };
 
-// the fit kernel is a cooperative launch: every CTA must be resident at once
-int lsm_fit_max_grid(int sms);
-cudaError_t launch_lsm_fit(const LsmFitArgs& A, int grid, cudaStream_t st);
+// The launch of a fit of C contracts on n paths: a cooperative launch, every CTA resident at once.
+struct LsmFitShape {
+    int grid = 0;
+    int64_t ppc = 0;      // LsmFitArgs::ppc
+    bool in_smem = false; // the paths' cashflows and lists fit in shared memory
+};
+cudaError_t lsm_fit_shape(int64_t n, int C, int sms, LsmFitShape* out);
+cudaError_t launch_lsm_fit(const LsmFitArgs& A, const LsmFitShape& shape, cudaStream_t st);
 cudaError_t launch_lsm_apply(const LsmArgs& A, int grid, cudaStream_t st);
 
 // One pass over the stored paths of one asset of a book (thoth_gpu.cu): a policy fitted and

@@ -71,16 +71,30 @@ FX_HD void fx_add(Fx128& a, double x)
     fx_add(a, lo, hi);
 }
 
-// add x when 0 <= x < FX_MAX_ADDEND, else set bad (negative, too large, inf or NaN):
-// integer tests on the bit pattern only
+// add x when 0 <= x < FX_MAX_ADDEND, else set bad (negative, too large, inf or NaN; the sum is
+// then worthless): integer tests on the bit pattern only. On the device without a branch: PTX
+// shifts by 64 or more give 0, so the left and the right shift of which only one applies are both
+// taken (by amounts that wrap to large ones where they do not apply) and combined. With branches
+// between the FP64 products of the callers, those ran several times a warp, for parts of it.
 FX_HD void fx_add_checked(Fx128& a, double x, bool& bad)
 {
     const uint64_t b = fx_bits(x);
+#ifdef __CUDA_ARCH__
+    bad |= b >= 0x4230000000000000ull && b != 0x8000000000000000ull;
+    const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+    const unsigned sh = (unsigned)((int)(b >> 52) & 0x7ff) - 1011u; // zero and subnormals: far below
+    unsigned long long l, r, hi;
+    asm("shl.b64 %0, %1, %2;" : "=l"(l) : "l"(mant), "r"(sh));
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(mant), "r"(0u - sh));
+    asm("shr.u64 %0, %1, %2;" : "=l"(hi) : "l"(mant), "r"(64u - sh));
+    fx_add(a, l | r, hi);
+#else
     if (b >= 0x4230000000000000ull) { // 2^36, or the sign bit set
         if ((b << 1) != 0) bad = true; // -0.0 adds nothing
         return;
     }
     fx_add(a, x);
+#endif
 }
 
 FX_HD int fx_clz64(uint64_t v)

@@ -1460,7 +1460,7 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + LSM_THREADS - 1) / LSM_THREADS,
                                                                  (int64_t)8 * g_dev.sms));
     const size_t tab = lsm_tab_bytes(M);
-    const size_t o_tab = 0, o_scr = align256(tab), scr_bytes = sizeof(float4) * (size_t)M;
+    const size_t o_tab = 0, o_scr = align256(tab), scr_bytes = sizeof(LsmScreen) * (size_t)M;
     const size_t o_acc = o_scr + align256(scr_bytes);
     const size_t acc_bytes = sizeof(Fx128) * (size_t)grid * LSM_NACC;
     const size_t o_ctl = o_acc + align256(acc_bytes);
@@ -1471,13 +1471,10 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     unsigned char* base = g_dev.lsm;
     unsigned char* h = g_dev.pinned;
     lsm_fill_tab(h, io);
-    // the single-precision screen of each date: b0, b1, b2 rounded to float, and 1 where the
-    // date has a regression (lsm_apply_kernel)
-    float4* scr = reinterpret_cast<float4*>(h + o_scr);
+    // the single-precision screen of each date
+    LsmScreen* scr = reinterpret_cast<LsmScreen*>(h + o_scr);
     for (int t = 0; t < M; t++)
-        scr[t] = io.fit_at[t] ? make_float4((float)io.beta[3 * (size_t)t], (float)io.beta[3 * (size_t)t + 1],
-                                            (float)io.beta[3 * (size_t)t + 2], 1.0f)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        scr[t] = lsm_screen(&io.beta[3 * (size_t)t], io.fit_at[t], io.strike, io.norm, (double)(float)io.strike / io.norm);
     cudaStream_t st = g_dev.stream;
     CUDA_TRY(cudaMemcpyAsync(base + o_tab, h, o_scr + scr_bytes, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(base + o_ctl, 0, sizeof(int), st));
@@ -1496,8 +1493,9 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     A.disc = A.df + M;
     A.beta = reinterpret_cast<double*>(base + o_tab) + 2 * (size_t)M;
     A.fit = reinterpret_cast<int*>(base + o_tab + sizeof(double) * 5 * (size_t)M);
-    A.screen = reinterpret_cast<const float4*>(base + o_scr);
+    A.screen = reinterpret_cast<const LsmScreen*>(base + o_scr);
     A.strike_f = (float)io.strike;
+    A.strike_lo = (float)((double)A.strike_f - io.strike);
     A.inv_norm_f = (float)A.inv_norm;
     A.acc = reinterpret_cast<Fx128*>(base + o_acc);
     A.status = reinterpret_cast<int*>(base + o_ctl);
@@ -1536,15 +1534,12 @@ int lsm_fit_batch_locked(const Plan& P, double sim_ms, LsmPass* const* io, int C
         Tmax = std::max(Tmax, io[k]->M);
     }
     const int64_t N = P.paths;
-    const int cap = lsm_fit_max_grid(g_dev.sms);
-    if (cap < 1) return fail(THOTH_GPU_E_CUDA, "no resident CTA for the exercise fit kernel");
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + LSM_THREADS - 1) / LSM_THREADS, cap));
-    const int64_t threads = (int64_t)grid * LSM_THREADS;
-    const int64_t seg_len = 32 * ((N + threads - 1) / threads);
-    const size_t n_list = (size_t)(grid * (LSM_THREADS / 32)) * (size_t)seg_len;
+    LsmFitShape shape;
+    CUDA_TRY(lsm_fit_shape(N, C, g_dev.sms, &shape));
+    const int grid = shape.grid;
     const size_t acc_bytes = sizeof(Fx128) * (size_t)grid * LSM_NACC;
-    // layout: [contracts][tables of every contract] (uploaded) | per contract: cf, val, lists,
-    // totals, result rows | control
+    // layout: [contracts][tables of every contract] (uploaded) | totals, control (zeroed) | per
+    // contract: exercise dates, result rows, and cashflows and lists where they are not shared
     size_t o = 0;
     auto take = [&](size_t bytes) {
         const size_t at = o;
@@ -1560,13 +1555,13 @@ int lsm_fit_batch_locked(const Plan& P, double sim_ms, LsmPass* const* io, int C
     for (int k = 0; k < C; k++) o_tot[k] = take(sizeof(unsigned long long) * 3 * (size_t)io[k]->M * LSM_PART);
     const size_t o_ctl = take(16);
     const size_t zero_bytes = o - o_zero;
-    std::vector<size_t> o_cf(C), o_val(C), o_cm(C), o_civ(C), o_cidx(C), o_acc(C);
+    std::vector<size_t> o_tau(C), o_cf(C), o_cm(C), o_cidx(C), o_acc(C);
     for (int k = 0; k < C; k++) {
-        o_cf[k] = take(sizeof(double) * (size_t)N);
-        o_val[k] = take(sizeof(double) * (size_t)N);
-        o_cm[k] = take(sizeof(double) * n_list);
-        o_civ[k] = take(sizeof(double) * n_list);
-        o_cidx[k] = take(sizeof(int32_t) * n_list);
+        const size_t own = shape.in_smem ? 0 : (size_t)N;
+        o_tau[k] = take(sizeof(int32_t) * (size_t)N);
+        o_cf[k] = take(sizeof(double) * own);
+        o_cm[k] = take(sizeof(double) * own);
+        o_cidx[k] = take(sizeof(int32_t) * own);
         o_acc[k] = take(acc_bytes);
     }
     rc = ensure_lsm(o);
@@ -1590,15 +1585,23 @@ int lsm_fit_batch_locked(const Plan& P, double sim_ms, LsmPass* const* io, int C
         K.strike = q.strike;
         K.norm = q.norm;
         K.inv_norm = 1.0 / q.norm;
+        K.inv_norm_lo = std::fma(-q.norm, K.inv_norm, 1.0) / q.norm;
+        uint64_t nb;
+        std::memcpy(&nb, &q.norm, sizeof nb);
+        K.short_norm = (nb & 0xff) == 0 && q.norm >= 0x1p-200 && q.norm <= 0x1p200;
+        K.strike_f = (float)q.strike;
+        K.strike_lo = (float)((double)K.strike_f - q.strike);
+        K.m0 = (double)K.strike_f / q.norm;
+        K.float_strike = (double)K.strike_f == q.strike;
+        K.inv_norm_f = (float)K.inv_norm;
         K.df = reinterpret_cast<const double*>(base + o_tab[k]);
         K.disc = K.df + M;
         K.beta = reinterpret_cast<double*>(base + o_tab[k]) + 2 * (size_t)M;
         K.fit = reinterpret_cast<int*>(base + o_tab[k] + sizeof(double) * 5 * (size_t)M);
+        K.tau = reinterpret_cast<int32_t*>(base + o_tau[k]);
         K.cf = reinterpret_cast<double*>(base + o_cf[k]);
-        K.val = reinterpret_cast<double*>(base + o_val[k]);
         K.c_idx = reinterpret_cast<int32_t*>(base + o_cidx[k]);
         K.c_m = reinterpret_cast<double*>(base + o_cm[k]);
-        K.c_iv = reinterpret_cast<double*>(base + o_civ[k]);
         K.tot = reinterpret_cast<unsigned long long*>(base + o_tot[k]);
         K.acc = reinterpret_cast<Fx128*>(base + o_acc[k]);
     }
@@ -1612,12 +1615,12 @@ int lsm_fit_batch_locked(const Plan& P, double sim_ms, LsmPass* const* io, int C
     A.C = C;
     A.Tmax = Tmax;
     A.ct = reinterpret_cast<const LsmContract*>(base + o_ct);
-    A.seg_len = seg_len;
-    A.bar = reinterpret_cast<unsigned*>(base + o_ctl);
-    A.done = reinterpret_cast<unsigned*>(base + o_ctl + 4);
+    A.ppc = shape.ppc;
+    A.bar_x = reinterpret_cast<unsigned*>(base + o_ctl);
+    A.bar_y = reinterpret_cast<unsigned*>(base + o_ctl + 4);
     A.status = reinterpret_cast<int*>(base + o_ctl + 8);
     CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
-    CUDA_TRY(launch_lsm_fit(A, grid, st));
+    CUDA_TRY(launch_lsm_fit(A, shape, st));
     CUDA_TRY(cudaEventRecord(g_dev.ev1, st));
     size_t hb = 0;
     CUDA_TRY(cudaMemcpyAsync(h + hb, base + o_ctl + 8, sizeof(int), cudaMemcpyDeviceToHost, st));
