@@ -604,6 +604,17 @@ struct PairLane {
 
 __host__ __device__ constexpr size_t ring_bytes(int threads, int LD) { return LD > 2 ? sizeof(uint32_t) * (size_t)threads * LD : 0; }
 
+// a low word, past L1: a CTA reads each once, and what a Heston or LSV book's shared memory leaves
+// of L1 holds the step program, which every warp reads at every step (Heston grid of 2^20 paths 2714
+// -> 2653 us, LSV barrier books 712 -> 697). Books that leave more of it share the words of
+// neighbouring CTAs there (paths stored, 2^20 x 365 steps: 0.3 ms slower past L1).
+__device__ __forceinline__ uint32_t load_word(const uint32_t* p)
+{
+    uint32_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ void copy_word(uint32_t dst, const uint32_t* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n\tcp.async.commit_group;" ::"r"(dst), "l"(src) : "memory");
@@ -641,7 +652,7 @@ __device__ __forceinline__ PairLane<LD> pair_lane(const DevPlan& P, const uint2*
 }
 
 // the next entry's low word, and the load of the one LD (or LD - 1) ahead
-template <int T, int LD>
+template <int T, int LD, bool STREAM = false>
 __device__ __forceinline__ uint32_t next_word(PairLane<LD>& L)
 {
     uint32_t w;
@@ -655,7 +666,7 @@ __device__ __forceinline__ uint32_t next_word(PairLane<LD>& L)
     } else {
         w = L.cur;
         L.cur = L.nxt;
-        L.nxt = __ldg(L.lo);
+        L.nxt = STREAM ? load_word(L.lo) : __ldg(L.lo);
     }
     L.lo += T;
     return w;
@@ -708,7 +719,7 @@ __device__ __forceinline__ void pair_gauss2(const DevPlan& P, uint2* hs_base, Pa
     if (L.hs == L.hs_end) next_chunk<TB>(P, hs_base, L);
     const uint4 h = *reinterpret_cast<const uint4*>(L.hs);
     L.hs += 2;
-    const uint32_t w0 = next_word<T, LD>(L), w1 = next_word<T, LD>(L);
+    const uint32_t w0 = next_word<T, LD, true>(L), w1 = next_word<T, LD, true>(L);
     quantile_quad(h.x ^ w0, h.y ^ w0, h.z ^ w1, h.w ^ w1, z0, z1);
 }
 
@@ -830,10 +841,13 @@ __device__ __forceinline__ StepRec program_rec(const DevPlan& P, const Program& 
 }
 
 // FAST: the book is in Sobol mode with every dimension a Sobol dimension, and stores no paths.
-// There each step's record is loaded at the step: loading it one step ahead holds eight more
-// registers across the step and measured slower (2.93 against 2.75 ms for the 2^20-path Heston
-// grid). The other pass loads it one step ahead, which measured faster where the paths are
-// stored (GBM, 2^20 paths x 252 steps: 1.11 against 1.23 ms).
+// There a GBM or Heston pass requests the next step's record after the bridge, so that the model's
+// step covers the load and the bridge, where registers are shortest, does not hold it (2^20-path
+// Heston grid: at the step 2653 us, a whole step ahead 2930, after the bridge 2606; ragged batch
+// 28.1 and 27.0 ms). The LSV step has no registers left for it (4-name LSV book: at the step 14.3
+// ms, after the bridge 14.9), so its record is loaded at the step. The pass that is not FAST loads
+// it one step ahead, which measured faster where the paths are stored (GBM, 2^20 paths x 252 steps:
+// 1.11 against 1.23 ms).
 // AT: the pass is asset a0's of a multi-asset book; else the book's only asset. MODEL M_SEQ: the
 // asset's model is looked up (the passes of such books that are not FAST).
 //
@@ -872,6 +886,7 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const
             if (valid[p]) P.path_out[n[p] - (uint64_t)P.skip - 1] = P.s0[aid];
 
     constexpr bool DEEP = LD > 2;
+    constexpr bool LATE = FAST && !DEEP && !SEQ && MODEL != M_LSV; // see above
     StepRec rec; // the next step's record
     const BridgeNode* const nodes = DEEP ? G.nodes : P.nodes;
     auto load_consts = [&](int i, float4& a, float4& b, float4& c, float4& d) {
@@ -889,7 +904,7 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const
             if (MODEL == M_LSV || (SEQ && model == M_LSV)) d = __ldg(cs + 3);
         }
     };
-    if constexpr (!FAST || DEEP) rec = program_rec<DEEP>(P, G, 1);
+    if constexpr (!FAST || DEEP || LATE) rec = program_rec<DEEP>(P, G, 1);
     // the draws of a node whose first dimension (factor 0) is dim
     auto draw = [&](int dim, float2& z0, float2& z1) {
         if constexpr (FAST && !AT && MODEL != M_GBM) {
@@ -902,11 +917,11 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const
     };
     for (int i = 1; i <= P.n_steps; ++i) {
         StepRec cur;
-        if constexpr (FAST && !DEEP) {
+        if constexpr (FAST && !DEEP && !LATE) {
             cur = load_rec(P, i);
         } else {
             cur = rec;
-            rec = program_rec<DEEP>(P, G, i + 1); // the record past the last step is padding
+            if constexpr (!LATE) rec = program_rec<DEEP>(P, G, i + 1); // the record past the last step is padding
         }
         // this step's constants, requested before the bridge work that covers their latency
         float4 c0 = u0, c1 = u1, c2 = u2, c3 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -981,6 +996,7 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const
                 nz1 = f2(quantile_u32(hash_u32(P.seed, n[0], d1)), quantile_u32(hash_u32(P.seed, n[1], d1)));
             }
         }
+        if constexpr (LATE) rec = program_rec<DEEP>(P, G, i + 1);
         // ---- the model's step of the log-spot (relative to S0) ----------------------
         float2 step;
         if (MODEL == M_GBM || (SEQ && model == M_GBM)) {
