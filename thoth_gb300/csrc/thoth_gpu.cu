@@ -1248,8 +1248,8 @@ Layout layout_of(const Plan& P, int grid)
     L.o_lo = (P.blob.bytes.size() + 255) & ~size_t(255);
     L.o_acc = L.o_lo + ((low_bytes(P) + 255) & ~size_t(255));
     L.o_out = L.o_acc + rows_bytes(P, grid);
-    L.o_st = L.o_out + ((sizeof(double) * n_acc + 255) & ~size_t(255));
-    L.total = L.o_st + 256;
+    L.o_st = L.o_out + sizeof(double) * n_acc; // behind the sums: one copy brings both back
+    L.total = (L.o_st + sizeof(int) + 255) & ~size_t(255);
     return L;
 }
 
@@ -1270,9 +1270,8 @@ int run_bound(Plan& P, unsigned char* base, const Layout& L, int grid, ThothBook
     CUDA_TRY(launch_book_alone(P.dp, P.variant, P.shape, grid, g_dev.sms, P.smem, st));
     CUDA_TRY(launch_reduce(P.dp.acc, grid, (int)n_acc, reinterpret_cast<double*>(base + L.o_out), st));
     CUDA_TRY(cudaEventRecord(g_dev.ev1, st));
-    CUDA_TRY(cudaMemcpyAsync(g_dev.pinned, base + L.o_out, sizeof(double) * n_acc, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(g_dev.pinned + sizeof(double) * n_acc, base + L.o_st, sizeof(int), cudaMemcpyDeviceToHost,
-                             st));
+    CUDA_TRY(cudaMemcpyAsync(g_dev.pinned, base + L.o_out, sizeof(double) * n_acc + sizeof(int),
+                             cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     float ms = 0;
     CUDA_TRY(cudaEventElapsedTime(&ms, g_dev.ev0, g_dev.ev1));
