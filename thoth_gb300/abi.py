@@ -296,45 +296,47 @@ class Book:
         na, npr = len(self.assets), len(self.products)
         A = (ThothAsset * max(na, 1))()
         for i, a in enumerate(self.assets):
-            A[i].model = a["model"]
-            A[i].spot = a["spot"]
-            A[i].carry = _ptr(a["carry"], C.c_double)
-            A[i].vol = a.get("vol", 0.0)
+            q = A[i]  # (indexing makes a new view each time)
+            q.model = a["model"]
+            q.spot = a["spot"]
+            q.carry = _ptr(a["carry"], C.c_double)
+            q.vol = a.get("vol", 0.0)
             for k in ("v0", "kappa", "theta", "xi", "rho"):
-                setattr(A[i], k, a.get(k, 0.0))
+                setattr(q, k, a.get(k, 0.0))
             if a["model"] == MODEL_LSV:
-                A[i].lev_points = a["lev_values"].shape[1]
-                A[i].lev_ln_step = _ptr(a["lev_ln_step"], C.c_double)
-                A[i].lev_offset = _ptr(a["lev_offset"], C.c_int64)
-                A[i].lev_values = _ptr(a["lev_values"], C.c_double)
+                q.lev_points = a["lev_values"].shape[1]
+                q.lev_ln_step = _ptr(a["lev_ln_step"], C.c_double)
+                q.lev_offset = _ptr(a["lev_offset"], C.c_int64)
+                q.lev_values = _ptr(a["lev_values"], C.c_double)
         P = (ThothProduct * max(npr, 1))()
         for i, p in enumerate(self.products):
-            P[i].kind = p["kind"]
-            P[i].option_type = p["option_type"]
-            P[i].asset = p["asset"]
-            P[i].maturity = p["maturity"]
-            P[i].strike = p["strike"]
-            P[i].zero_rate = p["zero_rate"]
-            P[i].fx = p["fx"]
-            P[i].quanto = p["quanto"]
-            if p["kind"] == BARRIER:
-                P[i].barrier_up = p["barrier_up"]
-                P[i].barrier_in = p["barrier_in"]
-                P[i].barrier_level = p["barrier_level"]
-                P[i].n_monitor = len(p["monitor"])
-                P[i].monitor = _ptr(p["monitor"], C.c_int32)
-            if p["kind"] == VARIANCE:
-                P[i].notional = p["notional"]
-                P[i].strike_variance = p["strike_variance"]
-                P[i].total_year_fraction = p["total_year_fraction"]
-                P[i].past_variance = p["past_variance"]
+            q, kind = P[i], p["kind"]
+            q.kind = kind
+            q.option_type = p["option_type"]
+            q.asset = p["asset"]
+            q.maturity = p["maturity"]
+            q.strike = p["strike"]
+            q.zero_rate = p["zero_rate"]
+            q.fx = p["fx"]
+            q.quanto = p["quanto"]
+            if kind == BARRIER:
+                q.barrier_up = p["barrier_up"]
+                q.barrier_in = p["barrier_in"]
+                q.barrier_level = p["barrier_level"]
+                q.n_monitor = len(p["monitor"])
+                q.monitor = _ptr(p["monitor"], C.c_int32)
+            if kind == VARIANCE:
+                q.notional = p["notional"]
+                q.strike_variance = p["strike_variance"]
+                q.total_year_fraction = p["total_year_fraction"]
+                q.past_variance = p["past_variance"]
                 if "obs" in p:
-                    P[i].n_obs = len(p["obs"])
-                    P[i].obs = _ptr(p["obs"], C.c_int32)
-            if p["kind"] == BASKET:
-                P[i].n_components = len(p["components"])
-                P[i].components = _ptr(p["components"], C.c_int32)
-                P[i].weights = _ptr(p["weights"], C.c_double)
+                    q.n_obs = len(p["obs"])
+                    q.obs = _ptr(p["obs"], C.c_int32)
+            if kind == BASKET:
+                q.n_components = len(p["components"])
+                q.components = _ptr(p["components"], C.c_int32)
+                q.weights = _ptr(p["weights"], C.c_double)
         d = ThothBookDesc()
         d.n_dates = self.n_dates
         d.days = _ptr(self.days, C.c_int32) if self.days is not None else None

@@ -317,12 +317,15 @@ bool build_bridge(const std::vector<double>& t, BridgeProgram& out, std::string&
         j = k + 1;
         if (j >= m) j = 0;
     }
-    // gap (left date, right date) -> build step; point date of each build step
-    std::map<std::pair<int, int>, int> gap;
-    std::vector<int> point(m);
+    // point date of each build step; the steps of each left date as a list (a right date halves the
+    // gap of the one before, so a list has log2(m) entries at most; an ordered map of the gaps took
+    // half of a plan's host time)
+    std::vector<int> point(m), of_left(m + 1, -1), next(m, -1);
     for (int i = 0; i < m; i++) {
         point[i] = bi[i] + 1;
-        if (i > 0) gap[{li[i], ri[i] + 1}] = i;
+        if (i == 0) continue;
+        next[i] = of_left[li[i]];
+        of_left[li[i]] = i;
     }
     auto node_of = [&](int s) {
         BridgeNode n;
@@ -335,6 +338,7 @@ bool build_bridge(const std::vector<double>& t, BridgeProgram& out, std::string&
     std::vector<int> stack; // pending dates
     out.prog.assign(m, StepProg{0, 0});
     out.nodes.clear();
+    out.nodes.reserve(m);
     int depth = 0;
     for (int i = 1; i <= m; i++) {
         StepProg sp{(int)out.nodes.size(), 0};
@@ -358,15 +362,16 @@ bool build_bridge(const std::vector<double>& t, BridgeProgram& out, std::string&
         }
         for (;;) {
             const int b = stack.back();
-            auto it = gap.find({i - 1, b});
-            if (it == gap.end()) {
+            int step = of_left[i - 1];
+            while (step >= 0 && ri[step] + 1 != b) step = next[step];
+            if (step < 0) {
                 err = "bridge program: no node for gap";
                 return false;
             }
-            out.nodes.push_back(node_of(it->second));
+            out.nodes.push_back(node_of(step));
             sp.count++;
-            if (point[it->second] == i) break;
-            stack.push_back(point[it->second]);
+            if (point[step] == i) break;
+            stack.push_back(point[step]);
         }
         depth = std::max(depth, (int)stack.size());
         out.prog[i - 1] = sp;
