@@ -20,9 +20,10 @@ constexpr int LSM_NACC = 3;
 
 // One date's exercise test in single precision (screen_exercise), with h = (S - K) / norm:
 // continuation a0 + a1 h + a2 h^2, and its error bound 2^-19 |iv| + e0 + e1 |h| + e2 h^2.
-struct LsmScreen {
+struct alignas(16) LsmScreen {
     float a0, a1, a2, e0, e1, e2;
     int fit; // 1 where the date has a regression
+    int pad;
 };
 
 // the screen of beta; m0 = (float) strike / norm. The expansion about the strike keeps the terms at
@@ -39,6 +40,7 @@ __host__ __device__ inline LsmScreen lsm_screen(const double* beta, int fit, dou
     s.a1 = (float)a1;
     s.a2 = (float)beta[2];
     s.fit = fit;
+    s.pad = 0;
     constexpr float U = 0x1p-19f, D = 0x1p-48f;
     const float k = fabsf((float)strike), q = fabsf((float)norm), m = fabsf((float)m0);
     const float b0 = fabsf((float)beta[0]), b1 = fabsf((float)beta[1]), b2 = fabsf(s.a2);
@@ -81,7 +83,7 @@ struct LsmArgs {
 // One contract of a batched fit: its exercise grid, payoff, discount tables, outputs and
 // scratch on the device.
 constexpr int LSM_MAX_CONTRACTS = 64;
-struct LsmContract {
+struct alignas(16) LsmContract {
     int M, call, min_itm, itm_bits; // as in LsmArgs
     double strike, norm, inv_norm;
     double inv_norm_lo;             // 1 / norm - inv_norm, rounded to nearest
