@@ -1084,7 +1084,7 @@ struct MinBlocks {
 // The work of one CTA of a book: tiles tile0, tile0 + tile_step, ... below P.n_tiles, every
 // product evaluated on each tile's paths, the FP64 sums in the row acc (zeroed here). A book's
 // own launch runs it with tile0 = blockIdx.x and tile_step = gridDim.x; the batch kernel runs
-// the same work items from a shared work list. Returns false when the cancel word stopped it.
+// the same work items from a shared work list. Returns false in thread 0 when it saw the cancel word set.
 template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
 __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_raw, int64_t tile0, int64_t tile_step,
                                           double* acc)
@@ -1134,8 +1134,10 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
         }
     }
 
-    // thread 0 reads the host-mapped cancel word one tile ahead, so its latency is not on the path
-    int cancel_ahead = (t == 0 && P.cancel != nullptr) ? *P.cancel : 0;
+    // thread 0 reads the host-mapped cancel word one tile ahead, so its latency is on no tile's path:
+    // a tile stops at the word read at the tile before, and the word read at the last tile counts
+    // when that tile is done (one-step GBM call 87 -> 78 us against a first tile that waits for it)
+    int cancel_ahead = 0;
     int ntile = 0;        // tiles done by this CTA
     int64_t nvalid = 0;   // valid paths of those tiles (few-product mode)
     for (int64_t tile = tile0; tile < P.n_tiles; tile += tile_step) {
@@ -1676,7 +1678,8 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
             acc[idx + 1] = d2 + 2.0 * c * d1 + n * c * c;
         }
     }
-    return true;
+    if (cancel_ahead) atomicExch(P.status, 1);
+    return !cancel_ahead;
 }
 
 template <int TB, int NA, int MODEL, bool UNIFORM, int PP, int LD = 2>
@@ -1706,13 +1709,14 @@ __global__ void __launch_bounds__((1 << TB) / PP, MinBlocks<TB, 1, PP>::value)
     static_assert(sizeof(DevPlan) % 8 == 0, "plans are copied in 8-byte words");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) DevPlan sp;
-    __shared__ int s_item, s_book, s_cur; // s_cur: the book whose plan is in sp
+    __shared__ int s_item, s_book, s_cur, s_stop; // s_cur: the book whose plan is in sp
     const int t = threadIdx.x;
     if (t == 0) s_cur = -1;
+    if (t == 0) s_stop = 0;
     for (;;) {
         __syncthreads(); // the previous item is done with shared memory
         if (t == 0) {
-            const int j = atomicAdd(next, 1);
+            const int j = s_stop ? n_items : atomicAdd(next, 1);
             int lo = 0;
             if (j < n_items) { // the last book whose first item is at or before j
                 int hi = n_books - 1;
@@ -1746,7 +1750,7 @@ __global__ void __launch_bounds__((1 << TB) / PP, MinBlocks<TB, 1, PP>::value)
         case 4: ok = book_body<TB, 1, M_HESTON, true, PP>(sp, smem_raw, r, bk.grid, acc); break;
         default: ok = book_body<TB, 1, M_GBM, true, PP>(sp, smem_raw, r, bk.grid, acc); break;
         }
-        if (!ok) break; // the book's cancel word is set: this CTA stops
+        if (t == 0) s_stop = !ok; // the cancel word is set: this CTA stops
     }
 }
 
