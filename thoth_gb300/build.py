@@ -34,7 +34,8 @@ FLAGS = {"kernels.cu": ["-ftz=true"], "book_batch.cu": ["-ftz=true"], "book_gbm.
          # oracle: no contraction of a * b + c into a fused multiply-add on the host
          "american_host.cu": ["-Xcompiler", "-ffp-contract=off"],
          "thoth_gpu.cu": ["-Xcompiler", "-ffp-contract=off"],
-         # the calibration ensemble rounds every expression as the reference does
+         # the book kernel's tail Gaussians round as the reference's do; the calibration writes its
+         # fused operations out
          "calib.cu": ["-fmad=false", "-Xcompiler", "-ffp-contract=off"]}
 
 

@@ -844,7 +844,7 @@ __device__ __forceinline__ StepRec program_rec(const DevPlan& P, const Program& 
 // There a GBM or Heston pass requests the next step's record after the bridge, so that the model's
 // step covers the load and the bridge, where registers are shortest, does not hold it (2^20-path
 // Heston grid: at the step 2653 us, a whole step ahead 2930, after the bridge 2606; ragged batch
-// 28.1 and 27.0 ms). The LSV step has no registers left for it (4-name LSV book: at the step 14.3
+// 28.1 and 27.0 ms). The LSV step has no registers left for it (5-name LSV book: at the step 14.3
 // ms, after the bridge 14.9), so its record is loaded at the step. The pass that is not FAST loads
 // it one step ahead, which measured faster where the paths are stored (GBM, 2^20 paths x 252 steps:
 // 1.11 against 1.23 ms).
