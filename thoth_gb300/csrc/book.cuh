@@ -399,21 +399,37 @@ __device__ __forceinline__ void bridge_step(const DevPlan& P, const Smem& S, con
 // step's record names (c3 = {1/ln_step, grid offset, first value as int bits}): the
 // layer's rows are uniform across the CTA and stay in L1 (staging the current layer in
 // shared memory measured slower)
+// SELECT: both ends select instead of branching, so that a thread's two lookups overlap (the pair
+// pass). The one-path loop of the other kernels branches (the correlated 5-name LSV book).
+template <bool SELECT>
 __device__ __forceinline__ void leverage(const DevPlan& P, int a, float4 c3, float x, float& L, float& dL)
 {
     const float2 mp = make_float2(c3.x, c3.y);
     const float* v = P.lev_values + __float_as_int(c3.z);
     const int npts = P.lev_points[a];
     const float f = fmaf(x, mp.x, mp.y);
-    // both ends select instead of branching, so that a thread's two lookups overlap
     const int last = npts - 1;
-    const int k = min(max((int)f, 0), last - 1);
-    const float w = f - (float)k;
-    const float v0 = __ldg(v + k), v1 = __ldg(v + k + 1);
-    const float mid = fmaf(w, v1 - v0, v0), slope = (v1 - v0) * mp.x;
-    const bool below = f <= 0.f, above = f >= (float)last;
-    L = below ? v0 : (above ? v1 : mid); // k is 0 below and last - 1 above
-    dL = below || above ? 0.f : slope;
+    if constexpr (SELECT) {
+        const int k = min(max((int)f, 0), last - 1);
+        const float w = f - (float)k;
+        const float v0 = __ldg(v + k), v1 = __ldg(v + k + 1);
+        const float mid = fmaf(w, v1 - v0, v0), slope = (v1 - v0) * mp.x;
+        const bool below = f <= 0.f, above = f >= (float)last;
+        L = below ? v0 : (above ? v1 : mid); // k is 0 below and last - 1 above
+        dL = below || above ? 0.f : slope;
+    } else if (f <= 0.f) {
+        L = __ldg(v);
+        dL = 0.f;
+    } else if (f >= (float)last) {
+        L = __ldg(v + last);
+        dL = 0.f;
+    } else {
+        const int k = (int)f;
+        const float w = f - (float)k;
+        const float v0 = __ldg(v + k), v1 = __ldg(v + k + 1);
+        L = fmaf(w, v1 - v0, v0);
+        dL = (v1 - v0) * mp.x;
+    }
 }
 
 __device__ __forceinline__ float intrinsic(const DevProduct& pr, float s)
@@ -929,8 +945,8 @@ __device__ __forceinline__ void pair_pass(const DevPlan& P, const Smem& S, const
         // LSV: the leverage at the step's start, requested before the bridge work (see book_kernel)
         float lvL[2] = {1.f, 1.f}, lvD[2] = {0.f, 0.f};
         if (MODEL == M_LSV || (SEQ && model == M_LSV)) {
-            leverage(P, aid, c3, X.x, lvL[0], lvD[0]);
-            leverage(P, aid, c3, X.y, lvL[1], lvD[1]);
+            leverage<true>(P, aid, c3, X.x, lvL[0], lvD[0]);
+            leverage<true>(P, aid, c3, X.y, lvL[1], lvD[1]);
         }
         // ---- Brownian bridge: normalised increments nz0 (spot), nz1 (variance) ----
         float2 nz0, nz1 = f2s(0.f);
@@ -1294,7 +1310,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                     const int ha = MODEL == M_SEQ ? a0 : 0;
                     if (MODEL == M_LSV || (MODEL == M_SEQ && P.model[ha] == M_LSV))
 #pragma unroll
-                        for (int p = 0; p < PP; ++p) leverage(P, ha, h3, x[p][0], lvL[p], lvD[p]);
+                        for (int p = 0; p < PP; ++p) leverage<false>(P, ha, h3, x[p][0], lvL[p], lvD[p]);
                 }
                 if (P.use_sobol) {
                     bridge_step<NA, T, PP, SEQ>(P, S, cur, sp, L, n, Wprev, top, nz, a0);
@@ -1397,7 +1413,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
                                     Lv = lvL[p];
                                     dL = lvD[p];
                                 } else {
-                                    leverage(P, aid, c3, x[p][a], Lv, dL);
+                                    leverage<false>(P, aid, c3, x[p][a], Lv, dL);
                                 }
                             }
                             const float s = vp + vc;
@@ -1444,7 +1460,8 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
 #pragma unroll
                     for (int p = 0; p < PP; ++p) {
                         const float step = stp[p];
-                        if ((cur.ev >> (4 * aid)) & 15u) apply_events(i, aid, t + p * TH, x[p][a], step, Wb[p][a], y[p][a]);
+                        // (any asset's events: its own bits cost the mixed kernel 5 %)
+                        if (cur.ev) apply_events(i, aid, t + p * TH, x[p][a], step, Wb[p][a], y[p][a]);
                         // stored paths: date-major, consecutive paths on consecutive threads
                         if (P.path_out && aid == P.path_asset && valid[p])
                             P.path_out[(size_t)i * P.path_ld + (n[p] - (uint64_t)P.skip - 1)] = P.s0[aid] * expf(x[p][a]);
