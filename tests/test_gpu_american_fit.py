@@ -61,3 +61,29 @@ def test_contracts_that_share_a_fit(gpu, paths, n):
         assert together[p]["premium"] == o["premium"] and together[p]["european"] == o["european"], p
         assert together[p]["fitted_dates"] == int(o["has_fit"].sum())
         np.testing.assert_array_equal(together[p]["beta"][:M][o["has_fit"]], o["beta"][o["has_fit"]])
+
+
+@pytest.mark.parametrize("paths,n,days,K,carry", [
+    (2, 1, DAYS, 1.0, 0.0),                              # one CTA, out of range on the first date walked
+    (128 * 152, 1, range(0, 91), 1.0, 0.0),              # every SM
+    (128 * 152 + 5, 1, range(0, 91), 1000.0 / 516, -2.0),  # in range at maturity, past it on the way to today
+    (300000, 3, range(0, 61), 1000.0 / 516, -2.0),       # contracts that share the launch
+    (120000, 20, range(0, 31), 1000.0 / 516, -2.0),      # paths in global memory
+])
+def test_moneyness_out_of_range_ends_the_fit(gpu, paths, n, days, K, carry):
+    """A call far in the money (m = S / K >= 512, so m^4 >= 2^36) is refused, whichever date and CTA
+    meets it first: every CTA's walkers and both its waiting warps leave the launch, on every repeat,
+    and the next fit is the same as before."""
+    good = vanilla_book(paths=5000)
+    before = gpu.price_american(good, 0)
+    b = abi.Book(days=np.asarray(list(days)), paths=paths)
+    a = b.add_gbm(1000.0, 0.3, carry)
+    for k in range(n):
+        b.add_vanilla(a, K * (1.0 + 0.001 * k), b.n_dates - 1 - k % 3, abi.CALL, zero_rate=0.02)
+    for _ in range(20):
+        with pytest.raises(gpu.ThothGpuError) as e:
+            gpu.price_american_book(b, list(range(n)), min_itm=1)
+        assert e.value.code == abi.THOTH_GPU_E_INVALID
+    after = gpu.price_american(good, 0)
+    assert after["premium"] == before["premium"] and after["trust"] == before["trust"]
+    np.testing.assert_array_equal(after["beta"], before["beta"])

@@ -118,7 +118,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 }
 
 // wait until *flag >= want; false (status 2) after 2 s, or soon when another CTA has failed: the
-// caller returns, so no wait outlives the limit
+// caller stops working and waits no more
 __device__ bool wait_for(const unsigned* flag, unsigned want, int* status)
 {
     const unsigned long long t0 = now_ns();
@@ -418,7 +418,10 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
 {
     extern __shared__ __align__(16) unsigned char fit_smem[];
     __shared__ Fx128 s_w[FIT_WARPS][LSM_NACC];
-    __shared__ int s_ok;
+    // What each of the two waiting warps tells the others when it gives up. s_stop, the solver's
+    // word for the whole CTA: set before the policy's barrier, read by the walkers behind it. s_lost,
+    // the factorer's: set before the factors' barrier, read by the solver behind it. Both stay set.
+    __shared__ int s_stop, s_lost;
     using Index = typename std::conditional<IN_SMEM, uint16_t, int32_t>::type;
     const int G = gridDim.x;
     const int C = A.C;
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
 
     for (int c = threadIdx.x; c < C; c += FIT_THREADS) s_ct[c] = A.ct[c];
     for (int i = threadIdx.x; i < C * FIT_SUMS * SUM_LIMBS; i += FIT_THREADS) s_limb[i] = 0;
-    if (threadIdx.x == 0) s_ok = 1;
+    if (threadIdx.x == 0) s_stop = s_lost = 0;
     __syncthreads();
 
     auto spots = [&](int t) -> const float* { // date t's spots of this CTA
@@ -492,11 +495,16 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
         if (lane == 0) ok = wait_for(bar, want, A.status);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         __syncwarp(); // lane 0's acquire orders the warp's reads of the totals
-        if (!ok) s_ok = 0;
         return ok != 0;
     };
+    // one reading for the warp of a word that another warp may be writing
+    auto told = [&](const int& word) { return __shfl_sync(0xffffffffu, *(const volatile int*)&word, 0) != 0; };
     auto total = [&](int c, int t, int i) { return fx_from3(s_ct[c].tot + ((size_t)t * LSM_PART + i) * 3); };
 
+    // A wait that fails takes no warp out of the loops: a named barrier counts its threads, so one
+    // that a warp no longer comes to would hold the others for good. Whoever gives up goes on through
+    // every barrier of the dates left without working, and all leave together behind the loops.
+    bool ok = true;
     if (warp == FIT_FACTORER) {
         // the moneyness sums of a date are complete while the CTAs still form its cashflow sums:
         // the normal equations' matrix is factored beside them
@@ -504,8 +512,12 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
         for (int t = A.Tmax - 2; t >= 1; --t) {
             phase += (unsigned)G;
             bar_sync<FIT_HANDOVER>(BAR_X + (t & 1));
-            publish(t, (t & 1) * FIT_X, 0, FIT_X, A.bar_x);
-            const bool ok = await(A.bar_x, phase);
+            ok = ok && !told(s_stop);
+            if (ok) {
+                publish(t, (t & 1) * FIT_X, 0, FIT_X, A.bar_x);
+                ok = await(A.bar_x, phase);
+                if (!ok) s_lost = 1;
+            }
             for (int c = lane; ok && c < C; c += 32) {
                 if (t > s_ct[c].M - 2) continue;
                 const Fx128 a1 = total(c, t, 0), a2 = total(c, t, 1), a3 = total(c, t, 2), a4 = total(c, t, 3);
@@ -516,17 +528,20 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
                     factor3(n, fx_to_double(a1), fx_to_double(a2), fx_to_double(a3), fx_to_double(a4), F);
             }
             bar_arrive<64>(BAR_FACTOR + (t & 1));
-            if (!ok) return;
         }
     } else if (warp == FIT_SOLVER) {
         unsigned phase = 0;
         for (int t = A.Tmax - 2; t >= 1; --t) {
             phase += (unsigned)G;
             bar_sync<FIT_HANDOVER>(BAR_Y);
-            publish(t, 2 * FIT_X, FIT_X, FIT_Y, A.bar_y);
-            bool ok = await(A.bar_y, phase);
+            if (ok) {
+                publish(t, 2 * FIT_X, FIT_X, FIT_Y, A.bar_y);
+                ok = await(A.bar_y, phase);
+            }
             bar_sync<64>(BAR_FACTOR + (t & 1));
-            ok = ok && *(volatile int*)&s_ok;
+            // (the factorer may be a date ahead: its word then stops the CTA a date early)
+            ok = ok && !told(s_lost);
+            if (!ok) s_stop = 1;
             for (int c = lane; ok && c < C; c += 32) {
                 const LsmContract& K = s_ct[c];
                 if (t > K.M - 2) continue;
@@ -551,7 +566,6 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
                 }
             }
             bar_arrive<FIT_HANDOVER>(BAR_POLICY);
-            if (!ok) return;
         }
     } else {
         // ---- the walkers -----------------------------------------------------------
@@ -731,23 +745,24 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
         for (int t = t0; t >= 1; --t) {
             if (t < t0) {
                 bar_sync<FIT_HANDOVER>(BAR_POLICY);
-                if (!s_ok) return;
+                ok = ok && !s_stop;
             }
-            roll(t);
-            // date t + 1's spots have been used: date t - 1's take their place
-            if (t > 1) request_spots(t - 1);
-            cashflow_sums(t);
+            if (ok) {
+                roll(t);
+                // date t + 1's spots have been used: date t - 1's take their place
+                if (t > 1) request_spots(t - 1);
+                cashflow_sums(t);
+            }
             bar_arrive<FIT_HANDOVER>(BAR_Y);
             if (t > 1) { // the next date's moneyness sums, while this date's policy is found
-                moneyness_sums(t - 1);
+                if (ok) moneyness_sums(t - 1);
                 bar_arrive<FIT_HANDOVER>(BAR_X + ((t - 1) & 1));
             }
         }
-        if (t0 >= 1) {
-            bar_sync<FIT_HANDOVER>(BAR_POLICY);
-            if (!s_ok) return;
-        }
+        if (t0 >= 1) bar_sync<FIT_HANDOVER>(BAR_POLICY);
     }
+    __syncthreads(); // every warp is out of the loops
+    if (s_stop) return;
 
     // the value of each path's earliest exercise (date 1's decision here), else of its maturity
     for (int c = 0; c < C; ++c) {
