@@ -141,3 +141,23 @@ def test_vanishing_vol_of_vol_keeps_its_errors_and_limits(gpu):
             continue
         L, _ = gpu.calibrate_leverage(c)
         np.testing.assert_allclose(L, oracle.calibrate_leverage(c), rtol=1e-9, atol=0)
+
+
+@pytest.mark.parametrize("particles", [300, 16384, 60000, 200000])  # few CTAs, most of the SMs, every one, in memory
+@pytest.mark.parametrize("heston", [
+    dict(v0=0.04, kappa=1.0, theta=0.04, xi=0.0, rho=0.0),  # no variance after the first step, on every CTA
+    dict(v0=1e9, kappa=2.0, theta=1e12, xi=1e5, rho=0.0),   # past 2^36 after some two weeks, CTA by CTA
+])
+def test_variance_out_of_range_ends_the_calibration(gpu, particles, heston):
+    """A variance that is not a number or past 2^36 is refused, whichever CTA meets it first and
+    wherever the others' waits are, on every repeat; the next calibration is the same as before."""
+    good = W.lsv_calibration(horizon_days=10, particles=particles)
+    before, _ = gpu.calibrate_leverage(good)
+    before = np.array(before)
+    for _ in range(20):
+        c = W.lsv_calibration(horizon_days=40, particles=particles, heston=heston)
+        with pytest.raises(gpu.ThothGpuError) as e:
+            gpu.calibrate_leverage(c)
+        assert e.value.code == abi.THOTH_GPU_E_INVALID
+    after, _ = gpu.calibrate_leverage(good)
+    np.testing.assert_array_equal(after, before)

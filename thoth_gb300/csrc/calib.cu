@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
     unsigned short* s_qi = reinterpret_cast<unsigned short*>(s_cnt);
     __shared__ int s_qn[2];    // how many
     __shared__ double s_bc[4]; // min ln S, bin width and its reciprocal, ensemble mean of v
-    __shared__ int s_ok; // 0: a wait failed; 1; 2: every particle at one spot
+    __shared__ int s_flat;             // every particle at one spot
+    __shared__ unsigned short s_span[2]; // the layer's points around the ensemble: first, one past the last
     const int T = G * CALIB_THREADS; // the CTAs past G have no particles and take no part in the rounds
     const int t = threadIdx.x, gt = blockIdx.x * CALIB_THREADS + t;
     const int lane = t & 31, warp = t >> 5;
@@ -493,8 +494,9 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
         // one thread a warp forms its share of the round's results: the bins' origin and width; their
         // reciprocal; the layer's points around the ensemble (below the lowest, above the highest);
         // the ensemble's mean
+        bool ok = true;
         if (lane == 0) {
-            const bool ok = wait_for(A.bar, round * (unsigned)G, A.status);
+            ok = wait_for(A.bar, round * (unsigned)G, A.status);
             if (ok && warp == 1) {
                 s_bc[3] = fx_to_double(fx_load3(A.vsum + 3 * (size_t)k)) * A.rP;
             } else if (ok) {
@@ -503,25 +505,24 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
                 if (warp == 0) {
                     s_bc[0] = gmn;
                     s_bc[1] = (gmx - gmn) * A.rbins;
-                    s_ok = gmx - gmn < 1e-10 ? 2 : 1;
+                    s_flat = gmx - gmn < 1e-10;
                 } else if (warp == 2) {
                     s_bc[2] = 1.0 / ((gmx - gmn) * A.rbins);
                 } else {
                     const double off = (double)A.offset[k], top = (double)A.points;
-                    s_min[0] = (long long)fmin(fmax(floor(fma(gmn, A.rln_step[k], -off)) - 1.0, 0.0), top - 1.0);
-                    s_max[0] = (long long)fmin(fmax(floor(fma(gmx, A.rln_step[k], -off)) + 3.0, 1.0), top);
+                    s_span[0] = (unsigned short)fmin(fmax(floor(fma(gmn, A.rln_step[k], -off)) - 1.0, 0.0), top - 1.0);
+                    s_span[1] = (unsigned short)fmin(fmax(floor(fma(gmx, A.rln_step[k], -off)) + 3.0, 1.0), top);
                 }
-            } else if (warp == 0) {
-                s_ok = 0;
             }
         }
-        __syncthreads();
-        if (!s_ok) return;
-        const bool flat = s_ok == 2;
+        // The four waits end apart, and where another CTA has failed some of them fail and others still
+        // find the count complete: the CTA goes on only if all four did, and so wrote their results
+        if (!__syncthreads_and(ok)) return;
+        const bool flat = s_flat != 0;
         const double bmn = s_bc[0], width = s_bc[1], rwidth = s_bc[2], fallback = s_bc[3];
         // the layer's points this CTA needs: those around the ensemble, or all to write out
-        const int i0 = writes ? 0 : (int)s_min[0];
-        const int i1 = writes ? A.points : (int)s_max[0];
+        const int i0 = writes ? 0 : s_span[0];
+        const int i1 = writes ? A.points : s_span[1];
 
         if (!flat) {
             // ---- round B: per-bin counts and sums of v ----
@@ -590,9 +591,8 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
             const double x0 = fma(0.5, width, bmn), ls = A.ln_step[k];
             const int64_t off = A.offset[k];
             for (int i = i0 + t; i < i1; i += CALIB_THREADS) s_layer[i] = ((double)(off + i) * ls - x0) * rwidth;
-            if (t == 0) s_ok = wait_for(A.bar, round * (unsigned)G, A.status);
-            __syncthreads();
-            if (!s_ok) return;
+            ok = t != 0 || wait_for(A.bar, round * (unsigned)G, A.status);
+            if (!__syncthreads_and(ok)) return;
             for (int b = t; b < bins; b += CALIB_THREADS) {
                 s_bsum[b] = fx_to_double(fx_load3(A.bsum + 3 * ((size_t)k * bins + b)));
                 s_cnt[b] = __ldcg(A.bcnt + (size_t)k * bins + b);
