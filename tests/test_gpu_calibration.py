@@ -161,3 +161,15 @@ def test_variance_out_of_range_ends_the_calibration(gpu, particles, heston):
         assert e.value.code == abi.THOTH_GPU_E_INVALID
     after, _ = gpu.calibrate_leverage(good)
     np.testing.assert_array_equal(after, before)
+
+
+def test_particles_lost_to_a_missing_local_vol_leave_the_others_as_they_are(gpu):
+    """Local vols that are not a number far below the money: the particles that come there are lost
+    (as the oracle's are), and the extremes, the bins and the layers of the others do not see them."""
+    c = W.lsv_calibration(horizon_days=30)
+    x = (c.offset[:, None] + np.arange(c.local_vol.shape[1])[None, :]) * c.ln_step[:, None]
+    c.local_vol = np.where(x < math.log(100.0) - 0.12, np.nan, c.local_vol)
+    L, _ = gpu.calibrate_leverage(c)
+    ref = oracle.calibrate_leverage(c)
+    assert np.isfinite(ref).any(axis=1).all() and np.isnan(ref).any()
+    np.testing.assert_allclose(L, ref, rtol=1e-9, atol=0, equal_nan=True)

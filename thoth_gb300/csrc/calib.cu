@@ -281,11 +281,16 @@ __device__ bool wait_for(const unsigned* flag, unsigned want, int* status)
     return true;
 }
 
-// a double's bit pattern as a signed integer with the same order
+// a double's bit pattern as a signed integer with the same order (not a number: not_a_number first)
 __device__ __forceinline__ long long order_key(double x)
 {
     const long long b = __double_as_longlong(x);
     return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+__device__ __forceinline__ bool not_a_number(double x)
+{
+    return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
 }
 
 __device__ __forceinline__ double from_key(long long k)
@@ -411,9 +416,11 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
                     q.lns = A.lns[p];
                     q.var = A.var[p];
                 }
-                const long long key = order_key(q.lns);
-                mn = min(mn, key);
-                mx = max(mx, key);
+                if (!not_a_number(q.lns)) { // a particle lost to a layer without a value moves no bin
+                    const long long key = order_key(q.lns);
+                    mn = min(mn, key);
+                    mx = max(mx, key);
+                }
                 fx_add_checked(sv, q.var, bad);
             }
 #pragma unroll
