@@ -173,3 +173,14 @@ def test_particles_lost_to_a_missing_local_vol_leave_the_others_as_they_are(gpu)
     ref = oracle.calibrate_leverage(c)
     assert np.isfinite(ref).any(axis=1).all() and np.isnan(ref).any()
     np.testing.assert_allclose(L, ref, rtol=1e-9, atol=0, equal_nan=True)
+
+
+def test_an_ensemble_lost_at_once_ends_at_the_upper_bound(gpu):
+    """Every particle outside the layer, at an end that has no local vol: no particle is left to form
+    a conditional variance, and the layers behind are the least variance's, at the upper bound."""
+    c = W.lsv_calibration(horizon_days=6, particles=300)
+    c.offset = np.ascontiguousarray(c.offset + 1000)  # the grid lies above the ensemble
+    c.local_vol[2, 0] = np.nan
+    L, _ = gpu.calibrate_leverage(c)
+    assert np.isnan(L[2, 0]) and np.isfinite(L[:2]).all()
+    assert (L[3:] == 10.0).all()

@@ -444,9 +444,11 @@ __global__ void __launch_bounds__(CALIB_THREADS, 4) lsv_calib_kernel(const Calib
                     cx = max(cx, s_max[w]);
                     fx_add(cs, s_sum[w]);
                 }
-                atomicMin(A.kmin + k, cm);
-                atomicMax(A.kmax + k, cx);
-                fx_red3(A.vsum + 3 * (size_t)k, cs);
+                if (cm <= cx) { // a CTA whose particles are all lost adds nothing
+                    atomicMin(A.kmin + k, cm);
+                    atomicMax(A.kmax + k, cx);
+                    fx_red3(A.vsum + 3 * (size_t)k, cs);
+                }
                 __threadfence();
             }
         }
