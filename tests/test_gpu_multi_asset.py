@@ -71,3 +71,32 @@ def test_assets_in_turn_slots_in_either_memory(gpu, models, n_products, paths, s
     for x in gpu.price_batch([b, book(models, 6, 200), b]):  # both books' slots in one batch buffer
         if len(x["premium"]) == n_products:
             assert np.array_equal(x["premium"], r["premium"]) and np.array_equal(x["trust"], r["trust"])
+
+
+def test_batch_slots_are_held_once_a_stream(gpu):
+    """Slots in global memory are a book's only while its kernel runs: a larger batch of such books
+    takes more plans, words and rows, but no more slots than its streams do, and prices as alone."""
+    import torch
+
+    def batch(n):
+        return [book(("lsv", "heston", "lsv", "gbm", "lsv"), 50, 2 ** 18, skip=k) for k in range(n)]
+
+    def grown(n):
+        gpu.debug_fail_allocations(0)  # drops the engine's working buffers
+        before = torch.cuda.mem_get_info()[0]
+        res = gpu.price_batch(batch(n))
+        return before - torch.cuda.mem_get_info()[0], res
+
+    b = batch(1)[0]
+    s = gpu.plan_summary(b)
+    assert s["variant"] == 6 and s["slots"] > 40
+    gpu.price_batch(batch(2))
+    # 1025 tiles on 513 CTAs at least (two tiles each)
+    slots = 4 * 257 * s["slots"] * 513
+    small, _ = grown(16)
+    large, res = grown(48)
+    assert large - small < 32 * slots / 2, (small, large, slots)
+    one = gpu.price_book(b)
+    np.testing.assert_array_equal(res[0]["premium"], one["premium"])
+    last = gpu.price_book(batch(48)[47])
+    np.testing.assert_array_equal(res[47]["premium"], last["premium"])

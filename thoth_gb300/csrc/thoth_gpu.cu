@@ -1227,19 +1227,24 @@ cudaError_t gather_low(const Plan& P, cudaStream_t st)
     return e;
 }
 
-// a book's per-CTA memory: its FP64 rows of sums, then (slots_global) its slots
+// a book's per-CTA memory: its FP64 rows of sums, and (slots_global) its slots, which only its
+// kernel uses
 size_t sums_bytes(const Plan& P, int grid) { return (sizeof(double) * (size_t)grid * P.dp.n_acc + 255) & ~size_t(255); }
-size_t rows_bytes(const Plan& P, int grid)
+size_t slots_bytes(const Plan& P, int grid)
 {
-    return sums_bytes(P, grid) + (P.slots_global ? (slot_row_bytes(P) * (size_t)grid + 255) & ~size_t(255) : 0);
+    return P.slots_global ? (slot_row_bytes(P) * (size_t)grid + 255) & ~size_t(255) : 0;
+}
+size_t rows_bytes(const Plan& P, int grid) { return sums_bytes(P, grid) + slots_bytes(P, grid); }
+
+// places them: regions of sums_bytes and slots_bytes bytes
+void bind_rows(Plan& P, unsigned char* sums, unsigned char* slots)
+{
+    P.dp.acc = reinterpret_cast<double*>(sums);
+    P.dp.slot_mem = P.slots_global ? reinterpret_cast<float*>(slots) : nullptr;
 }
 
-// places it at `rows` (a region of rows_bytes(P, grid) bytes)
-void bind_rows(Plan& P, unsigned char* rows, int grid)
-{
-    P.dp.acc = reinterpret_cast<double*>(rows);
-    P.dp.slot_mem = P.slots_global ? reinterpret_cast<float*>(rows + sums_bytes(P, grid)) : nullptr;
-}
+// one behind the other (a region of rows_bytes(P, grid) bytes)
+void bind_rows(Plan& P, unsigned char* rows, int grid) { bind_rows(P, rows, rows + sums_bytes(P, grid)); }
 
 // device layout of one priced book: [plan blob][low Sobol words][acc rows, slots][out][status]
 struct Layout {
@@ -1882,21 +1887,41 @@ static double item_cost(const Plan& P, int grid)
     return tiles * P.T * P.dp.n_steps * w;
 }
 
+// the books with launches of their own, on S streams at most by a longest-processing-time schedule:
+// books by decreasing path-steps, each onto the stream with the least work so far
+struct BatchSchedule {
+    std::vector<int> order;  // the books, as they are launched
+    std::vector<int> stream; // [n] each one's stream (-1: in the persistent launch)
+    int streams = 0;
+};
+
+static BatchSchedule batch_schedule(const std::vector<Plan>& plans, const std::vector<char>& member, int S, bool pers)
+{
+    BatchSchedule sc;
+    for (int b = 0; b < (int)plans.size(); b++)
+        if (!member[b]) sc.order.push_back(b);
+    std::stable_sort(sc.order.begin(), sc.order.end(),
+                     [&](int a, int c) { return batch_cost(plans[a]) > batch_cost(plans[c]); });
+    sc.streams = pers ? (int)std::min<size_t>(sc.order.size(), (size_t)S) : S;
+    sc.stream.assign(plans.size(), -1);
+    std::vector<double> load(std::max(sc.streams, 1), 0.0);
+    for (int b : sc.order) {
+        const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[k] += batch_cost(plans[b]);
+        sc.stream[b] = k;
+    }
+    return sc;
+}
+
 // the batch's device work as recorded into the graph: zero the status words (and the work
 // counter), then either the persistent launch with the other books on side streams, or each
-// book's gather, kernel and reduction on the stream chosen by a longest-processing-time
-// schedule (books by decreasing path-steps, each onto the stream with the least work so far)
+// book's gather, kernel and reduction on its stream
 static int record_batch(std::vector<Plan>& plans, const std::vector<int>& grid, const std::vector<size_t>& o_out,
-                        size_t o_sts, int S, cudaStream_t st, const BatchLaunch* BL)
+                        size_t o_sts, const BatchSchedule& sc, cudaStream_t st, const BatchLaunch* BL)
 {
     const int n = (int)plans.size();
     int launches = 0;
     CUDA_TRY(cudaMemsetAsync(g_batch.dev + o_sts, 0, sizeof(int) * (size_t)(n + 1), st));
-    std::vector<int> order;
-    for (int b = 0; b < n; b++)
-        if (!BL || !BL->member[b]) order.push_back(b);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int c) { return batch_cost(plans[a]) > batch_cost(plans[c]); });
     if (BL) {
         CUDA_TRY(launch_gather_low_batch(g_dev.sobol_lo, g_batch.dev + BL->o_gather, n, st));
         launches++;
@@ -1906,14 +1931,10 @@ static int record_batch(std::vector<Plan>& plans, const std::vector<int>& grid, 
                 launches++;
             }
     }
-    const int side = BL ? (int)std::min<size_t>(order.size(), (size_t)S) : S;
     CUDA_TRY(cudaEventRecord(g_batch.events[0], st));
-    for (int k = 0; k < side; k++) CUDA_TRY(cudaStreamWaitEvent(g_batch.streams[k], g_batch.events[0], 0));
-    std::vector<double> load(std::max(side, 1), 0.0);
-    for (int b : order) {
-        const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        load[k] += batch_cost(plans[b]);
-        cudaStream_t s = g_batch.streams[k];
+    for (int k = 0; k < sc.streams; k++) CUDA_TRY(cudaStreamWaitEvent(g_batch.streams[k], g_batch.events[0], 0));
+    for (int b : sc.order) {
+        cudaStream_t s = g_batch.streams[sc.stream[b]];
         if (!BL) {
             CUDA_TRY(gather_low(plans[b], s));
             launches += plans[b].dp.n_tail > 0 ? 2 : 1;
@@ -1933,7 +1954,7 @@ static int record_batch(std::vector<Plan>& plans, const std::vector<int>& grid, 
                                      BL->grid, BL->smem, st));
         launches++;
     }
-    for (int k = 0; k < side; k++) {
+    for (int k = 0; k < sc.streams; k++) {
         CUDA_TRY(cudaEventRecord(g_batch.events[k], g_batch.streams[k]));
         CUDA_TRY(cudaStreamWaitEvent(st, g_batch.events[k], 0));
     }
@@ -2014,13 +2035,22 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
                std::to_string(BL.items);
         for (int b : BL.books) sig += "," + std::to_string(b);
     }
-    // what is uploaded ends here; the books' low words, rows and slots are the device's own
+    // what is uploaded ends here; the books' low words and rows and the streams' slots are the
+    // device's own. Books on one stream run in turn and share its slots, so a batch holds at most
+    // as many regions as it has streams, whatever its size (at most SLOT_MAX_BYTES or so each).
     const size_t up_bytes = off;
     for (int b = 0; b < n; b++) {
         o_lo[b] = off;
         off += up(low_bytes(plans[b]));
         o_acc[b] = off;
-        off += rows_bytes(plans[b], grid[b]);
+        off += sums_bytes(plans[b], grid[b]);
+    }
+    const BatchSchedule sc = batch_schedule(plans, member, S, pers);
+    std::vector<size_t> o_slots(std::max(sc.streams, 1)), need(o_slots.size(), 0);
+    for (int b : sc.order) need[sc.stream[b]] = std::max(need[sc.stream[b]], slots_bytes(plans[b], grid[b]));
+    for (int k = 0; k < sc.streams; k++) {
+        o_slots[k] = off;
+        off += need[k];
     }
     // outputs and status words (then the work counter) contiguous at the end: one device->host copy
     const size_t o_outs = off;
@@ -2057,7 +2087,7 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         std::memcpy(g_batch.host + o_blob[b], plans[b].blob.bytes.data(), plans[b].blob.bytes.size());
         bind(plans[b], g_batch.dev + o_blob[b]);
         bind_low(plans[b], g_batch.dev + o_lo[b]);
-        bind_rows(plans[b], g_batch.dev + o_acc[b], grid[b]);
+        bind_rows(plans[b], g_batch.dev + o_acc[b], g_batch.dev + o_slots[std::max(sc.stream[b], 0)]);
         plans[b].dp.status = reinterpret_cast<int*>(g_batch.dev + o_st[b]);
         // the kernel parameters are baked into the graph: a replay needs them byte-equal
         sig.append(reinterpret_cast<const char*>(&plans[b].dp), sizeof(DevPlan));
@@ -2089,7 +2119,7 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
         // kernel attributes are set outside the capture
         for (int b = 0; b < n; b++) occupancy_of(plans[b]);
         CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        rc = record_batch(plans, grid, o_out, o_sts, S, st, pers ? &BL : nullptr);
+        rc = record_batch(plans, grid, o_out, o_sts, sc, st, pers ? &BL : nullptr);
         cudaGraph_t graph = nullptr;
         const cudaError_t ec = cudaStreamEndCapture(st, &graph); // always leave capture mode
         if (rc) {
