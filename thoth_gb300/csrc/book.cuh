@@ -1152,7 +1152,8 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
 
     // thread 0 reads the host-mapped cancel word one tile ahead, so its latency is on no tile's path:
     // a tile stops at the word read at the tile before, and the word read at the last tile counts
-    // when that tile is done (one-step GBM call 87 -> 78 us against a first tile that waits for it)
+    // when that tile is done (one-step GBM call 87 -> 78 us against a first tile that waits for it;
+    // a word set before the launch is the host's to see)
     int cancel_ahead = 0;
     int ntile = 0;        // tiles done by this CTA
     int64_t nvalid = 0;   // valid paths of those tiles (few-product mode)

@@ -1263,6 +1263,10 @@ Layout layout_of(const Plan& P, int grid)
     return L;
 }
 
+// a cancel requested before a call's launches ends it without them: a book kernel reads the word
+// while its first tile runs (book_body), so it would simulate a tile a CTA first
+bool cancel_requested() { return g_dev.ready && *(volatile int*)g_dev.cancel_host != 0; }
+
 // launch the book kernel and the reduction on a plan already bound to `base`,
 // copy the sums back and finalise the indicators
 int run_bound(Plan& P, unsigned char* base, const Layout& L, int grid, ThothBookResult* out, bool gather)
@@ -1274,6 +1278,7 @@ int run_bound(Plan& P, unsigned char* base, const Layout& L, int grid, ThothBook
     bind_low(P, base + L.o_lo);
     bind_rows(P, base + L.o_acc, grid);
     P.dp.status = reinterpret_cast<int*>(base + L.o_st);
+    if (cancel_requested()) return fail(THOTH_GPU_E_CANCELLED, "pricing cancelled");
     CUDA_TRY(cudaMemsetAsync(base + L.o_st, 0, sizeof(int), st));
     CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
     if (gather) CUDA_TRY(gather_low(P, st));
@@ -1739,8 +1744,8 @@ static int price_noalloc_locked(const ThothBookDesc* book, ThothBookResult* out)
     // call prices on that device as they do; before that, on the calling thread's current one
     if (g_dev.ready) CUDA_TRY(cudaSetDevice(g_dev.id));
     CUDA_TRY(cudaGetDevice(&dev));
-    // a cancel requested before the call ends it here, as at the first tile of the other entry points
-    if (g_dev.ready && *(volatile int*)g_dev.cancel_host) return fail(THOTH_GPU_E_CANCELLED, "pricing cancelled");
+    // a cancel requested before the call ends it here, as before the launches of the other entry points
+    if (cancel_requested()) return fail(THOTH_GPU_E_CANCELLED, "pricing cancelled");
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
     if (!(prop.major == 10 && prop.minor == 3))
@@ -2110,6 +2115,7 @@ static int price_batch_locked(const ThothBookDesc* books, int n, ThothBookResult
             std::memcpy(g_batch.host + BL.o_reduce + sizeof(BatchReduce) * (size_t)b, &r, sizeof r);
         }
     }
+    if (cancel_requested()) return fail(THOTH_GPU_E_CANCELLED, "pricing cancelled");
     cudaStream_t st = g_dev.stream;
     CUDA_TRY(cudaMemcpyAsync(g_batch.dev, g_batch.host, up_bytes, cudaMemcpyHostToDevice, st));
     if (g_batch.signature != sig || !g_batch.exec) {
@@ -2219,6 +2225,7 @@ static int autotune_book_locked(const ThothBookDesc* book, int reps, ThothTuneRe
         P.dp.status = reinterpret_cast<int*>(g_dev.arena + L.o_st);
         for (size_t c = 0; c < grids.size(); c++) {
             const int g = grids[c];
+            if (cancel_requested()) return fail(THOTH_GPU_E_CANCELLED, "autotune cancelled");
             CUDA_TRY(cudaMemsetAsync(g_dev.arena + L.o_st, 0, sizeof(int), st));
             CUDA_TRY(launch_book_alone(P.dp, P.variant, P.shape, g, g_dev.sms, P.smem, st)); // warm-up
             CUDA_TRY(cudaEventRecord(g_dev.ev0, st));
