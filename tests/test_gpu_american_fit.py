@@ -87,3 +87,15 @@ def test_moneyness_out_of_range_ends_the_fit(gpu, paths, n, days, K, carry):
     after = gpu.price_american(good, 0)
     assert after["premium"] == before["premium"] and after["trust"] == before["trust"]
     np.testing.assert_array_equal(after["beta"], before["beta"])
+
+
+@pytest.mark.parametrize("K,typ", [(55.0, abi.PUT), (260.0, abi.PUT), (99.9, abi.CALL)])
+def test_lists_of_every_length_in_global_memory(gpu, K, typ):
+    """Few, all and half of the paths in the money: blocks that are requested ahead of the walk end
+    inside, at and past a warp's share of the paths and of its list."""
+    b = vanilla_book(K=K, typ=typ, paths=1400003, days=[0, 120, 240, 365], r=0.08 if typ == abi.PUT else 0.02)
+    if typ == abi.CALL:
+        b.assets[0]["carry"] = b.assets[0]["carry"] - 0.06
+    r = gpu.price_american(b, 0)
+    S, _ = gpu.simulate_paths(b, 0)
+    assert_same_fit(r, am.fit(S, b.t, rates_of(b), K, typ == abi.CALL, K), b.n_dates)
