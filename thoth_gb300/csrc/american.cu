@@ -37,6 +37,8 @@
 
 #include <type_traits>
 
+using namespace lsm;
+
 namespace {
 
 constexpr unsigned long long BARRIER_LIMIT_NS = 2000000000ull; // 2 s
@@ -48,37 +50,6 @@ __device__ __forceinline__ bool in_the_money(float s, const K& A)
 {
     const int b = __float_as_int(s);
     return A.call ? b >= A.itm_bits : b <= A.itm_bits;
-}
-
-// S / norm rounded to nearest, from y = 1 / norm rounded to nearest (see moneyness_short for a norm
-// of few digits). q0 = RN(S y) may be
-// more than one ulp off near a power of two; one correction step q1 = RN(q0 + RN(S - norm q0) y)
-// brings it within one ulp, and then the remainder S - norm q1 is exact and the second step
-// q1 + r y rounded once is the correctly rounded quotient (P. Markstein, IBM J. Res. Dev.
-// 34(1), 1990: y within half an ulp of 1 / norm, q1 within one ulp of S / norm).
-// Five FP64 operations in place of a full division.
-template <class K>
-__device__ __forceinline__ double moneyness(double s, const K& A)
-{
-    const double y = A.inv_norm, b = A.norm;
-    const double q0 = __dmul_rn(s, y);
-    const double q1 = __fma_rn(__fma_rn(-q0, b, s), y, q0);
-    return __fma_rn(__fma_rn(-q1, b, s), y, q1);
-}
-
-// The same for a norm of at most 45 significant bits, from y and ylo = RN(1 / norm - y): the sum
-// before its one rounding is within 2^-105 of S / norm, and a quotient of a 24-bit by a 45-bit number
-// is never nearer than 2^-99 to a midpoint of two doubles (it would have to be a fraction with the
-// 54-bit midpoint's numerator), so it rounds as the quotient does. Two FP64 operations.
-__device__ __forceinline__ double moneyness_short(double s, double y, double ylo)
-{
-    return __fma_rn(s, y, __dmul_rn(s, ylo));
-}
-
-// b0 + b1 m + b2 m m, evaluated left to right
-__device__ __forceinline__ double continuation(double b0, double b1, double b2, double m)
-{
-    return __dadd_rn(__dadd_rn(b0, __dmul_rn(b1, m)), __dmul_rn(__dmul_rn(b2, m), m));
 }
 
 __device__ __forceinline__ void warp_sum(Fx128& a)
@@ -146,26 +117,6 @@ __device__ __forceinline__ Fx128 fx_from3(const unsigned long long* src)
     fx_add(r, l1 << 42, l1 >> 22);
     fx_add(r, 0, l2 << 20);
     return r;
-}
-
-// The exercise test iv >= b0 + b1 m + b2 m^2 (iv = phi (S - K), m = S / norm) of an
-// in-the-money spot sf, in single precision: 1 exercise, 0 hold, -1 too close to call.
-// With u = 2^-24, x = S - K_f (one rounding, relative) and h = x / norm, the inputs rounded to float
-// and the rounded operations leave iv with 2 u (|iv| + |K_f - K|), a0 with 2 u, a1 h with 6 u and
-// a2 h^2 with 9 u of their sizes, and the difference with one u of iv and c: below 10 u of each term,
-// against 32 u in the bound (lsm_screen), which also holds the reference's own rounding. So |d| above
-// the bound fixes the sign of the double-precision difference and hence the reference's test; inputs
-// too large for single precision give an infinite or NaN d or bound and come back undecided, as does
-// the thin band around the exercise boundary: the caller then runs the double-precision test.
-template <class K>
-__device__ __forceinline__ int screen_exercise(float sf, const LsmScreen& P, const K& A)
-{
-    const float x = sf - A.strike_f, v = x + A.strike_lo;
-    const float iv = A.call ? v : -v;
-    const float h = x * A.inv_norm_f, ah = fabsf(h);
-    const float d = iv - fmaf(fmaf(P.a2, h, P.a1), h, P.a0);
-    const float e = fmaf(fabsf(iv), 0x1p-19f, fmaf(fmaf(P.e2, ah, P.e1), ah, P.e0));
-    return d > e ? 1 : (d < -e ? 0 : -1);
 }
 
 // a float spot as a double, without the conversion's pass through the FP64 unit (out of line where
@@ -245,35 +196,6 @@ __device__ __forceinline__ void bar_arrive(int id)
 {
     __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(N) : "memory");
-}
-
-// A divisor and its reciprocal in two pieces: r = 1 / l rounded, rl = 1 / l - r rounded.
-struct Pivot {
-    double l, r, rl;
-};
-__device__ __forceinline__ Pivot pivot(double l)
-{
-    const double r = __ddiv_rn(1.0, l);
-    return Pivot{l, r, __dmul_rn(__fma_rn(-l, r, 1.0), r)};
-}
-
-// a / P.l from the two-piece reciprocal: within half an ulp and 2^-50 of one, so the correctly
-// rounded quotient unless a tie is nearer than that. `sure` stays set where the exact remainder
-// a - q l is below half an ulp of q (of the ulp below a power of two) times l by a clear margin,
-// which an integer comparison of its bits decides; elsewhere, and near the ends of the range, the
-// caller takes the division. Two dependent FP64 operations, the test beside the next ones: the
-// solver's chain of six divisions is on every date's critical path (a division takes about nine).
-__device__ __forceinline__ double divide_by(double a, const Pivot& P, bool& sure)
-{
-    const double q = __fma_rn(a, P.r, __dmul_rn(a, P.rl));
-    const unsigned long long rem = (unsigned long long)__double_as_longlong(__fma_rn(-q, P.l, a)) & 0x7fffffffffffffffull;
-    const unsigned long long qb = (unsigned long long)__double_as_longlong(q), lb = (unsigned long long)__double_as_longlong(P.l);
-    const int ea = (int)(__double2hiint(a) >> 20 & 0x7ff), eq = (int)(qb >> 52 & 0x7ff), el = (int)(lb >> 52 & 0x7ff);
-    // half an ulp of q times |l|, less 2^-19 of it; half that at a power of two
-    const long long half = (long long)(lb & 0x7fffffffffffffffull) - (1ll << 34) +
-                           ((long long)(eq - 1023 - 53 - ((qb << 12) == 0)) << 52);
-    sure &= (unsigned)(ea - 623) <= 800u && (unsigned)(el - 623) <= 800u && (long long)rem < half;
-    return q;
 }
 
 // the Cholesky factor of one date's normal equations

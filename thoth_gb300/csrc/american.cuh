@@ -2,7 +2,6 @@
 // launchers (american.cu), shared with the host pass in thoth_gpu.cu.
 #pragma once
 
-#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <vector>
@@ -10,6 +9,7 @@
 #include "thoth_gpu.h"
 
 #include "exact.cuh"
+#include "exercise.cuh"
 
 constexpr int LSM_THREADS = 512;
 // regression sums of one date: sum m, m^2, m^3, m^4, y, y m, y m^2 over the in-the-money
@@ -17,42 +17,6 @@ constexpr int LSM_THREADS = 512;
 constexpr int LSM_PART = 8;
 // per-CTA result sums: discounted exercise values, their squares, discounted maturity payoffs
 constexpr int LSM_NACC = 3;
-
-// One date's exercise test in single precision (screen_exercise), with h = (S - K) / norm:
-// continuation a0 + a1 h + a2 h^2, and its error bound 2^-19 |iv| + e0 + e1 |h| + e2 h^2.
-struct alignas(16) LsmScreen {
-    float a0, a1, a2, e0, e1, e2;
-    int fit; // 1 where the date has a regression
-    int pad;
-};
-
-// the screen of beta; m0 = (float) strike / norm. The expansion about the strike keeps the terms at
-// the size of the values that are compared: about 0 they are tens of times larger and cancel (near
-// the exercise boundary the polynomial hugs the payoff), and 4 % of the in-the-money paths of a daily
-// Heston put stayed open. The e's carry 2^-19 of each term (32 units of single precision; a term has
-// at most 10) and 2^-48 of the terms about 0, where the reference's own rounding and that of the
-// shift lie.
-__host__ __device__ inline LsmScreen lsm_screen(const double* beta, int fit, double strike, double norm, double m0)
-{
-    LsmScreen s;
-    const double a1 = fma(2.0 * beta[2], m0, beta[1]), a0 = fma(fma(beta[2], m0, beta[1]), m0, beta[0]);
-    s.a0 = (float)a0;
-    s.a1 = (float)a1;
-    s.a2 = (float)beta[2];
-    s.fit = fit;
-    s.pad = 0;
-    constexpr float U = 0x1p-19f, D = 0x1p-48f;
-    const float k = fabsf((float)strike), q = fabsf((float)norm), m = fabsf((float)m0);
-    const float b0 = fabsf((float)beta[0]), b1 = fabsf((float)beta[1]), b2 = fabsf(s.a2);
-    s.e0 = U * (fabsf(s.a0) + fabsf((float)((double)(float)strike - strike))) + D * (2.0f * k + b0 + (b1 + b2 * m) * m) +
-           1e-30f;
-    s.e1 = U * fabsf(s.a1) + D * (q + b1 + 2.0f * b2 * m);
-    s.e2 = U * b2;
-    // far from single precision's range: the test stays open
-    if (!(fmaxf(fmaxf(fmaxf(fabsf(s.a0), fabsf(s.a1)), fmaxf(b0, b1)), fmaxf(fmaxf(k, q), fmaxf(b2, m))) < 1e30f))
-        s.e0 = INFINITY;
-    return s;
-}
 
 // The frozen-policy apply of one contract (lsm_apply_kernel).
 struct LsmArgs {
@@ -73,8 +37,8 @@ struct LsmArgs {
     int* fit;             // [M] 1 where date t has a regression
     Fx128* acc;           // [grid][LSM_NACC] per-CTA result sums
     int* status;          // 0 ok; 3 an addend out of range
-    // apply only: the exercise test in single precision first (exercise_screened)
-    const LsmScreen* screen; // [M]
+    // apply only: the exercise test in single precision first (lsm::screen_exercise)
+    const lsm::LsmScreen* screen; // [M]
     float strike_f;       // strike rounded to float
     float strike_lo;      // strike_f - strike
     float inv_norm_f;     // 1 / norm rounded to float

@@ -1474,7 +1474,7 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + LSM_THREADS - 1) / LSM_THREADS,
                                                                  (int64_t)8 * g_dev.sms));
     const size_t tab = lsm_tab_bytes(M);
-    const size_t o_tab = 0, o_scr = align256(tab), scr_bytes = sizeof(LsmScreen) * (size_t)M;
+    const size_t o_tab = 0, o_scr = align256(tab), scr_bytes = sizeof(lsm::LsmScreen) * (size_t)M;
     const size_t o_acc = o_scr + align256(scr_bytes);
     const size_t acc_bytes = sizeof(Fx128) * (size_t)grid * LSM_NACC;
     const size_t o_ctl = o_acc + align256(acc_bytes);
@@ -1486,9 +1486,9 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     unsigned char* h = g_dev.pinned;
     lsm_fill_tab(h, io);
     // the single-precision screen of each date
-    LsmScreen* scr = reinterpret_cast<LsmScreen*>(h + o_scr);
+    lsm::LsmScreen* scr = reinterpret_cast<lsm::LsmScreen*>(h + o_scr);
     for (int t = 0; t < M; t++)
-        scr[t] = lsm_screen(&io.beta[3 * (size_t)t], io.fit_at[t], io.strike, io.norm, (double)(float)io.strike / io.norm);
+        scr[t] = lsm::lsm_screen(&io.beta[3 * (size_t)t], io.fit_at[t], io.strike, io.norm, (double)(float)io.strike / io.norm);
     cudaStream_t st = g_dev.stream;
     CUDA_TRY(cudaMemcpyAsync(base + o_tab, h, o_scr + scr_bytes, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(base + o_ctl, 0, sizeof(int), st));
@@ -1507,7 +1507,7 @@ int lsm_apply_locked(const Plan& P, double sim_ms, LsmPass& io)
     A.disc = A.df + M;
     A.beta = reinterpret_cast<double*>(base + o_tab) + 2 * (size_t)M;
     A.fit = reinterpret_cast<int*>(base + o_tab + sizeof(double) * 5 * (size_t)M);
-    A.screen = reinterpret_cast<const LsmScreen*>(base + o_scr);
+    A.screen = reinterpret_cast<const lsm::LsmScreen*>(base + o_scr);
     A.strike_f = (float)io.strike;
     A.strike_lo = (float)((double)A.strike_f - io.strike);
     A.inv_norm_f = (float)A.inv_norm;
@@ -1599,10 +1599,8 @@ int lsm_fit_batch_locked(const Plan& P, double sim_ms, LsmPass* const* io, int C
         K.strike = q.strike;
         K.norm = q.norm;
         K.inv_norm = 1.0 / q.norm;
-        K.inv_norm_lo = std::fma(-q.norm, K.inv_norm, 1.0) / q.norm;
-        uint64_t nb;
-        std::memcpy(&nb, &q.norm, sizeof nb);
-        K.short_norm = (nb & 0xff) == 0 && q.norm >= 0x1p-200 && q.norm <= 0x1p200;
+        K.inv_norm_lo = lsm::reciprocal_rest(q.norm, K.inv_norm);
+        K.short_norm = lsm::few_digits(q.norm);
         K.strike_f = (float)q.strike;
         K.strike_lo = (float)((double)K.strike_f - q.strike);
         K.m0 = (double)K.strike_f / q.norm;
