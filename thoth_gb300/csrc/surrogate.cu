@@ -3,6 +3,7 @@
 // tile (forward, head, backward for inputs and weights) and Adam.
 #include "engine.cuh"
 #include "phi.cuh"
+#include "surrogate.cuh"
 #include "tc.cuh"
 
 #include <cuda_bf16.h>
@@ -89,47 +90,7 @@ cudaError_t launch_tc_gemm_test(const void* A, const void* B, int N, int K, floa
     return cudaGetLastError();
 }
 
-
-// ===========================================================================
-// The surrogate MLP: 7 inputs (padded to 16) -> 4 x 128 SiLU -> 1.
-// Parameters (FP32 master, offsets in floats):
-//   W1 [128][16], b1[128], W2..W4 [128][128] + b[128], w5[128], b5[1]
-// BF16 copies of W1..W4 are the tensor-core operands, kept in global memory in the operand
-// layout (tc::cm_offset), so a CTA's copy of them is a plain block copy.
-// ===========================================================================
 namespace mlp {
-
-constexpr int H = 128;      // hidden width
-constexpr int KIN = 16;     // input features padded to one MMA K slice
-constexpr int ROWS = 128;   // rows per tile = MMA M
-constexpr int OFF_W1 = 0;
-constexpr int OFF_B1 = OFF_W1 + H * KIN;
-constexpr int OFF_W2 = OFF_B1 + H;
-constexpr int LAYER = H * H + H; // W + b of a hidden layer 2..4
-constexpr int OFF_W5 = OFF_W2 + 3 * LAYER;
-constexpr int OFF_B5 = OFF_W5 + H;
-constexpr int N_PARAMS = OFF_B5 + 1;
-constexpr int OFF_BF_W1 = 0;                 // bf16 weights, offsets in elements
-constexpr int OFF_BF_W2 = H * KIN;
-constexpr int N_BF = H * KIN + 3 * H * H;
-
-__host__ __device__ constexpr int w_off(int l) { return l == 1 ? OFF_W1 : OFF_W2 + (l - 2) * LAYER; }
-__host__ __device__ constexpr int b_off(int l) { return w_off(l) + H * (l == 1 ? KIN : H); }
-__host__ __device__ constexpr int bf_off(int l) { return l == 1 ? OFF_BF_W1 : OFF_BF_W2 + (l - 2) * H * H; }
-
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float dsilu(float z)
-{
-    const float s = __fdividef(1.0f, 1.0f + __expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
-
-struct Ctx {
-    uint64_t* mbar;
-    uint32_t tm;
-    uint32_t phase;
-    int* status;
-};
 
 // ---------------------------------------------------------------------------
 // One training tile: 128 rows of the batch through the whole network and back, one CTA.
@@ -158,20 +119,6 @@ struct Ctx {
 // (64 CTAs, 12 to 29 warps stalled on global memory per issue); as this kernel and Adam, 35 us with
 // its host work.
 // ---------------------------------------------------------------------------
-struct TileArgs {
-    const __nv_bfloat16* x; // [n][16] normalised inputs of the training set
-    const float* y;         // [n] targets
-    const float* w;         // [n] loss weights 1 / scale^2
-    const int* perm;        // row r of the batch is perm[first + r] (null: first + r)
-    int64_t first;
-    int rows;               // batch rows (multiple of 128)
-    const float* params;    // FP32 master
-    const __nv_bfloat16* wbf; // bf16 W1..W4 in the operand layout
-    float* part;            // per-tile partial gradients, [tiles][N_PARAMS]
-    float* loss_part;       // [tiles]
-    int* status;
-};
-
 constexpr int TILE_MAIN = 512; // the epilogue threads
 constexpr int TILE_THREADS = TILE_MAIN + H;
 constexpr uint32_t TILE_BUF = H * H * 2; // one 128 x 128 bf16 operand
@@ -721,32 +668,6 @@ constexpr int INFER_GROUP = 256;               // threads a tile
 constexpr int INFER_MAIN = INFER_TILES * INFER_GROUP;
 constexpr int INFER_LATTICE_THREADS = INFER_MAIN + ROWS; // and the scale's
 constexpr uint32_t INFER_TMEM_COLS = 512;      // a power of two >= 128 x INFER_TILES
-constexpr int MAX_MEMBERS = 64;
-
-struct LatticeTables {
-    const uint32_t* f_lm;  // [n_lm] feature words (bf16 hi, lo << 16), clipped and normalised
-    const uint32_t* f_T;   // [n_T]
-    const uint32_t* f_set; // [n_sets][5]
-    const double2* set_T;  // [n_sets][n_T] 1 / sd, sd / 2 of the price scale
-    const double2* lm;     // [n_lm] clipped log-moneyness, its exponential
-    const double* phi;     // [PHI_NODES][PHI_COEF]
-    double floor2;         // squared scale floor
-    uint32_t n_lm, n_T;
-};
-
-struct InferArgs {
-    const float* x;   // [n][7] normalised rows (not a lattice)
-    LatticeTables L;  // a lattice
-    int n;            // cells
-    int members;
-    float* y;         // [n] outputs, the members' mean
-    double* scale;    // [n] a lattice's price scale
-    float* price;     // [n] a lattice's prices
-    int* status;
-    const float* params[MAX_MEMBERS];
-    const __nv_bfloat16* wbf[MAX_MEMBERS];
-};
-
 __device__ __forceinline__ uint32_t feature_word(float v)
 {
     const __nv_bfloat16 h = __float2bfloat16(v), l = __float2bfloat16(v - __bfloat162float(h));
@@ -1025,27 +946,7 @@ cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfl
     return cudaGetLastError();
 }
 
-int mlp_n_params() { return mlp::N_PARAMS; }
-int mlp_n_bf() { return mlp::N_BF; }
-
-// ---------------------------------------------------------------------------
-// Lattice serving: the cells of n_sets parameter sets x n_T maturities x n_lm
-// log-moneyness, cell c = (set * n_T + j) * n_lm + k with raw features
-// (lm[k], T[j], kappa, theta, xi, rho, v0 of the set), clipped to the training
-// box and normalised, and the network's output scaled back to a price in units
-// of spot. Everything a cell needs is one word or number per axis value or per
-// (set, maturity); this kernel fills those tables, one thread an entry.
-// ---------------------------------------------------------------------------
-struct LatticeArgs {
-    const double* params; // [n_sets][5] kappa, theta, xi, rho, v0
-    const double* lms;    // [n_lm]
-    const double* Ts;     // [n_T]
-    double lo[7], hi[7];  // training box
-    int n_sets, n_lm, n_T;
-    uint32_t *f_lm, *f_T, *f_set;
-    double2 *set_T, *lm;
-};
-
+// the lattice's tables (LatticeArgs), one thread an entry
 __device__ __forceinline__ double clip(const LatticeArgs& A, int q, double f)
 {
     return fmin(fmax(f, A.lo[q]), A.hi[q]);

@@ -3,9 +3,7 @@
 // No reference counterpart: the reference has no learned pricer.
 #include "thoth_gpu.h"
 #include "phi.cuh"
-
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
+#include "surrogate.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -16,67 +14,6 @@
 #include <random>
 #include <string>
 #include <vector>
-
-namespace thoth {
-namespace mlp {
-struct TileArgs {
-    const __nv_bfloat16* x;
-    const float* y;
-    const float* w;
-    const int* perm;
-    int64_t first;
-    int rows;
-    const float* params;
-    const __nv_bfloat16* wbf;
-    float* part;
-    float* loss_part;
-    int* status;
-};
-} // namespace mlp
-cudaError_t mlp_train_prepare();
-cudaError_t mlp_train_tiles(const mlp::TileArgs& A, cudaStream_t st);
-cudaError_t mlp_adam(float* params, float* m, float* v, const float* part, int tiles, __nv_bfloat16* wbf, float lr,
-                     float b1, float b2, float eps, float bc1, float bc2, cudaStream_t st);
-cudaError_t mlp_gradient(const float* part, int tiles, float* grad, cudaStream_t st);
-cudaError_t mlp_loss(const float* loss_part, int tiles, float* loss, cudaStream_t st);
-cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfloat16* X, float* W, cudaStream_t st);
-cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t st);
-cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16* wbf, cudaStream_t st);
-int mlp_n_params();
-int mlp_n_bf();
-namespace mlp {
-constexpr int MAX_MEMBERS = 64;
-struct LatticeTables {
-    const uint32_t *f_lm, *f_T, *f_set;
-    const double2 *set_T, *lm;
-    const double* phi;
-    double floor2;
-    uint32_t n_lm, n_T;
-};
-struct InferArgs {
-    const float* x;
-    LatticeTables L;
-    int n, members;
-    float* y;
-    double* scale;
-    float* price;
-    int* status;
-    const float* params[MAX_MEMBERS];
-    const __nv_bfloat16* wbf[MAX_MEMBERS];
-};
-} // namespace mlp
-struct LatticeArgs {
-    const double* params;
-    const double* lms;
-    const double* Ts;
-    double lo[7], hi[7];
-    int n_sets, n_lm, n_T;
-    uint32_t *f_lm, *f_T, *f_set;
-    double2 *set_T, *lm;
-};
-cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st);
-cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st);
-} // namespace thoth
 
 using namespace thoth;
 
@@ -96,8 +33,7 @@ int sfail(int code, const std::string& m)
                          std::string(#expr) + ": " + cudaGetErrorString(e_));                                    \
     } while (0)
 
-constexpr int H = 128, KIN = 16, NF = 7;
-constexpr int OFF_W1 = 0, OFF_B1 = H * KIN, OFF_W2 = OFF_B1 + H, LAYER = H * H + H, OFF_W5 = OFF_W2 + 3 * LAYER;
+using mlp::H, mlp::KIN, mlp::NF, mlp::LAYER, mlp::OFF_W1, mlp::OFF_W2, mlp::OFF_W5;
 
 __nv_bfloat16 to_bf(float f)
 {
@@ -138,7 +74,7 @@ namespace {
 
 void host_params_to_bf(const std::vector<float>& p, std::vector<__nv_bfloat16>& w)
 {
-    w.resize((size_t)H * KIN + 3 * (size_t)H * H);
+    w.resize(mlp::N_BF);
     __nv_bfloat16* to = w.data();
     auto layer = [&](const float* from, int cols) { // the operand layout
         for (int kb = 0; kb < cols; kb += 8)
@@ -385,8 +321,8 @@ int thoth_gpu_surrogate_create(ThothSurrogate** out, uint64_t seed)
         if (!(p.major == 10 && p.minor == 3)) return sfail(THOTH_GPU_E_NODEVICE, "not an sm_103 device");
         ThothSurrogate* s = new ThothSurrogate();
         s->dev = dev;
-        s->np = mlp_n_params();
-        s->nbf = mlp_n_bf();
+        s->np = mlp::N_PARAMS;
+        s->nbf = mlp::N_BF;
         s->sms = p.multiProcessorCount;
         cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaMalloc(&s->params, sizeof(float) * s->np * 3);
@@ -457,7 +393,7 @@ int thoth_gpu_surrogate_destroy(ThothSurrogate* s)
     }
 }
 
-int thoth_gpu_surrogate_n_params(void) { return mlp_n_params(); }
+int thoth_gpu_surrogate_n_params(void) { return mlp::N_PARAMS; }
 
 int thoth_gpu_surrogate_get_params(ThothSurrogate* s, float* params)
 {
@@ -548,7 +484,7 @@ int thoth_gpu_surrogate_train_members(ThothSurrogate* const* members, int32_t k,
                                       uint64_t seed, int32_t avg_epochs, double lr_avg, double* final_loss)
 {
     try {
-        if (!members || k < 1 || k > 64 || !x || !y || n < 128 || epochs < 1 || batch < 128 || batch % 128 ||
+        if (!members || k < 1 || k > mlp::MAX_MEMBERS || !x || !y || n < 128 || epochs < 1 || batch < 128 || batch % 128 ||
             !(lr > 0))
             return sfail(THOTH_GPU_E_INVALID, "bad training arguments (batch must be a multiple of 128)");
         if (avg_epochs < 0 || avg_epochs >= epochs || (avg_epochs > 0 && !(lr_avg > 0 && lr_avg <= lr)))
@@ -568,8 +504,8 @@ int thoth_gpu_surrogate_train_members(ThothSurrogate* const* members, int32_t k,
                                        avg_epochs, lr_avg);
             if (rc) return rc;
         }
-        // the members' epochs interleaved: each member replays its own step graph on its own stream,
-        // so their kernels run side by side on the device
+        // the members' epochs interleaved: each member launches its steps on its own stream, so their
+        // kernels run side by side on the device
         for (int e = 0; e < epochs; e++)
             for (int j = 0; j < k; j++) {
                 const int rc = train_epoch(runs[j], e);
@@ -634,7 +570,7 @@ int thoth_gpu_surrogate_price_lattice_mean(ThothSurrogate* const* members, int32
                                            float* prices, double* device_ms)
 {
     try {
-        if (!members || k < 1 || k > 64 || !params || !lms || !Ts || !box_lo || !box_hi || !prices || n_sets < 1 ||
+        if (!members || k < 1 || k > mlp::MAX_MEMBERS || !params || !lms || !Ts || !box_lo || !box_hi || !prices || n_sets < 1 ||
             n_lm < 1 || n_T < 1 || !(floor > 0))
             return sfail(THOTH_GPU_E_INVALID, "bad lattice arguments");
         for (int j = 0; j < k; j++) {
