@@ -1175,6 +1175,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
         __syncthreads();
         if (s_cancel) {
             if (t == 0) atomicExch(P.status, 1);
+            if constexpr (LD > 2) copy_wait<0>();
             return false;
         }
         SobolLane<T, PP> L = sobol_lane<TB, PP>(P, S.hs, m);
@@ -1696,6 +1697,7 @@ __device__ __forceinline__ bool book_body(const DevPlan& P, unsigned char* smem_
             acc[idx + 1] = d2 + 2.0 * c * d1 + n * c * c;
         }
     }
+    if constexpr (LD > 2) copy_wait<0>(); // the last tile's copies of padding are still on their way into the ring
     if (cancel_ahead) atomicExch(P.status, 1);
     return !cancel_ahead;
 }
