@@ -541,7 +541,7 @@ int thoth_gpu_surrogate_train_avg(ThothSurrogate* s, const float* x, const float
                                   double lr_avg, double* final_loss);
 /* An ensemble's k members (1 <= k <= 64, distinct handles on one device) trained side by
  * side on the same set: member j as by thoth_gpu_surrogate_train_avg with data-order seed
- * seed + j (its initialisation is its own creation seed); each member replays its own step
+ * seed + j (its initialisation is its own creation seed); each member launches its own steps
  * on its own stream, so their kernels share the device. final_loss (may be null) holds k
  * values. */
 int thoth_gpu_surrogate_train_members(ThothSurrogate* const* members, int32_t k, const float* x, const float* y,
@@ -561,7 +561,7 @@ int thoth_gpu_surrogate_predict(ThothSurrogate* s, const float* x, int64_t n, fl
  * sqrt(bs^2 + floor^2), bs the Black-Scholes call (S = 1, r = q = 0) at the expected
  * average Heston variance theta + (v0 - theta)(1 - e^-kT)/(kT) over [0, T]. Only the
  * parameter sets and the lattice axes cross to the device and only the prices come back.
- * *device_ms: the three kernels' device time. */
+ * *device_ms: the kernels' device time. */
 int thoth_gpu_surrogate_price_lattice(ThothSurrogate* s, const double* params, int32_t n_sets, const double* lms,
                                       int32_t n_lm, const double* Ts, int32_t n_T, const double* box_lo,
                                       const double* box_hi, double floor, float* prices, double* device_ms);
@@ -576,8 +576,10 @@ int thoth_gpu_surrogate_price_lattice_mean(ThothSurrogate* const* members, int32
 const char* thoth_gpu_surrogate_last_error(void);
 
 /* Cooperative cancellation (reference: helpers/cancellation.hpp:9-15): a
- * running thoth_gpu_price_* call polls a host-mapped word between launches and
- * returns THOTH_GPU_E_CANCELLED. The flag is cleared by thoth_gpu_clear_cancel. */
+ * thoth_gpu_price_* call looks at a host-mapped word before its launches, and its
+ * kernels at each tile of paths, and returns THOTH_GPU_E_CANCELLED. A request that
+ * comes during the last tile may find the work done; the call still returns the
+ * error. The flag is cleared by thoth_gpu_clear_cancel. */
 int thoth_gpu_request_cancel(void);
 int thoth_gpu_clear_cancel(void);
 
