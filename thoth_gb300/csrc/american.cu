@@ -171,7 +171,7 @@ constexpr int FIT_THREADS = 32 * FIT_WARPS;
 constexpr int FIT_WALKERS = FIT_THREADS - 64;
 constexpr int FIT_MIN_PATHS = 128; // paths a CTA walks before the grid grows: a chunk a scheduler
 constexpr int FIT_SOLVER_CHUNKS = 24; // see lsm_fit_kernel
-constexpr int FIT_AHEAD = 512; // elements of a block requested ahead, paths in global memory
+constexpr int FIT_AHEAD = 256; // elements of a block requested ahead, paths in global memory (512: 2 % slower)
 constexpr int SUM_LIMBS = 5; // a warp's 128-bit sum in 26-bit limbs, added in shared memory
 
 constexpr int FIT_X = 5, FIT_Y = 3; // a date's moneyness sums (with the count), its cashflow sums
@@ -338,9 +338,10 @@ __device__ __noinline__ bool exercises_exactly(float sf, const FitPolicy* Q, con
 // IN_SMEM: the CTA's paths (spots of two dates, every contract's cashflows and in-the-money list)
 // live in shared memory, wherever they fit: 26 bytes a path of one contract, 18 more a contract. Else
 // in global memory, with the spots read from their rows; then 16 warps an SM have too few loads in
-// flight for the latency of DRAM, so each loop's next block is requested into L2 (ahead) and eight
-// chunks' loads go out together. 14 dates, one contract, the fit alone: 2^24 paths 7.07 ms without,
-// 5.7 with; 2^22 paths 1.45 and 1.15.
+// flight for the latency of DRAM, so each loop's next block is requested into L2 (ahead). 14 dates,
+// one contract, the fit alone: 2^24 paths 7.07 ms without, 5.6 with; 2^22 paths 1.44 and 1.14. (Eight
+// chunks' loads together instead of four: 1 % faster there, and 15 % slower where a warp has two or
+// three chunks, 64 contracts of 2^17 paths.)
 template <bool IN_SMEM>
 __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArgs A)
 {
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
                 double* const lm = list_m(K, c);
                 const FitScreen E = screen_of(K);
                 int nout = 0;
-#pragma unroll (IN_SMEM ? 4 : 8)
+#pragma unroll 4
                 for (int l0 = la; l0 < lb; l0 += 32) {
                     const int l = l0 + lane;
                     if (block_starts(l0 - la)) ahead(S, l0 + FIT_AHEAD, lb);
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) lsm_fit_kernel(const LsmFitArg
                 int32_t* const tau = K.tau + p0;
                 // without a branch from the screen to the product, so that the chunks' chains of
                 // single-precision operations overlap and an FP64 instruction serves a whole warp
-                constexpr int U = IN_SMEM ? 4 : 8;
+                constexpr int U = 4;
                 for (int l0 = la + lane; l0 - lane < lb; l0 += 32 * U) {
                     if (block_starts(l0 - lane - la)) {
                         ahead(cf, l0 - lane + FIT_AHEAD, lb);
