@@ -349,8 +349,9 @@ def american_section(G, flush, steps):
                            "sample": "oracle.american.fit on 2^15 Heston paths x 365 daily exercise dates "
                                      "(%.2f s)" % cpu_s,
                            "gpu_equals_oracle_on_sample": bool(G.price_american(sample, 0)["premium"] == o["premium"])}
-    out["note"] = ("fit = one cooperative launch, one publish/reduce/release per exercise date; FP64-issue and "
-                   "latency bound (GB300 runs FP64 at 1/64 of FP32): the paths are read once (fit_read_gbs)")
+    out["note"] = ("fit = one cooperative launch, two publishes per exercise date, every CTA solves from the totals; "
+                   "FP64-issue and latency bound (GB300 runs FP64 at 1/64 of FP32): the paths are read once "
+                   "(fit_read_gbs)")
     return out
 
 
@@ -384,8 +385,8 @@ def calibration_section(G):
     out["cpu_baseline"] = {"value": 16384 * 365 / cpu, "unit": "particle-steps/s", "cores": 1, "kind": "port",
                            "sample": "oracle.calibrate_leverage: 16384 particles x 365 daily layers (%.3f s)" % cpu}
     out["max_rel_diff_vs_oracle"] = float(np.max(np.abs(L / ref - 1.0)))
-    out["note"] = ("one cooperative launch, two exact publish-and-release rounds a date (extremes and sum of v, "
-                   "then the bins); FP64-latency bound; the Rng stream is the reference's, jumped per particle")
+    out["note"] = ("one cooperative launch, two exact rounds of all CTAs a date (extremes and sum of v, then the "
+                   "bins), every CTA forms the layer; FP64-latency bound; the Rng stream is the reference's, jumped per particle")
     return out
 
 
