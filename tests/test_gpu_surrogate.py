@@ -247,3 +247,40 @@ def test_lattice_cells_equal_the_same_rows(gpu, sets, n_lm, n_T, members):
         y = y * np.float32(1.0 / members)
     np.testing.assert_allclose(got, y.astype(np.float64) * S.price_scale(X), rtol=1.3e-7, atol=0)
     E.close()
+
+
+@pytest.mark.parametrize("floor", [1e-9, 1e-11, 1e-15, 1e-30])
+def test_lattice_scale_far_out_of_the_money(gpu, floor):
+    """The price scale sqrt(bs^2 + floor^2) under floors far below the trained one, against FP64 with a
+    distribution function good to its last digits in the tail. The network's output cancels in the
+    ratio of the prices under two floors, which holds their two roundings to single precision (6e-8
+    each)."""
+    import ctypes as C
+
+    from scipy.special import ndtr
+
+    m = S.Surrogate(seed=5)
+    P = S.sobol_params(40)
+    lms, Ts = np.linspace(-1.0, 1.0, 41), np.array([0.02, 0.1, 0.5, 2.0])
+    lo, hi = np.asarray(S.BOX_LO, dtype=np.float64).copy(), np.asarray(S.BOX_HI, dtype=np.float64).copy()
+    lo[0], hi[0], lo[1], hi[1] = -1.0, 1.0, 0.02, 2.0
+    ptr = lambda a: np.ascontiguousarray(a, dtype=np.float64).ctypes.data_as(C.POINTER(C.c_double))
+
+    def prices(f):
+        out, ms = np.zeros(len(P) * len(Ts) * len(lms), dtype=np.float32), C.c_double()
+        rc = m.L.thoth_gpu_surrogate_price_lattice(m.h, ptr(P), len(P), ptr(lms), len(lms), ptr(Ts), len(Ts), ptr(lo),
+                                                   ptr(hi), C.c_double(f), out.ctypes.data_as(C.POINTER(C.c_float)),
+                                                   C.byref(ms))
+        assert rc == 0
+        return out.astype(np.float64).reshape(len(P), len(Ts), len(lms))
+
+    Q = np.clip(P, lo[2:], hi[2:])
+    kT = Q[:, 0:1] * Ts[None, :]
+    var = Q[:, 1:2] + (Q[:, 4:5] - Q[:, 1:2]) * (1.0 - np.exp(-kT)) / kT
+    sd = np.sqrt(np.maximum(var, 1e-8) * Ts[None, :])[:, :, None]
+    d1 = -lms / sd + 0.5 * sd
+    bs = ndtr(d1) - np.exp(lms) * ndtr(d1 - sd)
+    assert (bs < 1e-20).any() and (bs > 1e-2).any()
+    want = np.sqrt(bs * bs + floor * floor) / np.sqrt(bs * bs + 1.0)
+    np.testing.assert_allclose(prices(floor) / prices(1.0), want, rtol=1.5e-7, atol=0)
+    m.close()

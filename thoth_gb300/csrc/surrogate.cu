@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(LATTICE ? INFER_LATTICE_THREADS : INFER_MAIN, 
 
     if (LATTICE && g == INFER_TILES) {
         // the price scale of every cell of this CTA's tiles
-        for (int tile0 = INFER_TILES * blockIdx.x; tile0 < tiles; tile0 += stride)
+        for (int tile0 = INFER_TILES * blockIdx.x; tile0 < tiles && !A.scale_done; tile0 += stride)
             for (int tile = tile0; tile < min(tile0 + INFER_TILES, tiles); ++tile) {
                 const uint32_t c = (uint32_t)tile * ROWS + (uint32_t)r;
                 if (c >= (uint32_t)A.n) break;
@@ -851,6 +851,19 @@ __global__ void __launch_bounds__(LATTICE ? INFER_LATTICE_THREADS : INFER_MAIN, 
                 A.price[c] = (float)((double)A.y[c] * A.scale[c]);
 }
 
+// the price scale of every cell by the library's distribution function (TABLE_FLOOR)
+__global__ void __launch_bounds__(256) lattice_scale_kernel(const InferArgs A)
+{
+    const uint32_t per = A.L.n_lm * A.L.n_T;
+    for (uint32_t c = blockIdx.x * 256 + threadIdx.x; c < (uint32_t)A.n; c += gridDim.x * 256) {
+        const uint32_t set = c / per, q = c % per, j = q / A.L.n_lm, k = q % A.L.n_lm;
+        const double2 v = A.L.set_T[(size_t)set * A.L.n_T + j], m = A.L.lm[k];
+        const double d1 = fma(-m.x, v.x, v.y);
+        const double bs = normcdf(d1) - m.y * normcdf(fma(-2.0, v.y, d1));
+        A.scale[c] = sqrt(fma(bs, bs, A.L.floor2));
+    }
+}
+
 } // namespace mlp
 
 // ---- launchers -----------------------------------------------------------------
@@ -992,6 +1005,12 @@ cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st)
 {
     const int64_t total = (int64_t)A.n_sets * (A.n_T + 5) + A.n_lm + A.n_T;
     lattice_tables_kernel<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8 * sms), 256, 0, st>>>(A);
+    return cudaGetLastError();
+}
+
+cudaError_t lattice_scale(const mlp::InferArgs& A, int sms, cudaStream_t st)
+{
+    mlp::lattice_scale_kernel<<<(unsigned)std::min((A.n + 255) / 256, 8 * sms), 256, 0, st>>>(A);
     return cudaGetLastError();
 }
 

@@ -71,6 +71,7 @@ struct InferArgs {
     int members;
     float* y;         // [n] outputs, the members' mean
     double* scale;    // [n] a lattice's price scale
+    int scale_done;   // 1: the scale is there already (lattice_scale)
     float* price;     // [n] a lattice's prices
     int* status;
     const float* params[MAX_MEMBERS];
@@ -107,6 +108,12 @@ cudaError_t mlp_pack_set(const float* x, const float* scale, int64_t n, __nv_bfl
 cudaError_t mlp_weight_avg(const float* params, float* avg, int k, cudaStream_t st);
 cudaError_t mlp_weight_avg_finish(float* params, const float* avg, __nv_bfloat16* wbf, cudaStream_t st);
 cudaError_t lattice_tables(const LatticeArgs& A, int sms, cudaStream_t st);
+// Below this floor the scale of a cell far out of the money is smaller than what the table of Phi holds
+// of it (its tail ends at 3e-18, and is good to 2e-10 there), and lattice_scale takes the library's
+// function for every cell. From 1e-9 on the prices are the same bits either way; at 1e-15 the table's
+// differed by 2e-6, at 1e-30 they had nothing in common with the scale.
+constexpr double TABLE_FLOOR = 1e-10;
+cudaError_t lattice_scale(const mlp::InferArgs& A, int sms, cudaStream_t st);
 cudaError_t mlp_infer(const mlp::InferArgs& A, bool lattice, int sms, cudaStream_t st);
 
 } // namespace thoth

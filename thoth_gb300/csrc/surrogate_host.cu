@@ -641,6 +641,8 @@ int thoth_gpu_surrogate_price_lattice_mean(ThothSurrogate* const* members, int32
         STRY(cudaMemsetAsync(s->status, 0, sizeof(int), s->st));
         STRY(cudaEventRecord(T.e0, s->st));
         STRY(lattice_tables(B, s->sms, s->st));
+        A.scale_done = floor < TABLE_FLOOR;
+        if (A.scale_done) STRY(lattice_scale(A, s->sms, s->st));
         STRY(mlp_infer(A, true, s->sms, s->st));
         STRY(cudaEventRecord(T.e1, s->st));
         return finish_infer(s, T, A.price, prices, n, device_ms);
